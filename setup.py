@@ -44,7 +44,7 @@ setup(
     version="0.1.0",
     description="Stick-breaking attention for NVIDIA B200 (sm_100a), hand-written CUDA behind a C ABI",
     packages=find_packages(include=["stickbreaking_attention_b200*"]),
-    package_data={"stickbreaking_attention_b200": ["libsb_b200.so", "csrc/*"]},
+    package_data={"stickbreaking_attention_b200": ["libsb_b200.so", "_sb_torch.so", "csrc/*"]},
     python_requires=">=3.10",
     install_requires=["torch"],
     cmdclass={"build_ext": BuildExt, "build_py": BuildPy},

@@ -1,4 +1,5 @@
-"""Builds ``libsb_b200.so`` (the C-ABI library with the sm_100a kernels) in-tree with nvcc.
+"""Builds ``libsb_b200.so`` (the C-ABI library with the sm_100a kernels) in-tree with nvcc, and ``_sb_torch.so`` (the
+native host path from torch tensors to that library) with the host compiler.
 
 Used by ``setup.py`` and by ``__graft_entry__.build()``; can be run directly::
 
@@ -18,6 +19,8 @@ import sys
 PKG_DIR = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(PKG_DIR, "csrc")
 LIB_PATH = os.path.join(PKG_DIR, "libsb_b200.so")
+EXT_PATH = os.path.join(PKG_DIR, "_sb_torch.so")
+EXT_SOURCE = "sb_torch.cpp"
 SOURCES = ("sb_api.cu", "sb_simt.cu", "sb_tc.cu", "sb_tc_fwd256.cu", "sb_tc_fwd128.cu", "sb_tc_bwd.cu")
 HEADERS = ("sb_common.cuh", "sb_ptx.cuh", "sb_tc_common.cuh", "sb_tc_fwd_rows.cuh", "../../include/sb_b200.h")
 NVCC_FLAGS = (
@@ -38,6 +41,26 @@ def _stale(target: str, deps) -> bool:
         return True
     t = os.path.getmtime(target)
     return any(os.path.exists(d) and os.path.getmtime(d) > t for d in deps)
+
+
+def _start_ext(force: bool):
+    """Starts the compilation of the torch binding; returns the process, or None if it is up to date."""
+    src = os.path.join(CSRC, EXT_SOURCE)
+    if not (force or _stale(EXT_PATH, [src, os.path.join(CSRC, "../../include/sb_b200.h")])):
+        return None
+    import sysconfig
+
+    import torch
+    root = os.path.dirname(torch.__file__)
+    cuda = os.path.dirname(os.path.dirname(os.path.realpath(find_nvcc())))
+    inc = [os.path.join(root, "include"), os.path.join(root, "include", "torch", "csrc", "api", "include"),
+           os.path.join(cuda, "include"), sysconfig.get_paths()["include"]]
+    cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden", "-w",
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", "-DTORCH_API_INCLUDE_EXTENSION_H",
+           "-DTORCH_EXTENSION_NAME=_sb_torch", *[f"-I{i}" for i in inc], src, "-o", EXT_PATH + ".tmp",
+           f"-L{os.path.join(root, 'lib')}", "-lc10", "-lc10_cuda", "-ltorch", "-ltorch_cpu", "-ltorch_cuda", "-ltorch_python",
+           f"-L{PKG_DIR}", "-l:libsb_b200.so", "-Wl,-rpath,$ORIGIN"]
+    return subprocess.Popen(cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
 
 
 def build(force: bool = False, verbose: bool = False) -> str:
@@ -65,6 +88,13 @@ def build(force: bool = False, verbose: bool = False) -> str:
     if force or procs or _stale(LIB_PATH, objs):
         cmd = [nvcc, "-shared", "-o", LIB_PATH, *objs, "-gencode", "arch=compute_100a,code=sm_100a"]
         subprocess.run(cmd, check=True)
+    ext = _start_ext(force)
+    if ext is not None:
+        out, _ = ext.communicate()
+        if ext.returncode != 0:
+            sys.stderr.write(out)
+            raise RuntimeError(f"the host compiler failed on {EXT_SOURCE}")
+        os.replace(EXT_PATH + ".tmp", EXT_PATH)
     return LIB_PATH
 
 

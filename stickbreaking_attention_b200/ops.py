@@ -23,7 +23,7 @@ from typing import Optional
 
 import torch
 
-from . import _cabi
+from . import _cabi, _sb_torch
 
 NAMESPACE = "stickbreaking_attention_b200"
 
@@ -35,8 +35,7 @@ class _Switches(threading.local):
 
 
 _state = _Switches()
-_launches = [0]   # process-wide: the backward's launches happen on autograd's thread
-_status_words: dict[int, torch.Tensor] = {}
+_launches = [0]   # process-wide; launches made through the ctypes calls below (the native host path counts its own)
 
 
 @contextlib.contextmanager
@@ -85,8 +84,8 @@ def switch_flags() -> int:
 
 
 def kernel_launches() -> int:
-    """Total kernel launches enqueued through this module since import (for benchmark accounting)."""
-    return _launches[0]
+    """Total kernel launches enqueued through this package since import (for benchmark accounting)."""
+    return _launches[0] + _sb_torch.launches()
 
 
 def set_backward_scratch_budget(nbytes: int) -> int:
@@ -99,12 +98,7 @@ def set_backward_scratch_budget(nbytes: int) -> int:
 
 
 def _status_word(device: torch.device) -> torch.Tensor:
-    idx = device.index if device.index is not None else torch.cuda.current_device()
-    word = _status_words.get(idx)
-    if word is None:
-        word = torch.zeros(4, dtype=torch.int32, device=device)
-        _status_words[idx] = word
-    return word
+    return _sb_torch.status_word(device.index if device.index is not None else torch.cuda.current_device())
 
 
 def check_status(device=None) -> None:
@@ -344,6 +338,25 @@ def _strip(cu_seqlens, leading_zero):
     return cu_seqlens[1:] if leading_zero else cu_seqlens
 
 
+def _native_fwd(q, k, v, cu_seqlens, max_seqlens, logit_scale, attend_current, leading_zero, fused):
+    return _sb_torch.forward(q, k, v, cu_seqlens, None if max_seqlens is None else int(max_seqlens), float(logit_scale),
+                             bool(attend_current), bool(leading_zero), fused, switch_flags())
+
+
+def _native_bwd(do, dr, q, k, v, cu_seqlens, max_seqlens, log_rem, logit_scale, attend_current, leading_zero, fused, switches):
+    return _sb_torch.backward(do, dr, q, k, v, cu_seqlens, None if max_seqlens is None else int(max_seqlens), log_rem,
+                              float(logit_scale), bool(attend_current), bool(leading_zero), fused,
+                              switch_flags() if switches is None else switches)
+
+
+def attention(q, k, v, cu_seqlens, max_seqlens, logit_scale, attend_current, leading_zero, fused=False):
+    """The differentiable operator behind the public functions, one native call (``csrc/sb_torch.cpp``): ``[o, rem]``, or
+    ``[o + rem[..., None] * v]`` if ``fused``; fixed-length when ``cu_seqlens`` is None.  The calling thread's switches
+    travel with the autograd node: the backward runs on a thread of autograd's, which does not see them."""
+    return _sb_torch.attention(q, k, v, cu_seqlens, None if max_seqlens is None else int(max_seqlens), float(logit_scale),
+                               bool(attend_current), bool(leading_zero), fused, switch_flags())
+
+
 def varlen_fwd(q, k, v, cu_seqlens, max_seqlens: Optional[int], logit_scale: float,
                attend_current: bool = False, leading_zero: bool = False, return_attention: bool = False):
     """Packed forward.  ``cu_seqlens`` holds sequence ends, preceded by a 0 iff ``leading_zero``.
@@ -353,6 +366,8 @@ def varlen_fwd(q, k, v, cu_seqlens, max_seqlens: Optional[int], logit_scale: flo
     ``W``, fp32 ``(heads, tokens, max_seqlens)``: row t holds the weights of token t over the keys of its own sequence,
     indexed from the sequence start, zeros elsewhere.  A debugging aid: O(tokens * max_seqlens) memory, and the call
     runs the CUDA-core kernels whatever the dtype."""
+    if not (return_attention or _compiling()):
+        return _native_fwd(q, k, v, cu_seqlens, max_seqlens, logit_scale, attend_current, leading_zero, False)
     q, k, v = _tma_ready(q), _tma_ready(k), _tma_ready(v)
     o = torch.empty_like(q)
     rem = torch.empty(q.shape[:-1], dtype=q.dtype, device=q.device)
@@ -364,11 +379,8 @@ def varlen_fwd(q, k, v, cu_seqlens, max_seqlens: Optional[int], logit_scale: flo
         _fwd_impl(False, q, k, v, ends, max_seqlens, logit_scale, attend_current, leading_zero, o, rem, log_rem,
                   attn=attn)
         return o, rem, log_rem, attn
-    if _compiling():
-        _op_varlen_fwd(q, k, v, ends, 0 if max_seqlens is None else int(max_seqlens), float(logit_scale),
-                       bool(attend_current), bool(leading_zero), o, rem, log_rem)
-    else:
-        _fwd_impl(False, q, k, v, ends, max_seqlens, logit_scale, attend_current, leading_zero, o, rem, log_rem)
+    _op_varlen_fwd(q, k, v, ends, 0 if max_seqlens is None else int(max_seqlens), float(logit_scale),
+                   bool(attend_current), bool(leading_zero), o, rem, log_rem)
     return o, rem, log_rem
 
 
@@ -376,22 +388,22 @@ def varlen_bwd(do, dr, q, k, v, cu_seqlens, max_seqlens: Optional[int], log_rem,
                attend_current: bool = False, leading_zero: bool = False, switches: Optional[int] = None):
     """Packed backward; returns ``(dq, dk, dv)`` in the dtype of the inputs.  ``switches``: the ``switch_flags()`` of
     the forward call (default: the calling thread's)."""
+    if not _compiling():
+        return _native_bwd(do, dr, q, k, v, cu_seqlens, max_seqlens, log_rem, logit_scale, attend_current, leading_zero, False,
+                           switches)
     q, k, v, do = _tma_ready(q), _tma_ready(k), _tma_ready(v), _tma_ready(do.to(q.dtype))
     dr = dr.to(q.dtype).contiguous()
     dq, dk, dv = torch.empty_like(q), torch.empty_like(k), torch.empty_like(v)
-    ends = _strip(cu_seqlens, leading_zero)
-    if _compiling():
-        _op_varlen_bwd(do, dr, q, k, v, ends, 0 if max_seqlens is None else int(max_seqlens), log_rem,
-                       float(logit_scale), bool(attend_current), bool(leading_zero), dq, dk, dv)
-    else:
-        _bwd_impl(False, do, dr, q, k, v, ends, max_seqlens, log_rem, logit_scale, attend_current,
-                  leading_zero, dq, dk, dv, switches=switches)
+    _op_varlen_bwd(do, dr, q, k, v, _strip(cu_seqlens, leading_zero), 0 if max_seqlens is None else int(max_seqlens), log_rem,
+                   float(logit_scale), bool(attend_current), bool(leading_zero), dq, dk, dv)
     return dq, dk, dv
 
 
 def attn_fwd(q, k, v, logit_scale: float, attend_current: bool = False, return_attention: bool = False):
     """Fixed-length ``(B,H,T,d)`` forward; returns ``(o, rem, log_rem)``, and with ``return_attention=True`` also the
     fp32 weights ``W (B,H,T,T)`` (see ``varlen_fwd``)."""
+    if not (return_attention or _compiling()):
+        return _native_fwd(q, k, v, None, None, logit_scale, attend_current, False, False)
     q, k, v = _tma_ready(q), _tma_ready(k), _tma_ready(v)
     o = torch.empty_like(q)
     rem = torch.empty(q.shape[:-1], dtype=q.dtype, device=q.device)
@@ -400,10 +412,7 @@ def attn_fwd(q, k, v, logit_scale: float, attend_current: bool = False, return_a
         attn = torch.zeros((*q.shape[:-1], q.shape[-2]), dtype=torch.float32, device=q.device)
         _fwd_impl(True, q, k, v, None, None, logit_scale, attend_current, False, o, rem, log_rem, attn=attn)
         return o, rem, log_rem, attn
-    if _compiling():
-        _op_attn_fwd(q, k, v, float(logit_scale), bool(attend_current), o, rem, log_rem)
-    else:
-        _fwd_impl(True, q, k, v, None, None, logit_scale, attend_current, False, o, rem, log_rem)
+    _op_attn_fwd(q, k, v, float(logit_scale), bool(attend_current), o, rem, log_rem)
     return o, rem, log_rem
 
 
@@ -411,14 +420,12 @@ def attn_bwd(do, dr, q, k, v, log_rem, logit_scale: float, attend_current: bool 
              switches: Optional[int] = None):
     """Fixed-length backward; returns ``(dq, dk, dv)`` in the dtype of the inputs (the reference
     forces dk and dv to bf16 here, ``sb_attn/sb_bwd.py:173-174``; this keeps the input dtype)."""
+    if not _compiling():
+        return _native_bwd(do, dr, q, k, v, None, None, log_rem, logit_scale, attend_current, False, False, switches)
     q, k, v, do = _tma_ready(q), _tma_ready(k), _tma_ready(v), _tma_ready(do.to(q.dtype))
     dr = dr.to(q.dtype).contiguous()
     dq, dk, dv = torch.empty_like(q), torch.empty_like(k), torch.empty_like(v)
-    if _compiling():
-        _op_attn_bwd(do, dr, q, k, v, log_rem, float(logit_scale), bool(attend_current), dq, dk, dv)
-    else:
-        _bwd_impl(True, do, dr, q, k, v, None, None, log_rem, logit_scale, attend_current, False, dq, dk, dv,
-                  switches=switches)
+    _op_attn_bwd(do, dr, q, k, v, log_rem, float(logit_scale), bool(attend_current), dq, dk, dv)
     return dq, dk, dv
 
 
@@ -426,28 +433,15 @@ def fused_fwd(q, k, v, cu_seqlens, max_seqlens, logit_scale, attend_current=Fals
     """Forward with the callers' usual next step folded in: returns ``(out, rem, log_rem)`` with
     ``out = o + rem[..., None] * v`` (``tests/test_varlen.py:101``, ``tests/test_attn.py:64`` of the reference).
     Fixed-length when ``cu_seqlens`` is None.  Always a direct call of the C ABI (``SB_FLAG_FUSE_REM_V``)."""
-    fixed = cu_seqlens is None
-    q, k, v = _tma_ready(q), _tma_ready(k), _tma_ready(v)
-    out = torch.empty_like(q)
-    rem = torch.empty(q.shape[:-1], dtype=q.dtype, device=q.device)
-    log_rem = torch.empty(q.shape[:-1], dtype=torch.float64, device=q.device)
-    ends = None if fixed else _strip(cu_seqlens, leading_zero)
-    _fwd_impl(fixed, q, k, v, ends, max_seqlens, logit_scale, attend_current, leading_zero and not fixed, out, rem,
-              log_rem, fuse_rem_v=True)
-    return out, rem, log_rem
+    return _native_fwd(q, k, v, cu_seqlens, max_seqlens, logit_scale, attend_current, leading_zero, True)
 
 
 def fused_bwd(dout, q, k, v, cu_seqlens, max_seqlens, log_rem, logit_scale, attend_current=False,
               leading_zero=False, switches=None):
     """Backward of ``fused_fwd``'s ``out``: ``<d_out, v>`` goes into the gradient of rem and ``rem * d_out`` into dv
     inside the library; returns ``(dq, dk, dv)``."""
-    fixed = cu_seqlens is None
-    q, k, v, dout = _tma_ready(q), _tma_ready(k), _tma_ready(v), _tma_ready(dout.to(q.dtype))
-    dq, dk, dv = torch.empty_like(q), torch.empty_like(k), torch.empty_like(v)
-    ends = None if fixed else _strip(cu_seqlens, leading_zero)
-    _bwd_impl(fixed, dout, None, q, k, v, ends, max_seqlens, log_rem, logit_scale, attend_current,
-              leading_zero and not fixed, dq, dk, dv, fuse_rem_v=True, switches=switches)
-    return dq, dk, dv
+    return _native_bwd(dout, None, q, k, v, cu_seqlens, max_seqlens, log_rem, logit_scale, attend_current, leading_zero, True,
+                       switches)
 
 
 def kernel_path(q, fixed: bool = False) -> int:

@@ -13,28 +13,13 @@ import torch
 from . import ops
 
 
-class StickBreakingAttention(torch.autograd.Function):
-    """Autograd glue of the packed operator (reference: ``sb_varlen/__init__.py:24-68``)."""
+class StickBreakingAttention:
+    """The reference's name for the differentiable operator (``sb_varlen/__init__.py:24-68``); the autograd node itself is
+    native (``csrc/sb_torch.cpp``)."""
 
     @staticmethod
-    def forward(ctx, q, k, v, cu_seqlens, max_seqlens, inv_temp, attend_current, leading_zero):
-        o, rem, log_rem = ops.varlen_fwd(q, k, v, cu_seqlens, max_seqlens, inv_temp,
-                                         attend_current=attend_current, leading_zero=leading_zero)
-        ctx.save_for_backward(q, k, v, log_rem, cu_seqlens)
-        ctx.logit_scale = inv_temp
-        ctx.max_seqlens = max_seqlens
-        ctx.attend_current = attend_current
-        ctx.leading_zero = leading_zero
-        ctx.switches = ops.switch_flags()   # the backward runs on autograd's thread: it gets the caller's switches
-        return o, rem
-
-    @staticmethod
-    def backward(ctx, do, drem):
-        q, k, v, log_rem, cu_seqlens = ctx.saved_tensors
-        dq, dk, dv = ops.varlen_bwd(do, drem, q, k, v, cu_seqlens, ctx.max_seqlens, log_rem,
-                                    ctx.logit_scale, attend_current=ctx.attend_current,
-                                    leading_zero=ctx.leading_zero, switches=ctx.switches)
-        return dq, dk, dv, None, None, None, None, None
+    def apply(q, k, v, cu_seqlens, max_seqlens, inv_temp, attend_current, leading_zero):
+        return sb_attn_varlen_(q, k, v, inv_temp, cu_seqlens, max_seqlens, attend_current, leading_zero)
 
 
 def sb_attn_varlen(q, k, v, cu_seqlens, max_seqlens=None, inv_temp=None, zero_start=True,
@@ -56,28 +41,8 @@ def sb_attn_varlen(q, k, v, cu_seqlens, max_seqlens=None, inv_temp=None, zero_st
 
 
 def sb_attn_varlen_(q, k, v, inv_temp, cu_seqlens, max_seqlens, attend_current, leading_zero=False):
-    return StickBreakingAttention.apply(q, k, v, cu_seqlens, max_seqlens, inv_temp, attend_current,
-                                        leading_zero)
-
-
-class StickBreakingAttentionFused(torch.autograd.Function):
-    """``out = o + rem[..., None] * v`` in one operator (forward epilogue and backward fold inside the kernels' C ABI)."""
-
-    @staticmethod
-    def forward(ctx, q, k, v, cu_seqlens, max_seqlens, inv_temp, attend_current, leading_zero):
-        out, _, log_rem = ops.fused_fwd(q, k, v, cu_seqlens, max_seqlens, inv_temp,
-                                        attend_current=attend_current, leading_zero=leading_zero)
-        ctx.save_for_backward(q, k, v, log_rem, cu_seqlens)
-        ctx.args = (max_seqlens, inv_temp, attend_current, leading_zero, ops.switch_flags())
-        return out
-
-    @staticmethod
-    def backward(ctx, dout):
-        q, k, v, log_rem, cu_seqlens = ctx.saved_tensors
-        max_seqlens, inv_temp, attend_current, leading_zero, switches = ctx.args
-        dq, dk, dv = ops.fused_bwd(dout, q, k, v, cu_seqlens, max_seqlens, log_rem, inv_temp,
-                                   attend_current=attend_current, leading_zero=leading_zero, switches=switches)
-        return dq, dk, dv, None, None, None, None, None
+    o, rem = ops.attention(q, k, v, cu_seqlens, max_seqlens, inv_temp, attend_current, leading_zero)
+    return o, rem
 
 
 def sb_attn_varlen_fused(q, k, v, cu_seqlens, max_seqlens=None, inv_temp=None, zero_start=True,
@@ -89,5 +54,4 @@ def sb_attn_varlen_fused(q, k, v, cu_seqlens, max_seqlens=None, inv_temp=None, z
     if torch.compiler.is_compiling():
         return ops.functional_fwd(q, k, v, cu_seqlens, max_seqlens, inv_temp, attend_current, bool(zero_start),
                                   fuse_rem_v=True)[0]
-    return StickBreakingAttentionFused.apply(q, k, v, cu_seqlens, max_seqlens, inv_temp, attend_current,
-                                             bool(zero_start))
+    return ops.attention(q, k, v, cu_seqlens, max_seqlens, inv_temp, attend_current, bool(zero_start), fused=True)[0]
