@@ -68,13 +68,13 @@ enum SbFlags {
   SB_FLAG_BWD_SKIP_DKV = 4, /* timing aid: sb_bwd enqueues only the dQ kernel                   */
   SB_FLAG_BWD_SKIP_DQ = 8,  /* timing aid: sb_bwd enqueues only the dK/dV kernel, which then reads
                             what a previous full sb_bwd left in the same workspace              */
-  SB_FLAG_BWD_RECOMPUTE = 16, /* small-workspace backward.  By default (16-bit tensors, head_dim up to 128)
-                            the dQ kernel stores its A and dz tiles -- 64 KiB per (query tile, key tile)
-                            pair and head, heads processed in chunks that fit the scratch budget (8 GiB
+  SB_FLAG_BWD_RECOMPUTE = 16, /* small-workspace backward.  By default the dQ kernel stores its A and dz
+                            tiles -- 64 KiB per (query tile, key tile) pair and head on the tensor-core
+                            path, 8 KiB per 32 x 32 pair on the CUDA-core path, heads processed in chunks that fit the scratch budget (8 GiB
                             unless sb_set_backward_scratch_budget changed it) -- and the dK/dV kernel is
                             two plain GEMMs over them.  With this flag, or when one head alone exceeds the
                             budget, the dK/dV kernel recomputes the tiles from boundary values (a few KiB
-                            per pair).  Same 16-bit tiles either way.                             */
+                            per pair).  Same tiles either way.                                    */
   SB_FLAG_FUSE_REM_V = 32,  /* the caller wants out = o + rem[..., None] * v, what every caller of the
                             reference computes right after the operator (tests/test_varlen.py:101,
                             tests/test_attn.py:64).  sb_fwd writes `out` to `o` (rem and log_rem as usual).

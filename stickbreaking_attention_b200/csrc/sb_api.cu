@@ -110,11 +110,12 @@ static int make_plan(const SbParams *p, Plan &pl, bool backward) {
   // the tensor-core path records the carried values four times per 128-key tile
   pl.bnd_halves = tc ? 4 : 1;   // keys 0, 32, 64, 96 of every 128-key tile
   pl.bnd_bytes_per_head = align_up((size_t)pl.pairs_cap * pl.tile * pl.bnd_halves * sizeof(float), 256);
-  // Stored-tiles mode (128-column head sizes): 64 KiB per (query tile, key tile) pair and head.  Taken when at least one
-  // head fits the budget and the caller did not ask for the small-workspace mode.
+  // Stored-tiles mode: A and dz of every (query tile, key tile) pair and head, 64 KiB of 16-bit values per 128 x 128 pair
+  // (CUDA-core path: 8 KiB of fp32 per 32 x 32 pair).  Taken when at least one head fits the budget and the caller did not
+  // ask for the small-workspace mode.
   const size_t budget = g_scratch_budget.load(std::memory_order_relaxed);
-  pl.az_bytes_per_head = (size_t)pl.pairs_cap * 2 * kTcTile * kTcTile * 2;
-  pl.store_az = backward && tc && !(p->flags & SB_FLAG_BWD_RECOMPUTE) && pl.az_bytes_per_head <= budget;
+  pl.az_bytes_per_head = (size_t)pl.pairs_cap * 2 * pl.tile * pl.tile * (tc ? 2 : 4);
+  pl.store_az = backward && !(p->flags & SB_FLAG_BWD_RECOMPUTE) && pl.az_bytes_per_head <= budget;
   const size_t per_head = pl.store_az ? pl.az_bytes_per_head : 2 * pl.bnd_bytes_per_head;
   size_t chunk = per_head ? budget / per_head : (size_t)p->heads;
   if (chunk < 1) chunk = 1;

@@ -52,6 +52,7 @@ struct KParams {
   float *bnd_r1;       // [head_cnt][pairs_cap][tile]  suffix sums of log(1-beta) at tile starts
   float *bnd_s2;       // [head_cnt][pairs_cap][tile]  prefix sums of G before each key tile
   unsigned short *az;  // stored-tiles mode: [head_cnt][pairs_cap][A, dz][128 query rows][128 keys], 16-bit; else null
+                       // (CUDA-core kernels: fp32, [head_cnt][pairs_cap][32 query rows][32 A, 32 dz])
   long long pairs_cap;
   float *attn;         // forward, CUDA-core kernels only: [batch][heads][tokens][attn_cols] attention weights, or null
   long long attn_cols;
@@ -163,6 +164,7 @@ int tc_tile(int head_dim, bool backward, int max_seqlen);   // rows per work ite
 cudaError_t launch_tc_fwd256(const KParams &p, int dtype, cudaStream_t s);
 cudaError_t launch_tc_fwd128(const KParams &p, int dtype, cudaStream_t s);
 cudaError_t sm_count(int *out);              // SMs of the current device (cached)
+cudaError_t allow_dynamic_smem(const void *kernel, int bytes);   // MaxDynamicSharedMemorySize, once per kernel and device
 
 constexpr size_t kTraceBytes = 8 * 1024 * 16;   // workspace tail reserved for the event log
 

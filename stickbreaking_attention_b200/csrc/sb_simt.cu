@@ -1,18 +1,6 @@
 // CUDA-core (fp32 FMA) kernels: the exact path for fp32 tensors and for head sizes the tensor-core
 // kernels do not take.  Also holds the two helper kernels every path uses: the sequence-table
 // builder and the tail zero-fill.
-//
-// Structure (shared with the tensor-core path):
-//   forward      one block per (sequence, 32-row query tile, head); key tiles are walked from the
-//                diagonal back to the sequence start while every row carries sum softplus(z), so the
-//                log-space suffix sum needs no second pass              (reference: _forward_one_row,
-//                sb_varlen_fwd.py:81-215)
-//   backward A   query-stationary, key tiles 0 -> diagonal: dQ, plus the per-(row, key tile)
-//                boundary values R1 (suffix sum of log(1-beta) from this key tile on) and S2 (prefix sum
-//                of G before this key tile)                             (reference: _backward_one_row,
-//                sb_varlen_bwd.py:297-481, which adds dK/dV under a spin lock instead)
-//   backward B   key-stationary: recomputes each tile from R1/S2 and accumulates dK, dV in registers;
-//                no atomics, no locks, fixed summation order.
 #include "sb_common.cuh"
 
 namespace sb {
@@ -289,322 +277,600 @@ cudaError_t launch_zero_tail(const KParams &p, int dtype, bool backward, cudaStr
 }
 
 // ------------------------------------------------------------------------------------------------
-// SIMT kernels.  256 threads; thread t owns output row t/8 and columns (t%8) + 8u.
+// CUDA-core kernels: fp32 arithmetic throughout, for fp32 tensors and head sizes the tensor-core kernels do not take.
 // ------------------------------------------------------------------------------------------------
-constexpr int kT = kSimtTile;   // 32
-constexpr int kLdS = kT + 1;
+// What bounds them: shared-memory operand traffic of the fp32 products.  A block is 128 threads; every product of a step
+// gives each thread a 4 x 4 patch of the result (4 x DP/16 for the accumulators), so that eight 16-byte shared loads feed
+// 64 FMAs.  A step is 32 query rows x 64 keys (forward, dQ) or 64 query rows x 32 keys (dK/dV): small enough for three or
+// four blocks per SM at head size 64, and for a few heads of a few hundred tokens to spread over the GPU.  The scans over
+// the keys of a row are shared by four (two) lanes with 16 keys each.  Next operands are requested while the other product
+// of the step runs: cp.async for fp32, registers for 16-bit tensors (which are widened on their way to shared memory).
+// Measured, forward + backward: 2 x 8 heads x 1024 tokens, head size 64, fp32: 447 us; one thread per row scanning
+// serially and one shared load per FMA before: 2290 us.
+constexpr int kT = kSimtTile;      // 32 rows or keys per tile
+constexpr int kStep = 2 * kT;      // keys (or query rows) per step
+constexpr int kSimtThreads = 128;
+constexpr int kLdS = kStep + 4;    // row stride of a score tile with 64 columns
+constexpr int kLdH = kT + 4;       // ... with 32 columns
+template <int DP> constexpr int kSimtBlocks = DP == 64 ? 3 : 1;   // blocks per SM the register allocation leaves room for
+template <int DP> constexpr int kLd = DP + 4;   // row stride of an operand tile: 16-byte rows, four banks apart
 
-__device__ __forceinline__ float softplus_f(float z) { return fmaxf(z, 0.f) + log1pf(expf(-fabsf(z))); }
-
-template <typename T>
-__device__ __forceinline__ void load_rows(float *dst, int ld, const TensorRef &t, const TileCoord &c, int h,
-                                          int tile_idx, int d) {
-  const T *base = reinterpret_cast<const T *>(t.ptr) + c.boff * t.sb + (long long)h * t.sh;
-  for (int e = threadIdx.x; e < kT * d; e += blockDim.x) {
-    const int r = e / d, x = e - r * d;
-    const int li = tile_idx * kT + r;
-    dst[r * ld + x] = li < c.len ? to_f32<T>(base[(c.tok0 + li) * t.st + x]) : 0.f;
-  }
+__device__ __forceinline__ void cp_async16(float *dst, const void *src, bool take) {
+  const uint32_t d = static_cast<uint32_t>(__cvta_generic_to_shared(dst));
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(take ? 16 : 0) : "memory");
 }
-
-// S[r][c] = scale * <A_r, B_c> for the 4 columns of this thread.
-__device__ __forceinline__ void tile_dot(float *S, const float *A, const float *B, int ld, int d, float scale) {
-  const int r = threadIdx.x >> 3, cg = threadIdx.x & 7;
-  float s0 = 0.f, s1 = 0.f, s2 = 0.f, s3 = 0.f;
-  const float *a = A + r * ld;
-  const float *b0 = B + cg * ld, *b1 = b0 + 8 * ld, *b2 = b0 + 16 * ld, *b3 = b0 + 24 * ld;
-  for (int x = 0; x < d; ++x) {
-    const float av = a[x];
-    s0 = fmaf(av, b0[x], s0); s1 = fmaf(av, b1[x], s1); s2 = fmaf(av, b2[x], s2); s3 = fmaf(av, b3[x], s3);
-  }
-  S[r * kLdS + cg] = s0 * scale; S[r * kLdS + cg + 8] = s1 * scale;
-  S[r * kLdS + cg + 16] = s2 * scale; S[r * kLdS + cg + 24] = s3 * scale;
+__device__ __forceinline__ void cp_async4(float *dst, const void *src, bool take) {
+  const uint32_t d = static_cast<uint32_t>(__cvta_generic_to_shared(dst));
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(d), "l"(src), "r"(take ? 4 : 0) : "memory");
 }
+__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
-template <typename T, int U>
-__global__ void __launch_bounds__(256) simt_fwd_kernel(KParams p) {
-  extern __shared__ float smem[];
-  if (p.hdr[0]) return;
-  TileCoord c;
-  if (!decode_tile(p, blockIdx.x, true, c)) return;
-  const int d = p.head_dim, ld = d + 1;
-  float *Qs = smem, *Ks = Qs + kT * ld, *Vs = Ks + kT * ld, *Ss = Vs + kT * ld;
-  const int h = p.head0 + blockIdx.y;
-  const int t = threadIdx.x, r = t >> 3, cg = t & 7;
-  const int I = c.idx;
+// A tile of ROWS rows of one tensor on its way into shared memory: issue() requests it, land() makes it visible to the
+// issuing thread's next barrier.  Rows outside [0, len) become zeros; columns past head_dim are zeroed once by clear().
+template <typename T, int DP, int ROWS>
+struct TileLoad {
+  static constexpr int kWords = ROWS * DP / 2 / kSimtThreads;   // 16-bit tensors: two elements per register
+  uint32_t w[sizeof(T) == 4 ? 1 : kWords];
 
-  load_rows<T>(Qs, ld, p.q, c, h, I, d);
-  float acc[U];
-#pragma unroll
-  for (int u = 0; u < U; ++u) acc[u] = 0.f;
-  float run_sp = 0.f;  // sum of softplus(z) over the key tiles already visited (rows of warp 0)
-
-  for (int J = I; J >= 0; --J) {
-    load_rows<T>(Ks, ld, p.k, c, h, J, d);
-    load_rows<T>(Vs, ld, p.v, c, h, J, d);
-    __syncthreads();
-    tile_dot(Ss, Qs, Ks, ld, d, p.scale);
-    __syncthreads();
-    if (t < kT) {
-      const int gi = I * kT + t;
-      float suffix = 0.f;
-      for (int j = kT - 1; j >= 0; --j) {
-        const int gj = J * kT + j;
-        const bool allowed = gi < c.len && (p.attend_current ? gj <= gi : gj < gi);
-        const float z = Ss[t * kLdS + j];
-        float a = 0.f;
-        if (allowed) {
-          suffix += softplus_f(z);
-          a = expf(z - run_sp - suffix);
+  __device__ __forceinline__ static const T *row_ptr(const TensorRef &t, const TileCoord &c, int h) {
+    return reinterpret_cast<const T *>(t.ptr) + c.boff * t.sb + (long long)h * t.sh + c.tok0 * t.st;
+  }
+  __device__ __forceinline__ void issue(float *dst, const TensorRef &t, const TileCoord &c, int h, int row0, int d, bool wide) {
+    const T *base = row_ptr(t, c, h);
+    if constexpr (sizeof(T) == 4) {
+      if (wide) {   // rows of whole 16-byte chunks
+#pragma unroll 4
+        for (int e = threadIdx.x; e < ROWS * (DP / 4); e += kSimtThreads) {
+          const int r = e / (DP / 4), x = (e % (DP / 4)) * 4, row = row0 + r;
+          const bool take = row >= 0 && row < c.len;
+          if (x < d) cp_async16(dst + r * kLd<DP> + x, base + (take ? row * t.st + x : 0), take);
         }
-        Ss[t * kLdS + j] = a;
+      } else {
+#pragma unroll 4
+        for (int e = threadIdx.x; e < ROWS * DP; e += kSimtThreads) {
+          const int r = e / DP, x = e % DP, row = row0 + r;
+          const bool take = row >= 0 && row < c.len;
+          if (x < d) cp_async4(dst + r * kLd<DP> + x, base + (take ? row * t.st + x : 0), take);
+        }
       }
-      run_sp += suffix;
-    }
-    __syncthreads();
-    if (p.attn != nullptr) {   // debugging aid: the attention weights of this tile, keys indexed inside the sequence
-      for (int e = t; e < kT * kT; e += blockDim.x) {
-        const int rr = e / kT, j = e - rr * kT;
-        const int gi = I * kT + rr, gj = J * kT + j;
-        if (gi < c.len && gj < c.len && gj < p.attn_cols)
-          p.attn[((c.boff * p.heads + h) * p.tokens + c.tok0 + gi) * p.attn_cols + gj] = Ss[rr * kLdS + j];
-      }
-    }
+    } else {
+      const unsigned short *b16 = reinterpret_cast<const unsigned short *>(base);
 #pragma unroll
-    for (int u = 0; u < U; ++u) {
-      const int x = cg + 8 * u;
-      if (x < d) {
-        float s = acc[u];
-        for (int j = 0; j < kT; ++j) s = fmaf(Ss[r * kLdS + j], Vs[j * ld + x], s);
-        acc[u] = s;
+      for (int i = 0; i < kWords; ++i) {
+        const int e = threadIdx.x + i * kSimtThreads;
+        const int r = e / (DP / 2), x = (e % (DP / 2)) * 2, row = row0 + r;
+        w[i] = 0u;
+        if (row >= 0 && row < c.len && x < d) {
+          const unsigned short *src = b16 + row * t.st + x;
+          if (wide) w[i] = *reinterpret_cast<const uint32_t *>(src);   // even head size, 4-byte aligned rows
+          else w[i] = (uint32_t)src[0] | (x + 1 < d ? (uint32_t)src[1] << 16 : 0u);
+        }
       }
     }
-    __syncthreads();
   }
+  __device__ __forceinline__ void land(float *dst) {
+    if constexpr (sizeof(T) == 4) {
+      cp_async_wait();
+    } else {
+#pragma unroll
+      for (int i = 0; i < kWords; ++i) {
+        const int e = threadIdx.x + i * kSimtThreads;
+        const int r = e / (DP / 2), x = (e % (DP / 2)) * 2;
+        const unsigned short lo = (unsigned short)(w[i] & 0xffffu), hi = (unsigned short)(w[i] >> 16);
+        *reinterpret_cast<float2 *>(dst + r * kLd<DP> + x) =
+            make_float2(to_f32<T>(*reinterpret_cast<const T *>(&lo)), to_f32<T>(*reinterpret_cast<const T *>(&hi)));
+      }
+    }
+  }
+};
+template <int DP, int ROWS>
+__device__ __forceinline__ void clear_tile(float *dst, int d) {   // columns past head_dim stay zero from here on
+  if (d == DP) return;
+  for (int e = threadIdx.x; e < ROWS * DP; e += kSimtThreads) dst[(e / DP) * kLd<DP> + e % DP] = 0.f;
+}
 
-  const int gi = I * kT + r;
-  if (p.fuse_rem_v) {   // out = o + rem * v: the row owners publish rem through the free score tile
-    if (t < kT) Ss[t * kLdS] = expf(-run_sp);
-    __syncthreads();
-  }
-  if (gi < c.len) {
-    T *o = reinterpret_cast<T *>(p.o.ptr) + c.boff * p.o.sb + (long long)h * p.o.sh + (c.tok0 + gi) * p.o.st;
-    const T *vrow = reinterpret_cast<const T *>(p.v.ptr) + c.boff * p.v.sb + (long long)h * p.v.sh + (c.tok0 + gi) * p.v.st;
-    const float rem_r = p.fuse_rem_v ? Ss[r * kLdS] : 0.f;
+// S[m][n] = mul * <A_m, B_n>, M x N with M N = 2048: thread (ty, tx) owns rows ty + i * (M / 4), columns tx + j * (N / 4).
+template <int DP, int M, int N>
+__device__ __forceinline__ void tile_dot(float *S, const float *A, const float *B, float mul) {
+  constexpr int kTx = N / 4, kTy = M / 4, kLdO = N + 4;
+  const int tx = threadIdx.x % kTx, ty = threadIdx.x / kTx;
+  float acc[4][4] = {};
+  const float *a = A + ty * kLd<DP>, *b = B + tx * kLd<DP>;
+#pragma unroll 4
+  for (int x = 0; x < DP; x += 4) {
+    float4 av[4], bv[4];
 #pragma unroll
-    for (int u = 0; u < U; ++u) {
-      const int x = cg + 8 * u;
-      if (x < d) o[x] = from_f32<T>(p.fuse_rem_v ? fmaf(rem_r, to_f32<T>(vrow[x]), acc[u]) : acc[u]);
+    for (int i = 0; i < 4; ++i) av[i] = *reinterpret_cast<const float4 *>(a + i * kTy * kLd<DP> + x);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) bv[j] = *reinterpret_cast<const float4 *>(b + j * kTx * kLd<DP> + x);
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        acc[i][j] = fmaf(av[i].x, bv[j].x, acc[i][j]);
+        acc[i][j] = fmaf(av[i].y, bv[j].y, acc[i][j]);
+        acc[i][j] = fmaf(av[i].z, bv[j].z, acc[i][j]);
+        acc[i][j] = fmaf(av[i].w, bv[j].w, acc[i][j]);
+      }
+  }
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) S[(ty + i * kTy) * kLdO + tx + j * kTx] = acc[i][j] * mul;
+}
+
+// acc (32 rows x DP, thread: rows 4 ty .. + 3, columns 4 tx + 64 u ..) += P (32 x 64) B (64 x DP)
+template <int DP>
+__device__ __forceinline__ void tile_pv(float (&acc)[4][DP / 16], const float *P, const float *B) {
+  const int tx = threadIdx.x % 16, ty = threadIdx.x / 16;
+  const float *pp = P + 4 * ty * kLdS, *b = B + 4 * tx;
+#pragma unroll 2
+  for (int k = 0; k < kStep; k += 4) {
+    float4 pv[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) pv[i] = *reinterpret_cast<const float4 *>(pp + i * kLdS + k);
+#pragma unroll
+    for (int kk = 0; kk < 4; ++kk) {
+#pragma unroll
+      for (int u = 0; u < DP / 64; ++u) {
+        const float4 bv = *reinterpret_cast<const float4 *>(b + (k + kk) * kLd<DP> + 64 * u);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const float s = kk == 0 ? pv[i].x : kk == 1 ? pv[i].y : kk == 2 ? pv[i].z : pv[i].w;
+          acc[i][4 * u] = fmaf(s, bv.x, acc[i][4 * u]);
+          acc[i][4 * u + 1] = fmaf(s, bv.y, acc[i][4 * u + 1]);
+          acc[i][4 * u + 2] = fmaf(s, bv.z, acc[i][4 * u + 2]);
+          acc[i][4 * u + 3] = fmaf(s, bv.w, acc[i][4 * u + 3]);
+        }
+      }
     }
   }
-  if (t < kT && I * kT + t < c.len) {
-    const long long idx = (c.boff * p.heads + h) * p.tokens + c.tok0 + I * kT + t;
-    reinterpret_cast<T *>(p.rem)[idx] = from_f32<T>(expf(-run_sp));
-    p.log_rem[idx] = -(double)run_sp * kLog2eD;
+}
+// acc (32 keys x DP) += P^T B with P (64 query rows x 32 keys), B (64 x DP)
+template <int DP>
+__device__ __forceinline__ void tile_ptb(float (&acc)[4][DP / 16], const float *P, const float *B) {
+  const int tx = threadIdx.x % 16, ty = threadIdx.x / 16;
+  const float *pp = P + 4 * ty, *b = B + 4 * tx;
+#pragma unroll 4
+  for (int k = 0; k < kStep; ++k) {
+    const float4 pv = *reinterpret_cast<const float4 *>(pp + k * kLdH);
+#pragma unroll
+    for (int u = 0; u < DP / 64; ++u) {
+      const float4 bv = *reinterpret_cast<const float4 *>(b + k * kLd<DP> + 64 * u);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const float s = i == 0 ? pv.x : i == 1 ? pv.y : i == 2 ? pv.z : pv.w;
+        acc[i][4 * u] = fmaf(s, bv.x, acc[i][4 * u]);
+        acc[i][4 * u + 1] = fmaf(s, bv.y, acc[i][4 * u + 1]);
+        acc[i][4 * u + 2] = fmaf(s, bv.z, acc[i][4 * u + 2]);
+        acc[i][4 * u + 3] = fmaf(s, bv.w, acc[i][4 * u + 3]);
+      }
+    }
   }
 }
 
-// Row pass of the backward: on entry Z holds z, P holds dP; on exit Z holds dz and P holds A.
-// r1 = sum of log(1-beta) over the allowed keys from this tile's first key on (<= 0).
-__device__ __forceinline__ void bwd_row_pass(float *Z, float *P, int row, int gi, int J, int len, int ac,
-                                             float r1, float gpre, float dr, float &sp_sum, float &g_sum) {
-  float spl = 0.f, gs = 0.f;
-  for (int j = 0; j < kT; ++j) {
-    const int gj = J * kT + j;
-    const bool allowed = gi < len && (ac ? gj <= gi : gj < gi);
-    const float z = Z[row * kLdS + j];
-    float a = 0.f, dz = 0.f;
-    if (allowed) {
-      a = expf(z + r1 + spl);
-      spl += softplus_f(z);
-      const float g = a * (P[row * kLdS + j] - dr);
-      gs += g;
-      const float beta = 1.f / (1.f + expf(-z));
-      dz = g - beta * (gpre + gs);
-    }
-    Z[row * kLdS + j] = dz;
-    P[row * kLdS + j] = a;
+// One lane's 16 keys of a row: beta and 1 - beta per key, and the sum of softplus(z) over the allowed ones.
+//   u = e^-|z|, t = 1 + u in (1, 2]:  beta = (z > 0 ? 1 : u) / t,  1 - beta = (z > 0 ? u : 1) / t,
+//   softplus(z) = max(z, 0) + log t;  16 factors t share one logarithm, and what rounding 1 + u to fp32 dropped comes back
+//   to first order ((u - (t - 1)) / t), so that the sum is as good as 16 log1p.
+// Keys [key0, key0 + 16) below `limit` are allowed, negative ones never.
+__device__ __forceinline__ float stick_segment(float (&z)[16], int key0, int limit, float (&beta)[16], float (&keep)[16]) {
+  float lin = 0.f, prod = 1.f, comp = 0.f;
+#pragma unroll
+  for (int j = 0; j < 16; ++j) {
+    const bool on = key0 + j >= 0 && key0 + j < limit;
+    const float u = expf(-fabsf(z[j])), t = 1.f + u, rt = __frcp_rn(t);
+    const bool pos = z[j] > 0.f;
+    beta[j] = on ? (pos ? rt : u * rt) : 0.f;
+    keep[j] = on ? (pos ? u * rt : rt) : 1.f;
+    lin += on && pos ? z[j] : 0.f;
+    prod *= on ? t : 1.f;
+    comp += on ? (u - (t - 1.f)) * rt : 0.f;
   }
-  sp_sum = spl;
-  g_sum = gs;
+  return lin + (logf(prod) + comp);
+}
+__device__ __forceinline__ void load16(float (&x)[16], const float *src) {
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const float4 f = *reinterpret_cast<const float4 *>(src + 4 * i);
+    x[4 * i] = f.x; x[4 * i + 1] = f.y; x[4 * i + 2] = f.z; x[4 * i + 3] = f.w;
+  }
+}
+__device__ __forceinline__ void store16(float *dst, const float (&x)[16]) {
+#pragma unroll
+  for (int i = 0; i < 4; ++i) *reinterpret_cast<float4 *>(dst + 4 * i) = make_float4(x[4 * i], x[4 * i + 1], x[4 * i + 2], x[4 * i + 3]);
 }
 
-template <typename T, int U>
-__global__ void __launch_bounds__(256) simt_bwd_dq_kernel(KParams p) {
-  extern __shared__ float smem[];
+// Forward: one block per (sequence, 32-row query tile, head), keys walked from the diagonal back to the sequence start in
+// steps of 64; every row carries sum softplus(z) over the keys already visited, in fp64 (reference: _forward_one_row,
+// sb_varlen_fwd.py:81-215).
+template <typename T, int DP>
+__global__ void __launch_bounds__(kSimtThreads, kSimtBlocks<DP>) simt_fwd_kernel(KParams p, bool wide) {
+  extern __shared__ float4 smem4[];
   if (p.hdr[0]) return;
   TileCoord c;
   if (!decode_tile(p, blockIdx.x, true, c)) return;
-  const int d = p.head_dim, ld = d + 1;
-  float *Qs = smem, *Gs = Qs + kT * ld, *Ks = Gs + kT * ld, *Vs = Ks + kT * ld;
-  float *Zs = Vs + kT * ld, *Ps = Zs + kT * kLdS;
-  const int hh = blockIdx.y, h = p.head0 + hh;
-  const int t = threadIdx.x, r = t >> 3, cg = t & 7;
-  const int I = c.idx;
+  const int d = p.head_dim, h = p.head0 + blockIdx.y, t = threadIdx.x;
+  float *Qs = reinterpret_cast<float *>(smem4), *Ks = Qs + kT * kLd<DP>, *Vs = Ks + kStep * kLd<DP>, *Ss = Vs + kStep * kLd<DP>;
+  const int row0 = c.idx * kT, ac = p.attend_current;
+  const int r = t >> 2, seg = t & 3, gi = row0 + r;   // the row this thread scans, and which 16 of the step's keys
+  const int limit = gi < c.len ? gi + ac : 0;
 
-  load_rows<T>(Qs, ld, p.q, c, h, I, d);
-  load_rows<T>(Gs, ld, p.d_o, c, h, I, d);
-  float acc[U];
+  clear_tile<DP, kT>(Qs, d);
+  clear_tile<DP, kStep>(Ks, d);
+  clear_tile<DP, kStep>(Vs, d);
+  if (d != DP) __syncthreads();
+  TileLoad<T, DP, kT> lq;
+  TileLoad<T, DP, kStep> lk, lv;
+  int key0 = row0 - kT;                     // first key of the step (negative: keys before the sequence, masked)
+  lq.issue(Qs, p.q, c, h, row0, d, wide);
+  lk.issue(Ks, p.k, c, h, key0, d, wide);
+  lq.land(Qs);
+  lk.land(Ks);
+  __syncthreads();
+  float acc[4][DP / 16] = {};
+  double run = 0.0;                         // sum of softplus(z) over the keys of the earlier steps
+  for (; key0 > -kStep; key0 -= kStep) {
+    lv.issue(Vs, p.v, c, h, key0, d, wide);
+    tile_dot<DP, kT, kStep>(Ss, Qs, Ks, p.scale);
+    lv.land(Vs);
+    __syncthreads();
+    const bool more = key0 > 0;
+    if (more) lk.issue(Ks, p.k, c, h, key0 - kStep, d, wide);
+    {
+      float z[16], beta[16], keep[16];
+      float *srow = Ss + r * kLdS + seg * 16;
+      load16(z, srow);
+      const float sp = stick_segment(z, key0 + seg * 16, limit, beta, keep);
+      float prod = 1.f;
 #pragma unroll
-  for (int u = 0; u < U; ++u) acc[u] = 0.f;
+      for (int j = 0; j < 16; ++j) prod *= keep[j];
+      // product over the lanes with later keys, then down the lane's own keys
+      const float p1 = __shfl_down_sync(0xffffffffu, prod, 1, 4), p2 = __shfl_down_sync(0xffffffffu, prod, 2, 4),
+                  p3 = __shfl_down_sync(0xffffffffu, prod, 3, 4);
+      float R = expf(-(float)run);
+      if (seg < 3) R *= p1;
+      if (seg < 2) R *= p2;
+      if (seg < 1) R *= p3;
+#pragma unroll
+      for (int j = 15; j >= 0; --j) {
+        z[j] = beta[j] * R;
+        R *= keep[j];
+      }
+      store16(srow, z);
+      float sum = sp + __shfl_xor_sync(0xffffffffu, sp, 1);
+      sum += __shfl_xor_sync(0xffffffffu, sum, 2);
+      run += (double)sum;
+    }
+    __syncthreads();
+    if (p.attn != nullptr) {   // debugging aid: the attention weights of this step, keys indexed inside the sequence
+      for (int e = t; e < kT * kStep; e += kSimtThreads) {
+        const int ri = row0 + e / kStep, gj = key0 + e % kStep;
+        if (ri < c.len && gj >= 0 && gj < c.len && gj < p.attn_cols)
+          p.attn[((c.boff * p.heads + h) * p.tokens + c.tok0 + ri) * p.attn_cols + gj] = Ss[(e / kStep) * kLdS + e % kStep];
+      }
+    }
+    tile_pv<DP>(acc, Ss, Vs);
+    if (more) lk.land(Ks);
+    __syncthreads();
+  }
+
+  const float rem = expf(-(float)run);
+  if (seg == 0 && gi < c.len) {
+    const long long idx = (c.boff * p.heads + h) * p.tokens + c.tok0 + gi;
+    reinterpret_cast<T *>(p.rem)[idx] = from_f32<T>(rem);
+    p.log_rem[idx] = -run * kLog2eD;
+  }
+  if (p.fuse_rem_v) {   // out = o + rem * v: the row owners publish rem through the free score tile
+    if (seg == 0) Ss[r] = rem;
+    __syncthreads();
+  }
+  const int tx = t % 16, ty = t / 16;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int row = row0 + 4 * ty + i;
+    if (row >= c.len) continue;
+    T *o = reinterpret_cast<T *>(p.o.ptr) + c.boff * p.o.sb + (long long)h * p.o.sh + (c.tok0 + row) * p.o.st;
+    const T *v = reinterpret_cast<const T *>(p.v.ptr) + c.boff * p.v.sb + (long long)h * p.v.sh + (c.tok0 + row) * p.v.st;
+#pragma unroll
+    for (int u = 0; u < DP / 64; ++u)
+#pragma unroll
+      for (int x = 0; x < 4; ++x) {
+        const int col = 64 * u + 4 * tx + x;
+        if (col < d) o[col] = from_f32<T>(p.fuse_rem_v ? fmaf(Ss[4 * ty + i], to_f32<T>(v[col]), acc[i][4 * u + x]) : acc[i][4 * u + x]);
+      }
+  }
+}
+
+// The backward of one lane's 16 keys: z, dP in; dz, A out.  LANES lanes share a row.
+// r1: minus the sum of softplus over the allowed keys from the step's first key on; gpre: sum of G over the keys before it.
+// On return r1_seg / g_seg hold the same two at this lane's first key and sp / gs the row's sums over the step.
+template <int LANES>
+__device__ __forceinline__ void bwd_segment(float (&z)[16], float (&dp)[16], int key0, int limit, double r1, float gpre, float dr,
+                                            double &r1_seg, float &g_seg, double &sp, float &gs) {
+  const int lane = threadIdx.x & (LANES - 1);
+  float beta[16], keep[16];
+  const float own = stick_segment(z, key0, limit, beta, keep);
+  double incl = own;                       // through this lane's last key
+#pragma unroll
+  for (int o = 1; o < LANES; o <<= 1) {
+    const double up = __shfl_up_sync(0xffffffffu, incl, o, LANES);
+    if (lane >= o) incl += up;
+  }
+  sp = __shfl_sync(0xffffffffu, incl, LANES - 1, LANES);
+  r1_seg = r1 + (incl - (double)own);
+  float W = expf((float)(r1 + incl));      // product of (1 - beta) over the keys after this lane's
+  float loc = 0.f;
+#pragma unroll
+  for (int j = 15; j >= 0; --j) {
+    const float a = beta[j] * W;
+    W *= keep[j];
+    z[j] = a;
+    dp[j] = a != 0.f ? a * (dp[j] - dr) : 0.f;   // a row or key outside the sequence carries nothing over
+  }
+#pragma unroll
+  for (int j = 0; j < 16; ++j) loc += dp[j];
+  float gi = loc;
+#pragma unroll
+  for (int o = 1; o < LANES; o <<= 1) {
+    const float up = __shfl_up_sync(0xffffffffu, gi, o, LANES);
+    if (lane >= o) gi += up;
+  }
+  gs = __shfl_sync(0xffffffffu, gi, LANES - 1, LANES);
+  const float before = __shfl_up_sync(0xffffffffu, gi, 1, LANES);
+  g_seg = gpre + (lane > 0 ? before : 0.f);
+  float C = g_seg;
+#pragma unroll
+  for (int j = 0; j < 16; ++j) {
+    const float g = dp[j];
+    C += g;
+    dp[j] = z[j];                          // A
+    z[j] = fmaf(-beta[j], C, g);           // dz
+  }
+}
+
+// dQ: query-stationary, keys from the sequence start to the diagonal (reference: _backward_one_row,
+// sb_varlen_bwd.py:297-481, which adds dK/dV under a spin lock instead).  Leaves A and dz of every (query tile, key tile)
+// pair in the workspace (p.az), or, where those would not fit the scratch budget, the carried R1 and S2 per pair and row.
+template <typename T, int DP>
+__global__ void __launch_bounds__(kSimtThreads, kSimtBlocks<DP>) simt_bwd_dq_kernel(KParams p, bool wide) {
+  extern __shared__ float4 smem4[];
+  if (p.hdr[0]) return;
+  TileCoord c;
+  if (!decode_tile(p, blockIdx.x, true, c)) return;
+  const int d = p.head_dim, hh = blockIdx.y, h = p.head0 + hh, t = threadIdx.x;
+  float *Qs = reinterpret_cast<float *>(smem4), *Gs = Qs + kT * kLd<DP>, *Ks = Gs + kT * kLd<DP>, *Vs = Ks + kStep * kLd<DP>;
+  float *Zs = Vs + kStep * kLd<DP>, *Ps = Zs + kT * kLdS;
+  const int I = c.idx, row0 = I * kT;
+  const int r = t >> 2, seg = t & 3, gi = row0 + r;
+  const int limit = gi < c.len ? gi + p.attend_current : 0;
+
+  clear_tile<DP, kT>(Qs, d);
+  clear_tile<DP, kT>(Gs, d);
+  clear_tile<DP, kStep>(Ks, d);
+  clear_tile<DP, kStep>(Vs, d);
+  if (d != DP) __syncthreads();
+  TileLoad<T, DP, kT> lq, lg;
+  TileLoad<T, DP, kStep> lk, lv;
+  lq.issue(Qs, p.q, c, h, row0, d, wide);
+  lg.issue(Gs, p.d_o, c, h, row0, d, wide);
+  lk.issue(Ks, p.k, c, h, 0, d, wide);
+  lq.land(Qs);
+  lg.land(Gs);
+  lk.land(Ks);
   double r1 = 0.0;
   float gpre = 0.f, dr = 0.f;
-  const int my_row = I * kT + t;
-  if (t < kT && my_row < c.len) {
-    const long long idx = (c.boff * p.heads + h) * p.tokens + c.tok0 + my_row;
+  if (gi < c.len) {
+    const long long idx = (c.boff * p.heads + h) * p.tokens + c.tok0 + gi;
     r1 = p.log_rem[idx] * kLn2D;
     dr = load_drem<T>(p, idx);
   }
-
-  for (int J = 0; J <= I; ++J) {
-    load_rows<T>(Ks, ld, p.k, c, h, J, d);
-    load_rows<T>(Vs, ld, p.v, c, h, J, d);
+  __syncthreads();
+  float acc[4][DP / 16] = {};
+  const long long pair0 = (long long)hh * p.pairs_cap + c.pair0 + (long long)I * (I + 1) / 2;
+  for (int key0 = 0; key0 <= row0; key0 += kStep) {
+    lv.issue(Vs, p.v, c, h, key0, d, wide);
+    tile_dot<DP, kT, kStep>(Zs, Qs, Ks, p.scale);
+    lv.land(Vs);
     __syncthreads();
-    tile_dot(Zs, Qs, Ks, ld, d, p.scale);
-    tile_dot(Ps, Gs, Vs, ld, d, 1.f);
+    tile_dot<DP, kT, kStep>(Ps, Gs, Vs, 1.f);
     __syncthreads();
-    if (t < kT) {
-      const long long slot = ((long long)hh * p.pairs_cap + c.pair0 + (long long)I * (I + 1) / 2 + J) * kT + t;
-      p.bnd_r1[slot] = (float)r1;
-      p.bnd_s2[slot] = gpre;
-      float sp_sum, g_sum;
-      bwd_row_pass(Zs, Ps, t, my_row, J, c.len, p.attend_current, (float)r1, gpre, dr, sp_sum, g_sum);
-      r1 += (double)sp_sum;
-      gpre += g_sum;
-    }
-    __syncthreads();
-#pragma unroll
-    for (int u = 0; u < U; ++u) {
-      const int x = cg + 8 * u;
-      if (x < d) {
-        float s = acc[u];
-        for (int j = 0; j < kT; ++j) s = fmaf(Zs[r * kLdS + j], Ks[j * ld + x], s);
-        acc[u] = s;
+    {
+      float z[16], dp[16];
+      float *zrow = Zs + r * kLdS + seg * 16;
+      load16(z, zrow);
+      load16(dp, Ps + r * kLdS + seg * 16);
+      double r1_seg, sp;
+      float g_seg, gs;
+      bwd_segment<4>(z, dp, key0 + seg * 16, limit, r1, gpre, dr, r1_seg, g_seg, sp, gs);
+      store16(zrow, z);
+      const int J = key0 / kT + (seg >> 1);
+      if (J <= I) {
+        if (p.az != nullptr) {
+          float *az = reinterpret_cast<float *>(p.az) + ((pair0 + J) * kT + r) * (2 * kT) + (seg & 1) * 16;   // row: A, then dz
+          store16(az, dp);
+          store16(az + kT, z);
+        } else if ((seg & 1) == 0) {
+          p.bnd_r1[(pair0 + J) * kT + r] = (float)r1_seg;
+          p.bnd_s2[(pair0 + J) * kT + r] = g_seg;
+        }
       }
+      r1 += sp;
+      gpre += gs;
     }
     __syncthreads();
+    const bool more = key0 + kStep <= row0;
+    tile_pv<DP>(acc, Zs, Ks);
+    __syncthreads();
+    if (more) {
+      lk.issue(Ks, p.k, c, h, key0 + kStep, d, wide);
+      lk.land(Ks);
+      __syncthreads();
+    }
   }
 
-  const int gi = I * kT + r;
-  if (gi < c.len) {
-    T *o = reinterpret_cast<T *>(p.dq.ptr) + c.boff * p.dq.sb + (long long)h * p.dq.sh + (c.tok0 + gi) * p.dq.st;
+  const int tx = t % 16, ty = t / 16;
 #pragma unroll
-    for (int u = 0; u < U; ++u) {
-      const int x = cg + 8 * u;
-      if (x < d) o[x] = from_f32<T>(acc[u] * p.scale);
-    }
+  for (int i = 0; i < 4; ++i) {
+    const int row = row0 + 4 * ty + i;
+    if (row >= c.len) continue;
+    T *o = reinterpret_cast<T *>(p.dq.ptr) + c.boff * p.dq.sb + (long long)h * p.dq.sh + (c.tok0 + row) * p.dq.st;
+#pragma unroll
+    for (int u = 0; u < DP / 64; ++u)
+#pragma unroll
+      for (int x = 0; x < 4; ++x) {
+        const int col = 64 * u + 4 * tx + x;
+        if (col < d) o[col] = from_f32<T>(acc[i][4 * u + x] * p.scale);
+      }
   }
 }
 
-template <typename T, int U>
-__global__ void __launch_bounds__(256) simt_bwd_dkv_kernel(KParams p) {
-  extern __shared__ float smem[];
+// dK, dV: key-stationary, one block per 32-key tile, query tiles diagonal -> end two at a time; accumulators in registers,
+// fixed summation order, no atomics.  kStored: A and dz come from the workspace; otherwise they are computed again.
+template <typename T, int DP, bool kStored>
+__global__ void __launch_bounds__(kSimtThreads, kSimtBlocks<DP>) simt_bwd_dkv_kernel(KParams p, bool wide) {
+  extern __shared__ float4 smem4[];
   if (p.hdr[0]) return;
   TileCoord c;
   if (!decode_tile(p, blockIdx.x, false, c)) return;
-  const int d = p.head_dim, ld = d + 1;
-  float *Qs = smem, *Gs = Qs + kT * ld, *Ks = Gs + kT * ld, *Vs = Ks + kT * ld;
-  float *Zs = Vs + kT * ld, *Ps = Zs + kT * kLdS;
-  const int hh = blockIdx.y, h = p.head0 + hh;
-  const int t = threadIdx.x, r = t >> 3, cg = t & 7;
+  const int d = p.head_dim, hh = blockIdx.y, h = p.head0 + hh, t = threadIdx.x;
+  float *Qs = reinterpret_cast<float *>(smem4), *Gs = Qs + kStep * kLd<DP>, *Zs = Gs + kStep * kLd<DP>, *Ps = Zs + kStep * kLdH;
+  float *Ks = Ps + kStep * kLdH, *Vs = Ks + kT * kLd<DP>;   // recomputation only
   const int J = c.idx;
 
-  load_rows<T>(Ks, ld, p.k, c, h, J, d);
-  load_rows<T>(Vs, ld, p.v, c, h, J, d);
-  float dk[U], dv[U];
+  clear_tile<DP, kStep>(Qs, d);
+  clear_tile<DP, kStep>(Gs, d);
+  TileLoad<T, DP, kStep> lq, lg;
+  if constexpr (!kStored) {
+    clear_tile<DP, kT>(Ks, d);
+    clear_tile<DP, kT>(Vs, d);
+    if (d != DP) __syncthreads();
+    TileLoad<T, DP, kT> lk, lv;
+    lk.issue(Ks, p.k, c, h, J * kT, d, wide);
+    lv.issue(Vs, p.v, c, h, J * kT, d, wide);
+    lk.land(Ks);
+    lv.land(Vs);
+  } else if (d != DP) {
+    __syncthreads();
+  }
+  float dk[4][DP / 16] = {}, dv[4][DP / 16] = {};
+  for (int I = J; I < c.n_tiles; I += 2) {
+    lq.issue(Qs, p.q, c, h, I * kT, d, wide);
+    lg.issue(Gs, p.d_o, c, h, I * kT, d, wide);
+    if constexpr (kStored) {   // 64 query rows x (32 A, 32 dz): 16 float4 per row
 #pragma unroll
-  for (int u = 0; u < U; ++u) { dk[u] = 0.f; dv[u] = 0.f; }
-
-  for (int I = J; I < c.n_tiles; ++I) {
-    load_rows<T>(Qs, ld, p.q, c, h, I, d);
-    load_rows<T>(Gs, ld, p.d_o, c, h, I, d);
-    __syncthreads();
-    tile_dot(Zs, Qs, Ks, ld, d, p.scale);
-    tile_dot(Ps, Gs, Vs, ld, d, 1.f);
-    __syncthreads();
-    if (t < kT) {
-      const int gi = I * kT + t;
-      float dr = 0.f;
-      if (gi < c.len)
-        dr = load_drem<T>(p, (c.boff * p.heads + h) * p.tokens + c.tok0 + gi);
-      const long long slot = ((long long)hh * p.pairs_cap + c.pair0 + (long long)I * (I + 1) / 2 + J) * kT + t;
-      float sp_sum, g_sum;
-      bwd_row_pass(Zs, Ps, t, gi, J, c.len, p.attend_current, p.bnd_r1[slot], p.bnd_s2[slot], dr, sp_sum, g_sum);
-    }
-    __syncthreads();
-#pragma unroll
-    for (int u = 0; u < U; ++u) {
-      const int x = cg + 8 * u;
-      if (x < d) {
-        float a = dk[u], b = dv[u];
-        for (int i = 0; i < kT; ++i) {
-          a = fmaf(Zs[i * kLdS + r], Qs[i * ld + x], a);
-          b = fmaf(Ps[i * kLdS + r], Gs[i * ld + x], b);
-        }
-        dk[u] = a; dv[u] = b;
+      for (int i = 0; i < kStep * 16 / kSimtThreads; ++i) {
+        const int e = t + i * kSimtThreads, row = e >> 4, x = (e & 15) * 4;
+        const int Ir = I + (row >> 5);
+        const bool take = Ir < c.n_tiles;
+        const long long pair = (long long)hh * p.pairs_cap + c.pair0 + (long long)Ir * (Ir + 1) / 2 + J;
+        const float *src = reinterpret_cast<const float *>(p.az) + (take ? (pair * kT + (row & 31)) * (2 * kT) + x : 0);
+        cp_async16((x < kT ? Ps + row * kLdH + x : Zs + row * kLdH + x - kT), src, take);
       }
+      lq.land(Qs);
+      lg.land(Gs);
+      cp_async_wait();
+      __syncthreads();
+    } else {
+      lq.land(Qs);
+      lg.land(Gs);
+      __syncthreads();
+      tile_dot<DP, kStep, kT>(Zs, Qs, Ks, p.scale);
+      tile_dot<DP, kStep, kT>(Ps, Gs, Vs, 1.f);
+      __syncthreads();
+      const int row = t >> 1, seg = t & 1, Ir = I + (row >> 5), gi = I * kT + row;
+      float r1 = 0.f, gpre = 0.f, dr = 0.f;
+      if (gi < c.len) {
+        const long long slot = ((long long)hh * p.pairs_cap + c.pair0 + (long long)Ir * (Ir + 1) / 2 + J) * kT + (row & 31);
+        r1 = p.bnd_r1[slot];
+        gpre = p.bnd_s2[slot];
+        dr = load_drem<T>(p, (c.boff * p.heads + h) * p.tokens + c.tok0 + gi);
+      }
+      float z[16], dp[16];
+      load16(z, Zs + row * kLdH + seg * 16);
+      load16(dp, Ps + row * kLdH + seg * 16);
+      double r1_seg, sp;
+      float g_seg, gs;
+      bwd_segment<2>(z, dp, J * kT + seg * 16, gi < c.len ? gi + p.attend_current : 0, r1, gpre, dr, r1_seg, g_seg, sp, gs);
+      store16(Zs + row * kLdH + seg * 16, z);
+      store16(Ps + row * kLdH + seg * 16, dp);
+      __syncthreads();
     }
+    tile_ptb<DP>(dk, Zs, Qs);
+    tile_ptb<DP>(dv, Ps, Gs);
     __syncthreads();
   }
 
-  const int gj = J * kT + r;
-  if (gj < c.len) {
-    T *ok = reinterpret_cast<T *>(p.dk.ptr) + c.boff * p.dk.sb + (long long)h * p.dk.sh + (c.tok0 + gj) * p.dk.st;
-    T *ov = reinterpret_cast<T *>(p.dv.ptr) + c.boff * p.dv.sb + (long long)h * p.dv.sh + (c.tok0 + gj) * p.dv.st;
+  const int tx = t % 16, ty = t / 16;
 #pragma unroll
-    for (int u = 0; u < U; ++u) {
-      const int x = cg + 8 * u;
-      if (x < d) { ok[x] = from_f32<T>(dk[u] * p.scale); ov[x] = from_f32<T>(dv[u]); }
-    }
+  for (int i = 0; i < 4; ++i) {
+    const int key = J * kT + 4 * ty + i;
+    if (key >= c.len) continue;
+    T *ok = reinterpret_cast<T *>(p.dk.ptr) + c.boff * p.dk.sb + (long long)h * p.dk.sh + (c.tok0 + key) * p.dk.st;
+    T *ov = reinterpret_cast<T *>(p.dv.ptr) + c.boff * p.dv.sb + (long long)h * p.dv.sh + (c.tok0 + key) * p.dv.st;
+#pragma unroll
+    for (int u = 0; u < DP / 64; ++u)
+#pragma unroll
+      for (int x = 0; x < 4; ++x) {
+        const int col = 64 * u + 4 * tx + x;
+        if (col < d) {
+          ok[col] = from_f32<T>(dk[i][4 * u + x] * p.scale);
+          ov[col] = from_f32<T>(dv[i][4 * u + x]);
+        }
+      }
   }
 }
 
 template <typename K>
-static cudaError_t launch_one(K kernel, const KParams &p, size_t smem, cudaStream_t s) {
-  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+static cudaError_t launch_one(K kernel, const KParams &p, size_t floats, bool wide, cudaStream_t s) {
+  const size_t smem = floats * sizeof(float);
+  cudaError_t e = allow_dynamic_smem(reinterpret_cast<const void *>(kernel), (int)smem);
   if (e != cudaSuccess) return e;
   dim3 grid(p.tiles_cap, p.head_cnt);
-  kernel<<<grid, 256, smem, s>>>(p);
+  kernel<<<grid, kSimtThreads, smem, s>>>(p, wide);
   return cudaGetLastError();
 }
 
+// Whether rows can be fetched in the loader's wide unit: 16 bytes of fp32, 4 bytes (two elements) of 16-bit tensors.
 template <typename T>
-static cudaError_t simt_fwd_t(const KParams &p, cudaStream_t s) {
-  const size_t smem = (size_t)(3 * kT * (p.head_dim + 1) + kT * kLdS) * sizeof(float);
-  if (p.head_dim <= 64) return launch_one(simt_fwd_kernel<T, 8>, p, smem, s);
-  if (p.head_dim <= 128) return launch_one(simt_fwd_kernel<T, 16>, p, smem, s);
-  return launch_one(simt_fwd_kernel<T, 32>, p, smem, s);
+static bool wide_rows(const TensorRef &t, int head_dim) {
+  const long long m = sizeof(T) == 4 ? 4 : 2;
+  return t.ptr == nullptr || (reinterpret_cast<uintptr_t>(t.ptr) % (m * sizeof(T)) == 0 && head_dim % m == 0 && t.sb % m == 0 &&
+                              t.sh % m == 0 && t.st % m == 0);
 }
 
-template <typename T>
-static cudaError_t simt_bwd_t(const KParams &p, cudaStream_t s) {
-  const size_t smem = (size_t)(4 * kT * (p.head_dim + 1) + 2 * kT * kLdS) * sizeof(float);
+template <typename T, int DP>
+static cudaError_t simt_run(const KParams &p, bool backward, cudaStream_t s) {
+  const bool wide = wide_rows<T>(p.q, p.head_dim) && wide_rows<T>(p.k, p.head_dim) && wide_rows<T>(p.v, p.head_dim) &&
+                    (!backward || wide_rows<T>(p.d_o, p.head_dim));
+  constexpr size_t kRow = kT * kLd<DP>;
+  if (!backward) return launch_one(simt_fwd_kernel<T, DP>, p, 5 * kRow + kT * kLdS, wide, s);
   cudaError_t e = cudaSuccess;
-  if (p.head_dim <= 64) {
-    if (!p.skip_dq) e = launch_one(simt_bwd_dq_kernel<T, 8>, p, smem, s);
-    if (e == cudaSuccess && !p.skip_dkv) e = launch_one(simt_bwd_dkv_kernel<T, 8>, p, smem, s);
-  } else if (p.head_dim <= 128) {
-    if (!p.skip_dq) e = launch_one(simt_bwd_dq_kernel<T, 16>, p, smem, s);
-    if (e == cudaSuccess && !p.skip_dkv) e = launch_one(simt_bwd_dkv_kernel<T, 16>, p, smem, s);
-  } else {
-    if (!p.skip_dq) e = launch_one(simt_bwd_dq_kernel<T, 32>, p, smem, s);
-    if (e == cudaSuccess && !p.skip_dkv) e = launch_one(simt_bwd_dkv_kernel<T, 32>, p, smem, s);
-  }
-  return e;
+  if (!p.skip_dq) e = launch_one(simt_bwd_dq_kernel<T, DP>, p, 6 * kRow + 2 * kT * kLdS, wide, s);
+  if (e != cudaSuccess || p.skip_dkv) return e;
+  if (p.az != nullptr) return launch_one(simt_bwd_dkv_kernel<T, DP, true>, p, 4 * kRow + 2 * kStep * kLdH, wide, s);
+  return launch_one(simt_bwd_dkv_kernel<T, DP, false>, p, 6 * kRow + 2 * kStep * kLdH, wide, s);
+}
+template <typename T>
+static cudaError_t simt_run_t(const KParams &p, bool backward, cudaStream_t s) {
+  if (p.head_dim <= 64) return simt_run<T, 64>(p, backward, s);
+  if (p.head_dim <= 128) return simt_run<T, 128>(p, backward, s);
+  return simt_run<T, 256>(p, backward, s);
+}
+static cudaError_t simt_dispatch(const KParams &p, int dtype, bool backward, cudaStream_t s) {
+  if (dtype == SB_DTYPE_F32) return simt_run_t<float>(p, backward, s);
+  if (dtype == SB_DTYPE_BF16) return simt_run_t<__nv_bfloat16>(p, backward, s);
+  return simt_run_t<__half>(p, backward, s);
 }
 
 cudaError_t launch_simt_fwd(const KParams &p, int dtype, cudaStream_t s, int *launches) {
   *launches += 1;
-  if (dtype == SB_DTYPE_F32) return simt_fwd_t<float>(p, s);
-  if (dtype == SB_DTYPE_BF16) return simt_fwd_t<__nv_bfloat16>(p, s);
-  return simt_fwd_t<__half>(p, s);
+  return simt_dispatch(p, dtype, false, s);
 }
 
 cudaError_t launch_simt_bwd(const KParams &p, int dtype, cudaStream_t s, int *launches) {
   *launches += (p.skip_dq ? 0 : 1) + (p.skip_dkv ? 0 : 1);
-  if (dtype == SB_DTYPE_F32) return simt_bwd_t<float>(p, s);
-  if (dtype == SB_DTYPE_BF16) return simt_bwd_t<__nv_bfloat16>(p, s);
-  return simt_bwd_t<__half>(p, s);
+  return simt_dispatch(p, dtype, true, s);
 }
 
 }  // namespace sb

@@ -337,6 +337,22 @@ def test_tokens_after_last_sequence_are_zero(sb, cuda_device, dtype):
         assert torch.all(t[:, 120:] == 0)
 
 
+@pytest.mark.parametrize("mode", ["stored", "recompute"])
+@pytest.mark.parametrize("d,dtype", [(64, torch.float32), (20, torch.float32), (33, torch.bfloat16), (50, torch.float16),
+                                     (128, torch.float32), (130, torch.float32), (200, torch.bfloat16)])
+def test_cuda_core_kernels_at_tile_edges(sb, cuda_device, d, dtype, mode):
+    """Sequence lengths around the 32-row tiles and 64-key steps, head sizes that fill the padded columns, exceed them by
+    little and leave rows unaligned, on both ways the dK/dV kernel gets its attention tiles."""
+    lengths = [1, 31, 32, 33, 63, 64, 65, 2, 97, 130]
+    cu = cu_of(lengths)
+    for ac, std in ((False, 1.0), (True, 3.0)):
+        q, k, v, do, drem = H.make_inputs((2, sum(lengths), d), dtype, seed=70 + d, std=std)
+        with sb.small_backward_workspace(mode == "recompute"), sb.force_simt():
+            got = H.run_varlen(sb, q, k, v, do, drem, cu, cuda_device, attend_current=ac, inv_temp=1 / (d ** 0.5 * std))
+        want = H.oracle_varlen(q, k, v, do, drem, cu, attend_current=ac, inv_temp=1 / (d ** 0.5 * std))
+        H.assert_parity(got, want, dtype, f"CUDA-core d={d} {mode} ac={ac}")
+
+
 @pytest.mark.parametrize("ac", [False, True])
 @pytest.mark.parametrize("shape", [(2, 3, 256, 64), (1, 7, 500, 50), (2, 2, 512, 32), (1, 2, 300, 16),
                                    (1, 2, 1024, 128), (4, 1, 130, 128)])
