@@ -86,9 +86,10 @@ enum SbFlags {
                             exactly 0 once the keys in between carry about 126 bits of -log2(1 - beta).  From
                             there on everything a row computes per score (p in the forward; A, G and dz in the
                             backward) is exactly 0, and the tensor-core kernels skip that arithmetic wherever it
-                            is 0 for all 32 rows of a warp: they keep only the running log-space sum.  Every MMA
-                            is still issued and the results are bit-identical.  With this flag the arithmetic is
-                            done for every score regardless.                                      */
+                            is 0 for all 32 rows of a warp: they keep only the running log-space sum.  With
+                            `tile_start` (below) whole tiles beyond that point are not visited either.  The
+                            results are bit-identical.  With this flag every tile is visited and the
+                            arithmetic is done for every score regardless.                        */
 };
 
 typedef struct SbTensor {
@@ -99,7 +100,8 @@ typedef struct SbTensor {
 } SbTensor;
 
 typedef struct SbParams {
-  int32_t struct_bytes; /* = sizeof(SbParams); checked                                          */
+  int32_t struct_bytes; /* = sizeof(SbParams); checked (a struct that ends before `tile_start`, as
+                         * callers built against an earlier header pass it, is taken too)       */
   int32_t dtype;        /* SbDtype of q,k,v,o,rem and all gradients                             */
   int32_t batch;        /* 1 for a packed variable-length batch                                 */
   int32_t heads;
@@ -137,6 +139,17 @@ typedef struct SbParams {
                          * key index.  A debugging aid: the call then runs the CUDA-core kernels, whatever *
                          * the dtype.                                                                       */
   int64_t attn_cols;    /* columns of attn_weights (>= the longest sequence to get every weight)          */
+
+  int32_t *tile_start;  /* optional saved state, forward out / backward in, NULL otherwise: int32                *
+                         * (batch, heads, tile_start_stride).  With it the forward is through with a group of 32 *
+                         * query rows where all of them have used their stick up (the product of (1 - beta) over *
+                         * the keys visited is exactly 0 in fp32: no earlier key can add anything to o, rem or a *
+                         * gradient), records here which key that was, and log_rem covers the visited keys only; *
+                         * the backward then starts at that key.  Results are the same bit for bit.              *
+                         * Without it, or with SB_FLAG_DENSE_ROW_PASS in the forward, every key is visited and   *
+                         * log_rem covers all of them.  Hand the same buffer (or NULL) to both calls, which have *
+                         * to take the same kernel path (sb_kernel_path).                                        */
+  int64_t tile_start_stride; /* elements per (batch, head): at least ceil(tokens / 32)                           */
 } SbParams;
 
 /* Scratch bytes sb_fwd (backward == 0) or sb_bwd (backward != 0) needs for these shapes.  Looks at

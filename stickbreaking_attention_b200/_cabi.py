@@ -48,6 +48,7 @@ class SbParams(ctypes.Structure):
         ("dq", SbTensor), ("dk", SbTensor), ("dv", SbTensor),
         ("workspace", ctypes.c_void_p), ("workspace_bytes", ctypes.c_size_t), ("status", ctypes.c_void_p),
         ("attn_weights", ctypes.c_void_p), ("attn_cols", ctypes.c_int64),
+        ("tile_start", ctypes.c_void_p), ("tile_start_stride", ctypes.c_int64),
     ]
 
 

@@ -1,5 +1,6 @@
 // C ABI of the library: argument checks, workspace layout, kernel selection, launches.
 #include <atomic>
+#include <cstddef>
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
@@ -19,6 +20,9 @@ static int fail(int code, const char *fmt, ...) {
   va_end(ap);
   return code;
 }
+
+// SbParams as callers built against the header without the saved tile starts pass it: valid up to `tile_start`.
+constexpr int kShortParams = (int)offsetof(SbParams, tile_start);
 
 static inline size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
 
@@ -63,7 +67,7 @@ static bool tma_friendly(const SbTensor &t, int esize) {
 
 static int make_plan(const SbParams *p, Plan &pl, bool backward) {
   if (p == nullptr) return fail(SB_ERR_ARGUMENT, "params is NULL");
-  if (p->struct_bytes != (int)sizeof(SbParams))
+  if (p->struct_bytes != (int)sizeof(SbParams) && p->struct_bytes != kShortParams)
     return fail(SB_ERR_ARGUMENT, "struct_bytes %d != sizeof(SbParams) %d", p->struct_bytes, (int)sizeof(SbParams));
   if (p->dtype < SB_DTYPE_F32 || p->dtype > SB_DTYPE_F16) return fail(SB_ERR_ARGUMENT, "unknown dtype %d", p->dtype);
   if (p->batch < 1 || p->batch > 65535 || p->heads < 1 || p->heads > 65535)
@@ -228,6 +232,12 @@ static int fill_kparams(const SbParams *p, const Plan &pl, bool backward, KParam
     k.attn_cols = p->attn_cols;
   }
   if (backward && k.fuse_rem_v) k.d_rem_fused = ws + pl.off_drem;
+  if (p->struct_bytes > kShortParams && p->tile_start != nullptr) {
+    if (p->tile_start_stride < (p->tokens + 31) / 32)
+      return fail(SB_ERR_ARGUMENT, "tile_start_stride %lld < ceil(tokens / 32)", (long long)p->tile_start_stride);
+    k.tile_start = p->tile_start;
+    k.tile_start_stride = p->tile_start_stride;
+  }
   k.status = p->status;
   return SB_OK;
 }
@@ -314,7 +324,9 @@ static int run_fwd_static_scratch(const SbParams *p, void *stream) {
   if ((rc = device_ok())) return rc;
   void *scratch = nullptr;
   if ((rc = static_scratch_address(&scratch))) return rc;
-  SbParams with_scratch = *p;
+  SbParams with_scratch;
+  memset(&with_scratch, 0, sizeof(with_scratch));
+  memcpy(&with_scratch, p, p->struct_bytes);   // make_plan has checked the size
   with_scratch.workspace = scratch;
   with_scratch.workspace_bytes = SB_STATIC_SCRATCH_BYTES;
   return run(&with_scratch, stream, false);

@@ -56,6 +56,8 @@ struct KParams {
   long long pairs_cap;
   float *attn;         // forward, CUDA-core kernels only: [batch][heads][tokens][attn_cols] attention weights, or null
   long long attn_cols;
+  int *tile_start;     // [batch * heads][tile_start_stride]: first key a group of 32 query rows reaches (see first_key), or null
+  long long tile_start_stride;
   int fuse_rem_v;      // forward writes o + rem * v; backward folds the two extra gradient terms in
   char *d_rem_fused;   // backward with fuse_rem_v: [batch][heads][tokens] d_rem + <d_out, v> in the tensors' dtype,
                        // written by the first kernel of the call; `d_rem` then points here for the other kernels
@@ -77,6 +79,56 @@ __device__ __forceinline__ long long load_cu(const KParams &p, int i) {
   return p.cu64 ? reinterpret_cast<const long long *>(p.cu)[i]
                 : (long long)reinterpret_cast<const int *>(p.cu)[i];
 }
+
+// Where the group of 32 query rows from row0 on (a multiple of 32, inside the sequence) stopped: keys before this one have
+// weight exactly 0 for all of them, and log_rem of these rows covers the keys from it on.  One entry per 32 tokens: a
+// sequence's first two groups always reach its first key and have none, the later groups of all packed sequences start at
+// least 32 tokens apart.
+__device__ __forceinline__ int *tile_start_entry(const KParams &p, const TileCoord &c, int h, int row0) {
+  return p.tile_start + (c.boff * p.heads + h) * p.tile_start_stride + ((c.tok0 + row0) >> 5);
+}
+__device__ __forceinline__ int first_key(const KParams &p, const TileCoord &c, int h, int row0) {
+  return p.tile_start == nullptr || row0 < 64 ? 0 : *tile_start_entry(p, c, h, row0);
+}
+// ... and where query tile I of `tile` rows did.
+__device__ __forceinline__ int tile_first_key(const KParams &p, const TileCoord &c, int h, int I, int tile) {
+  int first = first_key(p, c, h, I * tile);
+  for (int row0 = I * tile + 32; row0 < min((I + 1) * tile, c.len); row0 += 32) first = min(first, first_key(p, c, h, row0));
+  return first;
+}
+
+// The query tiles I = J + off that reach key tile J (the others stopped before it), as a bit per tile in shared memory for
+// the first kListBits of them; later ones are looked up.  Tile J itself always does.
+constexpr int kListBits = 8192;
+struct QueryList {
+  const KParams &p;
+  const TileCoord &c;
+  int h, J, tile, n;      // n: query tiles J .. n_tiles - 1
+  uint32_t *bits;         // [kListBits / 32]
+  __device__ __forceinline__ bool reaches(int off) const { return tile_first_key(p, c, h, J + off, tile) < (J + 1) * tile; }
+  // by all threads of the block, before a barrier; one global read per query tile, all in flight together
+  __device__ __forceinline__ void build() {
+    const int lim = min(n, kListBits), lane = threadIdx.x & 31, warps = blockDim.x >> 5;
+    for (int b = (threadIdx.x >> 5) * 32; b < lim; b += warps * 32) {
+      const uint32_t w = __ballot_sync(0xffffffffu, b + lane < n && reaches(b + lane));
+      if (lane == 0) bits[b >> 5] = w;
+    }
+  }
+  // first listed tile at or after `off`, n if there is none
+  __device__ __forceinline__ int next(int off) const {
+    while (off < n) {
+      if (off >= kListBits) {
+        if (reaches(off)) return off;
+        ++off;
+        continue;
+      }
+      const uint32_t w = bits[off >> 5] >> (off & 31);
+      if (w != 0) return off + __ffs(w) - 1;
+      off = (off | 31) + 1;
+    }
+    return n;
+  }
+};
 
 // Maps a work-item number to its sequence and tile.  Items are ordered by weight across ALL sequences: the tile with
 // the most key (or query) tiles to visit comes first, so that the blocks that run longest start earliest and the

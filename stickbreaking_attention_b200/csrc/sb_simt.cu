@@ -510,12 +510,14 @@ __global__ void __launch_bounds__(kSimtThreads, kSimtBlocks<DP>) simt_fwd_kernel
   __syncthreads();
   float acc[4][DP / 16] = {};
   double run = 0.0;                         // sum of softplus(z) over the keys of the earlier steps
+  const bool may_stop = p.tile_start != nullptr && !p.dense;
+  int reached = 0;                          // first key visited
   for (; key0 > -kStep; key0 -= kStep) {
     lv.issue(Vs, p.v, c, h, key0, d, wide);
     tile_dot<DP, kT, kStep>(Ss, Qs, Ks, p.scale);
     lv.land(Vs);
     __syncthreads();
-    const bool more = key0 > 0;
+    bool more = key0 > 0;
     if (more) lk.issue(Ks, p.k, c, h, key0 - kStep, d, wide);
     {
       float z[16], beta[16], keep[16];
@@ -542,7 +544,14 @@ __global__ void __launch_bounds__(kSimtThreads, kSimtBlocks<DP>) simt_fwd_kernel
       sum += __shfl_xor_sync(0xffffffffu, sum, 2);
       run += (double)sum;
     }
-    __syncthreads();
+    if (may_stop) {   // once every row's product has underflowed to 0, no earlier key has any weight
+      if (!__syncthreads_or(gi < c.len && expf(-(float)run) != 0.f) && more) {
+        more = false;
+        reached = key0;
+      }
+    } else {
+      __syncthreads();
+    }
     if (p.attn != nullptr) {   // debugging aid: the attention weights of this step, keys indexed inside the sequence
       for (int e = t; e < kT * kStep; e += kSimtThreads) {
         const int ri = row0 + e / kStep, gj = key0 + e % kStep;
@@ -551,9 +560,13 @@ __global__ void __launch_bounds__(kSimtThreads, kSimtBlocks<DP>) simt_fwd_kernel
       }
     }
     tile_pv<DP>(acc, Ss, Vs);
-    if (more) lk.land(Ks);
+    if (!more) break;
+    lk.land(Ks);
     __syncthreads();
   }
+  if constexpr (sizeof(T) == 4) cp_async_wait();   // keys requested before the stop was known
+  __syncthreads();
+  if (p.tile_start != nullptr && t == 0 && row0 >= 64) *tile_start_entry(p, c, h, row0) = reached;
 
   const float rem = expf(-(float)run);
   if (seg == 0 && gi < c.len) {
@@ -654,7 +667,8 @@ __global__ void __launch_bounds__(kSimtThreads, kSimtBlocks<DP>) simt_bwd_dq_ker
   TileLoad<T, DP, kStep> lk, lv;
   lq.issue(Qs, p.q, c, h, row0, d, wide);
   lg.issue(Gs, p.d_o, c, h, row0, d, wide);
-  lk.issue(Ks, p.k, c, h, 0, d, wide);
+  const int key_first = first_key(p, c, h, row0);
+  lk.issue(Ks, p.k, c, h, key_first, d, wide);
   lq.land(Qs);
   lg.land(Gs);
   lk.land(Ks);
@@ -668,7 +682,7 @@ __global__ void __launch_bounds__(kSimtThreads, kSimtBlocks<DP>) simt_bwd_dq_ker
   __syncthreads();
   float acc[4][DP / 16] = {};
   const long long pair0 = (long long)hh * p.pairs_cap + c.pair0 + (long long)I * (I + 1) / 2;
-  for (int key0 = 0; key0 <= row0; key0 += kStep) {
+  for (int key0 = key_first; key0 <= row0; key0 += kStep) {
     lv.issue(Vs, p.v, c, h, key0, d, wide);
     tile_dot<DP, kT, kStep>(Zs, Qs, Ks, p.scale);
     lv.land(Vs);
@@ -737,10 +751,13 @@ __global__ void __launch_bounds__(kSimtThreads, kSimtBlocks<DP>) simt_bwd_dkv_ke
   float *Qs = reinterpret_cast<float *>(smem4), *Gs = Qs + kStep * kLd<DP>, *Zs = Gs + kStep * kLd<DP>, *Ps = Zs + kStep * kLdH;
   float *Ks = Ps + kStep * kLdH, *Vs = Ks + kT * kLd<DP>;   // recomputation only
   const int J = c.idx;
+  __shared__ uint32_t list_bits[kListBits / 32];
+  QueryList list{p, c, h, J, kT, c.n_tiles - J, list_bits};
+  list.build();
 
   clear_tile<DP, kStep>(Qs, d);
   clear_tile<DP, kStep>(Gs, d);
-  TileLoad<T, DP, kStep> lq, lg;
+  TileLoad<T, DP, kT> lq, lg, lq1, lg1;
   if constexpr (!kStored) {
     clear_tile<DP, kT>(Ks, d);
     clear_tile<DP, kT>(Vs, d);
@@ -750,18 +767,21 @@ __global__ void __launch_bounds__(kSimtThreads, kSimtBlocks<DP>) simt_bwd_dkv_ke
     lv.issue(Vs, p.v, c, h, J * kT, d, wide);
     lk.land(Ks);
     lv.land(Vs);
-  } else if (d != DP) {
-    __syncthreads();
   }
+  __syncthreads();
   float dk[4][DP / 16] = {}, dv[4][DP / 16] = {};
-  for (int I = J; I < c.n_tiles; I += 2) {
-    lq.issue(Qs, p.q, c, h, I * kT, d, wide);
-    lg.issue(Gs, p.d_o, c, h, I * kT, d, wide);
+  for (int off = 0; off < list.n;) {   // two of the query tiles that reach this key tile per step
+    const int I0 = J + off, off1 = list.next(off + 1), I1 = J + off1;   // I1 == n_tiles: rows past the sequence, zeros
+    off = list.next(off1 + 1);
+    lq.issue(Qs, p.q, c, h, I0 * kT, d, wide);
+    lg.issue(Gs, p.d_o, c, h, I0 * kT, d, wide);
+    lq1.issue(Qs + kT * kLd<DP>, p.q, c, h, I1 * kT, d, wide);
+    lg1.issue(Gs + kT * kLd<DP>, p.d_o, c, h, I1 * kT, d, wide);
     if constexpr (kStored) {   // 64 query rows x (32 A, 32 dz): 16 float4 per row
 #pragma unroll
       for (int i = 0; i < kStep * 16 / kSimtThreads; ++i) {
         const int e = t + i * kSimtThreads, row = e >> 4, x = (e & 15) * 4;
-        const int Ir = I + (row >> 5);
+        const int Ir = row < kT ? I0 : I1;
         const bool take = Ir < c.n_tiles;
         const long long pair = (long long)hh * p.pairs_cap + c.pair0 + (long long)Ir * (Ir + 1) / 2 + J;
         const float *src = reinterpret_cast<const float *>(p.az) + (take ? (pair * kT + (row & 31)) * (2 * kT) + x : 0);
@@ -769,16 +789,20 @@ __global__ void __launch_bounds__(kSimtThreads, kSimtBlocks<DP>) simt_bwd_dkv_ke
       }
       lq.land(Qs);
       lg.land(Gs);
+      lq1.land(Qs + kT * kLd<DP>);
+      lg1.land(Gs + kT * kLd<DP>);
       cp_async_wait();
       __syncthreads();
     } else {
       lq.land(Qs);
       lg.land(Gs);
+      lq1.land(Qs + kT * kLd<DP>);
+      lg1.land(Gs + kT * kLd<DP>);
       __syncthreads();
       tile_dot<DP, kStep, kT>(Zs, Qs, Ks, p.scale);
       tile_dot<DP, kStep, kT>(Ps, Gs, Vs, 1.f);
       __syncthreads();
-      const int row = t >> 1, seg = t & 1, Ir = I + (row >> 5), gi = I * kT + row;
+      const int row = t >> 1, seg = t & 1, Ir = row < kT ? I0 : I1, gi = Ir * kT + (row & 31);
       float r1 = 0.f, gpre = 0.f, dr = 0.f;
       if (gi < c.len) {
         const long long slot = ((long long)hh * p.pairs_cap + c.pair0 + (long long)Ir * (Ir + 1) / 2 + J) * kT + (row & 31);

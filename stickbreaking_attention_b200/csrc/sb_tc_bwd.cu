@@ -39,6 +39,7 @@ __device__ __forceinline__ void bwd_row_chunk_values(const uint32_t (&s)[16], co
                                                      int ac, bool row_valid, float scale2, float r1, float gpre, float dr,
                                                      float &gs, float &logsum, float (&pa)[16], float (&pz)[16],
                                                      bool skip_zero = false) {
+  float chunk_log = 0.f;   // summed per chunk, like the forward's (see fwd256_row_chunk): the two agree bit for bit
   // columns (tile-local key indices) below `limit` are allowed: one compare per column, no branches
   const int limit = !row_valid ? -1 : (diag ? r + ac : 0x7fffffff);
   const float2 sc = make_float2(scale2, scale2), one = make_float2(1.f, 1.f);
@@ -46,7 +47,7 @@ __device__ __forceinline__ void bwd_row_chunk_values(const uint32_t (&s)[16], co
   float rpg[4], q23[4], ri1[4], ri3[4];
   float2 tt01[4], tt23[4], ppg[4];
 #pragma unroll
-  for (int g = 0; g < 4; ++g) {   // independent work in packed pairs (two fp32 per instruction)
+  for (int g = 3; g >= 0; --g) {   // independent work in packed pairs (two fp32 per instruction)
     const float2 x01 = mul2(make_float2(__uint_as_float(s[4 * g]), __uint_as_float(s[4 * g + 1])), sc);
     const float2 x23 = mul2(make_float2(__uint_as_float(s[4 * g + 2]), __uint_as_float(s[4 * g + 3])), sc);
     e01[g] = make_float2(ex2(fminf(x01.x, 30.f)), ex2(fminf(x01.y, 30.f)));
@@ -60,11 +61,12 @@ __device__ __forceinline__ void bwd_row_chunk_values(const uint32_t (&s)[16], co
       if (!(col + 3 < limit)) { e23[g].y = 0.f; t23.y = 1.f; }
     }
     const float2 pp = mul2(make_float2(t01.x, t23.x), make_float2(t01.y, t23.y));   // (t0 t1, t2 t3)
-    logsum += lg2(pp.x * pp.y);
+    chunk_log += lg2(pp.x * pp.y);
     tt01[g] = t01;
     tt23[g] = t23;
     ppg[g] = pp;
   }
+  logsum += chunk_log;
   if (!kMasked && skip_zero && __all_sync(0xffffffffu, ex2(r1 + logsum) == 0.f && gpre + gs == 0.f)) {
 #pragma unroll
     for (int i = 0; i < 16; ++i) { pa[i] = 0.f; pz[i] = 0.f; }
@@ -217,6 +219,20 @@ __device__ __forceinline__ bool strip_row_pass(uint32_t ts, uint32_t tp, int r, 
   return ok;
 }
 
+// The same for a strip before the first key of the warp's rows: dz (and the stored A) are zeros, the scores are not read.
+__device__ __forceinline__ void zero_strip_row(uint8_t *tile_z, int r, unsigned short *az_a, uint32_t empty_bar) {
+  const uint32_t z[8] = {0u, 0u, 0u, 0u, 0u, 0u, 0u, 0u};
+#pragma unroll
+  for (int c = 0; c < 64; c += 16) {
+    store_packed_chunk16(tile_z, r, c, z);
+    if (az_a != nullptr) store_packed_global16(az_a + c, z);
+  }
+  __syncwarp();
+  if ((threadIdx.x & 31) == 0) mbar_arrive(empty_bar);
+}
+// What is recorded as R1 (a log2) for such a strip: the product it starts a row with is 0, and so is all that follows.
+constexpr float kNothingLeft = -1e6f;
+
 // =======================================================================================================
 // dq kernel for head sizes 72..128: 256 query rows per CTA
 // =======================================================================================================
@@ -235,6 +251,7 @@ constexpr int kKvBox = kBN * 64 * 2;           // 64 keys x 64 columns
 constexpr int kKvTile = 2 * kKvBox;            // K or V sub-tile
 constexpr int kStageBytes = 2 * kKvTile;
 constexpr int kZBytes = kBM * kBN * 2;         // dz tile: 128 rows x 64 keys
+static_assert(kStages == 2, "stage = sub-tile mod 2");
 constexpr int kSmem = 1024 + 4 * kTileBytes + kStages * kStageBytes + 2 * kZBytes + 512;
 enum { bQG = 0, bKvFull = 1, bKvEmpty = 3, bSpFull = 5, bZFull = 7, bZEmpty = 9, bFirst = 11, bSpEmpty = 12, bDqFull = 14, bNum = 16 };
 }  // namespace dq2
@@ -273,6 +290,10 @@ tc_bwd_dq2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
   const int steps_b = b_active ? min(2 * Ia + 4, n_sub) : 0;
   const int n_steps = b_active ? steps_b : steps_a;
   const int issuers = b_active ? 2 : 1;
+  // the sub-tiles each tile starts at (even numbers: whole key tiles), and the block's: earlier keys have weight exactly 0
+  const int first_a = tile_first_key(p, c, p.head0 + hh_blk, Ia, kBM) / kBM * 2;
+  const int first_b = b_active ? tile_first_key(p, c, p.head0 + hh_blk, Ia + 1, kBM) / kBM * 2 : first_a;
+  const int first = min(first_a, first_b);
   int tr_cur = 0;   // cursor of this thread's event-log lane (diagnostics)
 
   if (threadIdx.x == 0) {
@@ -309,11 +330,11 @@ tc_bwd_dq2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
           tma_load_4d(sQ + w * 2 * kTileBytes + kb * kBoxBytes, &tm_q, bar(bQG), kb * 64, qrow + w * kBM, h, (int)c.boff);
           tma_load_4d(sQ + w * 2 * kTileBytes + kTileBytes + kb * kBoxBytes, &tm_g, bar(bQG), kb * 64, qrow + w * kBM, h, (int)c.boff);
         }
-      for (int t = 0; t < n_steps; ++t) {
+      for (int t = 0; t < n_steps - first; ++t) {
         const int st = t % kStages;
         if (t >= kStages && !wait_or_abort(bar(bKvEmpty + st), ((t / kStages) - 1) & 1, abort_flag, p, 510)) break;
         if (*abort_flag) break;
-        const int krow = (int)c.tok0 + t * kBN;
+        const int krow = (int)c.tok0 + (first + t) * kBN;
         const uint32_t dst = sKV + st * kStageBytes;
         mbar_arrive_expect_tx(bar(bKvFull + st), kStageBytes);
         for (int kb = 0; kb < 2; ++kb) {
@@ -330,17 +351,30 @@ tc_bwd_dq2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
       constexpr uint32_t idesc_dq = idesc_f16(kBM, D, kFp16, false, true);
       const uint32_t qaddr = sQ + w * 2 * kTileBytes, gaddr = qaddr + kTileBytes, zaddr = sZ + w * kZBytes;
       const uint32_t tS = tmem + w * 128, tP = tS + 64, tDQ = tmem + 256 + w * 128;
-      const int my_steps = w == 0 ? steps_a : steps_b;
-      auto issue_sp = [&](int t) {
-        const uint32_t kaddr = sKV + (t % kStages) * kStageBytes;
+      // this tile takes part in stages t_first .. t_end - 1 of the block's n_stages; u counts from its first one
+      const int n_stages = n_steps - first;
+      const int t_first = (w == 0 ? first_a : first_b) - first, t_end = (w == 0 ? steps_a : steps_b) - first;
+      const int my_steps = t_end - t_first;
+      auto issue_sp = [&](int u) {
+        const uint32_t kaddr = sKV + ((t_first + u) % kStages) * kStageBytes;
         mma_kmajor_kmajor<D, kBoxBytes, kKvBox>(tS, qaddr, kaddr, idesc_s, false);            // S = Q K^T
         mma_kmajor_kmajor<D, kBoxBytes, kKvBox>(tP, gaddr, kaddr + kKvTile, idesc_s, false);  // dP = dO V^T
         mma_commit(bar(bSpFull + w));
       };
-      bool ok = wait_or_abort(bar(bQG), 0, abort_flag, p, 520) && wait_or_abort(bar(bKvFull), 0, abort_flag, p, 521);
-      // tile b starts once tile a's first scores are done, so that one tile's MMAs fall into the other's row pass
+      bool ok = true;
+      // stages the tile does not read are released on its behalf once they have arrived
+      auto release = [&](int t, int t_stop) {
+        for (; ok && t < t_stop; ++t) {
+          ok = wait_or_abort(bar(bKvFull + t % kStages), (t / kStages) & 1, abort_flag, p, 524);
+          if (ok) mbar_arrive(bar(bKvEmpty + t % kStages));
+        }
+      };
+      release(0, t_first);
+      ok = ok && wait_or_abort(bar(bQG), 0, abort_flag, p, 520) &&
+           wait_or_abort(bar(bKvFull + t_first % kStages), (t_first / kStages) & 1, abort_flag, p, 521);
+      // if both tiles start at the same stage, tile b starts once tile a's first scores are done, so that one tile's MMAs fall into the other's row pass
       // (bFirst completes exactly once: this waiter does not follow the phases of tile a's own barriers)
-      if (ok && w == 1 && steps_a > 0) ok = wait_or_abort(bar(bFirst), 0, abort_flag, p, 525);
+      if (ok && w == 1 && first_a == first_b) ok = wait_or_abort(bar(bFirst), 0, abort_flag, p, 525);
       if (ok) {
         tc_fence_after();
         issue_sp(0);
@@ -350,7 +384,7 @@ tc_bwd_dq2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
         // the rows of step u have read their S/dP (they are still computing): the next scores go first ...
         if (u + 1 < my_steps) {
           ok = wait_or_abort(bar(bSpEmpty + w), u & 1, abort_flag, p, 526) &&
-               wait_or_abort(bar(bKvFull + (u + 1) % kStages), ((u + 1) / kStages) & 1, abort_flag, p, 523);
+               wait_or_abort(bar(bKvFull + (t_first + u + 1) % kStages), ((t_first + u + 1) / kStages) & 1, abort_flag, p, 523);
           if (!ok) break;
           trace_event(p, 1 + 3 * w, tr_cur, 2 + 16 * w, u + 1);
           tc_fence_after();
@@ -363,16 +397,12 @@ tc_bwd_dq2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
         trace_event(p, 1 + 3 * w, tr_cur, 6 + 16 * w, u);
         tc_fence_after();
         // dQ += dz K: dz [128 x 64] K-major, K sub-tile [64 keys x (2 x 64) columns] MN-major
-        mma_kmajor_mnmajor<kBN, kKvBox>(tDQ, zaddr, sKV + (u % kStages) * kStageBytes, idesc_dq, u > 0);
+        mma_kmajor_mnmajor<kBN, kKvBox>(tDQ, zaddr, sKV + ((t_first + u) % kStages) * kStageBytes, idesc_dq, u > 0);
         mma_commit(bar(bZEmpty + w));
-        mma_commit(bar(bKvEmpty + u % kStages));
+        mma_commit(bar(bKvEmpty + (t_first + u) % kStages));
       }
       if (ok) mma_commit(bar(bDqFull + w));   // this tile's dQ is complete: its rows store it while the other tile goes on
-      // tile a does not read the last sub-tiles: release them on its behalf once they have arrived
-      for (int t = my_steps; ok && t < n_steps; ++t) {
-        ok = wait_or_abort(bar(bKvFull + t % kStages), (t / kStages) & 1, abort_flag, p, 524);
-        if (ok) mbar_arrive(bar(bKvEmpty + t % kStages));
-      }
+      release(t_end, n_stages);   // tile a does not read the last sub-tiles
     }
   } else {
     // ------------------------------------------------ rows: warpgroup w owns query tile Ia + w
@@ -395,14 +425,17 @@ tc_bwd_dq2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
     const long long rec0 = ((long long)hh * p.pairs_cap + c.pair0 + (long long)I * (I + 1) / 2) * (4 * kBM) + r;
     const bool ragged = I * kBM + kBM > c.len;   // the sequence ends inside this tile
     bool ok = true;
-    for (int u = 0; u < my_steps && ok; ++u) {
+    // this warp's rows start at sub-tile u_warp (never, if they are past the sequence): before it, A and dz are zeros
+    const int u_warp = (gi & ~31) < c.len ? first_key(p, c, h, gi & ~31) / kBN : 0x7fffffff;
+    // u: 64-key sub-tile inside the sequence; the first one is even, so that phases and stages follow from u alone
+    for (int u = w == 0 ? first_a : first_b; u < my_steps && ok; ++u) {
       ok = wait_or_abort(bar(bSpFull + w), u & 1, abort_flag, p, 530);
       if (!ok) break;
-      if (threadIdx.x == 0 && u == 0) trace_block(p, 1);
       if (r == 0) trace_event(p, 2 + w, tr_cur, 4 + 16 * w, u);
       tc_fence_after();
       // the dz tile is still being read by the previous step's dQ MMAs: waited for inside the pass, before its first store
-      const uint32_t gate = u >= 1 ? bar(bZEmpty + w) : 0u, gate_parity = (u - 1) & 1;
+      // (in the tile's first step parity 1 is the phase before the barrier's first: no wait)
+      const uint32_t gate = bar(bZEmpty + w), gate_parity = (u + 1) & 1;
       const float r1f = (float)r1;
       float gs = 0.f, logsum = 0.f;
       bool pass_ok;
@@ -417,7 +450,10 @@ tc_bwd_dq2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
         // this warp's copy of the previous step's dz rows has left shared memory before they are rewritten
         if (lane == 0) tma_store_wait_read();
         __syncwarp();
-        if (on_diag || ragged)
+        if (u < u_warp) {
+          pass_ok = mbar_wait(gate, gate_parity);
+          zero_strip_row(gZ, r, az_a, bar(bSpEmpty + w));
+        } else if (on_diag || ragged)
           pass_ok = strip_row_pass<kFp16, false, true>(tS, tP, r, on_diag ? (u - 2 * I) * kBN : 0, on_diag, p.attend_current, valid,
                                                        scale2, r1f, gpre, dr, gs, logsum, nullptr, gZ, nullptr, nullptr,
                                                        bar(bSpEmpty + w), gate, gate_parity, az_a, az_z);
@@ -427,9 +463,14 @@ tc_bwd_dq2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
       } else {
         float *rec_r1 = p.bnd_r1 + rec0 + (long long)u * (2 * kBM);   // quarter 2 (u & 1) of key tile u >> 1
         float *rec_s2 = p.bnd_s2 + rec0 + (long long)u * (2 * kBM);
-        rec_r1[0] = r1f;
+        rec_r1[0] = u < u_warp ? kNothingLeft : r1f;
         rec_s2[0] = gpre;
-        if (on_diag)
+        if (u < u_warp) {
+          rec_r1[kBM] = kNothingLeft;
+          rec_s2[kBM] = 0.f;
+          pass_ok = mbar_wait(gate, gate_parity);
+          zero_strip_row(gZ, r, nullptr, bar(bSpEmpty + w));
+        } else if (on_diag)
           pass_ok = strip_row_pass<kFp16, false, true>(tS, tP, r, (u - 2 * I) * kBN, true, p.attend_current, true, scale2, r1f, gpre,
                                                        dr, gs, logsum, nullptr, gZ, rec_r1 + kBM, rec_s2 + kBM, bar(bSpEmpty + w),
                                                        gate, gate_parity);
@@ -448,7 +489,7 @@ tc_bwd_dq2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
       // the sequence ends inside this sub-tile: its dz columns behind the end are exact zeros, the K rows there are
       // not this sequence's (see zero_tile_rows) and are cleared before this step's dz K MMA is released
       if (c.len - u * kBN < kBN)
-        zero_tile_rows(gbase + (sKV - base) + (u % kStages) * kStageBytes, c.len - u * kBN, kBN, 2, kKvBox, r, kBM);
+        zero_tile_rows(gbase + (sKV - base) + (u & 1) * kStageBytes, c.len - u * kBN, kBN, 2, kKvBox, r, kBM);
       tc_fence_before();          // this step's TMEM reads are done before the slots are handed back
       fence_proxy_async_smem();
       __syncwarp();
@@ -527,7 +568,8 @@ constexpr int kBN = 64;
 constexpr int kTileBytes = kBM * 128 * 2;      // Q, dO, K or V tile: two 128 x 64 boxes
 constexpr int kStripOffset = kBN * 128;        // byte offset of strip 1 inside a box (64 rows of 128 bytes)
 constexpr int kAzBytes = kBM * kBN * 2;        // A or dz tile, 128 rows x 64 keys
-constexpr int kSmem = 1024 + 2 * kTileBytes + 4 * kTileBytes + 2 * kAzBytes + 512;
+constexpr int kSmem = 1024 + 2 * kTileBytes + 4 * kTileBytes + 2 * kAzBytes + 512 + kListBits / 8;
+static_assert(kSmem <= 232448, "shared memory per block");
 enum { bKV = 0, bQgFull = 1, bQgEmpty = 3, bSpFull = 5, bSpEmpty = 7, bAzFull = 9, bAzEmpty = 10, bOutFull = 11, bStaged = 12,
        bDrained = 14, bNum = 16 };
 }  // namespace dkv4
@@ -562,9 +604,10 @@ tc_bwd_dkv4_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int hh = hh_blk, h = p.head0 + hh;
-  const int cnt = c.n_tiles - J;               // query tiles J .. n_tiles-1
-  const int n_steps = cnt * n_halves;          // step g: query tile J + g / n_halves, strip g % n_halves
+  // step g: the (g / n_halves)-th query tile that reaches this key tile, strip g % n_halves
+  QueryList list{p, c, h, J, kBM, c.n_tiles - J, reinterpret_cast<uint32_t *>(gbase + (sBar - base) + 512)};
   const int hshift = n_halves - 1;
+  list.build();
   int tr_cur = 0;   // cursor of this thread's event-log lane (diagnostics)
 
   if (threadIdx.x == 0) {
@@ -600,11 +643,11 @@ tc_bwd_dkv4_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
         tma_load_4d(sK + kb * kBoxBytes, &tm_k, bar(bKV), kb * 64, krow, h, (int)c.boff);
         tma_load_4d(sV + kb * kBoxBytes, &tm_v, bar(bKV), kb * 64, krow, h, (int)c.boff);
       }
-      for (int u = 0; u < cnt; ++u) {
+      for (int u = 0, off = 0; off < list.n; ++u, off = list.next(off + 1)) {
         const int b = u & 1;
         if (u >= 2 && !wait_or_abort(bar(bQgEmpty + b), ((u >> 1) - 1) & 1, abort_flag, p, 610)) break;
         if (*abort_flag) break;
-        const int qrow = (int)c.tok0 + (J + u) * kBM;
+        const int qrow = (int)c.tok0 + (J + off) * kBM;
         const uint32_t dst = sQ + b * 2 * kTileBytes;
         trace_event(p, 0, tr_cur, 1, u);
         mbar_arrive_expect_tx(bar(bQgFull + b), 2 * kTileBytes);
@@ -619,7 +662,7 @@ tc_bwd_dkv4_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
     if (lane == 0) {
       constexpr uint32_t idesc_s = idesc_f16(kBM, kBN, kFp16, false, false);
       bool ok = wait_or_abort(bar(bKV), 0, abort_flag, p, 620);
-      for (int g = 0; ok && g < n_steps; ++g) {
+      for (int g = 0, off = 0; ok && off < list.n; off = (g & hshift) == hshift ? list.next(off + 1) : off, ++g) {
         const int u = g >> hshift, hf = g & hshift, b = u & 1, slot = g & 1;
         ok = wait_or_abort(bar(bQgFull + b), (u >> 1) & 1, abort_flag, p, 621);
         // the rows of step g-2 have read this S/dP slot
@@ -640,7 +683,7 @@ tc_bwd_dkv4_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
       constexpr uint32_t idesc_t = idesc_f16(kBM, kBN, kFp16, true, true);
       const uint64_t a0 = smem_desc_sw128(sAZ, 16, 1024), z0 = smem_desc_sw128(sAZ + kAzBytes, 16, 1024);
       bool ok = true;
-      for (int g = 0; ok && g < n_steps; ++g) {
+      for (int g = 0, off = 0; ok && off < list.n; off = (g & hshift) == hshift ? list.next(off + 1) : off, ++g) {
         const int u = g >> hshift, hf = g & hshift, b = u & 1;
         ok = wait_or_abort(bar(bAzFull), g & 1, abort_flag, p, 623);
         if (!ok) break;
@@ -672,8 +715,8 @@ tc_bwd_dkv4_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
     // the per-row start values of a step come from global memory: they are fetched one step ahead
     // (the gradient of rem stays a raw 16-bit value until the step that uses it, so that nothing in this step depends
     // on the load)
-    auto fetch = [&](int g, float &r1f, float &gpre, unsigned short &dr_raw) {
-      const int I = J + (g >> hshift), quarter = 2 * (g & hshift) + w;   // which 32-key quarter of the 128-key tile
+    auto fetch = [&](int I, int hf, float &r1f, float &gpre, unsigned short &dr_raw) {
+      const int quarter = 2 * hf + w;   // which 32-key quarter of the 128-key tile
       const int gi = I * kBM + r;
       const long long slot = (((long long)hh * p.pairs_cap + c.pair0 + (long long)I * (I + 1) / 2 + J) * 4 + quarter) * kBM + r;
       r1f = p.bnd_r1[slot];
@@ -685,15 +728,17 @@ tc_bwd_dkv4_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
     uint8_t *gZ = gA + kAzBytes;
     float nr1, ngpre;
     unsigned short ndr;
-    fetch(0, nr1, ngpre, ndr);
-    for (int g = 0; g < n_steps && ok; ++g) {
+    fetch(J, 0, nr1, ngpre, ndr);
+    int off = 0, off_next = 0;   // this step's and the next step's query tile
+    for (int g = 0; off < list.n && ok; ++g, off = off_next) {
       const int u = g >> hshift, hf = g & hshift, slot = g & 1;
-      const int I = J + u;
+      const int I = J + off;
+      off_next = hf == hshift ? list.next(off + 1) : off;
       const int quarter = 2 * hf + w;
       const bool valid = I * kBM + r < c.len;
       const float r1f = nr1, gpre = ngpre;
       const float dr = valid ? to_f32<T>(*reinterpret_cast<const T *>(&ndr)) : 0.f;
-      if (g + 1 < n_steps) fetch(g + 1, nr1, ngpre, ndr);
+      if (off_next < list.n) fetch(J + off_next, (g + 1) & hshift, nr1, ngpre, ndr);
       ok = wait_or_abort(bar(bSpFull + slot), (g >> 1) & 1, abort_flag, p, 630);
       if (!ok) break;
       if (threadIdx.x == 0 && g == 0) trace_block(p, 1);
@@ -849,7 +894,7 @@ constexpr int kRows = 32;                    // query rows per stage
 constexpr int kSub = kBM / kRows;            // stages per query tile
 constexpr int kBox = kRows * 64 * 2;         // kRows rows x 64 columns, 16-bit
 constexpr int kStageBytes = 8 * kBox;        // A, dz, Q, dO: two 64-column blocks each; also one 128 x 128 output tile
-constexpr int kSmem = 1024 + kStages * kStageBytes + 512;
+constexpr int kSmem = 1024 + kStages * kStageBytes + 512 + kListBits / 8;
 constexpr uint32_t kCols = 256;              // dK 0..127, dV 128..255
 enum { bFull = 0, bEmpty = 3, bOut = 6, bClean = 7, bLanded = 8, bNum = 9 };
 }  // namespace dkv5
@@ -868,14 +913,13 @@ tc_bwd_dkv5_kernel(const __grid_constant__ CUtensorMap tm_az, const __grid_const
   if (!decode_block(p, 1, false, c, hh)) return;
   const int h = p.head0 + hh;
   const int J = c.idx;                        // the 128-key tile
-  const int n_stages = kSub * (c.n_tiles - J);   // stage t: query tile J + t / kSub, rows (t % kSub) * kRows .. + kRows
   // The sequence may end inside the last query tile.  The A and dz rows behind the end are zeros in the workspace; the
-  // Q and dO rows there are not this sequence's (see zero_tile_rows).  Stages from t_clean on hold such rows: the
+  // Q and dO rows there are not this sequence's (see zero_tile_rows).  Stages that hold such rows are cleaned: the
   // issuer tells the epilogue warps, idle until the end, that such a stage has landed (bLanded; a barrier of its own,
   // because a parity wait on bFull only works for a waiter that follows every phase), they clear the rows and hand
   // the stage back through bClean.
   const int last_rows = c.len - (c.n_tiles - 1) * kBM;          // 1 .. 128 rows of the last query tile exist
-  const int t_clean = last_rows >= kBM ? n_stages : n_stages - (kSub - last_rows / kRows);
+  const int clean_from = last_rows / kRows;                     // first such stage of the last query tile
 
   const uint32_t raw = smem_u32(smem_raw);
   const uint32_t base = (raw + 1023u) & ~1023u;
@@ -883,8 +927,12 @@ tc_bwd_dkv5_kernel(const __grid_constant__ CUtensorMap tm_az, const __grid_const
   const uint32_t sBar = base + kStages * kStageBytes;
   Ctl *ctl = reinterpret_cast<Ctl *>(gbase + (sBar - base) + bNum * 8);
   volatile int *abort_flag = &ctl->abort;
+  volatile int *clean_stage = reinterpret_cast<volatile int *>(ctl + 1);
   auto bar = [&](int i) { return sBar + 8u * i; };
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  // the query tiles that reach this key tile, kSub stages each
+  QueryList list{p, c, h, J, kBM, c.n_tiles - J, reinterpret_cast<uint32_t *>(gbase + (sBar - base) + 512)};
+  list.build();
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < kStages; ++s) { mbar_init(bar(bFull + s), 1); mbar_init(bar(bEmpty + s), 1); }
@@ -906,11 +954,11 @@ tc_bwd_dkv5_kernel(const __grid_constant__ CUtensorMap tm_az, const __grid_const
   if (warp == 4) {
     if (lane == 0) {
       prefetch_tensormap(&tm_az); prefetch_tensormap(&tm_q); prefetch_tensormap(&tm_g);
-      for (int t = 0; t < n_stages; ++t) {
+      for (int t = 0, off = 0; off < list.n; ++t, off = t % kSub == 0 ? list.next(off + 1) : off) {
         const int st = t % kStages;
         if (t >= kStages && !wait_or_abort(bar(bEmpty + st), ((t / kStages) - 1) & 1, abort_flag, p, 640)) break;
         if (*abort_flag) break;
-        const int I = J + t / kSub, hq = t % kSub;
+        const int I = J + off, hq = t % kSub;
         const long long pair = c.pair0 + (long long)I * (I + 1) / 2 + J;
         const int az_row = (int)(pair * kBM) + hq * kRows;
         const int qrow = (int)c.tok0 + I * kBM + hq * kRows;
@@ -929,12 +977,14 @@ tc_bwd_dkv5_kernel(const __grid_constant__ CUtensorMap tm_az, const __grid_const
       // all operands MN-major: rows = query rows (the contraction), two 64-column blocks kBox apart
       constexpr uint32_t idesc = idesc_f16(kBM, D, kFp16, true, true);
       bool ok = true;
-      for (int t = 0; ok && t < n_stages; ++t) {
+      int cleaned = 0;
+      for (int t = 0, off = 0; ok && off < list.n; ++t, off = t % kSub == 0 ? list.next(off + 1) : off) {
         const int st = t % kStages;
         ok = wait_or_abort(bar(bFull + st), (t / kStages) & 1, abort_flag, p, 641);
-        if (ok && t >= t_clean) {
+        if (ok && off == list.n - 1 && t % kSub >= clean_from) {
+          *clean_stage = st;
           mbar_arrive(bar(bLanded));
-          ok = wait_or_abort(bar(bClean), (t - t_clean) & 1, abort_flag, p, 643);
+          ok = wait_or_abort(bar(bClean), cleaned++ & 1, abort_flag, p, 643);
         }
         if (!ok) break;
         tc_fence_after();
@@ -957,11 +1007,12 @@ tc_bwd_dkv5_kernel(const __grid_constant__ CUtensorMap tm_az, const __grid_const
     const int r = threadIdx.x;
     const uint32_t lane_off = (uint32_t)(warp * 32) << 16;
     bool ok = true;
-    for (int t = t_clean; ok && t < n_stages; ++t) {
-      const int st = t % kStages;
-      ok = wait_or_abort(bar(bLanded), (t - t_clean) & 1, abort_flag, p, 644);
+    const bool last_listed = list.next(list.n - 1) < list.n;
+    for (int hq = clean_from; ok && last_listed && hq < kSub; ++hq) {
+      ok = wait_or_abort(bar(bLanded), (hq - clean_from) & 1, abort_flag, p, 644);
       if (!ok) break;
-      int keep = last_rows - (t % kSub) * kRows;   // rows of this stage that belong to the sequence
+      const int st = *clean_stage;
+      int keep = last_rows - hq * kRows;   // rows of this stage that belong to the sequence
       keep = keep < 0 ? 0 : keep;
       zero_tile_rows(gbase + st * kStageBytes + 4 * kBox, keep, kRows, 4, kBox, r, kBM);   // Q and dO: boxes 4..7 of the stage
       fence_proxy_async_smem();

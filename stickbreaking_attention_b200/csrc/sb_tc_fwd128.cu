@@ -38,6 +38,12 @@ constexpr uint32_t kWorkerCols = 192;
 // barriers of one worker
 enum { bQ = 0, bQFree = 2, bKvFull = 4, bKvEmpty = 4 + kStages, bSFull = 4 + 2 * kStages, bPFull = bSFull + 2, bOFull = bSFull + 4,
        bOFree = bSFull + 5, bPerWorker = bSFull + 6 };
+struct Shared {                               // behind the barriers
+  Ctl ctl;
+  EarlyStop stop[2];                          // per worker
+  int kv_end[2][kStages];                     // per stage: stage number + 1 if it holds no keys but marks the end of its tile
+};
+static_assert(2 * bPerWorker * 8 + sizeof(Shared) <= kBarBytes, "barriers and control words");
 }  // namespace fwd128
 
 struct Fwd128Item {
@@ -67,7 +73,9 @@ __device__ __forceinline__ bool fwd128_item(const KParams &p, int it, int v, int
   return true;
 }
 
-template <bool kFp16>
+// kStop: tiles may stop early.  A tile of a sequence of up to 512 tokens has no four sub-tiles left by the time it could
+// (see may_stop_before), and the code for it costs short tiles 6 %: the launch leaves it out for such calls.
+template <bool kFp16, bool kStop>
 __global__ void __launch_bounds__(fwd128::kThreads, 1)
 tc_fwd128x2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                    const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_o, const KParams p) {
@@ -79,7 +87,8 @@ tc_fwd128x2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
   const uint32_t base = (raw + 1023u) & ~1023u;
   uint8_t *gbase = smem_raw + (base - raw);
   const uint32_t sBar = base + 2 * kWorkerBytes;
-  Ctl *ctl = reinterpret_cast<Ctl *>(gbase + (sBar - base) + 2 * bPerWorker * 8);
+  Shared *sh = reinterpret_cast<Shared *>(gbase + (sBar - base) + 2 * bPerWorker * 8);
+  Ctl *ctl = &sh->ctl;
   volatile int *abort_flag = &ctl->abort;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -96,9 +105,12 @@ tc_fwd128x2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
       auto b = [&](int i) { return sBar + 8u * (w * bPerWorker + i); };
       for (int i = 0; i < kQBufs; ++i) { mbar_init(b(bQ + i), 1); mbar_init(b(bQFree + i), 1); }
       for (int s = 0; s < kStages; ++s) { mbar_init(b(bKvFull + s), 1); mbar_init(b(bKvEmpty + s), 1); }
-      for (int s = 0; s < 2; ++s) { mbar_init(b(bSFull + s), 1); mbar_init(b(bPFull + s), 4); }
+      for (int s = 0; s < 2; ++s) { mbar_init(b(bSFull + s), 2); mbar_init(b(bPFull + s), 4); }   // S: commit and word
       mbar_init(b(bOFull), 1);
       mbar_init(b(bOFree), 4);
+      sh->stop[w].stopped = 0;
+      for (int i = 0; i < 4; ++i) sh->stop[w].through[i] = 0;
+      for (int s = 0; s < kStages; ++s) sh->kv_end[w][s] = 0;
     }
     ctl->abort = 0;
     fence_barrier_init();
@@ -112,6 +124,8 @@ tc_fwd128x2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
   tc_fence_after();
   const uint32_t tmem = ctl->tmem_base + wk * kWorkerCols;
 
+  volatile EarlyStop &stop = sh->stop[wk];
+  volatile int *kv_end = sh->kv_end[wk];
   Fwd128Item w;
   if (warp == 8 || warp == 11) {
     // ------------------------------------------------ TMA producer of this worker
@@ -127,10 +141,17 @@ tc_fwd128x2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
           tma_load_4d(sQ + qb * kQBytes + b * (kQBytes / 4), &tm_q, bar(bQ + qb), 0,
                       (int)w.c.tok0 + w.row0 + (wk ? 3 - b : b) * 32, w.h, (int)w.c.boff);
         bool ok = true;
+        int used = w.n_steps;   // stages this tile takes
         for (int t = 0; t < w.n_steps; ++t) {
           const int g = T + t, st = g % kStages;
           if (g >= kStages && !wait_or_abort(bar(bKvEmpty + st), ((g / kStages) - 1) & 1, abort_flag, p, 710)) { ok = false; break; }
           if (*abort_flag) { ok = false; break; }
+          if (kStop && stop.stopped == it + 1) {   // no more keys are wanted: mark the tile's end
+            kv_end[st] = g + 1;
+            mbar_arrive(bar(bKvFull + st));
+            used = t + 1;
+            break;
+          }
           const int krow = (int)w.c.tok0 + (w.s_top - t) * kBN;
           const uint32_t dst = sKV + st * kStageBytes;
           mbar_arrive_expect_tx(bar(bKvFull + st), kStageBytes);
@@ -138,7 +159,7 @@ tc_fwd128x2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
           tma_load_4d(dst + kKvTileBytes, &tm_v, bar(bKvFull + st), 0, krow, w.h, (int)w.c.boff);
         }
         if (!ok) break;
-        T += w.n_steps;
+        T += used;
       }
     }
   } else if (warp == 9 || warp == 10) {
@@ -155,14 +176,27 @@ tc_fwd128x2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
         // Iteration u issues S(u) and then P V of step u-1, so that the next scores are being computed while the
         // rows of the current step are processed.  S(u) reuses the TMEM slot of step u-2, whose P the P V MMA of
         // that step (issued earlier by this thread) has read.
-        for (int u = 0; ok && u <= w.n_steps; ++u) {
-          if (u < w.n_steps) {
+        int steps = w.n_steps, used = w.n_steps;   // steps computed and stages taken
+        bool early = false, halt = false;   // halt: the tile stops before step u (decided while the rows of step u - 2 worked)
+        for (int u = 0; ok && u <= steps; ++u) {
+          if (halt) {
+            early = true;
+            steps = u;
+            stop.stopped = it + 1;
+            stop.word[(U + u) & 1] = kStepStop;
+            mma_commit(bar(bQFree + qb));
+            mbar_arrive(bar(bSFull + ((U + u) & 1)));
+            mbar_arrive(bar(bSFull + ((U + u) & 1)));
+          } else if (u < w.n_steps) {
             const int g = T + u, st = g % kStages, gu = U + u;
             ok = wait_or_abort(bar(bKvFull + st), (g / kStages) & 1, abort_flag, p, 721);
             if (!ok) break;
             tc_fence_after();
             mma_kmajor_kmajor<D, kQBytes, kKvTileBytes>(tmem + (gu & 1) * 64, qaddr, sKV + st * kStageBytes, idesc_s, false);
             mma_commit(bar(bSFull + (gu & 1)));
+            stop.word[gu & 1] = st;
+            mbar_arrive(bar(bSFull + (gu & 1)));
+            halt = kStop && u >= 2 && u + 1 < w.n_steps && may_stop_before(w.s_top - u - 1) && all_through(stop, it, u - 2);
             if (u == w.n_steps - 1) mma_commit(bar(bQFree + qb));   // the tile's last read of Q
           }
           if (u >= 1) {
@@ -177,10 +211,19 @@ tc_fwd128x2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
             mma_commit(bar(bKvEmpty + st));
           }
         }
+        if (ok && early) {   // the stop word's slot has a P phase like every other; the rest of the tile's stages go unread
+          ok = wait_or_abort(bar(bPFull + ((U + steps) & 1)), ((U + steps) >> 1) & 1, abort_flag, p, 726);
+          for (int t = steps; ok && t < used; ++t) {
+            const int g = T + t, s = g % kStages;
+            ok = wait_or_abort(bar(bKvFull + s), (g / kStages) & 1, abort_flag, p, 724);
+            if (kv_end[s] == g + 1) used = t + 1;
+            if (ok) mbar_arrive(bar(bKvEmpty + s));
+          }
+        }
         if (!ok) break;
         mma_commit(bar(bOFull));   // this tile's O is complete
-        T += w.n_steps;
-        U += w.n_steps;
+        T += used;
+        U += steps + (early ? 1 : 0);
       }
     }
   } else {
@@ -191,7 +234,7 @@ tc_fwd128x2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
     const uint32_t lane_off = (uint32_t)((warp & 3) * 32) << 16;
     const float scale2 = p.scale * kLog2e;
     const int ac = p.attend_current;
-    int U = 0, S = 0;   // steps and K/V stages of the earlier tiles
+    int U = 0;   // steps of the earlier tiles
     bool ok = true;
     Fwd128Item w_next;
     bool have = fwd128_item(p, 0, v, V, w);
@@ -200,7 +243,10 @@ tc_fwd128x2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
       const int row = w.row0 + blk * 32 + lane;      // row index inside the sequence
       const int s_diag0 = 2 * w.c.idx;               // first sub-tile that reaches this tile's diagonal band
       const bool warp_live = (row & ~31) < w.c.len;  // a warp whose 32 rows all lie past the sequence end computes nothing
-      double run = 0.0;
+      LogSum run;
+      bool through = false;    // this warp is through with the tile, having got to sub-tile s_reached
+      int s_reached = 0;
+      int slots = w.n_steps;                         // S slots used
       if (lane == 0) tma_store_wait_read();          // the previous tile's O has left the staging tile
       __syncwarp();
       for (int u = 0; u < w.n_steps && ok; ++u) {
@@ -208,36 +254,53 @@ tc_fwd128x2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
         const int gu = U + u, buf = gu & 1;
         ok = wait_or_abort(bar(bSFull + buf), (gu >> 1) & 1, abort_flag, p, 730);
         if (!ok) break;
+        if (kStop && through && stop.word[buf] == kStepStop) {   // (a stop needs this warp's consent)
+          slots = u + 1;
+          __syncwarp();
+          if (lane == 0) mbar_arrive(bar(bPFull + buf));
+          break;
+        }
         tc_fence_after();
         const uint32_t ts = tmem + buf * 64 + lane_off;
         // the sequence ends inside this sub-tile: the V rows behind its end are not this sequence's (see
         // zero_tile_rows); their P columns are exact zeros, so the rows are cleared before this step's P V MMA
         const int tail_rows = w.c.len - s * kBN;
         if (tail_rows < kBN) {
-          zero_tile_rows(gbase + (sKV - base) + ((S + u) % kStages) * kStageBytes + kKvTileBytes, tail_rows, kBN, 1, kKvTileBytes, r, kBM);
+          zero_tile_rows(gbase + (sKV - base) + stop.word[buf] * kStageBytes + kKvTileBytes, tail_rows, kBN, 1, kKvTileBytes, r, kBM);
           fence_proxy_async_smem();
         }
-        float R = ex2(-(float)run);
+        bool done = through || !warp_live;
         float logsum = 0.f;
         // (the P rows of such a warp keep whatever the slot held: they only reach accumulator rows that are never stored)
-        if (!warp_live) {
-        } else if (s >= s_diag0) fwd256_row_pass<kFp16, true>(ts, s * kBN, row, ac, scale2, R, logsum, nullptr, r, ts + kPCol);
-        else fwd256_row_pass<kFp16, false>(ts, 0, 0, ac, scale2, R, logsum, nullptr, r, ts + kPCol, !p.dense);
-        run += (double)logsum;
+        if (through) {
+          fwd256_zero_row(ts + kPCol);
+        } else if (!warp_live) {
+        } else if (s >= s_diag0) fwd256_row_pass<kFp16, true>(ts, s * kBN, row, ac, scale2, run, logsum, ts + kPCol, true);
+        else done = fwd256_row_pass<kFp16, false>(ts, 0, 0, ac, scale2, run, logsum, ts + kPCol, row < w.c.len, !p.dense, kStop);
+        run.add(logsum);
         tmem_wait_st();
         tc_fence_before();          // this step's TMEM reads and its writes of P are done before the slot is handed back
         __syncwarp();
-        if (lane == 0) mbar_arrive(bar(bPFull + buf));
+        if (lane == 0) {
+          if (kStop && done && !through) publish_through(stop, warp & 3, it, u);
+          mbar_arrive(bar(bPFull + buf));
+        }
+        if (kStop && done && !through) {
+          through = true;
+          s_reached = s + 1;
+        }
       }
       // ---- epilogue: O (TMEM) -> global, rem, log_rem
       // While the last P V MMA finishes: rem and log_rem leave, and the next tile's table entries are fetched.
       const bool valid = row < w.c.len;
-      const float rem_f = ex2(-(float)run);
+      const float rem_f = run.stick();
       if (ok && valid) {
         const long long idx = (w.c.boff * p.heads + w.h) * p.tokens + w.c.tok0 + row;
         reinterpret_cast<T *>(p.rem)[idx] = from_f32<T>(rem_f);
-        p.log_rem[idx] = -run;
+        p.log_rem[idx] = -run.value();
       }
+      if (p.tile_start != nullptr && ok && warp_live && lane == 0 && row >= 64)
+        *tile_start_entry(p, w.c, w.h, row) = s_reached * kBN;
       const bool have_next = fwd128_item(p, it + 1, v, V, w_next);
       if (ok) ok = wait_or_abort(bar(bOFull), it & 1, abort_flag, p, 732);
       if (ok) {
@@ -264,8 +327,7 @@ tc_fwd128x2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
       tc_fence_before();            // the accumulator has been read: the next tile may overwrite it
       __syncwarp();
       if (lane == 0) mbar_arrive(bar(bOFree));
-      U += w.n_steps;
-      S += w.n_steps;
+      U += slots;
       w = w_next;
       have = have_next;
     }
@@ -277,7 +339,7 @@ tc_fwd128x2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
   if (warp == 9) tmem_dealloc(ctl->tmem_base, kTmemCols);
 }
 
-template <bool kFp16>
+template <bool kFp16, bool kStop>
 static cudaError_t launch128_t(const KParams &p, int dtype, cudaStream_t s) {
   CUtensorMap mq, mk, mv, mo;
   cudaError_t e;
@@ -289,14 +351,16 @@ static cudaError_t launch128_t(const KParams &p, int dtype, cudaStream_t s) {
   if ((e = sm_count(&sms)) != cudaSuccess) return e;
   const long long blocks = (item_blocks(p, 1) + 1) / 2;       // two workers per block
   const dim3 grid((unsigned)(blocks < sms ? blocks : sms));   // one resident block per SM
-  auto kernel = tc_fwd128x2_kernel<kFp16>;
+  auto kernel = tc_fwd128x2_kernel<kFp16, kStop>;
   if ((e = allow_dynamic_smem(reinterpret_cast<const void *>(kernel), fwd128::kSmem)) != cudaSuccess) return e;
   kernel<<<grid, fwd128::kThreads, fwd128::kSmem, s>>>(mq, mk, mv, mo, p);
   return cudaGetLastError();
 }
 
 cudaError_t launch_tc_fwd128(const KParams &p, int dtype, cudaStream_t s) {
-  return dtype == SB_DTYPE_F16 ? launch128_t<true>(p, dtype, s) : launch128_t<false>(p, dtype, s);
+  if (p.tile_start != nullptr && !p.dense && p.max_seqlen > 512)
+    return dtype == SB_DTYPE_F16 ? launch128_t<true, true>(p, dtype, s) : launch128_t<false, true>(p, dtype, s);
+  return dtype == SB_DTYPE_F16 ? launch128_t<true, false>(p, dtype, s) : launch128_t<false, false>(p, dtype, s);
 }
 
 }  // namespace sb

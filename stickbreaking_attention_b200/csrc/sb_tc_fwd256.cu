@@ -5,10 +5,10 @@
 // sub-tiles from its last needed key back to the sequence start.  Both tiles consume the same K/V stage, so K/V
 // is read once per 256 rows, and the two row-owning warpgroups (warps 0-3: tile a, warps 4-7: tile b) keep two
 // warps resident per scheduler so that one hides the other's dependent-issue and TMEM latency.
-//   warp 8    TMA producer: Q_a, Q_b once, then K/V sub-tiles into a 3-stage ring
+//   warp 8    TMA producer: Q_a, Q_b once, then K/V sub-tiles into a ring of stages
 //   warps 9,10 MMA issuers, one per tile: S_x = Q_x K^T (128x64) into a double-buffered TMEM slot, O_x += P_x V
 //   warps 0-7 one thread per query row: p = beta * R with the running product R of (1 - beta) over later keys,
-//             P written as a 16-bit [128 x 64] swizzled tile (double-buffered) for the second MMA
+//             P written back to tensor memory in 16 bits for the second MMA
 // TMEM columns: S_a[2] 0..127, S_b[2] 128..255, O_a 256..383, O_b 384..511.  All waits are bounded.
 #include "sb_tc_fwd_rows.cuh"
 
@@ -25,17 +25,24 @@ struct Cfg {
   static constexpr int kQBytes = kBM * D * 2;                  // one 128-row Q tile
   static constexpr int kKvTileBytes = kBoxes * kKvBoxBytes;    // K or V sub-tile: 64 keys x D columns
   static constexpr int kStageBytes = 2 * kKvTileBytes;         // K and V
-  // K/V ring: three stages at 128 columns fill the shared memory; at 64 columns six fit, and short sequences need
-  // them: a stage is reloaded only after both tiles' P V MMAs of its step, so with three stages the load for step
-  // s + 3 starts one row pass before its scores are wanted, which the ~2000 clk load latency does not always meet
-  static constexpr int kStages = D == 64 ? 6 : 3;
+  // K/V ring.  A stage is reloaded only after both tiles' P V MMAs of its step, and one tile runs a step ahead of the
+  // other, so that of n stages n - 2 hide the load latency: with three the event log shows every S MMA at 128 columns
+  // waiting ~1000 of 2800 clk for its keys.  Four fit next to one staging box per tile; at 64 columns six do.
+  static constexpr int kStages = D == 64 ? 6 : 4;
   // Q tiles of two items at 64 columns (there is room): the next item's Q is loaded while the current item still
   // reads its own, so a short item does not wait a load latency for its first scores
   static constexpr int kQBufs = D == 64 ? 2 : 1;
-  static constexpr int kSmem = 1024 + kQBufs * 2 * kQBytes + kStages * kStageBytes + 4 * kPBytes + kBarBytes;
+  static constexpr int kSmem = 1024 + kQBufs * 2 * kQBytes + kStages * kStageBytes + 2 * kPBytes + kBarBytes;
+  static_assert(kSmem <= 232448, "shared memory per block");
 };
-enum { bQ = 0, bKvFull = 1, bKvEmpty = 7, bSFull = 13, bQFree = 17, bOFree = 18, bPFull = 20, bPEmpty = 24, bOFull = 28, bQ2 = 30,
-       bQFree2 = 31, bNum = 32 };   // bQ2 / bQFree2: the second Q buffer
+enum { bQ = 0, bKvFull = 1, bKvEmpty = 7, bSFull = 13, bQFree = 17, bOFree = 18, bPFull = 20, bOFull = 24, bQ2 = 26,
+       bQFree2 = 27, bNum = 28 };   // bQ2 / bQFree2: the second Q buffer
+struct Shared {                     // behind the barriers
+  Ctl ctl;
+  EarlyStop stop[2];                // per tile
+  int kv_end[kMaxStages];           // per stage: stage number + 1 if it holds no keys but marks the end of its item
+};
+static_assert(bNum * 8 + sizeof(Shared) <= kBarBytes, "barriers and control words");
 static_assert(bKvEmpty - bKvFull == kMaxStages && bSFull - bKvEmpty == kMaxStages, "barrier slots per stage");
 // per-warpgroup barrier index: base + wg * 2 + buf
 }  // namespace fwd256
@@ -92,11 +99,13 @@ tc_fwd256_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
   uint8_t *gbase = smem_raw + (base - raw);
   const uint32_t sQ = base;                             // per buffer: Q_a, Q_b
   const uint32_t sKV = sQ + kQBufs * 2 * kQBytes;       // stages: K sub-tile then V sub-tile
-  const uint32_t sP = sKV + kStages * kStageBytes;      // P[wg][buf]
-  const uint32_t sBar = sP + 4 * kPBytes;
+  const uint32_t sP = sKV + kStages * kStageBytes;      // staging of O, one 128 x 64 box per tile
+  const uint32_t sBar = sP + 2 * kPBytes;
   uint8_t *gP = gbase + (sP - base);
-  Ctl *ctl = reinterpret_cast<Ctl *>(gbase + (sBar - base) + bNum * 8);
+  Shared *sh = reinterpret_cast<Shared *>(gbase + (sBar - base) + bNum * 8);
+  Ctl *ctl = &sh->ctl;
   volatile int *abort_flag = &ctl->abort;
+  const bool may_stop = p.tile_start != nullptr && !p.dense;
   auto bar = [&](int i) { return sBar + 8u * i; };
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -109,15 +118,19 @@ tc_fwd256_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
     mbar_init(bar(bQFree2), 2);
     for (int s = 0; s < kStages; ++s) { mbar_init(bar(bKvFull + s), 1); mbar_init(bar(bKvEmpty + s), 2); }
     for (int s = 0; s < 4; ++s) {
-      mbar_init(bar(bSFull + s), 1);
+      mbar_init(bar(bSFull + s), 2);   // the MMAs' commit, and the issuer itself (its word about the step)
       mbar_init(bar(bPFull + s), 4);
-      mbar_init(bar(bPEmpty + s), 1);
     }
     mbar_init(bar(bOFull), 1);
     mbar_init(bar(bOFull + 1), 1);
     mbar_init(bar(bOFree), 4);
     mbar_init(bar(bOFree + 1), 4);
     ctl->abort = 0;
+    for (int w = 0; w < 2; ++w) {
+      sh->stop[w].stopped = 0;
+      for (int i = 0; i < 4; ++i) sh->stop[w].through[i] = 0;
+    }
+    for (int s = 0; s < kStages; ++s) sh->kv_end[s] = 0;
     fence_barrier_init();
   }
   if (warp == 9) {
@@ -146,10 +159,18 @@ tc_fwd256_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
           for (int kb = 0; kb < kBoxes; ++kb)
             tma_load_4d(sQ + (qb * 2 + t) * kQBytes + kb * kBoxBytes, &tm_q, bar_q, kb * 64, qrow + t * kBM, w.h, (int)w.c.boff);
         bool ok = true;
+        int used = w.n_steps;   // stages this item takes
         for (int t = 0; t < w.n_steps; ++t) {
           const int g = T + t, st = g % kStages;
           if (g >= kStages && !wait_or_abort(bar(bKvEmpty + st), ((g / kStages) - 1) & 1, abort_flag, p, 310)) { ok = false; break; }
           if (*abort_flag) { ok = false; break; }
+          const volatile EarlyStop *stop = sh->stop;
+          if (stop[0].stopped == it + 1 && stop[1].stopped == it + 1) {   // no tile wants these keys: mark the item's end
+            *(volatile int *)&sh->kv_end[st] = g + 1;
+            mbar_arrive(bar(bKvFull + st));
+            used = t + 1;
+            break;
+          }
           const int krow = (int)w.c.tok0 + (w.s_top - t) * kBN;
           const uint32_t dst = sKV + st * kStageBytes;
           trace_event(p, 0, tr_cur, 1, t);
@@ -160,7 +181,7 @@ tc_fwd256_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
           }
         }
         if (!ok) break;
-        T += w.n_steps;
+        T += used;
       }
     }
   } else if (warp >= 9) {
@@ -173,14 +194,22 @@ tc_fwd256_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
       bool ok = true;
       for (int it = 0; ok && fwd256_item(p, it, w); ++it) {
         const bool active = wg == 0 || w.b_active;
-        const int t0 = active ? (wg == 0 ? w.t0_a : 0) : w.n_steps;   // stages this tile does not read
-        const int my_steps = w.n_steps - t0;
-        // release the unread stages on this tile's behalf, each once it has been filled
-        for (int t = 0; ok && t < t0; ++t) {
-          const int g = T + t;
-          ok = wait_or_abort(bar(bKvFull + g % kStages), (g / kStages) & 1, abort_flag, p, 324);
-          if (ok) mbar_arrive(bar(bKvEmpty + g % kStages));
-        }
+        const int t0 = active && wg == 0 ? w.t0_a : 0;
+        const int my_steps = active ? w.n_steps - t0 : 0;
+        volatile EarlyStop &stop = sh->stop[wg];
+        if (!active) stop.stopped = it + 1;
+        int used = w.n_steps;   // stages of this item; fewer if both tiles stop early
+        // releases stages t < t_end on this tile's behalf, each once it has been filled (or marked as the item's end)
+        auto release = [&](int t, int t_end) {
+          for (; ok && t < t_end; ++t) {
+            const int g = T + t, st = g % kStages;
+            ok = wait_or_abort(bar(bKvFull + st), (g / kStages) & 1, abort_flag, p, 324);
+            const bool end = *(volatile int *)&sh->kv_end[st] == g + 1;
+            if (ok) mbar_arrive(bar(bKvEmpty + st));
+            if (end) { used = t + 1; return; }
+          }
+        };
+        release(0, t0);
         const int qb = it % kQBufs, qn = it / kQBufs;
         const uint32_t qaddr = sQ + (qb * 2 + wg) * kQBytes, bar_qfree = bar(qb ? bQFree2 : bQFree);
         // (an idle issuer waits too: a parity wait is only meaningful for a waiter that follows every phase)
@@ -188,8 +217,19 @@ tc_fwd256_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
         // Iteration u issues S(u) and then P V of step u-1, so that the next scores are being computed while the
         // rows of the current step are processed.  S(u) reuses the TMEM slot of step u-2, whose rows were finished
         // before p_full(u-2) was signalled, and that was waited for in iteration u-1.
-        for (int u = 0; ok && active && u <= my_steps; ++u) {
-          if (u < my_steps) {
+        int steps = my_steps;          // steps computed
+        bool early = false, halt = false;   // halt: the tile stops before step u (decided while the rows of step u - 2 worked)
+        for (int u = 0; ok && active && u <= steps; ++u) {
+          if (halt) {
+            early = true;
+            steps = u;
+            stop.stopped = it + 1;
+            const int slot = (U + u) & 1;
+            stop.word[slot] = kStepStop;
+            mma_commit(bar_qfree);
+            mbar_arrive(bar(bSFull + wg * 2 + slot));
+            mbar_arrive(bar(bSFull + wg * 2 + slot));
+          } else if (u < my_steps) {
             const int g = T + t0 + u, st = g % kStages, gu = U + u;
             ok = wait_or_abort(bar(bKvFull + st), (g / kStages) & 1, abort_flag, p, 321);
             if (!ok) break;
@@ -198,6 +238,9 @@ tc_fwd256_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
             mma_kmajor_kmajor<D, kBoxBytes, kKvBoxBytes>(tmem + wg * 128 + (gu & 1) * 64, qaddr, sKV + st * kStageBytes, idesc_s,
                                                          false);
             mma_commit(bar(bSFull + wg * 2 + (gu & 1)));
+            stop.word[gu & 1] = st;
+            mbar_arrive(bar(bSFull + wg * 2 + (gu & 1)));
+            halt = may_stop && u >= 2 && u + 1 < my_steps && may_stop_before(w.s_top - t0 - u - 1) && all_through(stop, it, u - 2);
             if (u == my_steps - 1) mma_commit(bar_qfree);   // the item's last read of Q
             trace_event(p, 1 + 3 * wg, tr_cur, 3 + 16 * wg, t0 + u);
           }
@@ -210,23 +253,25 @@ tc_fwd256_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
             trace_event(p, 1 + 3 * wg, tr_cur, 6 + 16 * wg, t0 + up);
             tc_fence_after();
             // 16 keys per MMA; V: 64 rows x (2 x 64) columns, MN-major
-            if constexpr (kPTmem) {
-              mma_tmem_mnmajor<kBN, kKvBoxBytes>(tmem + 256 + wg * 128, tmem + wg * 128 + (gu & 1) * 64 + kPCol,
-                                                 sKV + st * kStageBytes + kKvTileBytes, idesc_pv, up > 0);
-            } else {
-              mma_kmajor_mnmajor<kBN, kKvBoxBytes>(tmem + 256 + wg * 128, sP + (wg * 2 + (gu & 1)) * kPBytes,
-                                                   sKV + st * kStageBytes + kKvTileBytes, idesc_pv, up > 0);
-              mma_commit(bar(bPEmpty + wg * 2 + (gu & 1)));
-            }
+            mma_tmem_mnmajor<kBN, kKvBoxBytes>(tmem + 256 + wg * 128, tmem + wg * 128 + (gu & 1) * 64 + kPCol,
+                                               sKV + st * kStageBytes + kKvTileBytes, idesc_pv, up > 0);
             mma_commit(bar(bKvEmpty + st));
             trace_event(p, 1 + 3 * wg, tr_cur, 7 + 16 * wg, t0 + up);
           }
         }
         if (!ok) break;
+        if (early) {   // the stop word's slot has a P phase like every other; the rest of the item's stages go unread
+          ok = wait_or_abort(bar(bPFull + wg * 2 + ((U + steps) & 1)), ((U + steps) >> 1) & 1, abort_flag, p, 326);
+          release(t0 + steps, w.n_steps);
+          if (!ok) break;
+        } else if (!active) {
+          release(0, w.n_steps);
+          if (!ok) break;
+        }
         if (!active) mma_commit(bar_qfree);   // after this thread's earlier MMAs, like every arrival on these two
         mma_commit(bar(bOFull + wg));   // this tile's O is complete (an idle tile: behind its earlier MMAs)
-        T += w.n_steps;
-        U += my_steps;
+        T += used;
+        U += steps + (early ? 1 : 0);
       }
     }
   } else {
@@ -237,7 +282,8 @@ tc_fwd256_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
     const uint32_t lane_off = (uint32_t)((warp & 3) * 32) << 16;
     const float scale2 = p.scale * kLog2e;
     const int ac = p.attend_current;
-    int U = 0, S = 0;   // this tile's steps and the K/V stages of the earlier items
+    int U = 0;   // this tile's steps of the earlier items
+    volatile EarlyStop &stop = sh->stop[wg];
     bool ok = true;
     Fwd256Item w_next;
     bool have = fwd256_item(p, 0, w);
@@ -248,56 +294,71 @@ tc_fwd256_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
       const int row = w.blk_row0 + wg * kBM + r;       // row index inside the sequence
       const int s_diag0 = 4 * w.c.idx + 2 * wg;        // first sub-tile that reaches this tile's diagonal band
       const bool warp_live = (row & ~31) < w.c.len;    // a warp whose 32 rows all lie past the sequence end computes nothing
-      double run = 0.0;
-      if (lane == 0) tma_store_wait_read();   // the previous item's O has left the P buffers
+      LogSum run;
+      bool through = false;    // this warp is through with the tile, having got to sub-tile s_reached
+      int s_reached = 0;
+      int slots = my_steps;                   // S slots used
+      if (lane == 0) tma_store_wait_read();   // the previous item's O has left the staging boxes
       __syncwarp();
       if ((threadIdx.x & 127) == 0) trace_event(p, 2 + wg, tr_cur, 40 + wg, it);
       for (int u = 0; u < my_steps && ok; ++u) {
         const int s = w.s_top - (t0 + u);
         const int gu = U + u, buf = gu & 1;
         ok = wait_or_abort(bar(bSFull + wg * 2 + buf), (gu >> 1) & 1, abort_flag, p, 330);
-        // a shared-memory P buffer is free once the P V MMA of two steps ago has read it; P in tensor memory needs no
-        // such wait: it overwrites scores of this very step, which the same thread has already loaded
-        if (!kPTmem && ok && gu >= 2) ok = wait_or_abort(bar(bPEmpty + wg * 2 + buf), ((gu >> 1) - 1) & 1, abort_flag, p, 331);
         if (!ok) break;
+        if (through && stop.word[buf] == kStepStop) {   // (a stop needs this warp's consent)
+          slots = u + 1;
+          __syncwarp();
+          if (lane == 0) mbar_arrive(bar(bPFull + wg * 2 + buf));
+          break;
+        }
         if (threadIdx.x == 128 && u == 0 && it == 0) trace_block(p, 1);
         if ((threadIdx.x & 127) == 0) trace_event(p, 2 + wg, tr_cur, 4 + 16 * wg, t0 + u);
         tc_fence_after();
         const uint32_t ts = tmem + wg * 128 + buf * 64 + lane_off;
-        uint8_t *tile_p = gP + (wg * 2 + buf) * kPBytes;
         // the sequence ends inside this sub-tile: the V rows behind its end are not this sequence's (see zero_tile_rows);
         // their P columns are exact zeros, so the rows are cleared before this step's P V MMA is released
         const int tail_rows = w.c.len - s * kBN;
         if (tail_rows < kBN) {
-          uint8_t *v_tile = gbase + (sKV - base) + ((S + t0 + u) % kStages) * kStageBytes + kKvTileBytes;
+          uint8_t *v_tile = gbase + (sKV - base) + stop.word[buf] * kStageBytes + kKvTileBytes;
           zero_tile_rows(v_tile, tail_rows, kBN, kBoxes, kKvBoxBytes, r, kBM);
           fence_proxy_async_smem();
         }
-        float R = ex2(-(float)run);
+        bool done = through || !warp_live;
         float logsum = 0.f;
         // 64 columns in chunks of 16, last chunk first; TMEM is read one chunk ahead of the arithmetic
         // (the P rows of such a warp keep whatever their buffer held: they only reach accumulator rows that are never stored)
-        if (!warp_live) {
-        } else if (s >= s_diag0) fwd256_row_pass<kFp16, true>(ts, s * kBN, row, ac, scale2, R, logsum, tile_p, r, ts + kPCol);
-        else fwd256_row_pass<kFp16, false>(ts, 0, 0, ac, scale2, R, logsum, tile_p, r, ts + kPCol, !p.dense);
-        run += (double)logsum;
-        if constexpr (kPTmem) tmem_wait_st();
-        tc_fence_before();          // this step's TMEM reads (and writes of P) are done before the slot is handed back
-        if constexpr (!kPTmem) fence_proxy_async_smem();
+        if (through) {
+          fwd256_zero_row(ts + kPCol);
+        } else if (!warp_live) {
+        } else if (s >= s_diag0) fwd256_row_pass<kFp16, true>(ts, s * kBN, row, ac, scale2, run, logsum, ts + kPCol, true);
+        else done = fwd256_row_pass<kFp16, false>(ts, 0, 0, ac, scale2, run, logsum, ts + kPCol, row < w.c.len, !p.dense, may_stop);
+        run.add(logsum);
+        tmem_wait_st();
+        tc_fence_before();          // this step's TMEM reads and writes of P are done before the slot is handed back
         __syncwarp();
-        if (lane == 0) mbar_arrive(bar(bPFull + wg * 2 + buf));
+        if (lane == 0) {
+          if (may_stop && done && !through) publish_through(stop, warp & 3, it, u);
+          mbar_arrive(bar(bPFull + wg * 2 + buf));
+        }
+        if (may_stop && done && !through) {
+          through = true;
+          s_reached = s + 1;
+        }
         if ((threadIdx.x & 127) == 0) trace_event(p, 2 + wg, tr_cur, 5 + 16 * wg, t0 + u);
       }
       // ---- epilogue: O (TMEM) -> global, rem, log_rem
       if ((threadIdx.x & 127) == 0) trace_event(p, 2 + wg, tr_cur, 42 + wg, it);
       // While the last P V MMA finishes: rem and log_rem leave, and the next item's table entries are fetched.
       const bool valid = row < w.c.len;
-      const float rem_f = ex2(-(float)run);
+      const float rem_f = run.stick();
       if (ok && my_steps > 0 && valid) {
         const long long idx = (w.c.boff * p.heads + w.h) * p.tokens + w.c.tok0 + row;
         reinterpret_cast<T *>(p.rem)[idx] = from_f32<T>(rem_f);
-        p.log_rem[idx] = -run;
+        p.log_rem[idx] = -run.value();
       }
+      if (p.tile_start != nullptr && ok && my_steps > 0 && warp_live && lane == 0 && row >= 64)
+        *tile_start_entry(p, w.c, w.h, row) = s_reached * kBN;
       const bool have_next = fwd256_item(p, it + 1, w_next);
       if (ok) ok = wait_or_abort(bar(bOFull + wg), it & 1, abort_flag, p, 332);
       if ((threadIdx.x & 127) == 0) trace_event(p, 2 + wg, tr_cur, 44 + wg, it);
@@ -309,16 +370,24 @@ tc_fwd256_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
                                                       (long long)w.h * p.v.sh + (w.c.tok0 + row) * p.v.st
                                                 : nullptr;
         if (tile_row0 + kBM <= w.c.len) {
-          // full tile: through this tile's two P buffers (all P V MMAs are done), one TMA store per warp and half
-          uint8_t *stage = gP + wg * 2 * kPBytes;
-          stage_acc_rows<D, kFp16>(tmem + 256 + wg * 128 + lane_off, stage, r, 1.f, vrow, rem_f, p.head_dim);
-          fence_proxy_async_smem();
-          __syncwarp();
-          if (lane == 0) {
-            const uint32_t src = sP + wg * 2 * kPBytes + (warp & 3) * 32 * 128;
-            const int trow = (int)w.c.tok0 + tile_row0 + (warp & 3) * 32;
-            for (int kb = 0; kb < kBoxes; ++kb) tma_store_4d(&tm_o, src + kb * kPBytes, kb * 64, trow, w.h, (int)w.c.boff);
-            tma_store_commit();
+          // full tile: 64 columns at a time through this tile's staging box, one TMA store per warp
+          uint8_t *stage = gP + wg * kPBytes;
+          const uint32_t src = sP + wg * kPBytes + (warp & 3) * 32 * 128;
+          const int trow = (int)w.c.tok0 + tile_row0 + (warp & 3) * 32;
+#pragma unroll 1
+          for (int kb = 0; kb < kBoxes; ++kb) {
+            if (kb > 0) {   // the warp's part of the box is rewritten
+              if (lane == 0) tma_store_wait_read();
+              __syncwarp();
+            }
+            stage_acc_rows<64, kFp16>(tmem + 256 + wg * 128 + kb * 64 + lane_off, stage, r, 1.f, vrow == nullptr ? nullptr : vrow + kb * 64,
+                                      rem_f, p.head_dim - kb * 64);
+            fence_proxy_async_smem();
+            __syncwarp();
+            if (lane == 0) {
+              tma_store_4d(&tm_o, src, kb * 64, trow, w.h, (int)w.c.boff);
+              tma_store_commit();
+            }
           }
         } else {
           // the sequence ends inside the tile: row by row, rows past the end are left alone
@@ -330,8 +399,7 @@ tc_fwd256_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
       __syncwarp();
       if (lane == 0) mbar_arrive(bar(bOFree + wg));
       if ((threadIdx.x & 127) == 0) trace_event(p, 2 + wg, tr_cur, 46 + wg, it);
-      U += my_steps;
-      S += w.n_steps;
+      U += slots;
       w = w_next;
       have = have_next;
     }

@@ -13,17 +13,25 @@ constexpr int kPBytes = kBM * kBN * 2;        // a 128 x 64 16-bit tile (the sta
 // packed row into columns 32..63 of the very S slot they have just read (key k of the step in column 32 + k / 2;
 // the chunks are read last column first, so every column written has been read before), and the MMA takes its A
 // operand from there.  The next S MMA into that slot is issued by the same thread after this P V MMA, and MMAs of
-// one thread execute in order.  With SB_FWD_P_SMEM the earlier hand-over through a swizzled shared-memory tile is built.
-#ifdef SB_FWD_P_SMEM
-constexpr bool kPTmem = false;
-#else
-constexpr bool kPTmem = true;
-#endif
+// one thread execute in order.
 constexpr uint32_t kPCol = 32;
 }  // namespace fwd256
 
 using fwd256::kPCol;
-using fwd256::kPTmem;
+
+// A row's sum of log2(1 + e) over the keys of the earlier sub-tiles, as an unevaluated pair of floats: exact for as long as
+// the sum's terms span less than 48 bits, and a few FMA-pipe operations on the way to the next sub-tile's start value where
+// fp64 takes a conversion, an addition and a conversion back.
+struct LogSum {
+  float hi = 0.f, lo = 0.f;
+  __device__ __forceinline__ void add(float x) {   // Knuth's two-sum
+    const float s = hi + x, b = s - hi;
+    lo += (hi - (s - b)) + (x - b);
+    hi = s;
+  }
+  __device__ __forceinline__ float stick() const { return ex2(-(hi + lo)); }   // product of (1 - beta) over those keys
+  __device__ __forceinline__ double value() const { return (double)hi + (double)lo; }
+};
 
 // One row, 16 consecutive key columns of a 64-key sub-tile, last column first.  key0: index inside the sequence of
 // the chunk's first column; row: index of this query row.
@@ -32,11 +40,14 @@ using fwd256::kPTmem;
 // R carries that product over everything after the current column.  Four columns share one reciprocal and one
 // logarithm of t0 t1 t2 t3; the four inclusive products follow from R, that reciprocal and partial products with
 // five multiplications, and beta itself is never formed.
+// The log-space sums are added up in the order the backward uses -- the groups of a chunk from the last to the first, the
+// chunks of a sub-tile from the first to the last, which is the way it walks: the two agree bit for bit, so that
+// the backward may start at any sub-tile from the fp64 sum of the sub-tiles after it (see `tile_start`).
 template <bool kFp16, bool kMasked>
 __device__ __forceinline__ void fwd256_row_chunk(const uint32_t (&v)[16], int c0, int key0, int row, int ac,
-                                                 float scale2, float &R, float &logsum, uint8_t *tile_p, int r,
-                                                 uint32_t tmem_p) {
+                                                 float scale2, float &R, float &logsum, uint32_t tmem_p) {
   float pr[16];
+  logsum = 0.f;
   const float2 sc = make_float2(scale2, scale2), one = make_float2(1.f, 1.f);
 #pragma unroll
   for (int g = 3; g >= 0; --g) {   // four columns at a time, last group first; independent work in packed pairs
@@ -67,33 +78,28 @@ __device__ __forceinline__ void fwd256_row_chunk(const uint32_t (&v)[16], int c0
     pr[4 * g + 2] = q23.x;
     pr[4 * g + 3] = q23.y;
   }
-  if constexpr (kPTmem) {   // 16 keys = 8 packed columns of this row's lane
-    uint32_t w[8];
-    pack_row_chunk16<kFp16>(pr, w);
-    tmem_st8(tmem_p + (c0 >> 1), w);
-  } else {
-    store_row_chunk16<kFp16>(tile_p, r, c0, pr);
-  }
+  uint32_t w[8];   // 16 keys = 8 packed columns of this row's lane
+  pack_row_chunk16<kFp16>(pr, w);
+  tmem_st8(tmem_p + (c0 >> 1), w);
 }
 
 // P of 32 key columns (from column c0 of the sub-tile on) set to zero without looking at the scores.
-template <bool kFp16>
-__device__ __forceinline__ void fwd256_zero_pair(int c0, uint8_t *tile_p, int r, uint32_t tmem_p) {
-  if constexpr (kPTmem) {
-    const uint32_t z[8] = {0u, 0u, 0u, 0u, 0u, 0u, 0u, 0u};
-    tmem_st8(tmem_p + (c0 >> 1), z);
-    tmem_st8(tmem_p + (c0 >> 1) + 8, z);
-  } else {
-    const float z[16] = {};
-    store_row_chunk16<kFp16>(tile_p, r, c0, z);
-    store_row_chunk16<kFp16>(tile_p, r, c0 + 16, z);
-  }
+__device__ __forceinline__ void fwd256_zero_pair(int c0, uint32_t tmem_p) {
+  const uint32_t z[8] = {0u, 0u, 0u, 0u, 0u, 0u, 0u, 0u};
+  tmem_st8(tmem_p + (c0 >> 1), z);
+  tmem_st8(tmem_p + (c0 >> 1) + 8, z);
+}
+
+__device__ __forceinline__ void fwd256_zero_row(uint32_t tmem_p) {
+  fwd256_zero_pair(0, tmem_p);
+  fwd256_zero_pair(32, tmem_p);
 }
 
 // One row of a 64-key sub-tile whose P is known to be exactly zero: only the log-space sum is formed, with the same
 // operations in the same order as fwd256_row_chunk, so that it is the same number bit for bit.
 __device__ __forceinline__ void fwd256_logsum_chunk(const uint32_t (&v)[16], float scale2, float &logsum) {
   const float2 sc = make_float2(scale2, scale2), one = make_float2(1.f, 1.f);
+  logsum = 0.f;
 #pragma unroll
   for (int g = 3; g >= 0; --g) {
     const float2 x01 = mul2(make_float2(__uint_as_float(v[4 * g]), __uint_as_float(v[4 * g + 1])), sc);
@@ -105,60 +111,108 @@ __device__ __forceinline__ void fwd256_logsum_chunk(const uint32_t (&v)[16], flo
     logsum += lg2(p01 * p23);
   }
 }
-template <bool kFp16>
-__device__ __forceinline__ void fwd256_logsum_pass(uint32_t ts, float scale2, float &logsum, uint8_t *tile_p, int r,
-                                                   uint32_t tmem_p) {
-  uint32_t va[16], vb[16];
-  tmem_ld16(ts + 48, va);
+// (The chunk of columns 48..63 has been requested into va.)
+__device__ __forceinline__ void fwd256_logsum_pass(uint32_t ts, float scale2, float &logsum, uint32_t tmem_p, uint32_t (&va)[16]) {
+  uint32_t vb[16];
+  float l3 = 0.f, l2 = 0.f;   // the chunks of the upper pair
 #pragma unroll 1
   for (int pair = 1; pair >= 0; --pair) {
+    float la, lb;
     tmem_wait_ld_regs(va);
     tmem_ld16(ts + pair * 32, vb);
-    fwd256_logsum_chunk(va, scale2, logsum);
+    fwd256_logsum_chunk(va, scale2, la);
     tmem_wait_ld_regs(vb);
     if (pair == 1) tmem_ld16(ts + 16, va);
-    fwd256_logsum_chunk(vb, scale2, logsum);
+    fwd256_logsum_chunk(vb, scale2, lb);
+    logsum = ((lb + la) + l2) + l3;
+    l3 = la;
+    l2 = lb;
   }
   // P is written last: its columns alias scores that have all been read by now
-  fwd256_zero_pair<kFp16>(32, tile_p, r, tmem_p);
-  fwd256_zero_pair<kFp16>(0, tile_p, r, tmem_p);
+  fwd256_zero_row(tmem_p);
 }
 
 // One row of a 64-key sub-tile.  In a masked sub-tile the columns from (last row of this warp) + ac on are masked for
 // every row of the warp (its 32 rows are consecutive and 32-aligned): such 32-column halves are not computed at all,
 // their P is zero and R and logsum stay as they are -- 6 of the 16 (warp, half) pairs of a diagonal 128 x 128 tile.
-// skip_zero: an unmasked sub-tile whose P is exactly zero for the whole warp (R has underflowed) only sums its logs.
+// An unmasked sub-tile whose P is exactly zero for all rows of the warp that exist (their product has underflowed) only
+// sums its logs (skip_zero), or not even that (drop_zero: log_rem is to cover the keys up to here only); the pass then
+// returns true.
 template <bool kFp16, bool kMasked>
-__device__ __forceinline__ void fwd256_row_pass(uint32_t ts, int key0, int row, int ac, float scale2, float &R,
-                                                float &logsum, uint8_t *tile_p, int r, uint32_t tmem_p,
-                                                bool skip_zero = false) {
-  if (!kMasked && skip_zero && __all_sync(0xffffffffu, R == 0.f)) {
-    // The product over the keys after this sub-tile has underflowed to exactly 0 for all 32 rows of the warp: every
-    // p of the sub-tile is e * 0 = 0 (e is finite: its exponent is clamped) and R stays 0.
-    fwd256_logsum_pass<kFp16>(ts, scale2, logsum, tile_p, r, tmem_p);
-    return;
-  }
+__device__ __forceinline__ bool fwd256_row_pass(uint32_t ts, int key0, int row, int ac, float scale2, const LogSum &sum,
+                                                float &logsum, uint32_t tmem_p, bool exists, bool skip_zero = false, bool drop_zero = false) {
+  float R;
+  uint32_t va[16], vb[16];
   int hi = 1;   // last 32-column half with an allowed key
   if (kMasked) {
     const int span = (row | 31) + ac - key0;   // the warp's rows may attend to columns [0, span) of this sub-tile
     hi = span > 32 ? 1 : (span > 0 ? 0 : -1);
-    if (hi < 1) fwd256_zero_pair<kFp16>(32, tile_p, r, tmem_p);
+    if (hi < 1) fwd256_zero_pair(32, tmem_p);
     if (hi < 0) {
-      fwd256_zero_pair<kFp16>(0, tile_p, r, tmem_p);
-      return;
+      fwd256_zero_pair(0, tmem_p);
+      return false;
+    }
+    tmem_ld16(ts + hi * 32 + 16, va);
+    R = sum.stick();
+  } else {
+    tmem_ld16(ts + 48, va);
+    R = sum.stick();   // (under the load's latency; the registers it fills must not cross a branch)
+    const bool zero = skip_zero && __all_sync(0xffffffffu, !exists || R == 0.f);
+    tmem_wait_ld_regs(va);
+    if (zero) {
+      // The product over the keys after this sub-tile has underflowed to exactly 0 for all rows of the warp: every p of
+      // the sub-tile is e * 0 = 0 (e is finite: its exponent is clamped).
+      if (drop_zero) fwd256_zero_row(tmem_p);
+      else fwd256_logsum_pass(ts, scale2, logsum, tmem_p, va);
+      return true;
     }
   }
-  uint32_t va[16], vb[16];
-  tmem_ld16(ts + hi * 32 + 16, va);
+  float l3 = 0.f, l2 = 0.f;   // log sums of the upper pair of chunks
 #pragma unroll 1
   for (int pair = hi; pair >= 0; --pair) {
+    float la, lb;
     tmem_wait_ld_regs(va);
     tmem_ld16(ts + pair * 32, vb);
-    fwd256_row_chunk<kFp16, kMasked>(va, pair * 32 + 16, key0 + pair * 32 + 16, row, ac, scale2, R, logsum, tile_p, r, tmem_p);
+    fwd256_row_chunk<kFp16, kMasked>(va, pair * 32 + 16, key0 + pair * 32 + 16, row, ac, scale2, R, la, tmem_p);
     tmem_wait_ld_regs(vb);
     if (pair == 1) tmem_ld16(ts + 16, va);
-    fwd256_row_chunk<kFp16, kMasked>(vb, pair * 32, key0 + pair * 32, row, ac, scale2, R, logsum, tile_p, r, tmem_p);
+    fwd256_row_chunk<kFp16, kMasked>(vb, pair * 32, key0 + pair * 32, row, ac, scale2, R, lb, tmem_p);
+    logsum = ((lb + la) + l2) + l3;
+    l3 = la;
+    l2 = lb;
   }
+  return false;
+}
+
+// ---- stopping early ------------------------------------------------------------------------------------------------
+// A row warp is through once the product R has underflowed to exactly 0 for all its rows: no earlier key can add anything
+// to O or rem.  From then on it only writes zeros for P, its log sum stays what it is, and the key it got to is recorded
+// for the backward.  Each of a query tile's four warps publishes its first step of zeros; the tile's MMA issuer stops
+// before step v if all four have done so by step v - 3 and tells the rows with the word that accompanies every step's
+// scores.  It looks when it has issued step v - 1's scores and would wait for step v - 2's P: it has waited for the P of
+// step v - 3, so the decision does not depend on timing, and nobody waits for it.  Three steps of zeros are cheap, and rows
+// that never finish pay nothing: the vote is the one the row pass takes anyway to skip its arithmetic.  (A vote on R at the
+// end of the pass and a decision right before step v's scores stop two steps earlier and cost every step of every row: +5 %
+// time on 4096-token sequences that never stop.)
+constexpr int kStepStop = -1;
+// No stop with fewer than three sub-tiles to go: what is left costs about as much as stopping and restarting the stream.
+__device__ __forceinline__ bool may_stop_before(int sub_tile) { return sub_tile >= 2; }
+struct EarlyStop {                            // shared memory, one per query tile
+  unsigned long long through[4];              // per row warp: (item + 1) << 32 | its first step of zeros
+  int word[2];                                // per S slot: K/V stage of the step, or kStepStop (read where it can matter)
+  int stopped;                                // item + 1: the tile wants no more keys of this item
+};
+__device__ __forceinline__ void publish_through(volatile EarlyStop &e, int warp, int item, int step) {
+  e.through[warp] = (unsigned long long)(unsigned)(item + 1) << 32 | (unsigned)step;
+}
+__device__ __forceinline__ bool all_through(const volatile EarlyStop &e, int item, int step) {
+  bool all = true;
+#pragma unroll
+  for (int w = 0; w < 4; ++w) {
+    const unsigned long long x = e.through[w];
+    all = all && (unsigned)(x >> 32) == (unsigned)(item + 1) && (int)(unsigned)x <= step;
+  }
+  return all;
 }
 
 }  // namespace sb

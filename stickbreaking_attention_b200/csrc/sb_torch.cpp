@@ -154,10 +154,29 @@ void launch(SbParams &p, bool backward, char *workspace, size_t bytes, const Ten
   g_launches.fetch_add(sb_last_launch_count(), std::memory_order_relaxed);
 }
 
-struct Forward { Tensor out, rem, log_rem; };
+// `state`: what the backward needs, one fp64 buffer -- log_rem (batch, heads, tokens) and, where the call keeps them, the
+// int32 tile starts (batch * heads, ceil(tokens / 32)) behind it.
+struct Forward { Tensor out, rem, state; };
+
+void attach_state(SbParams &p, double *state, bool tile_starts) {
+  const int64_t rows = (int64_t)p.batch * p.heads;
+  p.log_rem = state;
+  if (tile_starts) {
+    p.tile_start = reinterpret_cast<int32_t *>(state + rows * p.tokens);
+    p.tile_start_stride = (p.tokens + 31) / 32;
+  }
+}
+int64_t state_doubles(const SbParams &p) {
+  const int64_t rows = (int64_t)p.batch * p.heads;
+  return rows * p.tokens + (rows * ((p.tokens + 31) / 32) + 1) / 2;
+}
+
+// kLogRem: log_rem over all keys, as a tensor of the rows' shape; kState: the operator's own saved state; kNothing: no
+// backward will come, and the state is scratch like the rest and shares its allocation.
+enum class Keep { kNothing, kState, kLogRem };
 
 Forward run_forward(const Tensor &q_in, const Tensor &k_in, const Tensor &v_in, const std::optional<Tensor> &cu, const Call &c,
-                    bool keep_state) {
+                    Keep keep) {
   check_inputs(q_in, k_in, v_in, cu, c);
   c10::cuda::CUDAGuard guard(q_in.device());
   const Tensor q = tma_ready(q_in), k = tma_ready(k_in), v = tma_ready(v_in);
@@ -170,24 +189,21 @@ Forward run_forward(const Tensor &q_in, const Tensor &k_in, const Tensor &v_in, 
   p.o = arg(f.out, c.fixed);
   p.rem = f.rem.data_ptr();
   const size_t ws = (workspace_bytes(p, false) + 255) / 256 * 256;
-  // without a backward to come, log_rem is scratch like the rest and shares its allocation
   size_t bytes = ws;
-  if (keep_state) {
-    f.log_rem = empty_cuda(row_sizes, at::kDouble, q);
-    p.log_rem = static_cast<double *>(f.log_rem.data_ptr());
-  } else {
-    bytes += sizeof(double) * (size_t)(q.numel() / q.size(-1));
-  }
+  if (keep == Keep::kLogRem) f.state = empty_cuda(row_sizes, at::kDouble, q);
+  else if (keep == Keep::kState) f.state = empty_cuda({state_doubles(p)}, at::kDouble, q);
+  else bytes += sizeof(double) * (size_t)state_doubles(p);
   // freed on return: the caching allocator hands the block out again only behind this stream's work
   const Tensor scratch = empty_cuda({(int64_t)bytes}, at::kByte, q);
   char *base = static_cast<char *>(scratch.data_ptr());
-  if (!keep_state) p.log_rem = reinterpret_cast<double *>(base + ws);
+  attach_state(p, f.state.defined() ? static_cast<double *>(f.state.data_ptr()) : reinterpret_cast<double *>(base + ws),
+               keep != Keep::kLogRem);
   launch(p, false, base, ws, q);
   return f;
 }
 
 std::array<Tensor, 3> run_backward(const Tensor &dout_in, const Tensor &drem_in, const Tensor &q_in, const Tensor &k_in, const Tensor &v_in,
-                                   const std::optional<Tensor> &cu, const Tensor &log_rem, const Call &c) {
+                                   const std::optional<Tensor> &cu, const Tensor &state, bool tile_starts, const Call &c) {
   check_inputs(q_in, k_in, v_in, cu, c);
   c10::cuda::CUDAGuard guard(q_in.device());
   const Tensor q = tma_ready(q_in), k = tma_ready(k_in), v = tma_ready(v_in);
@@ -199,7 +215,7 @@ std::array<Tensor, 3> run_backward(const Tensor &dout_in, const Tensor &drem_in,
   const Tensor dq = empty_as(q), dk = empty_as(k), dv = empty_as(v);
   SbParams p;
   fill(p, q, k, v, cu, c);
-  p.log_rem = static_cast<double *>(log_rem.data_ptr());
+  attach_state(p, static_cast<double *>(state.data_ptr()), tile_starts);
   p.d_o = arg(dout, c.fixed);
   p.d_rem = drem.defined() ? drem.data_ptr() : nullptr;
   p.dq = arg(dq, c.fixed);
@@ -223,13 +239,13 @@ std::array<Tensor, 3> run_backward(const Tensor &dout_in, const Tensor &drem_in,
 
 // The operator's node in the autograd graph (reference: StickBreakingAttention.backward, sb_varlen/__init__.py:48-68).
 struct StickBreakingAttentionBackward : public torch::autograd::Node {
-  torch::autograd::SavedVariable q, k, v, log_rem, cu;
+  torch::autograd::SavedVariable q, k, v, state, cu;
   Call call{};
   bool released = false;
 
   std::string name() const override { return "StickBreakingAttentionBackward"; }
   void release_variables() override {
-    q.reset_data(); k.reset_data(); v.reset_data(); log_rem.reset_data(); cu.reset_data();
+    q.reset_data(); k.reset_data(); v.reset_data(); state.reset_data(); cu.reset_data();
     released = true;
   }
   variable_list apply(variable_list &&grads) override {
@@ -239,7 +255,8 @@ struct StickBreakingAttentionBackward : public torch::autograd::Node {
     at::AutoDispatchBelowADInplaceOrView below;   // plain tensors from here on: conversions and copies record nothing
     std::array<Tensor, 3> g;
     try {
-      g = run_backward(grads[0], grads.size() > 1 ? grads[1] : Tensor(), q.unpack(), k.unpack(), v.unpack(), ends, log_rem.unpack(), call);
+      g = run_backward(grads[0], grads.size() > 1 ? grads[1] : Tensor(), q.unpack(), k.unpack(), v.unpack(), ends, state.unpack(), true,
+                       call);
     } catch (const LibraryError &e) {   // on an autograd thread: the exception keeps its Python type on its way to the caller
       py::gil_scoped_acquire gil;
       set_python_error(e);
@@ -276,7 +293,7 @@ variable_list attention(const Tensor &q, const Tensor &k, const Tensor &v, const
   Forward f;
   {
     at::AutoDispatchBelowADInplaceOrView below;
-    f = run_forward(q, k, v, cu, c, grad);
+    f = run_forward(q, k, v, cu, c, grad ? Keep::kState : Keep::kNothing);
   }
   if (grad) {
     auto node = std::shared_ptr<StickBreakingAttentionBackward>(new StickBreakingAttentionBackward(), torch::autograd::deleteNode);
@@ -285,7 +302,7 @@ variable_list attention(const Tensor &q, const Tensor &k, const Tensor &v, const
     node->q = torch::autograd::SavedVariable(q, false);
     node->k = torch::autograd::SavedVariable(k, false);
     node->v = torch::autograd::SavedVariable(v, false);
-    node->log_rem = torch::autograd::SavedVariable(f.log_rem, false);
+    node->state = torch::autograd::SavedVariable(f.state, false);
     if (cu.has_value()) node->cu = torch::autograd::SavedVariable(*cu, false);
     torch::autograd::set_history(f.out, node);
     if (!fused) torch::autograd::set_history(f.rem, node);
@@ -299,15 +316,16 @@ std::tuple<Tensor, Tensor, Tensor> forward(const Tensor &q, const Tensor &k, con
                                            std::optional<int64_t> max_seqlens, double scale, bool attend_current, bool leading_zero,
                                            bool fused, int64_t flags) {
   at::AutoDispatchBelowADInplaceOrView below;
-  Forward f = run_forward(q, k, v, cu, make_call(!cu.has_value(), max_seqlens, scale, attend_current, leading_zero, fused, flags), true);
-  return {f.out, f.rem, f.log_rem};
+  Forward f = run_forward(q, k, v, cu, make_call(!cu.has_value(), max_seqlens, scale, attend_current, leading_zero, fused, flags),
+                          Keep::kLogRem);
+  return {f.out, f.rem, f.state};
 }
 std::tuple<Tensor, Tensor, Tensor> backward(const Tensor &dout, const std::optional<Tensor> &drem, const Tensor &q, const Tensor &k,
                                             const Tensor &v, const std::optional<Tensor> &cu, std::optional<int64_t> max_seqlens,
                                             const Tensor &log_rem, double scale, bool attend_current, bool leading_zero, bool fused,
                                             int64_t flags) {
   at::AutoDispatchBelowADInplaceOrView below;
-  std::array<Tensor, 3> g = run_backward(dout, drem.value_or(Tensor()), q, k, v, cu, log_rem,
+  std::array<Tensor, 3> g = run_backward(dout, drem.value_or(Tensor()), q, k, v, cu, log_rem, false,
                                          make_call(!cu.has_value(), max_seqlens, scale, attend_current, leading_zero, fused, flags));
   return {g[0], g[1], g[2]};
 }
