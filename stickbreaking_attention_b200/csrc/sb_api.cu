@@ -27,7 +27,7 @@ constexpr int kShortParams = (int)offsetof(SbParams, tile_start);
 static inline size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
 
 // Workspace layout, a pure function of the shapes:
-//   [hdr 256 B][tile_prefix int32 x (num_seq+1)][pair_prefix int64 x (num_seq+1)]
+//   [hdr 256 B][pair_prefix int64 x (num_seq+1)]
 //   packed batches: [order int2 x tiles][order2 (backward) int2 x tiles]
 //   backward, either: [A | dz tiles, 16-bit x chunk_heads x pairs_cap x 2 x 128 x 128]   (stored-tiles mode)
 //             or:     [R1 fp32 x chunk_heads x pairs_cap x halves x tile][S2 same]       (recompute mode)
@@ -39,7 +39,7 @@ struct Plan {
   int n_max;
   int max_seqlen;
   long long pairs_cap;
-  size_t off_tile_prefix, off_pair_prefix, off_order, off_order2, off_bnd, off_drem;
+  size_t off_pair_prefix, off_order, off_order2, off_bnd, off_drem;
   int bnd_halves;             // boundary records per (query tile, key tile) pair
   size_t bnd_bytes_per_head;  // one of the two arrays
   int chunk_heads;
@@ -105,8 +105,7 @@ static int make_plan(const SbParams *p, Plan &pl, bool backward) {
     pl.pairs_cap = ((long long)pl.tiles_cap * (pl.n_max + 1) + 1) / 2;
   }
   if (pl.tiles_cap < 1) pl.tiles_cap = 1;
-  pl.off_tile_prefix = 256;
-  pl.off_pair_prefix = align_up(pl.off_tile_prefix + sizeof(int) * (size_t)(p->num_seq + 1), 256);
+  pl.off_pair_prefix = 256;
   pl.off_order = align_up(pl.off_pair_prefix + sizeof(long long) * (size_t)(p->num_seq + 1), 256);
   const size_t order_bytes = p->cu_seqlens != nullptr ? align_up(sizeof(int2) * (size_t)pl.tiles_cap, 256) : 0;
   pl.off_order2 = pl.off_order + order_bytes;                       // every second tile: the backward's dq kernel
@@ -212,7 +211,6 @@ static int fill_kparams(const SbParams *p, const Plan &pl, bool backward, KParam
   k.tile = pl.tile; k.tiles_cap = pl.tiles_cap; k.n_max = pl.n_max; k.max_seqlen = pl.max_seqlen;
   char *ws = reinterpret_cast<char *>(p->workspace);
   k.hdr = reinterpret_cast<int *>(ws);
-  k.tile_prefix = reinterpret_cast<int *>(ws + pl.off_tile_prefix);
   k.pair_prefix = reinterpret_cast<long long *>(ws + pl.off_pair_prefix);
   if (p->cu_seqlens != nullptr) {
     k.order = reinterpret_cast<const int2 *>(ws + pl.off_order);
@@ -225,6 +223,13 @@ static int fill_kparams(const SbParams *p, const Plan &pl, bool backward, KParam
     k.bnd_s2 = reinterpret_cast<float *>(ws + pl.off_bnd + pl.bnd_bytes_per_head * pl.chunk_heads);
   }
   k.pairs_cap = pl.pairs_cap;
+  // Small packed batches: the kernels build their item tables themselves.  A block pays about a microsecond for it, so the
+  // backward's one-item blocks do so only while two rounds of them fill the GPU; the recomputing dK/dV kernel of the
+  // tensor-core path has no shared memory left for the table.
+  if (p->cu_seqlens != nullptr && p->num_seq <= kSmallSeqs && pl.tiles_cap <= kSmallItems) {
+    const bool tc = pl.path == SB_PATH_TCGEN05;
+    k.small_table = (!backward && tc) || ((long long)pl.tiles_cap * p->heads <= 2 * 148 * (tc ? 2 : 4) && (pl.store_az || !tc));
+  }
   k.fuse_rem_v = (p->flags & SB_FLAG_FUSE_REM_V) ? 1 : 0;
   if (!backward && p->attn_weights != nullptr) {
     if (p->attn_cols < 1) return fail(SB_ERR_ARGUMENT, "attn_cols must be >= 1 with attn_weights");
@@ -253,8 +258,7 @@ static int run(const SbParams *p, void *stream, bool backward) {
   if ((rc = fill_kparams(p, pl, backward, k))) return rc;
   if (p->tokens == 0) return SB_OK;
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
-  cudaError_t e = launch_prep(k, s);
-  g_launches += (p->cu_seqlens != nullptr && k.trace != nullptr) ? 2 : 1;   // prep kernel or header clear (both with the event log)
+  cudaError_t e = launch_prep(k, s, &g_launches);
   if (e != cudaSuccess) return fail(SB_ERR_CUDA, "prep launch: %s", cudaGetErrorString(e));
   if (backward && k.fuse_rem_v) {
     e = launch_fused_drem(k, p->dtype, s);
@@ -271,14 +275,9 @@ static int run(const SbParams *p, void *stream, bool backward) {
     else
       e = backward ? launch_simt_bwd(k, p->dtype, s, &g_launches) : launch_simt_fwd(k, p->dtype, s, &g_launches);
     if (e != cudaSuccess) return fail(SB_ERR_CUDA, "%s launch: %s", backward ? "backward" : "forward", cudaGetErrorString(e));
-    if (p->cu_seqlens != nullptr) {
-      e = launch_zero_tail(k, p->dtype, backward, s);
-      g_launches += 1;
-      if (e != cudaSuccess) return fail(SB_ERR_CUDA, "tail launch: %s", cudaGetErrorString(e));
-    }
   }
-  // the stored-tiles dK/dV kernel adds rem * d_out in its own epilogue; the other kernels leave it to one more pass
-  if (backward && k.fuse_rem_v && !k.skip_dkv && !(pl.path == SB_PATH_TCGEN05 && pl.store_az)) {
+  // the recomputing dK/dV kernel leaves rem * d_out to one more pass; the others add it in their own epilogue
+  if (backward && k.fuse_rem_v && !k.skip_dkv && pl.path == SB_PATH_TCGEN05 && !pl.store_az) {
     e = launch_fused_dv(k, p->dtype, s);
     g_launches += 1;
     if (e != cudaSuccess) return fail(SB_ERR_CUDA, "dv launch: %s", cudaGetErrorString(e));

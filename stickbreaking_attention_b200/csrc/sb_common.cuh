@@ -39,6 +39,7 @@ struct KParams {
   int check_leading_zero;  // the element before cu[0] must be 0
   int skip_dq, skip_dkv;   // timing aids: leave one of the two backward kernels out
   int dense;               // measuring aid: do the per-score arithmetic even where it is known to give exact zeros
+  int small_table;         // packed batches: every block builds the item table itself (see SmallTable)
   const int2 *order;       // packed batches: work items by descending weight, see decode_item
   const int2 *order2;      // the same for every second tile (backward only)
   int order_span;          // entries of one sequence that stay neighbours in order / order2 (>= 1)
@@ -46,9 +47,8 @@ struct KParams {
   int dbg;                 // experiments only (SbParams.reserved): 0 = normal arithmetic
   unsigned long long *trace;  // experiments only: event log of block (0,0) in the workspace tail, or nullptr
   // workspace views
-  int *hdr;            // [0] abort flag, [1] end of the last sequence (varlen), [2] / [3] entries of order / order2
-  int *tile_prefix;    // [num_seq + 1]  exclusive prefix of tiles per sequence (varlen)
-  long long *pair_prefix;  // [num_seq + 1] exclusive prefix of n(n+1)/2 (varlen)
+  int *hdr;            // [0] cu_seqlens refused, [1] end of the last sequence, [2] / [3] entries of order / order2
+  long long *pair_prefix;  // [num_seq] exclusive prefix of n(n+1)/2 (varlen)
   float *bnd_r1;       // [head_cnt][pairs_cap][tile]  suffix sums of log(1-beta) at tile starts
   float *bnd_s2;       // [head_cnt][pairs_cap][tile]  prefix sums of G before each key tile
   unsigned short *az;  // stored-tiles mode: [head_cnt][pairs_cap][A, dz][128 query rows][128 keys], 16-bit; else null
@@ -79,6 +79,16 @@ __device__ __forceinline__ long long load_cu(const KParams &p, int i) {
   return p.cu64 ? reinterpret_cast<const long long *>(p.cu)[i]
                 : (long long)reinterpret_cast<const int *>(p.cu)[i];
 }
+
+template <typename T> __device__ __forceinline__ float to_f32(T x);
+template <> __device__ __forceinline__ float to_f32<float>(float x) { return x; }
+template <> __device__ __forceinline__ float to_f32<__nv_bfloat16>(__nv_bfloat16 x) { return __bfloat162float(x); }
+template <> __device__ __forceinline__ float to_f32<__half>(__half x) { return __half2float(x); }
+
+template <typename T> __device__ __forceinline__ T from_f32(float x);
+template <> __device__ __forceinline__ float from_f32<float>(float x) { return x; }
+template <> __device__ __forceinline__ __nv_bfloat16 from_f32<__nv_bfloat16>(float x) { return __float2bfloat16_rn(x); }
+template <> __device__ __forceinline__ __half from_f32<__half>(float x) { return __float2half_rn(x); }
 
 // Where the group of 32 query rows from row0 on (a multiple of 32, inside the sequence) stopped: keys before this one have
 // weight exactly 0 for all of them, and log_rem of these rows covers the keys from it on.  One entry per 32 tokens: a
@@ -130,13 +140,71 @@ struct QueryList {
   }
 };
 
-// Maps a work-item number to its sequence and tile.  Items are ordered by weight across ALL sequences: the tile with
-// the most key (or query) tiles to visit comes first, so that the blocks that run longest start earliest and the
-// last blocks of a launch are the short ones.  For a packed batch the order is a table the prep kernel writes
-// (entries (sequence, k), k = tile index counted so that larger means heavier; `group` > 1 lists every group-th
-// tile only); for a fixed-length batch it is arithmetic.  `reverse`: the heavy tiles are the late ones (a query
-// tile sees all earlier keys); otherwise the early ones (a key tile is seen by all later queries).
-__device__ __forceinline__ bool decode_item(const KParams &p, int item, int group, bool reverse, TileCoord &c) {
+// ---- which work items there are ---------------------------------------------------------------------------------------
+// Work items (query or key tiles) are ordered by weight across ALL sequences: the tile with the most key (or query) tiles
+// to visit comes first, so that the blocks that run longest start earliest and the last blocks of a launch are the short
+// ones.  An entry is (sequence, k), k = tile index counted so that larger means heavier; `group` > 1 lists every group-th
+// tile only.  For a fixed-length batch the order is arithmetic.  For a packed batch it is a table, either written by a
+// kernel that runs first (p.order, p.order2, p.pair_prefix, p.hdr), or, for small calls (p.small_table), built by every
+// block for itself in shared memory: a launch and its hand-over cost more than the microsecond this takes.
+constexpr int kSmallSeqs = 128, kSmallItems = 256;
+struct SmallTable {                       // 1.5 KB: what the kernels' shared memory has left
+  uint32_t pair0[kSmallSeqs];             // first (query tile, key tile) pair of each sequence; while building: its entries
+  uint32_t order[kSmallItems];            // sequence << 16 | entry
+};
+
+__device__ __forceinline__ bool seq_valid(const KParams &p, long long start, long long end) {
+  return start >= 0 && end >= start && end <= p.tokens && end - start <= p.max_seqlen;
+}
+
+// By all threads of the block (at least kSmallSeqs of them); contains barriers.  Returns whether cu_seqlens was refused.
+__device__ __forceinline__ bool build_small_table(const KParams &p, int group, SmallTable &tb) {
+  const int t = threadIdx.x, span = p.order_span;
+  bool bad = false;
+  uint32_t n = 0;
+  if (t < p.num_seq) {
+    const long long start = t == 0 ? 0 : load_cu(p, t - 1), end = load_cu(p, t);
+    bad = !seq_valid(p, start, end);
+    n = bad ? 0 : (uint32_t)((end - start + p.tile - 1) / p.tile);
+    tb.pair0[t] = n;
+    if (bad && p.status != nullptr && blockIdx.x == 0) { p.status[0] = SB_DEV_BAD_CU_SEQLENS; p.status[1] = t; }
+  }
+  if (t == 0 && p.check_leading_zero && load_cu(p, -1) != 0) {
+    bad = true;
+    if (p.status != nullptr && blockIdx.x == 0) { p.status[0] = SB_DEV_BAD_CU_SEQLENS; p.status[1] = -1; }
+  }
+  if (__syncthreads_or(bad)) return true;
+  // Position of entry e of sequence s: the entries of heavier classes (a class is `span` consecutive entries), then those
+  // of the same class in the sequences before, then the heavier ones of its own.
+  for (int i = t; i < kSmallItems; i += blockDim.x) tb.order[i] = 0xffffffffu;
+  __syncthreads();
+  for (int s = 0, first = 0; s < p.num_seq; ++s) {
+    const int m = ((int)tb.pair0[s] + group - 1) / group;
+    for (int e = t - first % (int)blockDim.x; e < m; e += blockDim.x) {   // spread over the threads across sequences
+      if (e < 0) continue;
+      const int lo = e / span * span, hi = lo + span;
+      int pos = min(hi, m) - 1 - e;
+      for (int q = 0; q < p.num_seq; ++q) {
+        const int mq = ((int)tb.pair0[q] + group - 1) / group;
+        pos += max(mq - hi, 0);
+        if (q < s) pos += min(max(mq - lo, 0), span);
+      }
+      tb.order[pos] = (uint32_t)s << 16 | (uint32_t)(e * group);
+    }
+    first += m;
+  }
+  uint32_t before = 0;
+  if (t < p.num_seq)
+    for (int q = 0; q < t; ++q) before += tb.pair0[q] * (tb.pair0[q] + 1) / 2;
+  __syncthreads();
+  if (t < p.num_seq) tb.pair0[t] = before;
+  __syncthreads();
+  return false;
+}
+
+// `reverse`: the heavy tiles are the late ones (a query tile sees all earlier keys); otherwise the early ones (a key tile
+// is seen by all later queries).
+__device__ __forceinline__ bool decode_item(const KParams &p, const SmallTable &tb, int item, int group, bool reverse, TileCoord &c) {
   int s, k;
   if (p.cu == nullptr) {
     const int n = (int)((p.tokens + p.tile - 1) / p.tile);
@@ -151,29 +219,87 @@ __device__ __forceinline__ bool decode_item(const KParams &p, int item, int grou
     c.boff = s;
     c.pair0 = (long long)s * ((long long)n * (n + 1) / 2);
   } else {
-    if (item >= p.hdr[group == 1 ? 2 : 3]) return false;
-    const int2 e = (group == 1 ? p.order : p.order2)[item];
-    s = e.x;
-    k = e.y;
-    c.n_tiles = p.tile_prefix[s + 1] - p.tile_prefix[s];
+    if (p.small_table) {
+      if (item >= kSmallItems) return false;
+      const uint32_t e = tb.order[item];
+      if (e == 0xffffffffu) return false;
+      s = (int)(e >> 16);
+      k = (int)(e & 0xffffu);
+      c.pair0 = tb.pair0[s];
+    } else {
+      if (item >= p.hdr[group == 1 ? 2 : 3]) return false;
+      const int2 e = (group == 1 ? p.order : p.order2)[item];
+      s = e.x;
+      k = e.y;
+      c.pair0 = p.pair_prefix[s];
+    }
     c.tok0 = s == 0 ? 0 : load_cu(p, s - 1);
     c.len = (int)(load_cu(p, s) - c.tok0);
+    c.n_tiles = (c.len + p.tile - 1) / p.tile;
     c.boff = 0;
-    c.pair0 = p.pair_prefix[s];
   }
   c.seq = s;
   c.idx = reverse ? k : c.n_tiles - 1 - k;
   return true;
 }
-__device__ __forceinline__ bool decode_tile(const KParams &p, int item, bool reverse, TileCoord &c) {
-  return decode_item(p, item, 1, reverse, c);
-}
 // One-dimensional grids: block = item * head_cnt + head, so that equal-weight items of all heads are neighbours.
-__device__ __forceinline__ bool decode_block(const KParams &p, int group, bool reverse, TileCoord &c, int &hh) {
+__device__ __forceinline__ bool decode_block(const KParams &p, const SmallTable &tb, int group, bool reverse, TileCoord &c, int &hh) {
   const int item = blockIdx.x / p.head_cnt;
   hh = blockIdx.x - item * p.head_cnt;
-  return decode_item(p, item, group, reverse, c);
+  return decode_item(p, tb, item, group, reverse, c);
 }
+
+// ---- rows no sequence covers --------------------------------------------------------------------------------------------
+// Rows past the end of the last packed sequence get zeros.  When cu_seqlens was refused nothing is computed and every row
+// of the outputs is filled with NaN instead, so that a caller who does not look at the status word cannot mistake
+// uninitialised memory for results.  Both are done by whichever kernel writes the tensor, each block taking its share.
+// (By value and not inlined: a reference would have every kernel copy its parameters to local memory on entry.)
+struct FillJob {
+  long long tokens, first;   // rows [first, tokens) of heads [head0, head0 + head_cnt)
+  int head0, head_cnt, head_dim, block, blocks;
+  float value;
+};
+__device__ __forceinline__ FillJob fill_job(const KParams &p, long long first, bool refused, int block, int blocks) {
+  return FillJob{p.tokens, first, p.head0, p.head_cnt, p.head_dim, block, blocks, refused ? __int_as_float(0x7fc00000) : 0.f};
+}
+template <typename T>
+__device__ __noinline__ void fill_rows(TensorRef out, FillJob f) {
+  const long long rows = f.tokens - f.first, all = rows * f.head_cnt;
+  for (long long i = f.block; i < all; i += f.blocks) {
+    const long long h = i / rows, row = f.first + (i - h * rows);
+    T *o = reinterpret_cast<T *>(out.ptr) + (f.head0 + h) * out.sh + row * out.st;
+    for (int x = threadIdx.x; x < f.head_dim; x += blockDim.x) o[x] = from_f32<T>(f.value);
+  }
+}
+template <typename T>
+__device__ __noinline__ void fill_row_state(T *rem, double *log_rem, FillJob f) {
+  const long long rows = f.tokens - f.first, all = rows * f.head_cnt;
+  for (long long i = (long long)f.block * blockDim.x + threadIdx.x; i < all; i += (long long)f.blocks * blockDim.x) {
+    const long long h = i / rows, idx = (f.head0 + h) * f.tokens + f.first + (i - h * rows);
+    rem[idx] = from_f32<T>(f.value);
+    log_rem[idx] = (double)f.value;
+  }
+}
+template <typename T>
+__device__ __forceinline__ void fill_forward_rows(const KParams &p, long long first, bool refused, int block, int blocks) {
+  const FillJob f = fill_job(p, first, refused, block, blocks);
+  fill_rows<T>(p.o, f);
+  fill_row_state<T>(reinterpret_cast<T *>(p.rem), p.log_rem, f);
+}
+// A kernel's first step: its item table (by all threads; contains barriers for a small packed batch).  Returns the end of
+// the last sequence; `refused`: cu_seqlens was, nothing is to be computed and no row counts as covered.
+__device__ __forceinline__ long long open_table(const KParams &p, int group, SmallTable &tb, bool &refused) {
+  refused = false;
+  if (p.cu == nullptr) return p.tokens;
+  if (!p.small_table) {
+    const int4 h = *reinterpret_cast<const int4 *>(p.hdr);
+    refused = h.x != 0;
+    return h.y;
+  }
+  refused = build_small_table(p, group, tb);
+  return refused ? 0 : load_cu(p, p.num_seq - 1);
+}
+
 // Blocks to launch for such a grid (an upper bound for packed batches: surplus blocks leave at once).
 inline long long item_blocks(const KParams &p, int group) {
   long long items;
@@ -186,16 +312,6 @@ inline long long item_blocks(const KParams &p, int group) {
   return items * p.head_cnt;
 }
 
-template <typename T> __device__ __forceinline__ float to_f32(T x);
-template <> __device__ __forceinline__ float to_f32<float>(float x) { return x; }
-template <> __device__ __forceinline__ float to_f32<__nv_bfloat16>(__nv_bfloat16 x) { return __bfloat162float(x); }
-template <> __device__ __forceinline__ float to_f32<__half>(__half x) { return __half2float(x); }
-
-template <typename T> __device__ __forceinline__ T from_f32(float x);
-template <> __device__ __forceinline__ float from_f32<float>(float x) { return x; }
-template <> __device__ __forceinline__ __nv_bfloat16 from_f32<__nv_bfloat16>(float x) { return __float2bfloat16_rn(x); }
-template <> __device__ __forceinline__ __half from_f32<__half>(float x) { return __float2half_rn(x); }
-
 // Upstream gradient of rem for row `idx` of the (batch, heads, tokens) array.
 template <typename T>
 __device__ __forceinline__ float load_drem(const KParams &p, long long idx) {
@@ -205,8 +321,7 @@ __device__ __forceinline__ float load_drem(const KParams &p, long long idx) {
 // Host-side launch helpers implemented in the .cu files; all return cudaError_t of the launch.
 cudaError_t launch_fused_drem(const KParams &p, int dtype, cudaStream_t s);   // fills d_rem_fused (all heads)
 cudaError_t launch_fused_dv(const KParams &p, int dtype, cudaStream_t s);     // dv += rem * d_out (all heads)
-cudaError_t launch_prep(const KParams &p, cudaStream_t s);
-cudaError_t launch_zero_tail(const KParams &p, int dtype, bool backward, cudaStream_t s);
+cudaError_t launch_prep(const KParams &p, cudaStream_t s, int *launches);   // the sequence table, where the call needs one
 cudaError_t launch_simt_fwd(const KParams &p, int dtype, cudaStream_t s, int *launches);
 cudaError_t launch_simt_bwd(const KParams &p, int dtype, cudaStream_t s, int *launches);
 cudaError_t launch_tc_fwd(const KParams &p, int dtype, cudaStream_t s, int *launches);

@@ -1,26 +1,58 @@
 // CUDA-core (fp32 FMA) kernels: the exact path for fp32 tensors and for head sizes the tensor-core
-// kernels do not take.  Also holds the two helper kernels every path uses: the sequence-table
-// builder and the tail zero-fill.
+// kernels do not take.  Also holds the sequence-table builder and the elementwise kernels of the fused form.
 #include "sb_common.cuh"
 
 namespace sb {
 
 // ------------------------------------------------------------------------------------------------
-// Sequence table: exclusive prefix of tiles per sequence and of (query tile, key tile) pairs.
+// Sequence table of the larger packed batches: the first (query tile, key tile) pair of every sequence, and the work items
+// by descending weight (see decode_item).
 // ------------------------------------------------------------------------------------------------
-// Work items by descending weight (see decode_item): a counting sort over classes of `order_span` consecutive tiles
-// (counted in units of `group`), the heaviest class first.  The tiles of one sequence inside a class stay neighbours
-// (they read the same keys or queries at about the same time and share them through L2); the order of the
-// sequences inside a class is whatever the shared-memory atomics give, which does not matter.
+// The order is a counting sort over classes of `order_span` consecutive tiles (counted in units of `group`), the heaviest
+// class first.  The tiles of one sequence inside a class stay neighbours (they read the same keys or queries at about the
+// same time and share them through L2); the order of the sequences inside a class is whatever the shared-memory atomics
+// give, which does not matter.
+// One block: what bounds it is latency, so every phase is a few steps of 1024 threads.  Sequences of few classes are taken
+// one per thread, with one atomic per warp and class; long ones one per warp.  One 131072-token sequence: 8.3 us (one thread
+// per sequence and serial prefix sums before: 82 us); 1024 sequences of up to 512 tokens: 9.4 us (16.3).
 constexpr int kMaxClasses = 8192;
-__device__ __forceinline__ int seq_tiles(const KParams &p, int s) {
-  const long long start = s == 0 ? 0 : load_cu(p, s - 1);
-  const long long len = load_cu(p, s) - start;
-  if (len < 0 || len > p.max_seqlen) return 0;
-  return (int)((len + p.tile - 1) / p.tile);
+constexpr int kPrepThreads = 1024;
+
+// Exclusive prefix sum over the block's threads; `total` is the sum over all of them.
+template <typename V>
+__device__ __forceinline__ V block_exclusive_scan(V x, V *s_warp, V &total) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  V incl = x;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const V up = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += up;
+  }
+  if (lane == 31) s_warp[warp] = incl;
+  __syncthreads();
+  if (warp == 0) {
+    V w = lane < kPrepThreads / 32 ? s_warp[lane] : V(0);
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const V up = __shfl_up_sync(0xffffffffu, w, o);
+      if (lane >= o) w += up;
+    }
+    s_warp[lane] = w;
+  }
+  __syncthreads();
+  total = s_warp[kPrepThreads / 32 - 1];
+  const V before = (warp > 0 ? s_warp[warp - 1] : V(0)) + incl - x;
+  __syncthreads();
+  return before;
 }
-__device__ void build_order(const KParams &p, int group, int2 *out, int hdr_slot, int *s_cls) {
-  const int t = threadIdx.x;
+
+__device__ __forceinline__ int seq_tiles(const KParams &p, int s) {
+  const long long start = s == 0 ? 0 : load_cu(p, s - 1), end = load_cu(p, s);
+  return (int)((end - start + p.tile - 1) / p.tile);
+}
+
+__device__ void build_order(const KParams &p, int group, int2 *out, int hdr_slot, int *s_cls, int *s_warp) {
+  const int t = threadIdx.x, lane = t & 31;
   const int span = p.order_span;                         // entries of one sequence that stay neighbours
   const int m_max = (p.n_max + group - 1) / group;       // entries of the longest sequence
   const int c_max = (m_max + span - 1) / span;           // classes
@@ -34,135 +66,110 @@ __device__ void build_order(const KParams &p, int group, int2 *out, int hdr_slot
     __syncthreads();
     return;
   }
-  for (int j = t; j < c_max; j += blockDim.x) s_cls[j] = 0;
+  const bool wide = c_max > 8;   // a warp per sequence, a lane per class; otherwise a thread per sequence
+  for (int j = t; j < c_max; j += kPrepThreads) s_cls[j] = 0;
   __syncthreads();
-  for (int s = t; s < p.num_seq; s += blockDim.x) {   // entries per class
-    const int m = (seq_tiles(p, s) + group - 1) / group;
-    for (int cl = 0; cl * span < m; ++cl) atomicAdd(&s_cls[cl], min(span, m - cl * span));
-  }
-  __syncthreads();
-  if (t == 0) {   // -> first position of every class, the heaviest class first
-    int pos = 0;
-    for (int cl = c_max - 1; cl >= 0; --cl) {
-      const int n = s_cls[cl];
-      s_cls[cl] = pos;
-      pos += n;
-    }
-    p.hdr[hdr_slot] = pos;
-  }
-  __syncthreads();
-  for (int s = t; s < p.num_seq; s += blockDim.x) {
-    const int m = (seq_tiles(p, s) + group - 1) / group;
-    for (int cl = 0; cl * span < m; ++cl) {
-      const int n = min(span, m - cl * span);
-      const int pos = atomicAdd(&s_cls[cl], n);
-      for (int i = 0; i < n; ++i) out[pos + i] = make_int2(s, (cl * span + n - 1 - i) * group);   // heaviest first
-    }
-  }
-  __syncthreads();
-}
-
-__global__ void __launch_bounds__(256) prep_kernel(KParams p) {
-  __shared__ int s_cls[kMaxClasses];
-  __shared__ long long s_tiles[256];
-  __shared__ long long s_pairs[256];
-  const int t = threadIdx.x;
-  if (t < 8) p.hdr[t] = 0;   // the header is this kernel's to initialise (a fixed-length batch uses clear_hdr_kernel)
-  __syncthreads();
-  const int per = (p.num_seq + 255) / 256;
-  const int s0 = t * per, s1 = min(p.num_seq, s0 + per);
-  const int busy = (p.num_seq + per - 1) / per;   // threads that own sequences
-  long long tiles = 0, pairs = 0;
-  int bad = -1;
-  for (int s = s0; s < s1; ++s) {
-    const long long start = s == 0 ? 0 : load_cu(p, s - 1);
-    const long long end = load_cu(p, s);
-    const long long len = end - start;
-    if (len < 0 || end > p.tokens || start < 0 || len > p.max_seqlen) { if (bad < 0) bad = s; continue; }
-    const long long n = (len + p.tile - 1) / p.tile;
-    tiles += n;
-    pairs += n * (n + 1) / 2;
-  }
-  s_tiles[t] = tiles;
-  s_pairs[t] = pairs;
-  if (bad >= 0) {
-    p.hdr[0] = 1;
-    if (p.status != nullptr) { p.status[0] = SB_DEV_BAD_CU_SEQLENS; p.status[1] = bad; }
-  }
-  __syncthreads();
-  if (t == 0) {
-    if (p.check_leading_zero && load_cu(p, -1) != 0) {
-      p.hdr[0] = 1;
-      if (p.status != nullptr) { p.status[0] = SB_DEV_BAD_CU_SEQLENS; p.status[1] = -1; }
-    }
-    long long a = 0, b = 0;
-    for (int i = 0; i < busy; ++i) {
-      const long long x = s_tiles[i], y = s_pairs[i];
-      s_tiles[i] = a; s_pairs[i] = b;
-      a += x; b += y;
-    }
-    p.tile_prefix[p.num_seq] = (int)a;
-    p.pair_prefix[p.num_seq] = b;
-    p.hdr[1] = p.num_seq > 0 ? (int)load_cu(p, p.num_seq - 1) : 0;
-    if (a > p.tiles_cap || b > p.pairs_cap) p.hdr[0] = 1;  // cannot happen for valid cu_seqlens
-  }
-  __syncthreads();
-  tiles = s_tiles[t];
-  pairs = s_pairs[t];
-  for (int s = s0; s < s1; ++s) {
-    p.tile_prefix[s] = (int)tiles;
-    p.pair_prefix[s] = pairs;
-    const long long start = s == 0 ? 0 : load_cu(p, s - 1);
-    const long long len = load_cu(p, s) - start;
-    if (len < 0 || len > p.max_seqlen) continue;
-    const long long n = (len + p.tile - 1) / p.tile;
-    tiles += n;
-    pairs += n * (n + 1) / 2;
-  }
-  __syncthreads();
-  if (p.hdr[0]) return;   // bad cu_seqlens: no kernel will look at the order
-  build_order(p, 1, const_cast<int2 *>(p.order), 2, s_cls);
-  if (p.order2 != nullptr) build_order(p, 2, const_cast<int2 *>(p.order2), 3, s_cls);
-}
-
-__global__ void clear_hdr_kernel(int *hdr, unsigned long long *trace) {
-  if (threadIdx.x < 8) hdr[threadIdx.x] = 0;
-  if (trace != nullptr)
-    for (int i = threadIdx.x; i < (int)(kTraceBytes / 8); i += blockDim.x) trace[i] = 0;
-}
-
-cudaError_t launch_prep(const KParams &p, cudaStream_t s) {
-  if (p.cu == nullptr || p.trace != nullptr) clear_hdr_kernel<<<1, 32, 0, s>>>(p.hdr, p.trace);
-  if (p.cu != nullptr) prep_kernel<<<1, 256, 0, s>>>(p);
-  return cudaGetLastError();
-}
-
-// Rows past the end of the last packed sequence belong to no sequence: write zeros there.  When the sequence table
-// was refused (bad cu_seqlens: every other kernel of the call has returned at once), every row of the outputs is
-// filled with NaN instead, so that a caller who does not look at the status word cannot mistake uninitialised memory
-// for results.
-template <typename T>
-__global__ void zero_tail_kernel(KParams p, bool backward) {
-  const bool refused = p.hdr[0] != 0;
-  const long long first = refused ? 0 : p.hdr[1];
-  const float fill = refused ? __int_as_float(0x7fc00000) : 0.f;
-  const int h = p.head0 + blockIdx.y;
-  const int d = p.head_dim;
-  for (long long row = first + blockIdx.x; row < p.tokens; row += gridDim.x) {
-    if (!backward) {
-      T *o = reinterpret_cast<T *>(p.o.ptr) + h * p.o.sh + row * p.o.st;
-      for (int x = threadIdx.x; x < d; x += blockDim.x) o[x] = from_f32<T>(fill);
-      if (threadIdx.x == 0) {
-        reinterpret_cast<T *>(p.rem)[(long long)h * p.tokens + row] = from_f32<T>(fill);
-        p.log_rem[(long long)h * p.tokens + row] = (double)fill;
+  // one sweep counts the entries of every class, a second one writes them
+  auto sweep = [&](bool write) {
+    const int step = wide ? kPrepThreads / 32 : kPrepThreads;
+    for (int s0 = 0; s0 < p.num_seq; s0 += step) {
+      const int s = s0 + (wide ? t >> 5 : t);
+      const int m = s < p.num_seq ? (seq_tiles(p, s) + group - 1) / group : 0;
+      if (wide) {
+        for (int cl = lane; cl * span < m; cl += 32) {
+          const int n = min(span, m - cl * span), pos = atomicAdd(&s_cls[cl], n);
+          if (write)
+            for (int i = 0; i < n; ++i) out[pos + i] = make_int2(s, (cl * span + n - 1 - i) * group);   // heaviest first
+        }
+      } else {
+        for (int cl = 0; cl < c_max; ++cl) {   // the same class in all lanes: one atomic per warp
+          const int n = min(span, max(m - cl * span, 0));
+          int incl = n;
+#pragma unroll
+          for (int o = 1; o < 32; o <<= 1) {
+            const int up = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += up;
+          }
+          const int sum = __shfl_sync(0xffffffffu, incl, 31);
+          if (sum == 0) break;
+          int base = 0;
+          if (lane == 0) base = atomicAdd(&s_cls[cl], sum);
+          const int pos = __shfl_sync(0xffffffffu, base, 0) + incl - n;
+          if (write)
+            for (int i = 0; i < n; ++i) out[pos + i] = make_int2(s, (cl * span + n - 1 - i) * group);
+        }
       }
-    } else {
-      T *a = reinterpret_cast<T *>(p.dq.ptr) + h * p.dq.sh + row * p.dq.st;
-      T *b = reinterpret_cast<T *>(p.dk.ptr) + h * p.dk.sh + row * p.dk.st;
-      T *c = reinterpret_cast<T *>(p.dv.ptr) + h * p.dv.sh + row * p.dv.st;
-      for (int x = threadIdx.x; x < d; x += blockDim.x) { a[x] = b[x] = c[x] = from_f32<T>(fill); }
     }
+  };
+  sweep(false);
+  __syncthreads();
+  // -> first position of every class, the heaviest class first
+  int base = 0;
+  for (int j0 = 0; j0 < c_max; j0 += kPrepThreads) {
+    const int cl = c_max - 1 - (j0 + t);
+    const int n = cl >= 0 ? s_cls[cl] : 0;
+    int total;
+    const int before = block_exclusive_scan(n, s_warp, total);
+    if (cl >= 0) s_cls[cl] = base + before;
+    base += total;
   }
+  if (t == 0) p.hdr[hdr_slot] = base;
+  __syncthreads();
+  sweep(true);
+  __syncthreads();
+}
+
+__global__ void __launch_bounds__(kPrepThreads) prep_kernel(KParams p) {
+  __shared__ int s_cls[kMaxClasses];
+  __shared__ long long s_warp[32];
+  const int t = threadIdx.x;
+  const int per = (p.num_seq + kPrepThreads - 1) / kPrepThreads;
+  const int s0 = min(p.num_seq, t * per), s1 = min(p.num_seq, s0 + per);
+  long long tiles = 0, pairs = 0;
+  int bad = -2;
+  if (t == 0 && p.check_leading_zero && load_cu(p, -1) != 0) bad = -1;
+  for (int s = s0; s < s1; ++s) {
+    const long long start = s == 0 ? 0 : load_cu(p, s - 1), end = load_cu(p, s);
+    if (!seq_valid(p, start, end)) { if (bad == -2) bad = s; continue; }
+    const long long n = (end - start + p.tile - 1) / p.tile;
+    tiles += n;
+    pairs += n * (n + 1) / 2;
+  }
+  long long all_tiles, all_pairs;
+  block_exclusive_scan(tiles, s_warp, all_tiles);
+  long long before = block_exclusive_scan(pairs, s_warp, all_pairs);
+  // (more than the workspace holds cannot happen for valid cu_seqlens)
+  const bool refused = __syncthreads_or(bad != -2) || all_tiles > p.tiles_cap || all_pairs > p.pairs_cap;
+  if (bad != -2 && p.status != nullptr) { p.status[0] = SB_DEV_BAD_CU_SEQLENS; p.status[1] = bad; }
+  if (t == 0) {
+    p.hdr[0] = refused ? 1 : 0;
+    p.hdr[1] = refused ? 0 : (int)load_cu(p, p.num_seq - 1);
+  }
+  if (refused) return;   // no kernel will look at the table
+  for (int s = s0; s < s1; ++s) {
+    p.pair_prefix[s] = before;
+    const long long n = seq_tiles(p, s);
+    before += n * (n + 1) / 2;
+  }
+  int *s_warp_i = reinterpret_cast<int *>(s_warp);
+  build_order(p, 1, const_cast<int2 *>(p.order), 2, s_cls, s_warp_i);
+  if (p.order2 != nullptr) build_order(p, 2, const_cast<int2 *>(p.order2), 3, s_cls, s_warp_i);
+}
+
+#ifdef SB_TRACE
+__global__ void clear_trace_kernel(unsigned long long *trace) {
+  for (int i = threadIdx.x; i < (int)(kTraceBytes / 8); i += blockDim.x) trace[i] = 0;
+}
+#endif
+
+cudaError_t launch_prep(const KParams &p, cudaStream_t s, int *launches) {
+#ifdef SB_TRACE
+  if (p.trace != nullptr) clear_trace_kernel<<<1, 32, 0, s>>>(p.trace);
+#endif
+  if (p.cu == nullptr || p.small_table) return cudaSuccess;
+  *launches += 1;
+  prep_kernel<<<1, kPrepThreads, 0, s>>>(p);
+  return cudaGetLastError();
 }
 
 // Backward with out = o + rem * v: the upstream gradient of rem gains <d_out, v> per row, and dv gains rem * d_out
@@ -208,7 +215,7 @@ __global__ void __launch_bounds__(256) fused_drem_kernel(KParams p, int group) {
 
 template <typename T, int kVec>
 __global__ void __launch_bounds__(256) fused_dv_kernel(KParams p, int group) {
-  if (p.hdr[0]) return;
+  if (p.cu != nullptr && p.hdr[0]) return;   // (a small call's table never comes with this kernel)
   const long long covered = p.cu != nullptr ? (long long)p.hdr[1] : p.tokens;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int rows_per_warp = 32 / group;
@@ -265,15 +272,6 @@ cudaError_t launch_fused_dv(const KParams &p, int dtype, cudaStream_t s) {
   if (dtype == SB_DTYPE_F32) return launch_fused_t<float, true>(p, s);
   if (dtype == SB_DTYPE_BF16) return launch_fused_t<__nv_bfloat16, true>(p, s);
   return launch_fused_t<__half, true>(p, s);
-}
-
-cudaError_t launch_zero_tail(const KParams &p, int dtype, bool backward, cudaStream_t s) {
-  if (p.cu == nullptr) return cudaSuccess;
-  dim3 grid(32, p.head_cnt);
-  if (dtype == SB_DTYPE_F32) zero_tail_kernel<float><<<grid, 128, 0, s>>>(p, backward);
-  else if (dtype == SB_DTYPE_BF16) zero_tail_kernel<__nv_bfloat16><<<grid, 128, 0, s>>>(p, backward);
-  else zero_tail_kernel<__half><<<grid, 128, 0, s>>>(p, backward);
-  return cudaGetLastError();
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -485,11 +483,15 @@ __device__ __forceinline__ void store16(float *dst, const float (&x)[16]) {
 // steps of 64; every row carries sum softplus(z) over the keys already visited, in fp64 (reference: _forward_one_row,
 // sb_varlen_fwd.py:81-215).
 template <typename T, int DP>
-__global__ void __launch_bounds__(kSimtThreads, kSimtBlocks<DP>) simt_fwd_kernel(KParams p, bool wide) {
+__global__ void __launch_bounds__(kSimtThreads, kSimtBlocks<DP>) simt_fwd_kernel(const __grid_constant__ KParams p, bool wide) {
   extern __shared__ float4 smem4[];
-  if (p.hdr[0]) return;
+  __shared__ SmallTable tb;
+  bool refused;
+  const long long covered = open_table(p, 1, tb, refused);
+  const int block = blockIdx.y * gridDim.x + blockIdx.x, blocks = gridDim.x * gridDim.y;
+  if (covered < p.tokens) fill_forward_rows<T>(p, covered, refused, block, blocks);
   TileCoord c;
-  if (!decode_tile(p, blockIdx.x, true, c)) return;
+  if (refused || !decode_item(p, tb, blockIdx.x, 1, true, c)) return;
   const int d = p.head_dim, h = p.head0 + blockIdx.y, t = threadIdx.x;
   float *Qs = reinterpret_cast<float *>(smem4), *Ks = Qs + kT * kLd<DP>, *Vs = Ks + kStep * kLd<DP>, *Ss = Vs + kStep * kLd<DP>;
   const int row0 = c.idx * kT, ac = p.attend_current;
@@ -646,11 +648,15 @@ __device__ __forceinline__ void bwd_segment(float (&z)[16], float (&dp)[16], int
 // sb_varlen_bwd.py:297-481, which adds dK/dV under a spin lock instead).  Leaves A and dz of every (query tile, key tile)
 // pair in the workspace (p.az), or, where those would not fit the scratch budget, the carried R1 and S2 per pair and row.
 template <typename T, int DP>
-__global__ void __launch_bounds__(kSimtThreads, kSimtBlocks<DP>) simt_bwd_dq_kernel(KParams p, bool wide) {
+__global__ void __launch_bounds__(kSimtThreads, kSimtBlocks<DP>) simt_bwd_dq_kernel(const __grid_constant__ KParams p, bool wide) {
   extern __shared__ float4 smem4[];
-  if (p.hdr[0]) return;
+  __shared__ SmallTable tb;
+  bool refused;
+  const long long covered = open_table(p, 1, tb, refused);
+  const int block = blockIdx.y * gridDim.x + blockIdx.x, blocks = gridDim.x * gridDim.y;
+  if (covered < p.tokens) fill_rows<T>(p.dq, fill_job(p, covered, refused, block, blocks));
   TileCoord c;
-  if (!decode_tile(p, blockIdx.x, true, c)) return;
+  if (refused || !decode_item(p, tb, blockIdx.x, 1, true, c)) return;
   const int d = p.head_dim, hh = blockIdx.y, h = p.head0 + hh, t = threadIdx.x;
   float *Qs = reinterpret_cast<float *>(smem4), *Gs = Qs + kT * kLd<DP>, *Ks = Gs + kT * kLd<DP>, *Vs = Ks + kStep * kLd<DP>;
   float *Zs = Vs + kStep * kLd<DP>, *Ps = Zs + kT * kLdS;
@@ -742,11 +748,18 @@ __global__ void __launch_bounds__(kSimtThreads, kSimtBlocks<DP>) simt_bwd_dq_ker
 // dK, dV: key-stationary, one block per 32-key tile, query tiles diagonal -> end two at a time; accumulators in registers,
 // fixed summation order, no atomics.  kStored: A and dz come from the workspace; otherwise they are computed again.
 template <typename T, int DP, bool kStored>
-__global__ void __launch_bounds__(kSimtThreads, kSimtBlocks<DP>) simt_bwd_dkv_kernel(KParams p, bool wide) {
+__global__ void __launch_bounds__(kSimtThreads, kSimtBlocks<DP>) simt_bwd_dkv_kernel(const __grid_constant__ KParams p, bool wide) {
   extern __shared__ float4 smem4[];
-  if (p.hdr[0]) return;
+  __shared__ SmallTable tb;
+  bool refused;
+  const long long covered = open_table(p, 1, tb, refused);
+  const int block = blockIdx.y * gridDim.x + blockIdx.x, blocks = gridDim.x * gridDim.y;
+  if (covered < p.tokens) {
+    fill_rows<T>(p.dk, fill_job(p, covered, refused, block, blocks));
+    fill_rows<T>(p.dv, fill_job(p, covered, refused, block, blocks));
+  }
   TileCoord c;
-  if (!decode_tile(p, blockIdx.x, false, c)) return;
+  if (refused || !decode_item(p, tb, blockIdx.x, 1, false, c)) return;
   const int d = p.head_dim, hh = blockIdx.y, h = p.head0 + hh, t = threadIdx.x;
   float *Qs = reinterpret_cast<float *>(smem4), *Gs = Qs + kStep * kLd<DP>, *Zs = Gs + kStep * kLd<DP>, *Ps = Zs + kStep * kLdH;
   float *Ks = Ps + kStep * kLdH, *Vs = Ks + kT * kLd<DP>;   // recomputation only
@@ -832,6 +845,9 @@ __global__ void __launch_bounds__(kSimtThreads, kSimtBlocks<DP>) simt_bwd_dkv_ke
     if (key >= c.len) continue;
     T *ok = reinterpret_cast<T *>(p.dk.ptr) + c.boff * p.dk.sb + (long long)h * p.dk.sh + (c.tok0 + key) * p.dk.st;
     T *ov = reinterpret_cast<T *>(p.dv.ptr) + c.boff * p.dv.sb + (long long)h * p.dv.sh + (c.tok0 + key) * p.dv.st;
+    // out = o + rem * v was requested: dV gains rem * d_out on its own row (rem = 2^log_rem)
+    const T *g = reinterpret_cast<const T *>(p.d_o.ptr) + c.boff * p.d_o.sb + (long long)h * p.d_o.sh + (c.tok0 + key) * p.d_o.st;
+    const float rem = p.fuse_rem_v ? exp2f((float)p.log_rem[(c.boff * p.heads + h) * p.tokens + c.tok0 + key]) : 0.f;
 #pragma unroll
     for (int u = 0; u < DP / 64; ++u)
 #pragma unroll
@@ -839,7 +855,7 @@ __global__ void __launch_bounds__(kSimtThreads, kSimtBlocks<DP>) simt_bwd_dkv_ke
         const int col = 64 * u + 4 * tx + x;
         if (col < d) {
           ok[col] = from_f32<T>(dk[i][4 * u + x] * p.scale);
-          ov[col] = from_f32<T>(dv[i][4 * u + x]);
+          ov[col] = from_f32<T>(p.fuse_rem_v ? fmaf(rem, to_f32<T>(g[col]), dv[i][4 * u + x]) : dv[i][4 * u + x]);
         }
       }
   }

@@ -252,7 +252,8 @@ constexpr int kKvTile = 2 * kKvBox;            // K or V sub-tile
 constexpr int kStageBytes = 2 * kKvTile;
 constexpr int kZBytes = kBM * kBN * 2;         // dz tile: 128 rows x 64 keys
 static_assert(kStages == 2, "stage = sub-tile mod 2");
-constexpr int kSmem = 1024 + 4 * kTileBytes + kStages * kStageBytes + 2 * kZBytes + 512;
+constexpr int kSmem = 1024 + 4 * kTileBytes + kStages * kStageBytes + 2 * kZBytes + 512 + (int)sizeof(SmallTable);
+static_assert(kSmem <= 232448, "shared memory per block");
 enum { bQG = 0, bKvFull = 1, bKvEmpty = 3, bSpFull = 5, bZFull = 7, bZEmpty = 9, bFirst = 11, bSpEmpty = 12, bDqFull = 14, bNum = 16 };
 }  // namespace dq2
 
@@ -265,13 +266,6 @@ tc_bwd_dq2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
   constexpr int D = 128;
   extern __shared__ uint8_t smem_raw[];
   if (threadIdx.x == 0) trace_block(p, 0);
-  if (p.hdr[0]) return;
-  TileCoord c;
-  int hh_blk;
-  if (!decode_block(p, 2, true, c, hh_blk)) return;   // c.idx: the even tile of the pair (idx, idx + 1)
-  const int Ia = c.idx;
-  const bool b_active = Ia + 1 < c.n_tiles;
-
   const uint32_t raw = smem_u32(smem_raw);
   const uint32_t base = (raw + 1023u) & ~1023u;
   uint8_t *gbase = smem_raw + (base - raw);
@@ -279,6 +273,15 @@ tc_bwd_dq2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
   const uint32_t sKV = sQ + 4 * kTileBytes;     // stage: K sub-tile then V sub-tile
   const uint32_t sZ = sKV + kStages * kStageBytes;
   const uint32_t sBar = sZ + 2 * kZBytes;
+  SmallTable &tb = *reinterpret_cast<SmallTable *>(gbase + (sBar - base) + 512);
+  bool refused;
+  const long long covered = open_table(p, 2, tb, refused);
+  if (covered < p.tokens) fill_rows<typename std::conditional<kFp16, __half, __nv_bfloat16>::type>(p.dq, fill_job(p, covered, refused, blockIdx.x, gridDim.x));
+  TileCoord c;
+  int hh_blk;
+  if (refused || !decode_block(p, tb, 2, true, c, hh_blk)) return;   // c.idx: the even tile of the pair (idx, idx + 1)
+  const int Ia = c.idx;
+  const bool b_active = Ia + 1 < c.n_tiles;
   Ctl *ctl = reinterpret_cast<Ctl *>(gbase + (sBar - base) + bNum * 8);
   volatile int *abort_flag = &ctl->abort;
   auto bar = [&](int i) { return sBar + 8u * i; };
@@ -583,10 +586,17 @@ tc_bwd_dkv4_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
   constexpr int D = 128;
   extern __shared__ uint8_t smem_raw[];
   if (threadIdx.x == 0) trace_block(p, 0);
-  if (p.hdr[0]) return;
+  SmallTable &tb = *reinterpret_cast<SmallTable *>(smem_raw);   // never used: the launch sees to that, there is no room for it
+  bool refused;
+  const long long covered = open_table(p, 1, tb, refused);
+  if (covered < p.tokens) {
+    using T = typename std::conditional<kFp16, __half, __nv_bfloat16>::type;
+    fill_rows<T>(p.dk, fill_job(p, covered, refused, blockIdx.x, gridDim.x));
+    fill_rows<T>(p.dv, fill_job(p, covered, refused, blockIdx.x, gridDim.x));
+  }
   TileCoord c;
   int hh_blk;
-  if (!decode_block(p, 1, false, c, hh_blk)) return;
+  if (refused || !decode_block(p, tb, 1, false, c, hh_blk)) return;
   const int J = c.idx;                         // the 128-key tile
   const int n_halves = J * kBM + kBN < c.len ? 2 : 1;   // the sequence may end inside the first strip
 
@@ -894,7 +904,7 @@ constexpr int kRows = 32;                    // query rows per stage
 constexpr int kSub = kBM / kRows;            // stages per query tile
 constexpr int kBox = kRows * 64 * 2;         // kRows rows x 64 columns, 16-bit
 constexpr int kStageBytes = 8 * kBox;        // A, dz, Q, dO: two 64-column blocks each; also one 128 x 128 output tile
-constexpr int kSmem = 1024 + kStages * kStageBytes + 512 + kListBits / 8;
+constexpr int kSmem = 1024 + kStages * kStageBytes + 512 + kListBits / 8 + (int)sizeof(SmallTable);
 constexpr uint32_t kCols = 256;              // dK 0..127, dV 128..255
 enum { bFull = 0, bEmpty = 3, bOut = 6, bClean = 7, bLanded = 8, bNum = 9 };
 }  // namespace dkv5
@@ -907,10 +917,21 @@ tc_bwd_dkv5_kernel(const __grid_constant__ CUtensorMap tm_az, const __grid_const
   using namespace dkv5;
   constexpr int D = 128;
   extern __shared__ uint8_t smem_raw[];
-  if (p.hdr[0]) return;
+  const uint32_t raw = smem_u32(smem_raw);
+  const uint32_t base = (raw + 1023u) & ~1023u;
+  uint8_t *gbase = smem_raw + (base - raw);
+  const uint32_t sBar = base + kStages * kStageBytes;
+  SmallTable &tb = *reinterpret_cast<SmallTable *>(gbase + (sBar - base) + 512 + kListBits / 8);
+  bool refused;
+  const long long covered = open_table(p, 1, tb, refused);
+  if (covered < p.tokens) {
+    using T = typename std::conditional<kFp16, __half, __nv_bfloat16>::type;
+    fill_rows<T>(p.dk, fill_job(p, covered, refused, blockIdx.x, gridDim.x));
+    fill_rows<T>(p.dv, fill_job(p, covered, refused, blockIdx.x, gridDim.x));
+  }
   TileCoord c;
   int hh;
-  if (!decode_block(p, 1, false, c, hh)) return;
+  if (refused || !decode_block(p, tb, 1, false, c, hh)) return;
   const int h = p.head0 + hh;
   const int J = c.idx;                        // the 128-key tile
   // The sequence may end inside the last query tile.  The A and dz rows behind the end are zeros in the workspace; the
@@ -921,10 +942,6 @@ tc_bwd_dkv5_kernel(const __grid_constant__ CUtensorMap tm_az, const __grid_const
   const int last_rows = c.len - (c.n_tiles - 1) * kBM;          // 1 .. 128 rows of the last query tile exist
   const int clean_from = last_rows / kRows;                     // first such stage of the last query tile
 
-  const uint32_t raw = smem_u32(smem_raw);
-  const uint32_t base = (raw + 1023u) & ~1023u;
-  uint8_t *gbase = smem_raw + (base - raw);
-  const uint32_t sBar = base + kStages * kStageBytes;
   Ctl *ctl = reinterpret_cast<Ctl *>(gbase + (sBar - base) + bNum * 8);
   volatile int *abort_flag = &ctl->abort;
   volatile int *clean_stage = reinterpret_cast<volatile int *>(ctl + 1);

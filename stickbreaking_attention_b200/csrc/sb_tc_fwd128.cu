@@ -33,7 +33,7 @@ constexpr int kQBufs = 2;
 constexpr int kOBytes = kBM * D * 2;          // staging tile of the O epilogue
 constexpr int kWorkerBytes = kQBufs * kQBytes + kStages * kStageBytes + kOBytes;
 constexpr int kBarBytes = 512;
-constexpr int kSmem = 1024 + 2 * kWorkerBytes + kBarBytes;
+constexpr int kSmem = 1024 + 2 * kWorkerBytes + kBarBytes + (int)sizeof(SmallTable);
 constexpr uint32_t kWorkerCols = 192;
 // barriers of one worker
 enum { bQ = 0, bQFree = 2, bKvFull = 4, bKvEmpty = 4 + kStages, bSFull = 4 + 2 * kStages, bPFull = bSFull + 2, bOFull = bSFull + 4,
@@ -65,10 +65,10 @@ __device__ __forceinline__ void fwd128_finish(const KParams &p, long long lin, l
   w.s_top = min(2 * w.c.idx + 1, n_sub - 1);
   w.n_steps = w.s_top + 1;
 }
-__device__ __forceinline__ bool fwd128_item(const KParams &p, int it, int v, int V, Fwd128Item &w) {
+__device__ __forceinline__ bool fwd128_item(const KParams &p, const SmallTable &tb, int it, int v, int V, Fwd128Item &w) {
   const long long lin = fwd128_lin(it, v, V);
   const long long item = lin / p.head_cnt;
-  if (item > 0x7fffffffLL || !decode_item(p, (int)item, 1, true, w.c)) return false;
+  if (item > 0x7fffffffLL || !decode_item(p, tb, (int)item, 1, true, w.c)) return false;
   fwd128_finish(p, lin, item, w);
   return true;
 }
@@ -78,15 +78,18 @@ __device__ __forceinline__ bool fwd128_item(const KParams &p, int it, int v, int
 template <bool kFp16, bool kStop>
 __global__ void __launch_bounds__(fwd128::kThreads, 1)
 tc_fwd128x2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
-                   const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_o, const KParams p) {
+                   const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_o, const __grid_constant__ KParams p) {
   using namespace fwd128;
   extern __shared__ uint8_t smem_raw[];
-  if (p.hdr[0]) return;
-
   const uint32_t raw = smem_u32(smem_raw);
   const uint32_t base = (raw + 1023u) & ~1023u;
   uint8_t *gbase = smem_raw + (base - raw);
   const uint32_t sBar = base + 2 * kWorkerBytes;
+  SmallTable &tb = *reinterpret_cast<SmallTable *>(gbase + (sBar - base) + kBarBytes);
+  bool refused;
+  const long long covered = open_table(p, 1, tb, refused);
+  if (covered < p.tokens) fill_forward_rows<typename std::conditional<kFp16, __half, __nv_bfloat16>::type>(p, covered, refused, blockIdx.x, gridDim.x);
+  if (refused) return;
   Shared *sh = reinterpret_cast<Shared *>(gbase + (sBar - base) + 2 * bPerWorker * 8);
   Ctl *ctl = &sh->ctl;
   volatile int *abort_flag = &ctl->abort;
@@ -132,7 +135,7 @@ tc_fwd128x2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
     if (lane == 0) {
       prefetch_tensormap(&tm_q); prefetch_tensormap(&tm_k); prefetch_tensormap(&tm_v);
       int T = 0;   // K/V stages filled so far
-      for (int it = 0; fwd128_item(p, it, v, V, w); ++it) {
+      for (int it = 0; fwd128_item(p, tb, it, v, V, w); ++it) {
         const int qb = it % kQBufs, qn = it / kQBufs;
         // the buffer's previous tile is no longer read once its last S MMA has finished
         if (qn >= 1 && !wait_or_abort(bar(bQFree + qb), (qn - 1) & 1, abort_flag, p, 711)) break;
@@ -169,7 +172,7 @@ tc_fwd128x2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
       constexpr uint32_t idesc_pv = idesc_f16(kBM, D, kFp16, false, true);
       int T = 0, U = 0;   // K/V stages and steps of the earlier tiles
       bool ok = true;
-      for (int it = 0; ok && fwd128_item(p, it, v, V, w); ++it) {
+      for (int it = 0; ok && fwd128_item(p, tb, it, v, V, w); ++it) {
         const int qb = it % kQBufs, qn = it / kQBufs;
         ok = wait_or_abort(bar(bQ + qb), qn & 1, abort_flag, p, 720);
         const uint32_t qaddr = sQ + qb * kQBytes;
@@ -237,7 +240,7 @@ tc_fwd128x2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
     int U = 0;   // steps of the earlier tiles
     bool ok = true;
     Fwd128Item w_next;
-    bool have = fwd128_item(p, 0, v, V, w);
+    bool have = fwd128_item(p, tb, 0, v, V, w);
     uint8_t *stage = gbase + (sO - base);
     for (int it = 0; ok && have; ++it) {
       const int row = w.row0 + blk * 32 + lane;      // row index inside the sequence
@@ -301,7 +304,7 @@ tc_fwd128x2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
       }
       if (p.tile_start != nullptr && ok && warp_live && lane == 0 && row >= 64)
         *tile_start_entry(p, w.c, w.h, row) = s_reached * kBN;
-      const bool have_next = fwd128_item(p, it + 1, v, V, w_next);
+      const bool have_next = fwd128_item(p, tb, it + 1, v, V, w_next);
       if (ok) ok = wait_or_abort(bar(bOFull), it & 1, abort_flag, p, 732);
       if (ok) {
         tc_fence_after();

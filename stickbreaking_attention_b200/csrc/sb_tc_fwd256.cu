@@ -32,7 +32,7 @@ struct Cfg {
   // Q tiles of two items at 64 columns (there is room): the next item's Q is loaded while the current item still
   // reads its own, so a short item does not wait a load latency for its first scores
   static constexpr int kQBufs = D == 64 ? 2 : 1;
-  static constexpr int kSmem = 1024 + kQBufs * 2 * kQBytes + kStages * kStageBytes + 2 * kPBytes + kBarBytes;
+  static constexpr int kSmem = 1024 + kQBufs * 2 * kQBytes + kStages * kStageBytes + 2 * kPBytes + kBarBytes + (int)sizeof(SmallTable);
   static_assert(kSmem <= 232448, "shared memory per block");
 };
 enum { bQ = 0, bKvFull = 1, bKvEmpty = 7, bSFull = 13, bQFree = 17, bOFree = 18, bPFull = 20, bOFull = 24, bQ2 = 26,
@@ -60,11 +60,11 @@ struct Fwd256Item {
 
 // Item number `it` of this block: the launch holds one block per SM; blocks walk the weight-ordered item list in a
 // boustrophedon (even rounds left to right, odd rounds right to left), which evens out the sums of the weights.
-__device__ __forceinline__ bool fwd256_item(const KParams &p, int it, Fwd256Item &w) {
+__device__ __forceinline__ bool fwd256_item(const KParams &p, const SmallTable &tb, int it, Fwd256Item &w) {
   const long long G = gridDim.x;
   const long long lin = (long long)it * G + ((it & 1) ? G - 1 - blockIdx.x : blockIdx.x);
   const long long item = lin / p.head_cnt;
-  if (item > 0x7fffffffLL || !decode_item(p, (int)item, 1, true, w.c)) return false;
+  if (item > 0x7fffffffLL || !decode_item(p, tb, (int)item, 1, true, w.c)) return false;
   w.h = p.head0 + (int)(lin - item * p.head_cnt);
   const int m = w.c.idx;
   const int n_sub = (w.c.len + fwd256::kBN - 1) / fwd256::kBN;   // 64-key sub-tiles of the sequence
@@ -85,15 +85,13 @@ __device__ __forceinline__ bool fwd256_item(const KParams &p, int it, Fwd256Item
 template <int D, bool kFp16>
 __global__ void __launch_bounds__(fwd256::kThreads, 1)
 tc_fwd256_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
-                 const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_o, const KParams p) {
+                 const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_o, const __grid_constant__ KParams p) {
   using namespace fwd256;
   using C = Cfg<D>;
   constexpr int kQBytes = C::kQBytes, kKvTileBytes = C::kKvTileBytes, kStageBytes = C::kStageBytes, kBoxes = C::kBoxes;
   constexpr int kStages = C::kStages, kQBufs = C::kQBufs;
   extern __shared__ uint8_t smem_raw[];
   if (threadIdx.x == 0) trace_block(p, 0);
-  if (p.hdr[0]) return;
-
   const uint32_t raw = smem_u32(smem_raw);
   const uint32_t base = (raw + 1023u) & ~1023u;
   uint8_t *gbase = smem_raw + (base - raw);
@@ -102,6 +100,11 @@ tc_fwd256_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
   const uint32_t sP = sKV + kStages * kStageBytes;      // staging of O, one 128 x 64 box per tile
   const uint32_t sBar = sP + 2 * kPBytes;
   uint8_t *gP = gbase + (sP - base);
+  SmallTable &tb = *reinterpret_cast<SmallTable *>(gbase + (sBar - base) + kBarBytes);
+  bool refused;
+  const long long covered = open_table(p, 1, tb, refused);
+  if (covered < p.tokens) fill_forward_rows<typename std::conditional<kFp16, __half, __nv_bfloat16>::type>(p, covered, refused, blockIdx.x, gridDim.x);
+  if (refused) return;
   Shared *sh = reinterpret_cast<Shared *>(gbase + (sBar - base) + bNum * 8);
   Ctl *ctl = &sh->ctl;
   volatile int *abort_flag = &ctl->abort;
@@ -148,7 +151,7 @@ tc_fwd256_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
     if (lane == 0) {
       prefetch_tensormap(&tm_q); prefetch_tensormap(&tm_k); prefetch_tensormap(&tm_v);
       int T = 0;   // K/V stages filled so far
-      for (int it = 0; fwd256_item(p, it, w); ++it) {
+      for (int it = 0; fwd256_item(p, tb, it, w); ++it) {
         // the Q buffer's previous item (kQBufs items back) is no longer read once both issuers have finished its last S MMAs
         const int qb = it % kQBufs, qn = it / kQBufs;     // buffer and how many items it has held before
         const uint32_t bar_q = bar(qb ? bQ2 : bQ), bar_qfree = bar(qb ? bQFree2 : bQFree);
@@ -192,7 +195,7 @@ tc_fwd256_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
       constexpr uint32_t idesc_pv = idesc_f16(kBM, D, kFp16, false, true);
       int T = 0, U = 0;   // K/V stages and this tile's steps of the earlier items
       bool ok = true;
-      for (int it = 0; ok && fwd256_item(p, it, w); ++it) {
+      for (int it = 0; ok && fwd256_item(p, tb, it, w); ++it) {
         const bool active = wg == 0 || w.b_active;
         const int t0 = active && wg == 0 ? w.t0_a : 0;
         const int my_steps = active ? w.n_steps - t0 : 0;
@@ -286,7 +289,7 @@ tc_fwd256_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
     volatile EarlyStop &stop = sh->stop[wg];
     bool ok = true;
     Fwd256Item w_next;
-    bool have = fwd256_item(p, 0, w);
+    bool have = fwd256_item(p, tb, 0, w);
     for (int it = 0; ok && have; ++it) {
       const bool active = wg == 0 || w.b_active;
       const int t0 = wg == 0 ? w.t0_a : 0;
@@ -295,8 +298,7 @@ tc_fwd256_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
       const int s_diag0 = 4 * w.c.idx + 2 * wg;        // first sub-tile that reaches this tile's diagonal band
       const bool warp_live = (row & ~31) < w.c.len;    // a warp whose 32 rows all lie past the sequence end computes nothing
       LogSum run;
-      bool through = false;    // this warp is through with the tile, having got to sub-tile s_reached
-      int s_reached = 0;
+      int s_reached = -1;      // >= 0: this warp is through with the tile, having got to this sub-tile
       int slots = my_steps;                   // S slots used
       if (lane == 0) tma_store_wait_read();   // the previous item's O has left the staging boxes
       __syncwarp();
@@ -306,7 +308,7 @@ tc_fwd256_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
         const int gu = U + u, buf = gu & 1;
         ok = wait_or_abort(bar(bSFull + wg * 2 + buf), (gu >> 1) & 1, abort_flag, p, 330);
         if (!ok) break;
-        if (through && stop.word[buf] == kStepStop) {   // (a stop needs this warp's consent)
+        if (s_reached >= 0 && stop.word[buf] == kStepStop) {   // (a stop needs this warp's consent)
           slots = u + 1;
           __syncwarp();
           if (lane == 0) mbar_arrive(bar(bPFull + wg * 2 + buf));
@@ -324,11 +326,11 @@ tc_fwd256_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
           zero_tile_rows(v_tile, tail_rows, kBN, kBoxes, kKvBoxBytes, r, kBM);
           fence_proxy_async_smem();
         }
-        bool done = through || !warp_live;
+        bool done = !warp_live;
         float logsum = 0.f;
         // 64 columns in chunks of 16, last chunk first; TMEM is read one chunk ahead of the arithmetic
         // (the P rows of such a warp keep whatever their buffer held: they only reach accumulator rows that are never stored)
-        if (through) {
+        if (s_reached >= 0) {
           fwd256_zero_row(ts + kPCol);
         } else if (!warp_live) {
         } else if (s >= s_diag0) fwd256_row_pass<kFp16, true>(ts, s * kBN, row, ac, scale2, run, logsum, ts + kPCol, true);
@@ -338,13 +340,10 @@ tc_fwd256_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
         tc_fence_before();          // this step's TMEM reads and writes of P are done before the slot is handed back
         __syncwarp();
         if (lane == 0) {
-          if (may_stop && done && !through) publish_through(stop, warp & 3, it, u);
+          if (may_stop && done && s_reached < 0) publish_through(stop, warp & 3, it, u);
           mbar_arrive(bar(bPFull + wg * 2 + buf));
         }
-        if (may_stop && done && !through) {
-          through = true;
-          s_reached = s + 1;
-        }
+        if (may_stop && done && s_reached < 0) s_reached = s + 1;
         if ((threadIdx.x & 127) == 0) trace_event(p, 2 + wg, tr_cur, 5 + 16 * wg, t0 + u);
       }
       // ---- epilogue: O (TMEM) -> global, rem, log_rem
@@ -358,8 +357,8 @@ tc_fwd256_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
         p.log_rem[idx] = -run.value();
       }
       if (p.tile_start != nullptr && ok && my_steps > 0 && warp_live && lane == 0 && row >= 64)
-        *tile_start_entry(p, w.c, w.h, row) = s_reached * kBN;
-      const bool have_next = fwd256_item(p, it + 1, w_next);
+        *tile_start_entry(p, w.c, w.h, row) = max(s_reached, 0) * kBN;
+      const bool have_next = fwd256_item(p, tb, it + 1, w_next);
       if (ok) ok = wait_or_abort(bar(bOFull + wg), it & 1, abort_flag, p, 332);
       if ((threadIdx.x & 127) == 0) trace_event(p, 2 + wg, tr_cur, 44 + wg, it);
       if (ok && my_steps > 0) {

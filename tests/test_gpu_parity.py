@@ -353,6 +353,19 @@ def test_cuda_core_kernels_at_tile_edges(sb, cuda_device, d, dtype, mode):
         H.assert_parity(got, want, dtype, f"CUDA-core d={d} {mode} ac={ac}")
 
 
+@pytest.mark.parametrize("dtype,d", [(torch.bfloat16, 64), (torch.bfloat16, 128), (torch.float32, 32)])
+@pytest.mark.parametrize("lengths", [[1], [300, 0, 5] * 20, [7] * 128, [7] * 129, [40] * 120 + [900], [1100, 1] * 3, [1500, 1, 130, 300]])
+def test_item_tables_at_their_limits(sb, cuda_device, dtype, d, lengths):
+    """Packed batches around the limits up to which the kernels build their work tables themselves (128 sequences, 256
+    tiles), with empty sequences and tokens after the last one."""
+    tokens, cu = sum(lengths), cu_of(lengths)
+    q, k, v, do, drem = H.make_inputs((2, tokens + 9, d), dtype, seed=len(lengths) + d)
+    got = H.run_varlen(sb, q, k, v, do, drem, cu, cuda_device, max_seqlens=max(lengths))
+    want = H.oracle_varlen(*(t[:, :tokens] for t in (q, k, v, do, drem)), cu)
+    H.assert_parity([t[:, :tokens] for t in got], want, dtype, f"{len(lengths)} sequences, d={d}")
+    assert all((t[:, tokens:] == 0).all() for t in got)
+
+
 @pytest.mark.parametrize("ac", [False, True])
 @pytest.mark.parametrize("shape", [(2, 3, 256, 64), (1, 7, 500, 50), (2, 2, 512, 32), (1, 2, 300, 16),
                                    (1, 2, 1024, 128), (4, 1, 130, 128)])
