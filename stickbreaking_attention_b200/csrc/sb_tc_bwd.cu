@@ -34,85 +34,101 @@ namespace sb {
 // the chunk -- has underflowed to exactly 0 and the prefix of G is still exactly 0, for all 32 rows of the warp, every
 // A, G and dz of the chunk is exactly 0 (e, the reciprocals and dP - dR are finite): only the log-space sum is formed,
 // with the same operations as otherwise, and the rest is not computed.
-template <bool kMasked>
-__device__ __forceinline__ void bwd_row_chunk_values(const uint32_t (&s)[16], const uint32_t (&dp)[16], int mc0, int r, bool diag,
-                                                     int ac, bool row_valid, float scale2, float r1, float gpre, float dr,
-                                                     float &gs, float &logsum, float (&pa)[16], float (&pz)[16],
-                                                     bool skip_zero = false) {
+// Packed pairs (two fp32 per instruction) are used where a pair sits in adjacent registers anyway -- accumulator columns and
+// what is computed column by column from them.  Products across columns stay scalar: pairing their operands up costs as many
+// register moves as the packed instruction saves.
+struct BwdChunk {
+  float2 be01[4], be23[4];   // beta
+  float pa[16];              // A
+  bool zero;                 // the chunk is known to be zero for all rows of the warp
+};
+
+// Sweeps 1 and 2, which do not need dP; `between` runs where the fewest registers are in use and half of sweep 2 is left.
+template <bool kMasked, class Between>
+__device__ __forceinline__ void bwd_chunk_weights(const uint32_t (&s)[16], int mc0, int limit, float scale2, float r1, float g_before,
+                                                  float &logsum, BwdChunk &c, bool skip_zero, Between between) {
   float chunk_log = 0.f;   // summed per chunk, like the forward's (see fwd256_row_chunk): the two agree bit for bit
-  // columns (tile-local key indices) below `limit` are allowed: one compare per column, no branches
-  const int limit = !row_valid ? -1 : (diag ? r + ac : 0x7fffffff);
   const float2 sc = make_float2(scale2, scale2), one = make_float2(1.f, 1.f);
-  float2 e01[4], e23[4], be01[4], be23[4];
-  float rpg[4], q23[4], ri1[4], ri3[4];
-  float2 tt01[4], tt23[4], ppg[4];
+  float2 e01[4], e23[4], t01[4], t23[4];
 #pragma unroll
-  for (int g = 3; g >= 0; --g) {   // independent work in packed pairs (two fp32 per instruction)
+  for (int g = 3; g >= 0; --g) {
     const float2 x01 = mul2(make_float2(__uint_as_float(s[4 * g]), __uint_as_float(s[4 * g + 1])), sc);
     const float2 x23 = mul2(make_float2(__uint_as_float(s[4 * g + 2]), __uint_as_float(s[4 * g + 3])), sc);
     e01[g] = make_float2(ex2(fminf(x01.x, 30.f)), ex2(fminf(x01.y, 30.f)));
     e23[g] = make_float2(ex2(fminf(x23.x, 30.f)), ex2(fminf(x23.y, 30.f)));
-    float2 t01 = add2(e01[g], one), t23 = add2(e23[g], one);
+    t01[g] = add2(e01[g], one);
+    t23[g] = add2(e23[g], one);
     if (kMasked) {
       const int col = mc0 + 4 * g;
-      if (!(col < limit)) { e01[g].x = 0.f; t01.x = 1.f; }
-      if (!(col + 1 < limit)) { e01[g].y = 0.f; t01.y = 1.f; }
-      if (!(col + 2 < limit)) { e23[g].x = 0.f; t23.x = 1.f; }
-      if (!(col + 3 < limit)) { e23[g].y = 0.f; t23.y = 1.f; }
+      if (!(col < limit)) { e01[g].x = 0.f; t01[g].x = 1.f; }
+      if (!(col + 1 < limit)) { e01[g].y = 0.f; t01[g].y = 1.f; }
+      if (!(col + 2 < limit)) { e23[g].x = 0.f; t23[g].x = 1.f; }
+      if (!(col + 3 < limit)) { e23[g].y = 0.f; t23[g].y = 1.f; }
     }
-    const float2 pp = mul2(make_float2(t01.x, t23.x), make_float2(t01.y, t23.y));   // (t0 t1, t2 t3)
-    chunk_log += lg2(pp.x * pp.y);
-    tt01[g] = t01;
-    tt23[g] = t23;
-    ppg[g] = pp;
+    chunk_log += lg2((t01[g].x * t01[g].y) * (t23[g].x * t23[g].y));
   }
   logsum += chunk_log;
-  if (!kMasked && skip_zero && __all_sync(0xffffffffu, ex2(r1 + logsum) == 0.f && gpre + gs == 0.f)) {
+  c.zero = !kMasked && skip_zero && __all_sync(0xffffffffu, ex2(r1 + logsum) == 0.f && g_before == 0.f);
+  if (c.zero) {
 #pragma unroll
-    for (int i = 0; i < 16; ++i) { pa[i] = 0.f; pz[i] = 0.f; }
+    for (int i = 0; i < 16; ++i) c.pa[i] = 0.f;
+    between();
     return;
   }
+  float rpg[4], i23[4], ri1[4], ri3[4];
 #pragma unroll
   for (int g = 0; g < 4; ++g) {
-    const float2 t01 = tt01[g], t23 = tt23[g], pp = ppg[g];
-    const float rp = rcp(pp.x * pp.y);
-    const float2 ab = mul2(make_float2(rp, rp), make_float2(pp.y, pp.x));           // (1 / t0 t1, 1 / t2 t3)
-    const float2 ri01 = mul2(make_float2(ab.x, ab.x), make_float2(t01.y, t01.x));   // (1/t0, 1/t1)
-    const float2 ri23 = mul2(make_float2(ab.y, ab.y), make_float2(t23.y, t23.x));   // (1/t2, 1/t3)
-    be01[g] = mul2(e01[g], ri01);
-    be23[g] = mul2(e23[g], ri23);
+    const float p01 = t01[g].x * t01[g].y, p23 = t23[g].x * t23[g].y;
+    const float rp = rcp(p01 * p23);
+    const float i01 = rp * p23;                 // 1 / t0 t1
+    i23[g] = rp * p01;                          // 1 / t2 t3
+    const float2 ri01 = make_float2(i01 * t01[g].y, i01 * t01[g].x);
+    const float2 ri23 = make_float2(i23[g] * t23[g].y, i23[g] * t23[g].x);
+    c.be01[g] = mul2(e01[g], ri01);
+    c.be23[g] = mul2(e23[g], ri23);
     rpg[g] = rp;
-    q23[g] = ab.y;
     ri1[g] = ri01.y;
     ri3[g] = ri23.y;
   }
+  between();
   float wend = ex2(r1 + logsum);   // product of (1 - beta) over everything after the chunk
 #pragma unroll
   for (int g = 3; g >= 0; --g) {
-    const float2 w32 = mul2(make_float2(wend, wend), make_float2(ri3[g], q23[g]));   // inclusive products at columns 3, 2
-    const float w1 = w32.y * ri1[g];                                                  // at column 1
-    wend *= rpg[g];                                                                   // at column 0 = after the previous group
-    const float2 a01 = mul2(e01[g], make_float2(wend, w1));
-    const float2 a23 = mul2(e23[g], make_float2(w32.y, w32.x));
-    pa[4 * g] = a01.x;
-    pa[4 * g + 1] = a01.y;
-    pa[4 * g + 2] = a23.x;
-    pa[4 * g + 3] = a23.y;
+    const float2 w23 = make_float2(wend * i23[g], wend * ri3[g]);   // inclusive products at columns 2, 3
+    wend *= rpg[g];                                                  // at column 0 = after the previous group
+    const float2 w01 = make_float2(wend, w23.x * ri1[g]);
+    const float2 a01 = mul2(e01[g], w01);
+    const float2 a23 = mul2(e23[g], w23);
+    c.pa[4 * g] = a01.x;
+    c.pa[4 * g + 1] = a01.y;
+    c.pa[4 * g + 2] = a23.x;
+    c.pa[4 * g + 3] = a23.y;
+  }
+}
+
+// Sweep 3.  On entry `gs` is the pass's sum of G before the chunk; pz: dz.
+template <bool kMasked>
+__device__ __forceinline__ void bwd_chunk_dz(const uint32_t (&dp)[16], int mc0, int limit, float gpre, float dr, float &gs, BwdChunk &c,
+                                             float (&pz)[16]) {
+  if (!kMasked && c.zero) {
+#pragma unroll
+    for (int i = 0; i < 16; ++i) pz[i] = 0.f;
+    return;
   }
   const float2 ndr = make_float2(-dr, -dr);
   float cb = gpre + gs, csum = 0.f;   // C before the group; the chunk's own sum of G
 #pragma unroll
   for (int g = 0; g < 4; ++g) {
-    float2 g01 = mul2(make_float2(pa[4 * g], pa[4 * g + 1]),
+    float2 g01 = mul2(make_float2(c.pa[4 * g], c.pa[4 * g + 1]),
                       add2(make_float2(__uint_as_float(dp[4 * g]), __uint_as_float(dp[4 * g + 1])), ndr));
-    float2 g23 = mul2(make_float2(pa[4 * g + 2], pa[4 * g + 3]),
+    float2 g23 = mul2(make_float2(c.pa[4 * g + 2], c.pa[4 * g + 3]),
                       add2(make_float2(__uint_as_float(dp[4 * g + 2]), __uint_as_float(dp[4 * g + 3])), ndr));
     if (kMasked) {   // rows past the sequence end carry arbitrary values: select, do not rely on 0 * x
       const int col = mc0 + 4 * g;
-      if (!(col < limit)) { g01.x = 0.f; pa[4 * g] = 0.f; }
-      if (!(col + 1 < limit)) { g01.y = 0.f; pa[4 * g + 1] = 0.f; }
-      if (!(col + 2 < limit)) { g23.x = 0.f; pa[4 * g + 2] = 0.f; }
-      if (!(col + 3 < limit)) { g23.y = 0.f; pa[4 * g + 3] = 0.f; }
+      if (!(col < limit)) { g01.x = 0.f; c.pa[4 * g] = 0.f; }
+      if (!(col + 1 < limit)) { g01.y = 0.f; c.pa[4 * g + 1] = 0.f; }
+      if (!(col + 2 < limit)) { g23.x = 0.f; c.pa[4 * g + 2] = 0.f; }
+      if (!(col + 3 < limit)) { g23.y = 0.f; c.pa[4 * g + 3] = 0.f; }
     }
     const float t1 = g01.x + g01.y, t23 = g23.x + g23.y;
     const float tg = t1 + t23;
@@ -120,150 +136,187 @@ __device__ __forceinline__ void bwd_row_chunk_values(const uint32_t (&s)[16], co
     const float c2v = c1v + g23.x;
     cb += tg;
     csum += tg;
-    const float2 z01 = fma2(make_float2(-be01[g].x, -be01[g].y), make_float2(c0v, c1v), g01);
-    const float2 z23 = fma2(make_float2(-be23[g].x, -be23[g].y), make_float2(c2v, cb), g23);
-    pz[4 * g] = z01.x;
-    pz[4 * g + 1] = z01.y;
-    pz[4 * g + 2] = z23.x;
-    pz[4 * g + 3] = z23.y;
+    pz[4 * g] = fmaf(-c.be01[g].x, c0v, g01.x);
+    pz[4 * g + 1] = fmaf(-c.be01[g].y, c1v, g01.y);
+    pz[4 * g + 2] = fmaf(-c.be23[g].x, c2v, g23.x);
+    pz[4 * g + 3] = fmaf(-c.be23[g].y, cb, g23.y);
     if (kMasked) {
 #pragma unroll
-      for (int i = 0; i < 4; ++i) pz[4 * g + i] = row_valid ? pz[4 * g + i] : 0.f;
+      for (int i = 0; i < 4; ++i) pz[4 * g + i] = limit >= 0 ? pz[4 * g + i] : 0.f;
     }
   }
   gs += csum;
 }
 
-// The same, written to the 16-bit A (optional) and dz tiles; c0 addresses the output tile.
-template <bool kFp16, bool kStoreA, bool kMasked>
-__device__ __forceinline__ void bwd_row_chunk(const uint32_t (&s)[16], const uint32_t (&dp)[16], int c0, int mc0, int r, bool diag,
-                                              int ac, bool row_valid, float scale2, float r1, float gpre, float dr,
-                                              float &gs, float &logsum, uint8_t *tile_a, uint8_t *tile_z,
-                                              bool skip_zero = false) {
-  float pa[16], pz[16];
-  bwd_row_chunk_values<kMasked>(s, dp, mc0, r, diag, ac, row_valid, scale2, r1, gpre, dr, gs, logsum, pa, pz, skip_zero);
-  if constexpr (kStoreA) store_row_chunk16<kFp16>(tile_a, r, c0, pa);
+// columns (tile-local key indices) below the limit are allowed: one compare per column, no branches
+__device__ __forceinline__ int chunk_limit(bool row_valid, bool diag, int r, int ac) {
+  return !row_valid ? -1 : (diag ? r + ac : 0x7fffffff);
+}
+
+// All three sweeps, A and dz written to the 16-bit tiles; c0 addresses the output tiles.
+template <bool kFp16, bool kMasked>
+__device__ __forceinline__ void bwd_row_chunk(const uint32_t (&s)[16], const uint32_t (&dp)[16], int c0, int mc0, int r, int limit,
+                                              float scale2, float r1, float gpre, float dr, float &gs, float &logsum, uint8_t *tile_a,
+                                              uint8_t *tile_z, bool skip_zero = false) {
+  BwdChunk c;
+  float pz[16];
+  bwd_chunk_weights<kMasked>(s, mc0, limit, scale2, r1, gpre + gs, logsum, c, skip_zero, [] {});
+  bwd_chunk_dz<kMasked>(dp, mc0, limit, gpre, dr, gs, c, pz);
+  store_row_chunk16<kFp16>(tile_a, r, c0, c.pa);
   store_row_chunk16<kFp16>(tile_z, r, c0, pz);
 }
 
-// One row of a 64-key strip: four 16-column chunks, TMEM read one chunk ahead.  mc0: key index of the strip's first
-// column inside its 128-key tile (for the diagonal mask).  empty_bar (optional) is signalled, one arrival per warp,
-// once the last S/dP columns are in registers; gate_bar (optional) is waited for before the first store to the
-// output tiles, i.e. after the first chunk's arithmetic.  az_a / az_z (optional): this row's 64 values of the stored
-// A and dz tiles in global memory (plain row-major, 16-bit), written next to the shared-memory dz tile (the caller may
-// instead copy the finished dz tile out of shared memory).
-// Returns false if the gate wait gave up.
-template <bool kFp16, bool kStoreA, bool kMasked>
-__device__ __forceinline__ bool strip_row_pass(uint32_t ts, uint32_t tp, int r, int mc0, bool diag, int ac, bool row_valid,
-                                              float scale2, float r1, float gpre, float dr, float &gs, float &logsum,
-                                              uint8_t *tile_a, uint8_t *tile_z, float *mid_r1 = nullptr,
-                                              float *mid_s2 = nullptr, uint32_t empty_bar = 0, uint32_t gate_bar = 0,
-                                              uint32_t gate_parity = 0, unsigned short *az_a = nullptr,
-                                              unsigned short *az_z = nullptr, bool skip_zero = false) {
-  uint32_t s0[16], d0[16], s1[16], d1[16];
+// One row of a 64-key sub-tile of the dq kernel: four 16-column chunks.  What a pair of chunks still needs is requested
+// together in the first one's sweep 2, the second chunk's dP into the registers of the first one's scores, so that 48
+// registers do for everything in flight, and the last S and dP columns are in registers after two thirds of the pass:
+// bSpEmpty is signalled then (one arrival per warp), and the next sub-tile's scores are computed under the rest.  dP is not
+// waited for before half of the first chunk is done.
+// mc0: key index of the sub-tile's first column inside its 128-key tile (for the diagonal mask).  The dz tile of the
+// sub-tile before is waited for before the first store to it (in a tile's first sub-tile, an even one, that is the phase
+// before the barrier's first: no wait).  Returns false if a wait gave up.
+namespace dq2 {
+constexpr int kMaxStages = 4;
+enum { bQG = 0, bKvFull = 1, bKvEmpty = bKvFull + kMaxStages, bSFull = bKvEmpty + kMaxStages, bDpFull = bSFull + 2, bZFull = bDpFull + 2,
+       bZEmpty = bZFull + 2, bFirst = bZEmpty + 2, bSpEmpty = bFirst + 1, bDqFull = bSpEmpty + 2, bNum = bDqFull + 2 };
+}  // namespace dq2
+// `bars`: the dq kernel's barriers, offset by the tile's number.  out: stored-tiles mode: this row's 64 values of A in the
+// workspace; otherwise this row's record of R1 at the sub-tile's first key (S2 is `s2_off` floats further, both again kBM
+// floats further for the key 32 columns on).
+template <bool kFp16, bool kMasked, bool kStored>
+__device__ __forceinline__ bool strip_row_pass(uint32_t ts, uint32_t tp, int r, int u, int mc0, int limit, float scale2, float r1, float gpre,
+                                              float dr, float &gs, float &logsum, uint8_t *tile_z, uint32_t bars, void *out,
+                                              long long s2_off, bool skip_zero = false) {
+  uint32_t s0[16], s1[16], d[16];
   bool ok = true;
+  auto store = [&](int c0, const BwdChunk &c, const float (&pz)[16]) {
+    uint32_t wz[8];
+    pack_row_chunk16<kFp16>(pz, wz);
+    store_packed_chunk16(tile_z, r, c0, wz);
+    if constexpr (kStored) {
+      uint32_t wa[8];
+      pack_row_chunk16<kFp16>(c.pa, wa);
+      store_packed_global16(reinterpret_cast<unsigned short *>(out) + c0, wa);
+    }
+  };
   tmem_ld16(ts, s0);
-  tmem_ld16(tp, d0);
 #pragma unroll 1
   for (int pair = 0; pair < 2; ++pair) {
     const int c0 = pair * 32;
-    tmem_wait_ld_regs(s0, d0);
-    tmem_ld16(ts + c0 + 16, s1);
-    tmem_ld16(tp + c0 + 16, d1);
+    tmem_wait_ld_regs(s0);
     {
-      float pa[16], pz[16];
-      bwd_row_chunk_values<kMasked>(s0, d0, mc0 + c0, r, diag, ac, row_valid, scale2, r1, gpre, dr, gs, logsum, pa, pz, skip_zero);
-      if (pair == 0 && gate_bar != 0) {
-        ok = mbar_wait(gate_bar, gate_parity);
+      BwdChunk c;
+      bwd_chunk_weights<kMasked>(s0, mc0 + c0, limit, scale2, r1, gpre + gs, logsum, c, skip_zero, [&] {
+        if (pair == 0) {
+          ok = mbar_wait(bars + 8u * dq2::bDpFull, u & 1);
+          tc_fence_after();
+        }
+        tmem_ld16(tp + c0, d);
+        tmem_ld16(ts + c0 + 16, s1);
+        tmem_ld16(tp + c0 + 16, s0);
+      });
+      tmem_wait_ld_regs(d, s0);
+      asm volatile("" : "+r"(s1[0]), "+r"(s1[1]), "+r"(s1[2]), "+r"(s1[3]), "+r"(s1[4]), "+r"(s1[5]), "+r"(s1[6]), "+r"(s1[7]), "+r"(s1[8]),
+                   "+r"(s1[9]), "+r"(s1[10]), "+r"(s1[11]), "+r"(s1[12]), "+r"(s1[13]), "+r"(s1[14]), "+r"(s1[15])::"memory");
+      if (pair == 0) {
+        ok = mbar_wait(bars + 8u * dq2::bZEmpty, (u + 1) & 1) && ok;   // the previous sub-tile's dz has been read
         tc_fence_after();
+      } else {               // the last columns are in registers: the S / dP slots can be overwritten
+        tc_fence_before();
+        __syncwarp();
+        if ((threadIdx.x & 31) == 0) mbar_arrive(bars + 8u * dq2::bSpEmpty);
       }
-      if constexpr (kStoreA) store_row_chunk16<kFp16>(tile_a, r, c0, pa);
-      uint32_t wz[8];
-      pack_row_chunk16<kFp16>(pz, wz);
-      store_packed_chunk16(tile_z, r, c0, wz);
-      if (az_a != nullptr) {
-        uint32_t wa[8];
-        pack_row_chunk16<kFp16>(pa, wa);
-        store_packed_global16(az_a + c0, wa);
-        if (az_z != nullptr) store_packed_global16(az_z + c0, wz);
-      }
+      float pz[16];
+      bwd_chunk_dz<kMasked>(d, mc0 + c0, limit, gpre, dr, gs, c, pz);
+      store(c0, c, pz);
     }
-    tmem_wait_ld_regs(s1, d1);
+    {
+      BwdChunk c;
+      float pz[16];
+      bwd_chunk_weights<kMasked>(s1, mc0 + c0 + 16, limit, scale2, r1, gpre + gs, logsum, c, skip_zero, [] {});
+      bwd_chunk_dz<kMasked>(s0, mc0 + c0 + 16, limit, gpre, dr, gs, c, pz);
+      store(c0 + 16, c, pz);
+    }
     if (pair == 0) {
       tmem_ld16(ts + 32, s0);
-      tmem_ld16(tp + 32, d0);
-    } else if (empty_bar != 0) {   // the last columns are in registers: the S/dP slots can be overwritten
-      tc_fence_before();
-      __syncwarp();
-      if ((threadIdx.x & 31) == 0) mbar_arrive(empty_bar);
-    }
-    {
-      float pa[16], pz[16];
-      bwd_row_chunk_values<kMasked>(s1, d1, mc0 + c0 + 16, r, diag, ac, row_valid, scale2, r1, gpre, dr, gs, logsum, pa, pz, skip_zero);
-      if constexpr (kStoreA) store_row_chunk16<kFp16>(tile_a, r, c0 + 16, pa);
-      uint32_t wz[8];
-      pack_row_chunk16<kFp16>(pz, wz);
-      store_packed_chunk16(tile_z, r, c0 + 16, wz);
-      if (az_a != nullptr) {
-        uint32_t wa[8];
-        pack_row_chunk16<kFp16>(pa, wa);
-        store_packed_global16(az_a + c0 + 16, wa);
-        if (az_z != nullptr) store_packed_global16(az_z + c0 + 16, wz);
+      if constexpr (!kStored) {   // the carried values after 32 of the 64 columns
+        float *rec = reinterpret_cast<float *>(out) + kBM;
+        rec[0] = r1 + logsum;
+        rec[s2_off] = gpre + gs;
       }
-    }
-    if (pair == 0 && mid_r1 != nullptr) {   // the carried values after 32 of the 64 columns
-      *mid_r1 = r1 + logsum;
-      *mid_s2 = gpre + gs;
     }
   }
   return ok;
 }
 
-// The same for a strip before the first key of the warp's rows: dz (and the stored A) are zeros, the scores are not read.
-__device__ __forceinline__ void zero_strip_row(uint8_t *tile_z, int r, unsigned short *az_a, uint32_t empty_bar) {
+// What is recorded as R1 (a log2) where a row has not started: the product is 0, and so is all that follows from it.
+constexpr float kNothingLeft = -1e6f;
+
+// The same for a sub-tile before the first key of the warp's rows: dz (and the stored A) are zeros, the scores are not read.
+template <bool kStored>
+__device__ __forceinline__ bool zero_strip_row(uint8_t *tile_z, int r, int u, uint32_t bars, void *out, long long s2_off) {
   const uint32_t z[8] = {0u, 0u, 0u, 0u, 0u, 0u, 0u, 0u};
+  const bool ok = mbar_wait(bars + 8u * dq2::bDpFull, u & 1) && mbar_wait(bars + 8u * dq2::bZEmpty, (u + 1) & 1);   // (every phase is followed)
 #pragma unroll
   for (int c = 0; c < 64; c += 16) {
     store_packed_chunk16(tile_z, r, c, z);
-    if (az_a != nullptr) store_packed_global16(az_a + c, z);
+    if constexpr (kStored) store_packed_global16(reinterpret_cast<unsigned short *>(out) + c, z);
+  }
+  if constexpr (!kStored) {
+    float *rec = reinterpret_cast<float *>(out) + kBM;
+    rec[0] = kNothingLeft;
+    rec[s2_off] = 0.f;
   }
   __syncwarp();
-  if ((threadIdx.x & 31) == 0) mbar_arrive(empty_bar);
+  if ((threadIdx.x & 31) == 0) mbar_arrive(bars + 8u * dq2::bSpEmpty);
+  return ok;
 }
-// What is recorded as R1 (a log2) for such a strip: the product it starts a row with is 0, and so is all that follows.
-constexpr float kNothingLeft = -1e6f;
 
 // =======================================================================================================
-// dq kernel for head sizes 72..128: 256 query rows per CTA
+// dq kernel: 256 query rows per CTA
 // =======================================================================================================
-// Two adjacent 128-row query tiles (a, b) share one stream of 64-key K/V sub-tiles, walked from the sequence start
-// to tile b's diagonal.  Each tile has its own row-owning warpgroup (warps 0-3 / 4-7), MMA issuer (warps 9 / 10),
+// Two adjacent 128-row query tiles (a, b) share one stream of 64-key K/V sub-tiles, walked from the first key their rows
+// reach to tile b's diagonal.  Each tile has its own row-owning warpgroup (warps 0-3 / 4-7), MMA issuer (warps 9 / 10),
 // S/dP slots and dQ accumulator in TMEM and dz tile in shared memory.  Per sub-tile and tile: S = Q K^T and
 // dP = dO V^T (128 x 64), the row pass (which also records R1/S2 at the sub-tile's first key, i.e. at keys 0 and 64
 // of every 128-key tile), then dQ += dz K.
 // TMEM columns: S_a 0, dP_a 64, S_b 128, dP_b 192, dQ_a 256, dQ_b 384.
+// What bounds it: the row arithmetic (~2700 clk per sub-tile of both tiles in isolation, ~4200 here) and the MMAs'
+// shared-memory operand traffic (~80 clk per 128 x 64 x 16 instruction, ~3300 clk at 128 columns), so the two have to
+// overlap although S and dP fill all the tensor memory there is and cannot be double-buffered: rows start on S alone, dP
+// has until the middle of the first chunk, and both slots are handed back after two thirds of the pass (see strip_row_pass).
 namespace dq2 {
 constexpr int kThreads = 352;
 constexpr int kBN = 64;
-constexpr int kStages = 2;
-constexpr int kTileBytes = kBM * 128 * 2;      // Q or dO tile
 constexpr int kKvBox = kBN * 64 * 2;           // 64 keys x 64 columns
-constexpr int kKvTile = 2 * kKvBox;            // K or V sub-tile
-constexpr int kStageBytes = 2 * kKvTile;
 constexpr int kZBytes = kBM * kBN * 2;         // dz tile: 128 rows x 64 keys
-static_assert(kStages == 2, "stage = sub-tile mod 2");
-constexpr int kSmem = 1024 + 4 * kTileBytes + kStages * kStageBytes + 2 * kZBytes + 512 + (int)sizeof(SmallTable);
-static_assert(kSmem <= 232448, "shared memory per block");
-enum { bQG = 0, bKvFull = 1, bKvEmpty = 3, bSpFull = 5, bZFull = 7, bZEmpty = 9, bFirst = 11, bSpEmpty = 12, bDqFull = 14, bNum = 16 };
+template <int D>                               // head size rounded up to 64 or 128
+struct Cfg {
+  static constexpr int kBoxes = D / 64;
+  static constexpr int kTileBytes = kBoxes * kBoxBytes;   // Q or dO tile
+  static constexpr int kKvTile = kBoxes * kKvBox;         // K or V sub-tile
+  static constexpr int kStageBytes = 2 * kKvTile;
+  static constexpr int kStages = D == 64 ? 4 : 2;         // what shared memory holds
+  static constexpr int kSmem = 1024 + 4 * kTileBytes + kStages * kStageBytes + 2 * kZBytes + 512 + (int)sizeof(SmallTable);
+  static_assert(kSmem <= 232448, "shared memory per block");
+};
+// What the rows need again after their loop, kept out of their registers meanwhile.
+struct Shared {
+  Ctl ctl;
+  int first;     // the sub-tile in stage 0
+  int h, hh, len, idx;
+  long long tok0, boff, pair0;
+};
+static_assert(bNum * 8 + sizeof(Shared) <= 512, "barriers and control words");
 }  // namespace dq2
 
-template <bool kFp16>
+template <int D, bool kFp16, bool kStored>
 __global__ void __launch_bounds__(dq2::kThreads, 1)
 tc_bwd_dq2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                   const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_g,
                   const __grid_constant__ CUtensorMap tm_dq, const __grid_constant__ CUtensorMap tm_az, const KParams p) {
   using namespace dq2;
-  constexpr int D = 128;
+  using C = Cfg<D>;
+  constexpr int kTileBytes = C::kTileBytes, kKvTile = C::kKvTile, kStageBytes = C::kStageBytes, kStages = C::kStages, kBoxes = C::kBoxes;
   extern __shared__ uint8_t smem_raw[];
   if (threadIdx.x == 0) trace_block(p, 0);
   const uint32_t raw = smem_u32(smem_raw);
@@ -282,7 +335,8 @@ tc_bwd_dq2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
   if (refused || !decode_block(p, tb, 2, true, c, hh_blk)) return;   // c.idx: the even tile of the pair (idx, idx + 1)
   const int Ia = c.idx;
   const bool b_active = Ia + 1 < c.n_tiles;
-  Ctl *ctl = reinterpret_cast<Ctl *>(gbase + (sBar - base) + bNum * 8);
+  Shared *sh = reinterpret_cast<Shared *>(gbase + (sBar - base) + bNum * 8);
+  Ctl *ctl = &sh->ctl;
   volatile int *abort_flag = &ctl->abort;
   auto bar = [&](int i) { return sBar + 8u * i; };
 
@@ -304,14 +358,17 @@ tc_bwd_dq2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
     mbar_init(bar(bFirst), 1);
     for (int s = 0; s < kStages; ++s) { mbar_init(bar(bKvFull + s), 1); mbar_init(bar(bKvEmpty + s), issuers); }
     for (int w = 0; w < 2; ++w) {
-      mbar_init(bar(bSpFull + w), 1);
+      mbar_init(bar(bSFull + w), 1);
+      mbar_init(bar(bDpFull + w), 1);
       mbar_init(bar(bZFull + w), 4);
-      mbar_init(bar(bZEmpty + w), 1);
+      mbar_init(bar(bZEmpty + w), kStored ? 2 : 1);   // the dQ MMAs have read the dz tile, and it has left for the workspace
       mbar_init(bar(bSpEmpty + w), 4);
     }
     mbar_init(bar(bDqFull), 1);
     mbar_init(bar(bDqFull + 1), 1);
     ctl->abort = 0;
+    sh->first = first; sh->h = h; sh->hh = hh; sh->len = c.len; sh->idx = Ia;
+    sh->tok0 = c.tok0; sh->boff = c.boff; sh->pair0 = c.pair0;
     fence_barrier_init();
   }
   if (warp == 9) {
@@ -329,7 +386,7 @@ tc_bwd_dq2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
       const int qrow = (int)c.tok0 + Ia * kBM;
       mbar_arrive_expect_tx(bar(bQG), 4 * kTileBytes);
       for (int w = 0; w < 2; ++w)
-        for (int kb = 0; kb < 2; ++kb) {
+        for (int kb = 0; kb < kBoxes; ++kb) {
           tma_load_4d(sQ + w * 2 * kTileBytes + kb * kBoxBytes, &tm_q, bar(bQG), kb * 64, qrow + w * kBM, h, (int)c.boff);
           tma_load_4d(sQ + w * 2 * kTileBytes + kTileBytes + kb * kBoxBytes, &tm_g, bar(bQG), kb * 64, qrow + w * kBM, h, (int)c.boff);
         }
@@ -340,7 +397,7 @@ tc_bwd_dq2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
         const int krow = (int)c.tok0 + (first + t) * kBN;
         const uint32_t dst = sKV + st * kStageBytes;
         mbar_arrive_expect_tx(bar(bKvFull + st), kStageBytes);
-        for (int kb = 0; kb < 2; ++kb) {
+        for (int kb = 0; kb < kBoxes; ++kb) {
           tma_load_4d(dst + kb * kKvBox, &tm_k, bar(bKvFull + st), kb * 64, krow, h, (int)c.boff);
           tma_load_4d(dst + kKvTile + kb * kKvBox, &tm_v, bar(bKvFull + st), kb * 64, krow, h, (int)c.boff);
         }
@@ -358,11 +415,13 @@ tc_bwd_dq2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
       const int n_stages = n_steps - first;
       const int t_first = (w == 0 ? first_a : first_b) - first, t_end = (w == 0 ? steps_a : steps_b) - first;
       const int my_steps = t_end - t_first;
+      const int z_row = (int)((c.pair0 + (long long)(Ia + w) * (Ia + w + 1) / 2) * kBM);   // of the stored dz tiles
       auto issue_sp = [&](int u) {
         const uint32_t kaddr = sKV + ((t_first + u) % kStages) * kStageBytes;
         mma_kmajor_kmajor<D, kBoxBytes, kKvBox>(tS, qaddr, kaddr, idesc_s, false);            // S = Q K^T
+        mma_commit(bar(bSFull + w));
         mma_kmajor_kmajor<D, kBoxBytes, kKvBox>(tP, gaddr, kaddr + kKvTile, idesc_s, false);  // dP = dO V^T
-        mma_commit(bar(bSpFull + w));
+        mma_commit(bar(bDpFull + w));
       };
       bool ok = true;
       // stages the tile does not read are released on its behalf once they have arrived
@@ -403,9 +462,19 @@ tc_bwd_dq2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
         mma_kmajor_mnmajor<kBN, kKvBox>(tDQ, zaddr, sKV + ((t_first + u) % kStages) * kStageBytes, idesc_dq, u > 0);
         mma_commit(bar(bZEmpty + w));
         mma_commit(bar(bKvEmpty + (t_first + u) % kStages));
+        if constexpr (kStored) {
+          // The dz tile also leaves for the workspace.  (Issued by the row warps, 32 rows each, these stores held every one of
+          // them up for ~900 clk a step; this thread has nothing to do before two thirds of the next pass.)
+          const int ub = u + (w == 0 ? first_a : first_b);   // sub-tile inside the sequence
+          tma_store_4d(&tm_az, zaddr, (ub & 1) * kBN, z_row + (ub >> 1) * kBM, 1, hh);
+          tma_store_commit();
+          tma_store_wait_read();
+          mbar_arrive(bar(bZEmpty + w));
+        }
       }
       if (ok) mma_commit(bar(bDqFull + w));   // this tile's dQ is complete: its rows store it while the other tile goes on
       release(t_end, n_stages);   // tile a does not read the last sub-tiles
+      if constexpr (kStored) tma_store_wait_all();
     }
   } else {
     // ------------------------------------------------ rows: warpgroup w owns query tile Ia + w
@@ -414,111 +483,96 @@ tc_bwd_dq2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
     const int r = threadIdx.x & 127;
     const uint32_t lane_off = (uint32_t)((warp & 3) * 32) << 16;
     const float scale2 = p.scale * kLog2e;
-    const int I = Ia + w;
+    const volatile Shared &item = *sh;
+    const int I = Ia + w, row0 = I * kBM;
     const int my_steps = w == 0 ? steps_a : steps_b;
-    const int gi = I * kBM + r;
-    const bool valid = gi < c.len;
-    const long long idx = (c.boff * p.heads + h) * p.tokens + c.tok0 + gi;
-    double r1 = (valid && my_steps > 0) ? p.log_rem[idx] : 0.0;   // sum of log2(1-beta) over the keys from the current one on
-    const float dr = (valid && my_steps > 0) ? load_drem<T>(p, idx) : 0.f;
-    float gpre = 0.f;
+    const bool valid = row0 + r < c.len;
+    const long long idx = (c.boff * p.heads + h) * p.tokens + c.tok0 + row0 + r;
+    // sum of log2(1 - beta) over the keys from the current sub-tile on, as an unevaluated pair (see LogSum in the forward)
+    float r1 = 0.f, r1_lo = 0.f, dr = 0.f, gpre = 0.f;
+    if (valid && my_steps > 0) {
+      const double total = p.log_rem[idx];
+      r1 = (float)total;
+      r1_lo = (float)(total - (double)r1);
+      dr = load_drem<T>(p, idx);
+    }
     uint8_t *gZ = gbase + (sZ - base) + w * kZBytes;
     const uint32_t tS = tmem + w * 128 + lane_off, tP = tS + 64;
-    // boundary records: [pair (I, J)][half][row]; sub-tile u is half u & 1 of key tile u >> 1
-    const long long rec0 = ((long long)hh * p.pairs_cap + c.pair0 + (long long)I * (I + 1) / 2) * (4 * kBM) + r;
-    const bool ragged = I * kBM + kBM > c.len;   // the sequence ends inside this tile
-    bool ok = true;
+    const uint32_t bars = sBar + 8u * w;
+    // this row's part of the workspace for sub-tile 0: A, or the boundary records [pair (I, J)][quarter of the key tile][row]
+    const long long pair00 = (long long)(kStored ? 2 * hh : hh) * p.pairs_cap + c.pair0 + (long long)I * (I + 1) / 2;
+    char *out = kStored ? reinterpret_cast<char *>(p.az + (pair00 * kBM + r) * kBM) : reinterpret_cast<char *>(p.bnd_r1 + pair00 * (4 * kBM) + r);
+    const bool ragged = row0 + kBM > c.len;      // the sequence ends inside this tile
+    const int u_diag = 2 * I, u_tail = c.len / kBN;   // a sub-tile with rows past the sequence is number u_tail
     // this warp's rows start at sub-tile u_warp (never, if they are past the sequence): before it, A and dz are zeros
-    const int u_warp = (gi & ~31) < c.len ? first_key(p, c, h, gi & ~31) / kBN : 0x7fffffff;
-    // u: 64-key sub-tile inside the sequence; the first one is even, so that phases and stages follow from u alone
+    const int u_warp = row0 + (r & ~31) < c.len ? first_key(p, c, h, row0 + (r & ~31)) / kBN : 0x7fffffff;
+    bool ok = true;
+    // u: 64-key sub-tile inside the sequence; the first one is even, so that phases follow from u alone
     for (int u = w == 0 ? first_a : first_b; u < my_steps && ok; ++u) {
-      ok = wait_or_abort(bar(bSpFull + w), u & 1, abort_flag, p, 530);
+      ok = wait_or_abort(bars + 8u * bSFull, u & 1, abort_flag, p, 530);
       if (!ok) break;
       if (r == 0) trace_event(p, 2 + w, tr_cur, 4 + 16 * w, u);
       tc_fence_after();
-      // the dz tile is still being read by the previous step's dQ MMAs: waited for inside the pass, before its first store
-      // (in the tile's first step parity 1 is the phase before the barrier's first: no wait)
-      const uint32_t gate = bar(bZEmpty + w), gate_parity = (u + 1) & 1;
-      const float r1f = (float)r1;
+      const float r1f = r1 + r1_lo;
       float gs = 0.f, logsum = 0.f;
       bool pass_ok;
       // a tile with rows past the sequence end takes the masking variant throughout: those rows must be zero in the
       // stored tiles (the dK/dV GEMMs sum over all 128 query rows)
-      const bool on_diag = u >= 2 * I;
-      if (p.az != nullptr) {
-        // stored-tiles mode: this row's 64 values of A and dz for key tile u >> 1, half u & 1
-        const long long pair = c.pair0 + (long long)I * (I + 1) / 2 + (u >> 1);
-        unsigned short *az_a = p.az + ((((long long)hh * 2) * p.pairs_cap + pair) * kBM + r) * kBM + (u & 1) * kBN;
-        unsigned short *az_z = nullptr;   // the dz tile leaves by TMA below
-        // this warp's copy of the previous step's dz rows has left shared memory before they are rewritten
-        if (lane == 0) tma_store_wait_read();
-        __syncwarp();
-        if (u < u_warp) {
-          pass_ok = mbar_wait(gate, gate_parity);
-          zero_strip_row(gZ, r, az_a, bar(bSpEmpty + w));
-        } else if (on_diag || ragged)
-          pass_ok = strip_row_pass<kFp16, false, true>(tS, tP, r, on_diag ? (u - 2 * I) * kBN : 0, on_diag, p.attend_current, valid,
-                                                       scale2, r1f, gpre, dr, gs, logsum, nullptr, gZ, nullptr, nullptr,
-                                                       bar(bSpEmpty + w), gate, gate_parity, az_a, az_z);
-        else
-          pass_ok = strip_row_pass<kFp16, false, false>(tS, tP, r, 0, false, 0, true, scale2, r1f, gpre, dr, gs, logsum, nullptr, gZ,
-                                                        nullptr, nullptr, bar(bSpEmpty + w), gate, gate_parity, az_a, az_z, !p.dense);
+      const bool on_diag = u >= u_diag;
+      void *dst;
+      long long s2_off = 0;
+      if constexpr (kStored) {
+        dst = out + ((long long)(u >> 1) * (kBM * kBM) + (u & 1) * kBN) * 2;
       } else {
-        float *rec_r1 = p.bnd_r1 + rec0 + (long long)u * (2 * kBM);   // quarter 2 (u & 1) of key tile u >> 1
-        float *rec_s2 = p.bnd_s2 + rec0 + (long long)u * (2 * kBM);
-        rec_r1[0] = u < u_warp ? kNothingLeft : r1f;
-        rec_s2[0] = gpre;
-        if (u < u_warp) {
-          rec_r1[kBM] = kNothingLeft;
-          rec_s2[kBM] = 0.f;
-          pass_ok = mbar_wait(gate, gate_parity);
-          zero_strip_row(gZ, r, nullptr, bar(bSpEmpty + w));
-        } else if (on_diag)
-          pass_ok = strip_row_pass<kFp16, false, true>(tS, tP, r, (u - 2 * I) * kBN, true, p.attend_current, true, scale2, r1f, gpre,
-                                                       dr, gs, logsum, nullptr, gZ, rec_r1 + kBM, rec_s2 + kBM, bar(bSpEmpty + w),
-                                                       gate, gate_parity);
-        else
-          pass_ok = strip_row_pass<kFp16, false, false>(tS, tP, r, 0, false, 0, true, scale2, r1f, gpre, dr, gs, logsum, nullptr, gZ,
-                                                        rec_r1 + kBM, rec_s2 + kBM, bar(bSpEmpty + w), gate, gate_parity, nullptr,
-                                                        nullptr, !p.dense);
+        dst = out + (long long)u * (2 * kBM * sizeof(float));
+        s2_off = p.bnd_s2 - p.bnd_r1;
+        reinterpret_cast<float *>(dst)[0] = u < u_warp ? kNothingLeft : r1f;
+        reinterpret_cast<float *>(dst)[s2_off] = gpre;
       }
-      if (!pass_ok) {   // the bounded wait inside the pass gave up
+      if (u < u_warp)
+        pass_ok = zero_strip_row<kStored>(gZ, r, u, bars, dst, s2_off);
+      else if (on_diag || (kStored && ragged))
+        pass_ok = strip_row_pass<kFp16, true, kStored>(tS, tP, r, u, on_diag ? (u - u_diag) * kBN : 0,
+                                                       chunk_limit(valid || !kStored, on_diag, r, p.attend_current), scale2, r1f, gpre, dr,
+                                                       gs, logsum, gZ, bars, dst, s2_off);
+      else
+        pass_ok = strip_row_pass<kFp16, false, kStored>(tS, tP, r, u, 0, 0, scale2, r1f, gpre, dr, gs, logsum, gZ, bars, dst, s2_off, !p.dense);
+      if (!pass_ok) {   // a bounded wait inside the pass gave up
         *abort_flag = 1;
         if (p.status != nullptr) { p.status[0] = SB_DEV_WAIT_TIMEOUT; p.status[1] = 531; }
         ok = false;
       }
-      r1 += (double)logsum;
+      {   // r1 += logsum
+        const float sum = r1 + logsum, b = sum - r1;
+        r1_lo += (r1 - (sum - b)) + (logsum - b);
+        r1 = sum;
+      }
       gpre += gs;
       // the sequence ends inside this sub-tile: its dz columns behind the end are exact zeros, the K rows there are
       // not this sequence's (see zero_tile_rows) and are cleared before this step's dz K MMA is released
-      if (c.len - u * kBN < kBN)
-        zero_tile_rows(gbase + (sKV - base) + (u & 1) * kStageBytes, c.len - u * kBN, kBN, 2, kKvBox, r, kBM);
+      if (u == u_tail)
+        zero_tile_rows(gbase + (sKV - base) + ((u - item.first) % kStages) * kStageBytes, item.len - u * kBN, kBN, kBoxes, kKvBox, r, kBM);
       tc_fence_before();          // this step's TMEM reads are done before the slots are handed back
       fence_proxy_async_smem();
       __syncwarp();
       if (r == 0) trace_event(p, 2 + w, tr_cur, 5 + 16 * w, u);
-      if (lane == 0) {
-        mbar_arrive(bar(bZFull + w));
-        if (p.az != nullptr) {   // stored-tiles mode: this warp's 32 rows x 64 keys of dz, out of the shared-memory tile
-          const long long pair = c.pair0 + (long long)I * (I + 1) / 2 + (u >> 1);
-          tma_store_4d(&tm_az, sZ + w * kZBytes + (warp & 3) * 32 * 128, (u & 1) * kBN, (int)(pair * kBM) + (warp & 3) * 32, 1, hh);
-          tma_store_commit();
-        }
-      }
+      if (lane == 0) mbar_arrive(bars + 8u * bZFull);
     }
-    if (lane == 0) tma_store_wait_read();   // the dz buffer is reused by the epilogue
-    __syncwarp();
+    // the dz buffer is reused by the epilogue: its last tile has been read (in stored-tiles mode by the store as well)
+    if (ok && my_steps > 0) ok = wait_or_abort(bars + 8u * bZEmpty, (my_steps - 1) & 1, abort_flag, p, 533);
     if (ok && my_steps > 0) ok = wait_or_abort(bar(bDqFull + w), 0, abort_flag, p, 532);
     if (ok && my_steps > 0) {
       tc_fence_after();
       const uint32_t t_acc = tmem + 256 + w * 128 + lane_off;
-      if (I * kBM + kBM <= c.len) {
+      const long long tok0 = item.tok0, boff = item.boff;
+      const int hd = item.h, tile_row0 = (item.idx + w) * kBM;
+      if (tile_row0 + kBM <= item.len) {
         // full tile: two 64-column halves through this tile's dz buffer (its last dQ MMA is done), one TMA store per
         // warp and half -- full lines instead of 16 bytes per thread and row
         const uint32_t src = sZ + w * kZBytes + (warp & 3) * 32 * 128;
-        const int trow = (int)c.tok0 + I * kBM + (warp & 3) * 32;
+        const int trow = (int)tok0 + tile_row0 + (warp & 3) * 32;
 #pragma unroll 1
-        for (int half = 0; half < (p.head_dim > 64 ? 2 : 1); ++half) {   // columns past head_dim do not exist
+        for (int half = 0; half < (D > 64 && p.head_dim > 64 ? 2 : 1); ++half) {   // columns past head_dim do not exist
 #pragma unroll 1
           for (int ch = 0; ch < 2; ++ch) {
             uint32_t v[32];
@@ -532,7 +586,7 @@ tc_bwd_dq2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
           fence_proxy_async_smem();
           __syncwarp();
           if (lane == 0) {
-            tma_store_4d(&tm_dq, src, half * 64, trow, h, (int)c.boff);
+            tma_store_4d(&tm_dq, src, half * 64, trow, hd, (int)boff);
             tma_store_commit();
             tma_store_wait_read();   // the buffer is rewritten by the next half
           }
@@ -541,8 +595,8 @@ tc_bwd_dq2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
         if (lane == 0) tma_store_wait_all();
       } else {
         // the sequence ends inside the tile: row by row, rows past the end are left alone
-        T *grow = reinterpret_cast<T *>(p.dq.ptr) + c.boff * p.dq.sb + (long long)h * p.dq.sh + (c.tok0 + gi) * p.dq.st;
-        store_acc_rows<D, kFp16, T>(t_acc, grow, valid, p.head_dim, p.scale);
+        T *grow = reinterpret_cast<T *>(p.dq.ptr) + boff * p.dq.sb + (long long)hd * p.dq.sh + (tok0 + tile_row0 + r) * p.dq.st;
+        store_acc_rows<D, kFp16, T>(t_acc, grow, tile_row0 + r < item.len, p.head_dim, p.scale);
       }
     }
   }
@@ -768,18 +822,23 @@ tc_bwd_dkv4_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
         tmem_wait_ld_regs(s0, d0);
         tmem_ld16(tS + 16, s1);
         tmem_ld16(tP + 16, d1);
+        const int limit = chunk_limit(valid, diag, r, p.attend_current);
         {
-          float pa[16], pz[16];
-          if (masked)
-            bwd_row_chunk_values<true>(s0, d0, quarter * 32, r, diag, p.attend_current, valid, scale2, r1f, gpre, dr, gs, logsum, pa, pz);
-          else
-            bwd_row_chunk_values<false>(s0, d0, 0, r, false, 0, true, scale2, r1f, gpre, dr, gs, logsum, pa, pz, !p.dense);
+          BwdChunk k;
+          float pz[16];
+          if (masked) {
+            bwd_chunk_weights<true>(s0, quarter * 32, limit, scale2, r1f, gpre, logsum, k, false, [] {});
+            bwd_chunk_dz<true>(d0, quarter * 32, limit, gpre, dr, gs, k, pz);
+          } else {
+            bwd_chunk_weights<false>(s0, 0, limit, scale2, r1f, gpre, logsum, k, !p.dense, [] {});
+            bwd_chunk_dz<false>(d0, 0, limit, gpre, dr, gs, k, pz);
+          }
           // the A/dz tiles are still being read by the previous step's MMAs
           if (g >= 1) {
             ok = wait_or_abort(bar(bAzEmpty), (g - 1) & 1, abort_flag, p, 631);
             tc_fence_after();
           }
-          store_row_chunk16<kFp16>(gA, r, w * 32, pa);
+          store_row_chunk16<kFp16>(gA, r, w * 32, k.pa);
           store_row_chunk16<kFp16>(gZ, r, w * 32, pz);
         }
         tmem_wait_ld_regs(s1, d1);
@@ -787,11 +846,9 @@ tc_bwd_dkv4_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
         __syncwarp();
         if (lane == 0) mbar_arrive(bar(bSpEmpty + slot));
         if (masked)
-          bwd_row_chunk<kFp16, true, true>(s1, d1, w * 32 + 16, quarter * 32 + 16, r, diag, p.attend_current, valid, scale2, r1f,
-                                           gpre, dr, gs, logsum, gA, gZ);
+          bwd_row_chunk<kFp16, true>(s1, d1, w * 32 + 16, quarter * 32 + 16, r, limit, scale2, r1f, gpre, dr, gs, logsum, gA, gZ);
         else
-          bwd_row_chunk<kFp16, true, false>(s1, d1, w * 32 + 16, 0, r, false, 0, true, scale2, r1f, gpre, dr, gs, logsum, gA, gZ,
-                                            !p.dense);
+          bwd_row_chunk<kFp16, false>(s1, d1, w * 32 + 16, 0, r, limit, scale2, r1f, gpre, dr, gs, logsum, gA, gZ, !p.dense);
       } else {
         if (g >= 1) {
           ok = wait_or_abort(bar(bAzEmpty), (g - 1) & 1, abort_flag, p, 631);
@@ -1092,17 +1149,19 @@ static cudaError_t launch_bwd_t(const KParams &p, int dtype, cudaStream_t s) {
   if ((e = make_tile_map(&mg, p.d_o, p, dtype)) != cudaSuccess) return e;
   const dim3 grid((unsigned)item_blocks(p, 1)), grid_pairs((unsigned)item_blocks(p, 2));
   if (!p.skip_dq) {
-    auto kernel = tc_bwd_dq2_kernel<kFp16>;
-    e = allow_dynamic_smem(reinterpret_cast<const void *>(kernel), dq2::kSmem);
-    if (e != cudaSuccess) return e;
+    const bool narrow = p.head_dim <= 64;
+    auto kernel = p.az != nullptr ? (narrow ? tc_bwd_dq2_kernel<64, kFp16, true> : tc_bwd_dq2_kernel<128, kFp16, true>)
+                                  : (narrow ? tc_bwd_dq2_kernel<64, kFp16, false> : tc_bwd_dq2_kernel<128, kFp16, false>);
+    const int smem = narrow ? dq2::Cfg<64>::kSmem : dq2::Cfg<128>::kSmem;
+    if ((e = allow_dynamic_smem(reinterpret_cast<const void *>(kernel), smem)) != cudaSuccess) return e;
     CUtensorMap mk64, mv64;   // 64-row boxes: the kernel streams 64-key sub-tiles
     if ((e = make_tile_map(&mk64, p.k, p, dtype, 64)) != cudaSuccess) return e;
     if ((e = make_tile_map(&mv64, p.v, p, dtype, 64)) != cudaSuccess) return e;
-    CUtensorMap mdq, maz32;   // stores: 32 rows per warp
+    CUtensorMap mdq, maz128;   // stores: dQ 32 rows per warp, dz one tile at a time
     if ((e = make_tile_map(&mdq, p.dq, p, dtype, 32)) != cudaSuccess) return e;
-    if (p.az != nullptr) { if ((e = make_az_map(&maz32, p, dtype, 32)) != cudaSuccess) return e; }
-    else maz32 = mdq;         // not used
-    kernel<<<grid_pairs, dq2::kThreads, dq2::kSmem, s>>>(mq, mk64, mv64, mg, mdq, maz32, p);
+    if (p.az != nullptr) { if ((e = make_az_map(&maz128, p, dtype, kBM)) != cudaSuccess) return e; }
+    else maz128 = mdq;         // not used
+    kernel<<<grid_pairs, dq2::kThreads, smem, s>>>(mq, mk64, mv64, mg, mdq, maz128, p);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
   }
   if (!p.skip_dkv && p.az != nullptr) {
@@ -1130,8 +1189,7 @@ static cudaError_t launch_bwd_t(const KParams &p, int dtype, cudaStream_t s) {
   return cudaSuccess;
 }
 
-// Every head size up to 128 runs the same 128-column kernels: TMA fills the columns past head_dim with zeros, and the
-// row passes, which bound these kernels, do not depend on the head size.
+// TMA fills the columns past head_dim with zeros, so every head size up to 128 runs the 64- or 128-column kernels.
 cudaError_t launch_tc_bwd(const KParams &p, int dtype, cudaStream_t s, int *launches) {
   *launches += (p.skip_dq ? 0 : 1) + (p.skip_dkv ? 0 : 1);
   return dtype == SB_DTYPE_F16 ? launch_bwd_t<true>(p, dtype, s) : launch_bwd_t<false>(p, dtype, s);
