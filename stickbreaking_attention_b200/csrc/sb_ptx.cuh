@@ -205,6 +205,13 @@ __device__ __forceinline__ void tmem_wait_ld_regs(uint32_t (&a)[32], uint32_t (&
       : "memory");
 }
 
+// ---- register hand-over between the warpgroups of a block (every warp of a warpgroup executes the same one) ----------
+// The shares have to add up to no more than the block was launched with.
+template <int kRegs>
+__device__ __forceinline__ void reg_inc() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kRegs)); }
+template <int kRegs>
+__device__ __forceinline__ void reg_dec() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kRegs)); }
+
 // ---- descriptors ---------------------------------------------------------------------------------------
 // Shared-memory matrix descriptor (64 bit): start address >> 4 in bits [0,14), leading-dimension byte
 // offset >> 4 in [16,30), stride-dimension byte offset >> 4 in [32,46), descriptor version 1 in [46,48),

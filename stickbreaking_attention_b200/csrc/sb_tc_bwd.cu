@@ -30,7 +30,7 @@ namespace sb {
 // kMasked tiles (the diagonal one, or one with rows past the sequence end) zero what is not allowed.
 // The chunk is kept to 16 columns so that the unrolled code of all variants stays inside the instruction cache.
 // mc0: key index of the first column inside the 128-key tile (for the diagonal mask).
-// skip_zero (unmasked chunks only): where the product of (1 - beta) at the END of the chunk -- its largest value in
+// kSkip (unmasked chunks only): where the product of (1 - beta) at the END of the chunk -- its largest value in
 // the chunk -- has underflowed to exactly 0 and the prefix of G is still exactly 0, for all 32 rows of the warp, every
 // A, G and dz of the chunk is exactly 0 (e, the reciprocals and dP - dR are finite): only the log-space sum is formed,
 // with the same operations as otherwise, and the rest is not computed.
@@ -44,9 +44,9 @@ struct BwdChunk {
 };
 
 // Sweeps 1 and 2, which do not need dP; `between` runs where the fewest registers are in use and half of sweep 2 is left.
-template <bool kMasked, class Between>
+template <bool kMasked, bool kSkip, class Between>
 __device__ __forceinline__ void bwd_chunk_weights(const uint32_t (&s)[16], int mc0, int limit, float scale2, float r1, float g_before,
-                                                  float &logsum, BwdChunk &c, bool skip_zero, Between between) {
+                                                  float &logsum, BwdChunk &c, Between between, bool may_skip = true) {
   float chunk_log = 0.f;   // summed per chunk, like the forward's (see fwd256_row_chunk): the two agree bit for bit
   const float2 sc = make_float2(scale2, scale2), one = make_float2(1.f, 1.f);
   float2 e01[4], e23[4], t01[4], t23[4];
@@ -68,7 +68,7 @@ __device__ __forceinline__ void bwd_chunk_weights(const uint32_t (&s)[16], int m
     chunk_log += lg2((t01[g].x * t01[g].y) * (t23[g].x * t23[g].y));
   }
   logsum += chunk_log;
-  c.zero = !kMasked && skip_zero && __all_sync(0xffffffffu, ex2(r1 + logsum) == 0.f && g_before == 0.f);
+  c.zero = kSkip && may_skip && __all_sync(0xffffffffu, ex2(r1 + logsum) == 0.f && g_before == 0.f);
   if (c.zero) {
 #pragma unroll
     for (int i = 0; i < 16; ++i) c.pa[i] = 0.f;
@@ -107,10 +107,10 @@ __device__ __forceinline__ void bwd_chunk_weights(const uint32_t (&s)[16], int m
 }
 
 // Sweep 3.  On entry `gs` is the pass's sum of G before the chunk; pz: dz.
-template <bool kMasked>
+template <bool kMasked, bool kSkip>
 __device__ __forceinline__ void bwd_chunk_dz(const uint32_t (&dp)[16], int mc0, int limit, float gpre, float dr, float &gs, BwdChunk &c,
                                              float (&pz)[16]) {
-  if (!kMasked && c.zero) {
+  if (kSkip && c.zero) {
 #pragma unroll
     for (int i = 0; i < 16; ++i) pz[i] = 0.f;
     return;
@@ -154,14 +154,14 @@ __device__ __forceinline__ int chunk_limit(bool row_valid, bool diag, int r, int
 }
 
 // All three sweeps, A and dz written to the 16-bit tiles; c0 addresses the output tiles.
-template <bool kFp16, bool kMasked>
+template <bool kFp16, bool kMasked, bool kSkip>
 __device__ __forceinline__ void bwd_row_chunk(const uint32_t (&s)[16], const uint32_t (&dp)[16], int c0, int mc0, int r, int limit,
                                               float scale2, float r1, float gpre, float dr, float &gs, float &logsum, uint8_t *tile_a,
-                                              uint8_t *tile_z, bool skip_zero = false) {
+                                              uint8_t *tile_z, bool may_skip = true) {
   BwdChunk c;
   float pz[16];
-  bwd_chunk_weights<kMasked>(s, mc0, limit, scale2, r1, gpre + gs, logsum, c, skip_zero, [] {});
-  bwd_chunk_dz<kMasked>(dp, mc0, limit, gpre, dr, gs, c, pz);
+  bwd_chunk_weights<kMasked, kSkip>(s, mc0, limit, scale2, r1, gpre + gs, logsum, c, [] {}, may_skip);
+  bwd_chunk_dz<kMasked, kSkip>(dp, mc0, limit, gpre, dr, gs, c, pz);
   store_row_chunk16<kFp16>(tile_a, r, c0, c.pa);
   store_row_chunk16<kFp16>(tile_z, r, c0, pz);
 }
@@ -182,10 +182,10 @@ enum { bQG = 0, bKvFull = 1, bKvEmpty = bKvFull + kMaxStages, bSFull = bKvEmpty 
 // `bars`: the dq kernel's barriers, offset by the tile's number.  out: stored-tiles mode: this row's 64 values of A in the
 // workspace; otherwise this row's record of R1 at the sub-tile's first key (S2 is `s2_off` floats further, both again kBM
 // floats further for the key 32 columns on).
-template <bool kFp16, bool kMasked, bool kStored>
+template <bool kFp16, bool kMasked, bool kStored, bool kSkip>
 __device__ __forceinline__ bool strip_row_pass(uint32_t ts, uint32_t tp, int r, int u, int mc0, int limit, float scale2, float r1, float gpre,
                                               float dr, float &gs, float &logsum, uint8_t *tile_z, uint32_t bars, void *out,
-                                              long long s2_off, bool skip_zero = false) {
+                                              long long s2_off) {
   uint32_t s0[16], s1[16], d[16];
   bool ok = true;
   auto store = [&](int c0, const BwdChunk &c, const float (&pz)[16]) {
@@ -205,7 +205,7 @@ __device__ __forceinline__ bool strip_row_pass(uint32_t ts, uint32_t tp, int r, 
     tmem_wait_ld_regs(s0);
     {
       BwdChunk c;
-      bwd_chunk_weights<kMasked>(s0, mc0 + c0, limit, scale2, r1, gpre + gs, logsum, c, skip_zero, [&] {
+      bwd_chunk_weights<kMasked, kSkip>(s0, mc0 + c0, limit, scale2, r1, gpre + gs, logsum, c, [&] {
         if (pair == 0) {
           ok = mbar_wait(bars + 8u * dq2::bDpFull, u & 1);
           tc_fence_after();
@@ -226,14 +226,14 @@ __device__ __forceinline__ bool strip_row_pass(uint32_t ts, uint32_t tp, int r, 
         if ((threadIdx.x & 31) == 0) mbar_arrive(bars + 8u * dq2::bSpEmpty);
       }
       float pz[16];
-      bwd_chunk_dz<kMasked>(d, mc0 + c0, limit, gpre, dr, gs, c, pz);
+      bwd_chunk_dz<kMasked, kSkip>(d, mc0 + c0, limit, gpre, dr, gs, c, pz);
       store(c0, c, pz);
     }
     {
       BwdChunk c;
       float pz[16];
-      bwd_chunk_weights<kMasked>(s1, mc0 + c0 + 16, limit, scale2, r1, gpre + gs, logsum, c, skip_zero, [] {});
-      bwd_chunk_dz<kMasked>(s0, mc0 + c0 + 16, limit, gpre, dr, gs, c, pz);
+      bwd_chunk_weights<kMasked, kSkip>(s1, mc0 + c0 + 16, limit, scale2, r1, gpre + gs, logsum, c, [] {});
+      bwd_chunk_dz<kMasked, kSkip>(s0, mc0 + c0 + 16, limit, gpre, dr, gs, c, pz);
       store(c0 + 16, c, pz);
     }
     if (pair == 0) {
@@ -285,7 +285,7 @@ __device__ __forceinline__ bool zero_strip_row(uint8_t *tile_z, int r, int u, ui
 // overlap although S and dP fill all the tensor memory there is and cannot be double-buffered: rows start on S alone, dP
 // has until the middle of the first chunk, and both slots are handed back after two thirds of the pass (see strip_row_pass).
 namespace dq2 {
-constexpr int kThreads = 352;
+constexpr int kThreads = 384;   // three warpgroups (one warp idles)
 constexpr int kBN = 64;
 constexpr int kKvBox = kBN * 64 * 2;           // 64 keys x 64 columns
 constexpr int kZBytes = kBM * kBN * 2;         // dz tile: 128 rows x 64 keys
@@ -380,6 +380,10 @@ tc_bwd_dq2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
   tc_fence_after();
   const uint32_t tmem = ctl->tmem_base;
 
+  // The row warps take over registers the other warpgroup does not need (8 x 32 x 216 + 4 x 32 x 64 of the launch's
+  // 12 x 32 x 168): at 168 they spill.
+  if (warp >= 8) {
+  reg_dec<64>();
   if (warp == 8) {
     if (lane == 0) {
       prefetch_tensormap(&tm_q); prefetch_tensormap(&tm_k); prefetch_tensormap(&tm_v); prefetch_tensormap(&tm_g);
@@ -403,7 +407,7 @@ tc_bwd_dq2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
         }
       }
     }
-  } else if (warp >= 9) {
+  } else if (warp == 9 || warp == 10) {
     // ------------------------------------------------ MMA issuers, one per tile
     const int w = warp - 9;
     if (lane == 0 && w < issuers) {
@@ -476,7 +480,9 @@ tc_bwd_dq2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
       release(t_end, n_stages);   // tile a does not read the last sub-tiles
       if constexpr (kStored) tma_store_wait_all();
     }
+  }
   } else {
+    reg_inc<216>();
     // ------------------------------------------------ rows: warpgroup w owns query tile Ia + w
     using T = typename std::conditional<kFp16, __half, __nv_bfloat16>::type;
     const int w = warp >> 2;
@@ -506,6 +512,9 @@ tc_bwd_dq2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
     const int u_diag = 2 * I, u_tail = c.len / kBN;   // a sub-tile with rows past the sequence is number u_tail
     // this warp's rows start at sub-tile u_warp (never, if they are past the sequence): before it, A and dz are zeros
     const int u_warp = row0 + (r & ~31) < c.len ? first_key(p, c, h, row0 + (r & ~31)) / kBN : 0x7fffffff;
+    // Where the forward has said where each warp's rows start, hardly a chunk of zeros is left, and the test for them costs
+    // every chunk a tenth of its instructions.
+    const bool skip = p.tile_start == nullptr && !p.dense;
     bool ok = true;
     // u: 64-key sub-tile inside the sequence; the first one is even, so that phases follow from u alone
     for (int u = w == 0 ? first_a : first_b; u < my_steps && ok; ++u) {
@@ -532,11 +541,13 @@ tc_bwd_dq2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
       if (u < u_warp)
         pass_ok = zero_strip_row<kStored>(gZ, r, u, bars, dst, s2_off);
       else if (on_diag || (kStored && ragged))
-        pass_ok = strip_row_pass<kFp16, true, kStored>(tS, tP, r, u, on_diag ? (u - u_diag) * kBN : 0,
+        pass_ok = strip_row_pass<kFp16, true, kStored, false>(tS, tP, r, u, on_diag ? (u - u_diag) * kBN : 0,
                                                        chunk_limit(valid || !kStored, on_diag, r, p.attend_current), scale2, r1f, gpre, dr,
                                                        gs, logsum, gZ, bars, dst, s2_off);
+      else if (skip)
+        pass_ok = strip_row_pass<kFp16, false, kStored, true>(tS, tP, r, u, 0, 0, scale2, r1f, gpre, dr, gs, logsum, gZ, bars, dst, s2_off);
       else
-        pass_ok = strip_row_pass<kFp16, false, kStored>(tS, tP, r, u, 0, 0, scale2, r1f, gpre, dr, gs, logsum, gZ, bars, dst, s2_off, !p.dense);
+        pass_ok = strip_row_pass<kFp16, false, kStored, false>(tS, tP, r, u, 0, 0, scale2, r1f, gpre, dr, gs, logsum, gZ, bars, dst, s2_off);
       if (!pass_ok) {   // a bounded wait inside the pass gave up
         *abort_flag = 1;
         if (p.status != nullptr) { p.status[0] = SB_DEV_WAIT_TIMEOUT; p.status[1] = 531; }
@@ -827,11 +838,11 @@ tc_bwd_dkv4_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
           BwdChunk k;
           float pz[16];
           if (masked) {
-            bwd_chunk_weights<true>(s0, quarter * 32, limit, scale2, r1f, gpre, logsum, k, false, [] {});
-            bwd_chunk_dz<true>(d0, quarter * 32, limit, gpre, dr, gs, k, pz);
+            bwd_chunk_weights<true, false>(s0, quarter * 32, limit, scale2, r1f, gpre, logsum, k, [] {});
+            bwd_chunk_dz<true, false>(d0, quarter * 32, limit, gpre, dr, gs, k, pz);
           } else {
-            bwd_chunk_weights<false>(s0, 0, limit, scale2, r1f, gpre, logsum, k, !p.dense, [] {});
-            bwd_chunk_dz<false>(d0, 0, limit, gpre, dr, gs, k, pz);
+            bwd_chunk_weights<false, true>(s0, 0, limit, scale2, r1f, gpre, logsum, k, [] {}, !p.dense);
+            bwd_chunk_dz<false, true>(d0, 0, limit, gpre, dr, gs, k, pz);
           }
           // the A/dz tiles are still being read by the previous step's MMAs
           if (g >= 1) {
@@ -846,9 +857,9 @@ tc_bwd_dkv4_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
         __syncwarp();
         if (lane == 0) mbar_arrive(bar(bSpEmpty + slot));
         if (masked)
-          bwd_row_chunk<kFp16, true>(s1, d1, w * 32 + 16, quarter * 32 + 16, r, limit, scale2, r1f, gpre, dr, gs, logsum, gA, gZ);
+          bwd_row_chunk<kFp16, true, false>(s1, d1, w * 32 + 16, quarter * 32 + 16, r, limit, scale2, r1f, gpre, dr, gs, logsum, gA, gZ);
         else
-          bwd_row_chunk<kFp16, false>(s1, d1, w * 32 + 16, 0, r, limit, scale2, r1f, gpre, dr, gs, logsum, gA, gZ, !p.dense);
+          bwd_row_chunk<kFp16, false, true>(s1, d1, w * 32 + 16, 0, r, limit, scale2, r1f, gpre, dr, gs, logsum, gA, gZ, !p.dense);
       } else {
         if (g >= 1) {
           ok = wait_or_abort(bar(bAzEmpty), (g - 1) & 1, abort_flag, p, 631);
