@@ -21,6 +21,14 @@
 
 namespace sb {
 
+struct Fwd128Item {
+  TileCoord c;
+  int h;          // head
+  int row0;       // first row of the tile inside the sequence
+  int s_top;      // sub-tile of step 0; step t handles sub-tile s_top - t
+  int n_steps;    // 0: no such item
+};
+
 namespace fwd128 {
 constexpr int kThreads = 384;
 constexpr int D = 64;                         // columns (head sizes below 64: TMA fills the rest with zeros)
@@ -32,45 +40,35 @@ constexpr int kStages = 3;                    // (a fourth stage fits and was me
 constexpr int kQBufs = 2;
 constexpr int kOBytes = kBM * D * 2;          // staging tile of the O epilogue
 constexpr int kWorkerBytes = kQBufs * kQBytes + kStages * kStageBytes + kOBytes;
-constexpr int kBarBytes = 512;
+constexpr int kBarBytes = 1024;
 constexpr int kSmem = 1024 + 2 * kWorkerBytes + kBarBytes + (int)sizeof(SmallTable);
 constexpr uint32_t kWorkerCols = 192;
+constexpr int kRecords = 4;
 // barriers of one worker
 enum { bQ = 0, bQFree = 2, bKvFull = 4, bKvEmpty = 4 + kStages, bSFull = 4 + 2 * kStages, bPFull = bSFull + 2, bOFull = bSFull + 4,
-       bOFree = bSFull + 5, bPerWorker = bSFull + 6 };
+       bOFree = bSFull + 5, bItem = bSFull + 6, bPerWorker = bItem + kRecords };
 struct Shared {                               // behind the barriers
   Ctl ctl;
   EarlyStop stop[2];                          // per worker
+  // The items, looked up by the producer (two dependent reads of global memory, ~1400 clk) and read by the issuer and the
+  // rows, which are up to three items behind.
+  Fwd128Item item[2][kRecords];
   int kv_end[2][kStages];                     // per stage: stage number + 1 if it holds no keys but marks the end of its tile
 };
 static_assert(2 * bPerWorker * 8 + sizeof(Shared) <= kBarBytes, "barriers and control words");
 }  // namespace fwd128
 
-struct Fwd128Item {
-  TileCoord c;
-  int h;          // head
-  int row0;       // first row of the tile inside the sequence
-  int s_top;      // sub-tile of step 0; step t handles sub-tile s_top - t
-  int n_steps;
-};
-
 // Item number `it` of worker v out of V: the workers walk the weight-ordered tile list in a boustrophedon.
-__device__ __forceinline__ long long fwd128_lin(int it, int v, int V) {
-  return (long long)it * V + ((it & 1) ? V - 1 - v : v);
-}
-__device__ __forceinline__ void fwd128_finish(const KParams &p, long long lin, long long item, Fwd128Item &w) {
+__device__ __forceinline__ void fwd128_item(const KParams &p, const SmallTable &tb, int it, int v, int V, Fwd128Item &w) {
+  const long long lin = (long long)it * V + ((it & 1) ? V - 1 - v : v);
+  const long long item = lin / p.head_cnt;
+  w.n_steps = 0;
+  if (item > 0x7fffffffLL || !decode_item(p, tb, (int)item, 1, true, w.c)) return;
   w.h = p.head0 + (int)(lin - item * p.head_cnt);
   const int n_sub = (w.c.len + fwd128::kBN - 1) / fwd128::kBN;
   w.row0 = w.c.idx * kBM;
   w.s_top = min(2 * w.c.idx + 1, n_sub - 1);
   w.n_steps = w.s_top + 1;
-}
-__device__ __forceinline__ bool fwd128_item(const KParams &p, const SmallTable &tb, int it, int v, int V, Fwd128Item &w) {
-  const long long lin = fwd128_lin(it, v, V);
-  const long long item = lin / p.head_cnt;
-  if (item > 0x7fffffffLL || !decode_item(p, tb, (int)item, 1, true, w.c)) return false;
-  fwd128_finish(p, lin, item, w);
-  return true;
 }
 
 // kStop: tiles may stop early.  A tile of a sequence of up to 512 tokens has no four sub-tiles left by the time it could
@@ -106,6 +104,7 @@ tc_fwd128x2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
   if (threadIdx.x == 0) {
     for (int w = 0; w < 2; ++w) {
       auto b = [&](int i) { return sBar + 8u * (w * bPerWorker + i); };
+      for (int i = 0; i < kRecords; ++i) mbar_init(b(bItem + i), 1);
       for (int i = 0; i < kQBufs; ++i) { mbar_init(b(bQ + i), 1); mbar_init(b(bQFree + i), 1); }
       for (int s = 0; s < kStages; ++s) { mbar_init(b(bKvFull + s), 1); mbar_init(b(bKvEmpty + s), 1); }
       for (int s = 0; s < 2; ++s) { mbar_init(b(bSFull + s), 2); mbar_init(b(bPFull + s), 4); }   // S: commit and word
@@ -130,12 +129,22 @@ tc_fwd128x2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
   volatile EarlyStop &stop = sh->stop[wk];
   volatile int *kv_end = sh->kv_end[wk];
   Fwd128Item w;
+  Fwd128Item *records = sh->item[wk];
+  auto next_item = [&](int it) {   // waits for item `it`; false if there is none or the wait gave up
+    if (!wait_or_abort(bar(bItem + it % kRecords), (it / kRecords) & 1, abort_flag, p, 709)) return false;
+    w = records[it % kRecords];
+    return w.n_steps > 0;
+  };
   if (warp == 8 || warp == 11) {
     // ------------------------------------------------ TMA producer of this worker
     if (lane == 0) {
       prefetch_tensormap(&tm_q); prefetch_tensormap(&tm_k); prefetch_tensormap(&tm_v);
       int T = 0;   // K/V stages filled so far
-      for (int it = 0; fwd128_item(p, tb, it, v, V, w); ++it) {
+      for (int it = 0;; ++it) {
+        fwd128_item(p, tb, it, v, V, w);
+        records[it % kRecords] = w;
+        mbar_arrive(bar(bItem + it % kRecords));
+        if (w.n_steps == 0) break;
         const int qb = it % kQBufs, qn = it / kQBufs;
         // the buffer's previous tile is no longer read once its last S MMA has finished
         if (qn >= 1 && !wait_or_abort(bar(bQFree + qb), (qn - 1) & 1, abort_flag, p, 711)) break;
@@ -172,7 +181,7 @@ tc_fwd128x2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
       constexpr uint32_t idesc_pv = idesc_f16(kBM, D, kFp16, false, true);
       int T = 0, U = 0;   // K/V stages and steps of the earlier tiles
       bool ok = true;
-      for (int it = 0; ok && fwd128_item(p, tb, it, v, V, w); ++it) {
+      for (int it = 0; ok && next_item(it); ++it) {
         const int qb = it % kQBufs, qn = it / kQBufs;
         ok = wait_or_abort(bar(bQ + qb), qn & 1, abort_flag, p, 720);
         const uint32_t qaddr = sQ + qb * kQBytes;
@@ -239,10 +248,8 @@ tc_fwd128x2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
     const int ac = p.attend_current;
     int U = 0;   // steps of the earlier tiles
     bool ok = true;
-    Fwd128Item w_next;
-    bool have = fwd128_item(p, tb, 0, v, V, w);
     uint8_t *stage = gbase + (sO - base);
-    for (int it = 0; ok && have; ++it) {
+    for (int it = 0; ok && next_item(it); ++it) {
       const int row = w.row0 + blk * 32 + lane;      // row index inside the sequence
       const int s_diag0 = 2 * w.c.idx;               // first sub-tile that reaches this tile's diagonal band
       const bool warp_live = (row & ~31) < w.c.len;  // a warp whose 32 rows all lie past the sequence end computes nothing
@@ -294,7 +301,7 @@ tc_fwd128x2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
         }
       }
       // ---- epilogue: O (TMEM) -> global, rem, log_rem
-      // While the last P V MMA finishes: rem and log_rem leave, and the next tile's table entries are fetched.
+      // While the last P V MMA finishes: rem and log_rem leave.
       const bool valid = row < w.c.len;
       const float rem_f = run.stick();
       if (ok && valid) {
@@ -304,7 +311,6 @@ tc_fwd128x2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
       }
       if (p.tile_start != nullptr && ok && warp_live && lane == 0 && row >= 64)
         *tile_start_entry(p, w.c, w.h, row) = s_reached * kBN;
-      const bool have_next = fwd128_item(p, tb, it + 1, v, V, w_next);
       if (ok) ok = wait_or_abort(bar(bOFull), it & 1, abort_flag, p, 732);
       if (ok) {
         tc_fence_after();
@@ -331,8 +337,6 @@ tc_fwd128x2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
       __syncwarp();
       if (lane == 0) mbar_arrive(bar(bOFree));
       U += slots;
-      w = w_next;
-      have = have_next;
     }
     if (lane == 0) tma_store_wait_all();
   }
