@@ -230,6 +230,12 @@ static int fill_kparams(const SbParams *p, const Plan &pl, bool backward, KParam
     const bool tc = pl.path == SB_PATH_TCGEN05;
     k.small_table = (!backward && tc) || ((long long)pl.tiles_cap * p->heads <= 2 * 148 * (tc ? 2 : 4) && (pl.store_az || !tc));
   }
+  // Short sequences, forward, larger batches: the workers draw their items, and then the tiles of a sequence (eight at most:
+  // see tc_tile) can be neighbours and share K/V through L2 (DRAM reads -38 %, time -1 %).
+  if (!backward && pl.tile == kTcTile && pl.path == SB_PATH_TCGEN05 && p->cu_seqlens != nullptr && !k.small_table) {
+    k.order_span = 8;
+    k.item_counter = reinterpret_cast<unsigned *>(k.hdr + 4);
+  }
   k.fuse_rem_v = (p->flags & SB_FLAG_FUSE_REM_V) ? 1 : 0;
   if (!backward && p->attn_weights != nullptr) {
     if (p->attn_cols < 1) return fail(SB_ERR_ARGUMENT, "attn_cols must be >= 1 with attn_weights");

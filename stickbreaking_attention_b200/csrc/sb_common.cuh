@@ -48,6 +48,7 @@ struct KParams {
   unsigned long long *trace;  // experiments only: event log of block (0,0) in the workspace tail, or nullptr
   // workspace views
   int *hdr;            // [0] cu_seqlens refused, [1] end of the last sequence, [2] / [3] entries of order / order2
+  unsigned *item_counter;  // hdr[4]: items the workers of a persistent kernel have drawn, or null: fixed assignment
   long long *pair_prefix;  // [num_seq] exclusive prefix of n(n+1)/2 (varlen)
   float *bnd_r1;       // [head_cnt][pairs_cap][tile]  suffix sums of log(1-beta) at tile starts
   float *bnd_s2;       // [head_cnt][pairs_cap][tile]  prefix sums of G before each key tile

@@ -143,6 +143,7 @@ __global__ void __launch_bounds__(kPrepThreads) prep_kernel(KParams p) {
   if (bad != -2 && p.status != nullptr) { p.status[0] = SB_DEV_BAD_CU_SEQLENS; p.status[1] = bad; }
   if (t == 0) {
     p.hdr[0] = refused ? 1 : 0;
+    p.hdr[4] = 0;
     p.hdr[1] = refused ? 0 : (int)load_cu(p, p.num_seq - 1);
   }
   if (refused) return;   // no kernel will look at the table

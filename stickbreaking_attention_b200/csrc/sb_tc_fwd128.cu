@@ -58,9 +58,11 @@ struct Shared {                               // behind the barriers
 static_assert(2 * bPerWorker * 8 + sizeof(Shared) <= kBarBytes, "barriers and control words");
 }  // namespace fwd128
 
-// Item number `it` of worker v out of V: the workers walk the weight-ordered tile list in a boustrophedon.
+// Item number `it` of worker v out of V.  With a table written by a kernel that ran first, the workers draw from a counter:
+// the tiles of a sequence are neighbours in the list then and share their keys through L2, and a fixed assignment of items
+// in that order would leave the workers up to 10 % apart.  Otherwise they walk the weight-ordered list in a boustrophedon.
 __device__ __forceinline__ void fwd128_item(const KParams &p, const SmallTable &tb, int it, int v, int V, Fwd128Item &w) {
-  const long long lin = (long long)it * V + ((it & 1) ? V - 1 - v : v);
+  const long long lin = p.item_counter != nullptr ? (long long)atomicAdd(p.item_counter, 1u) : (long long)it * V + ((it & 1) ? V - 1 - v : v);
   const long long item = lin / p.head_cnt;
   w.n_steps = 0;
   if (item > 0x7fffffffLL || !decode_item(p, tb, (int)item, 1, true, w.c)) return;
