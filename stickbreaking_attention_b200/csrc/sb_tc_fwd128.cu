@@ -256,22 +256,16 @@ tc_fwd128x2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
       const int s_diag0 = 2 * w.c.idx;               // first sub-tile that reaches this tile's diagonal band
       const bool warp_live = (row & ~31) < w.c.len;  // a warp whose 32 rows all lie past the sequence end computes nothing
       LogSum run;
-      bool through = false;    // this warp is through with the tile, having got to sub-tile s_reached
-      int s_reached = 0;
+      int s_reached = -1;      // >= 0: this warp is through with the tile, having got to this sub-tile
       int slots = w.n_steps;                         // S slots used
       if (lane == 0) tma_store_wait_read();          // the previous tile's O has left the staging tile
       __syncwarp();
-      for (int u = 0; u < w.n_steps && ok; ++u) {
+      int u = 0;
+      for (; u < w.n_steps && ok && (!kStop || s_reached < 0); ++u) {
         const int s = w.s_top - u;
         const int gu = U + u, buf = gu & 1;
         ok = wait_or_abort(bar(bSFull + buf), (gu >> 1) & 1, abort_flag, p, 730);
         if (!ok) break;
-        if (kStop && through && stop.word[buf] == kStepStop) {   // (a stop needs this warp's consent)
-          slots = u + 1;
-          __syncwarp();
-          if (lane == 0) mbar_arrive(bar(bPFull + buf));
-          break;
-        }
         tc_fence_after();
         const uint32_t ts = tmem + buf * 64 + lane_off;
         // the sequence ends inside this sub-tile: the V rows behind its end are not this sequence's (see
@@ -281,12 +275,10 @@ tc_fwd128x2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
           zero_tile_rows(gbase + (sKV - base) + stop.word[buf] * kStageBytes + kKvTileBytes, tail_rows, kBN, 1, kKvTileBytes, r, kBM);
           fence_proxy_async_smem();
         }
-        bool done = through || !warp_live;
+        bool done = !warp_live;
         float logsum = 0.f;
         // (the P rows of such a warp keep whatever the slot held: they only reach accumulator rows that are never stored)
-        if (through) {
-          fwd256_zero_row(ts + kPCol);
-        } else if (!warp_live) {
+        if (done) {
         } else if (s >= s_diag0) fwd256_row_pass<kFp16, true>(ts, s * kBN, row, ac, scale2, run, logsum, ts + kPCol, true);
         else done = fwd256_row_pass<kFp16, false>(ts, 0, 0, ac, scale2, run, logsum, ts + kPCol, row < w.c.len, !p.dense, kStop);
         run.add(logsum);
@@ -294,12 +286,28 @@ tc_fwd128x2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
         tc_fence_before();          // this step's TMEM reads and its writes of P are done before the slot is handed back
         __syncwarp();
         if (lane == 0) {
-          if (kStop && done && !through) publish_through(stop, warp & 3, it, u);
+          if (kStop && done) publish_through(stop, warp & 3, it, u);
           mbar_arrive(bar(bPFull + buf));
         }
-        if (kStop && done && !through) {
-          through = true;
-          s_reached = s + 1;
+        if (kStop && done) s_reached = s + 1;
+      }
+      // through: zeros for P until the other warps of the tile are as well (the sequence's tail is behind these steps)
+      for (; kStop && u < w.n_steps && ok; ++u) {
+        const int gu = U + u, buf = gu & 1;
+        ok = wait_or_abort(bar(bSFull + buf), (gu >> 1) & 1, abort_flag, p, 731);
+        if (!ok) break;
+        const bool halt = stop.word[buf] == kStepStop;
+        if (!halt) {
+          tc_fence_after();
+          fwd256_zero_row(tmem + buf * 64 + lane_off + kPCol);
+          tmem_wait_st();
+          tc_fence_before();
+        }
+        __syncwarp();
+        if (lane == 0) mbar_arrive(bar(bPFull + buf));
+        if (halt) {
+          slots = u + 1;
+          break;
         }
       }
       // ---- epilogue: O (TMEM) -> global, rem, log_rem
@@ -312,7 +320,7 @@ tc_fwd128x2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
         p.log_rem[idx] = -run.value();
       }
       if (p.tile_start != nullptr && ok && warp_live && lane == 0 && row >= 64)
-        *tile_start_entry(p, w.c, w.h, row) = s_reached * kBN;
+        *tile_start_entry(p, w.c, w.h, row) = max(s_reached, 0) * kBN;
       if (ok) ok = wait_or_abort(bar(bOFull), it & 1, abort_flag, p, 732);
       if (ok) {
         tc_fence_after();
