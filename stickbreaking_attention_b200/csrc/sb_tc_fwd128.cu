@@ -191,7 +191,7 @@ tc_fwd128x2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
         // rows of the current step are processed.  S(u) reuses the TMEM slot of step u-2, whose P the P V MMA of
         // that step (issued earlier by this thread) has read.
         int steps = w.n_steps, used = w.n_steps;   // steps computed and stages taken
-        bool early = false, halt = false;   // halt: the tile stops before step u (decided while the rows of step u - 2 worked)
+        bool early = false, halt = false;   // halt: the tile stops before step u
         for (int u = 0; ok && u <= steps; ++u) {
           if (halt) {
             early = true;
@@ -210,7 +210,7 @@ tc_fwd128x2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
             mma_commit(bar(bSFull + (gu & 1)));
             stop.word[gu & 1] = st;
             mbar_arrive(bar(bSFull + (gu & 1)));
-            halt = kStop && u >= 2 && u + 1 < w.n_steps && may_stop_before(w.s_top - u - 1) && all_through(stop, it, u - 2);
+            halt = kStop && u >= 2 && u + 1 < w.n_steps && may_stop_before(w.s_top - u - 1) && all_through(stop, it);
             if (u == w.n_steps - 1) mma_commit(bar(bQFree + qb));   // the tile's last read of Q
           }
           if (u >= 1) {
@@ -286,7 +286,7 @@ tc_fwd128x2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
         tc_fence_before();          // this step's TMEM reads and its writes of P are done before the slot is handed back
         __syncwarp();
         if (lane == 0) {
-          if (kStop && done) publish_through(stop, warp & 3, it, u);
+          if (kStop && done) publish_through(stop, warp & 3, it);
           mbar_arrive(bar(bPFull + buf));
         }
         if (kStop && done) s_reached = s + 1;

@@ -221,7 +221,7 @@ tc_fwd256_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
         // rows of the current step are processed.  S(u) reuses the TMEM slot of step u-2, whose rows were finished
         // before p_full(u-2) was signalled, and that was waited for in iteration u-1.
         int steps = my_steps;          // steps computed
-        bool early = false, halt = false;   // halt: the tile stops before step u (decided while the rows of step u - 2 worked)
+        bool early = false, halt = false;   // halt: the tile stops before step u
         for (int u = 0; ok && active && u <= steps; ++u) {
           if (halt) {
             early = true;
@@ -243,7 +243,7 @@ tc_fwd256_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
             mma_commit(bar(bSFull + wg * 2 + (gu & 1)));
             stop.word[gu & 1] = st;
             mbar_arrive(bar(bSFull + wg * 2 + (gu & 1)));
-            halt = may_stop && u >= 2 && u + 1 < my_steps && may_stop_before(w.s_top - t0 - u - 1) && all_through(stop, it, u - 2);
+            halt = may_stop && u >= 2 && u + 1 < my_steps && may_stop_before(w.s_top - t0 - u - 1) && all_through(stop, it);
             if (u == my_steps - 1) mma_commit(bar_qfree);   // the item's last read of Q
             trace_event(p, 1 + 3 * wg, tr_cur, 3 + 16 * wg, t0 + u);
           }
@@ -334,7 +334,7 @@ tc_fwd256_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
         tc_fence_before();          // this step's TMEM reads and writes of P are done before the slot is handed back
         __syncwarp();
         if (lane == 0) {
-          if (may_stop && done) publish_through(stop, warp & 3, it, u);
+          if (may_stop && done) publish_through(stop, warp & 3, it);
           mbar_arrive(bar(bPFull + wg * 2 + buf));
         }
         if (may_stop && done) s_reached = s + 1;

@@ -187,32 +187,28 @@ __device__ __forceinline__ bool fwd256_row_pass(uint32_t ts, int key0, int row, 
 // ---- stopping early ------------------------------------------------------------------------------------------------
 // A row warp is through once the product R has underflowed to exactly 0 for all its rows: no earlier key can add anything
 // to O or rem.  From then on it only writes zeros for P, its log sum stays what it is, and the key it got to is recorded
-// for the backward.  Each of a query tile's four warps publishes its first step of zeros; the tile's MMA issuer stops
-// before step v if all four have done so by step v - 3 and tells the rows with the word that accompanies every step's
-// scores.  It looks when it has issued step v - 1's scores and would wait for step v - 2's P: it has waited for the P of
-// step v - 3, so the decision does not depend on timing, and nobody waits for it.  Three steps of zeros are cheap, and rows
-// that never finish pay nothing: the vote is the one the row pass takes anyway to skip its arithmetic.  (A vote on R at the
-// end of the pass and a decision right before step v's scores stop two steps earlier and cost every step of every row: +5 %
-// time on 4096-token sequences that never stop.)
+// for the backward.  Each of a query tile's four warps publishes that it is through; once all four are, the tile's MMA
+// issuer, who looks after each step's scores have been issued, stops before the next step and tells the rows with the word
+// that accompanies every step's scores.  Where exactly it stops depends on timing, what is stored does not: the steps in
+// between are zeros.  Rows that never finish pay nothing: the vote is the one the row pass takes anyway to skip its
+// arithmetic, and the issuer's look is one 16-byte read.
 constexpr int kStepStop = -1;
 // No stop with fewer than three sub-tiles to go: what is left costs about as much as stopping and restarting the stream.
 __device__ __forceinline__ bool may_stop_before(int sub_tile) { return sub_tile >= 2; }
-struct EarlyStop {                            // shared memory, one per query tile
-  unsigned long long through[4];              // per row warp: (item + 1) << 32 | its first step of zeros
+struct alignas(16) EarlyStop {                // shared memory, one per query tile
+  int through[4];                             // per row warp: the last item it was through with, plus one
   int word[2];                                // per S slot: K/V stage of the step, or kStepStop (read where it can matter)
   int stopped;                                // item + 1: the tile wants no more keys of this item
 };
-__device__ __forceinline__ void publish_through(volatile EarlyStop &e, int warp, int item, int step) {
-  e.through[warp] = (unsigned long long)(unsigned)(item + 1) << 32 | (unsigned)step;
-}
-__device__ __forceinline__ bool all_through(const volatile EarlyStop &e, int item, int step) {
-  bool all = true;
-#pragma unroll
-  for (int w = 0; w < 4; ++w) {
-    const unsigned long long x = e.through[w];
-    all = all && (unsigned)(x >> 32) == (unsigned)(item + 1) && (int)(unsigned)x <= step;
-  }
-  return all;
+__device__ __forceinline__ void publish_through(volatile EarlyStop &e, int warp, int item) { e.through[warp] = item + 1; }
+__device__ __forceinline__ bool all_through(const volatile EarlyStop &e, int item) {
+  uint32_t a, b, c, d;
+  asm volatile("ld.volatile.shared.v4.u32 {%0, %1, %2, %3}, [%4];"
+               : "=r"(a), "=r"(b), "=r"(c), "=r"(d)
+               : "r"(smem_u32(const_cast<const int *>(&e.through[0])))
+               : "memory");
+  const uint32_t t = (uint32_t)item + 1u;
+  return ((a ^ t) | (b ^ t) | (c ^ t) | (d ^ t)) == 0u;
 }
 
 }  // namespace sb
