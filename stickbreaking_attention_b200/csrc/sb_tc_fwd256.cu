@@ -27,8 +27,9 @@ struct Cfg {
   static constexpr int kStageBytes = 2 * kKvTileBytes;         // K and V
   // K/V ring.  A stage is reloaded only after both tiles' P V MMAs of its step, and one tile runs a step ahead of the
   // other, so that of n stages n - 2 hide the load latency: with three the event log shows every S MMA at 128 columns
-  // waiting ~1000 of 2800 clk for its keys.  Four fit next to one staging box per tile; at 64 columns six do.
-  static constexpr int kStages = D == 64 ? 6 : 4;
+  // waiting ~1000 of 2800 clk for its keys.  Four fit next to one staging box per tile; at 64 columns six would, and are 1 %
+  // slower (more keys in flight than L2 likes).
+  static constexpr int kStages = 4;
   // Q tiles of two items at 64 columns (there is room): the next item's Q is loaded while the current item still
   // reads its own, so a short item does not wait a load latency for its first scores
   static constexpr int kQBufs = D == 64 ? 2 : 1;
