@@ -261,7 +261,7 @@ tc_fwd128x2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
       if (lane == 0) tma_store_wait_read();          // the previous tile's O has left the staging tile
       __syncwarp();
       int u = 0;
-      for (; u < w.n_steps && ok && (!kStop || s_reached < 0); ++u) {
+      for (; u < w.n_steps && ok; ++u) {
         const int s = w.s_top - u;
         const int gu = U + u, buf = gu & 1;
         ok = wait_or_abort(bar(bSFull + buf), (gu >> 1) & 1, abort_flag, p, 730);
@@ -275,39 +275,46 @@ tc_fwd128x2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
           zero_tile_rows(gbase + (sKV - base) + stop.word[buf] * kStageBytes + kKvTileBytes, tail_rows, kBN, 1, kKvTileBytes, r, kBM);
           fence_proxy_async_smem();
         }
-        bool done = !warp_live;
         float logsum = 0.f;
-        // (the P rows of such a warp keep whatever the slot held: they only reach accumulator rows that are never stored)
-        if (done) {
-        } else if (s >= s_diag0) fwd256_row_pass<kFp16, true>(ts, s * kBN, row, ac, scale2, run, logsum, ts + kPCol, true);
-        else done = fwd256_row_pass<kFp16, false>(ts, 0, 0, ac, scale2, run, logsum, ts + kPCol, row < w.c.len, !p.dense, kStop);
+        // (the P rows of a warp that is not live keep whatever was there: they only reach accumulator rows that are never stored)
+        if (!warp_live) {
+          if (kStop) break;
+        } else if (s >= s_diag0) {
+          fwd256_row_pass<kFp16, true>(ts, s * kBN, row, ac, scale2, run, logsum, ts + kPCol, true);
+        } else if (fwd256_row_pass<kFp16, false>(ts, 0, 0, ac, scale2, run, logsum, ts + kPCol, row < w.c.len, !p.dense, kStop)) {
+          break;
+        }
         run.add(logsum);
         tmem_wait_st();
         tc_fence_before();          // this step's TMEM reads and its writes of P are done before the slot is handed back
         __syncwarp();
-        if (lane == 0) {
-          if (kStop && done) publish_through(stop, warp & 3, it);
-          mbar_arrive(bar(bPFull + buf));
-        }
-        if (kStop && done) s_reached = s + 1;
-      }
-      // through: zeros for P until the other warps of the tile are as well (the sequence's tail is behind these steps)
-      for (; kStop && u < w.n_steps && ok; ++u) {
-        const int gu = U + u, buf = gu & 1;
-        ok = wait_or_abort(bar(bSFull + buf), (gu >> 1) & 1, abort_flag, p, 731);
-        if (!ok) break;
-        const bool halt = stop.word[buf] == kStepStop;
-        if (!halt) {
-          tc_fence_after();
-          fwd256_zero_row(tmem + buf * 64 + lane_off + kPCol);
-          tmem_wait_st();
-          tc_fence_before();
-        }
-        __syncwarp();
         if (lane == 0) mbar_arrive(bar(bPFull + buf));
-        if (halt) {
-          slots = u + 1;
-          break;
+      }
+      // Through (the scores of step u are there, and count for nothing): zeros for P until the other warps of the tile are as
+      // well.  The sequence's tail is behind these steps.
+      if (kStop && u < w.n_steps && ok) {
+        s_reached = w.s_top - u + 1;
+        if (lane == 0) publish_through(stop, warp & 3, it);
+        for (bool first = true; u < w.n_steps && ok; ++u, first = false) {
+          const int gu = U + u, buf = gu & 1;
+          bool halt = false;
+          if (!first) {
+            ok = wait_or_abort(bar(bSFull + buf), (gu >> 1) & 1, abort_flag, p, 331);
+            if (!ok) break;
+            halt = stop.word[buf] == kStepStop;
+          }
+          if (!halt) {
+            tc_fence_after();
+            fwd256_zero_row(tmem + buf * 64 + lane_off + kPCol);
+            tmem_wait_st();
+            tc_fence_before();
+          }
+          __syncwarp();
+          if (lane == 0) mbar_arrive(bar(bPFull + buf));
+          if (halt) {
+            slots = u + 1;
+            break;
+          }
         }
       }
       // ---- epilogue: O (TMEM) -> global, rem, log_rem

@@ -304,9 +304,9 @@ tc_fwd256_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
       if (lane == 0) tma_store_wait_read();   // the previous item's O has left the staging boxes
       __syncwarp();
       if ((threadIdx.x & 127) == 0) trace_event(p, 2 + wg, tr_cur, 40 + wg, it);
-      // (two loops: with the steps of a warp that is through inside the first one, every step of every warp took 5 % longer)
+      // (two loops: with the steps of a warp that is through in the first one, every step of every warp took 5 % longer)
       int u = 0;
-      for (; u < my_steps && ok && s_reached < 0; ++u) {
+      for (; u < my_steps && ok; ++u) {
         const int s = w.s_top - (t0 + u);
         const int gu = U + u, buf = gu & 1;
         ok = wait_or_abort(bar(bSFull + wg * 2 + buf), (gu >> 1) & 1, abort_flag, p, 330);
@@ -323,41 +323,47 @@ tc_fwd256_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
           zero_tile_rows(v_tile, tail_rows, kBN, kBoxes, kKvBoxBytes, r, kBM);
           fence_proxy_async_smem();
         }
-        bool done = !warp_live;
         float logsum = 0.f;
-        // 64 columns in chunks of 16, last chunk first; TMEM is read one chunk ahead of the arithmetic
-        // (the P rows of such a warp keep whatever their buffer held: they only reach accumulator rows that are never stored)
-        if (done) {
-        } else if (s >= s_diag0) fwd256_row_pass<kFp16, true>(ts, s * kBN, row, ac, scale2, run, logsum, ts + kPCol, true);
-        else done = fwd256_row_pass<kFp16, false>(ts, 0, 0, ac, scale2, run, logsum, ts + kPCol, row < w.c.len, !p.dense, may_stop);
+        // (the P rows of a warp that is not live keep whatever was there: they only reach accumulator rows that are never stored)
+        if (!warp_live) {
+          if (may_stop) break;
+        } else if (s >= s_diag0) {
+          fwd256_row_pass<kFp16, true>(ts, s * kBN, row, ac, scale2, run, logsum, ts + kPCol, true);
+        } else if (fwd256_row_pass<kFp16, false>(ts, 0, 0, ac, scale2, run, logsum, ts + kPCol, row < w.c.len, !p.dense, may_stop)) {
+          break;
+        }
         run.add(logsum);
         tmem_wait_st();
         tc_fence_before();          // this step's TMEM reads and writes of P are done before the slot is handed back
         __syncwarp();
-        if (lane == 0) {
-          if (may_stop && done) publish_through(stop, warp & 3, it);
-          mbar_arrive(bar(bPFull + wg * 2 + buf));
-        }
-        if (may_stop && done) s_reached = s + 1;
+        if (lane == 0) mbar_arrive(bar(bPFull + wg * 2 + buf));
         if ((threadIdx.x & 127) == 0) trace_event(p, 2 + wg, tr_cur, 5 + 16 * wg, t0 + u);
       }
-      // through: zeros for P until the other warps of the tile are as well (the sequence's tail is behind these steps)
-      for (; u < my_steps && ok; ++u) {
-        const int gu = U + u, buf = gu & 1;
-        ok = wait_or_abort(bar(bSFull + wg * 2 + buf), (gu >> 1) & 1, abort_flag, p, 331);
-        if (!ok) break;
-        const bool halt = stop.word[buf] == kStepStop;
-        if (!halt) {
-          tc_fence_after();
-          fwd256_zero_row(tmem + wg * 128 + buf * 64 + lane_off + kPCol);
-          tmem_wait_st();
-          tc_fence_before();
-        }
-        __syncwarp();
-        if (lane == 0) mbar_arrive(bar(bPFull + wg * 2 + buf));
-        if (halt) {
-          slots = u + 1;
-          break;
+      // Through (the scores of step u are there, and count for nothing): zeros for P until the other warps of the tile are as
+      // well.  The sequence's tail is behind these steps.
+      if (may_stop && u < my_steps && ok) {
+        s_reached = w.s_top - (t0 + u) + 1;
+        if (lane == 0) publish_through(stop, warp & 3, it);
+        for (bool first = true; u < my_steps && ok; ++u, first = false) {
+          const int gu = U + u, buf = gu & 1;
+          bool halt = false;
+          if (!first) {
+            ok = wait_or_abort(bar(bSFull + wg * 2 + buf), (gu >> 1) & 1, abort_flag, p, 331);
+            if (!ok) break;
+            halt = stop.word[buf] == kStepStop;
+          }
+          if (!halt) {
+            tc_fence_after();
+            fwd256_zero_row(tmem + wg * 128 + buf * 64 + lane_off + kPCol);
+            tmem_wait_st();
+            tc_fence_before();
+          }
+          __syncwarp();
+          if (lane == 0) mbar_arrive(bar(bPFull + wg * 2 + buf));
+          if (halt) {
+            slots = u + 1;
+            break;
+          }
         }
       }
       // ---- epilogue: O (TMEM) -> global, rem, log_rem

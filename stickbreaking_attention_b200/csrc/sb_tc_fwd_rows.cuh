@@ -136,8 +136,7 @@ __device__ __forceinline__ void fwd256_logsum_pass(uint32_t ts, float scale2, fl
 // every row of the warp (its 32 rows are consecutive and 32-aligned): such 32-column halves are not computed at all,
 // their P is zero and R and logsum stay as they are -- 6 of the 16 (warp, half) pairs of a diagonal 128 x 128 tile.
 // An unmasked sub-tile whose P is exactly zero for all rows of the warp that exist (their product has underflowed) only
-// sums its logs (skip_zero), or not even that (drop_zero: log_rem is to cover the keys up to here only); the pass then
-// returns true.
+// sums its logs (skip_zero).  drop_zero: it does nothing instead and returns true, log_rem is to cover the keys up to here.
 template <bool kFp16, bool kMasked>
 __device__ __forceinline__ bool fwd256_row_pass(uint32_t ts, int key0, int row, int ac, float scale2, const LogSum &sum,
                                                 float &logsum, uint32_t tmem_p, bool exists, bool skip_zero = false, bool drop_zero = false) {
@@ -162,9 +161,9 @@ __device__ __forceinline__ bool fwd256_row_pass(uint32_t ts, int key0, int row, 
     if (zero) {
       // The product over the keys after this sub-tile has underflowed to exactly 0 for all rows of the warp: every p of
       // the sub-tile is e * 0 = 0 (e is finite: its exponent is clamped).
-      if (drop_zero) fwd256_zero_row(tmem_p);
-      else fwd256_logsum_pass(ts, scale2, logsum, tmem_p, va);
-      return true;
+      if (drop_zero) return true;
+      fwd256_logsum_pass(ts, scale2, logsum, tmem_p, va);
+      return false;
     }
   }
   float l3 = 0.f, l2 = 0.f;   // log sums of the upper pair of chunks
