@@ -508,67 +508,94 @@ tc_bwd_dq2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
     // this row's part of the workspace for sub-tile 0: A, or the boundary records [pair (I, J)][quarter of the key tile][row]
     const long long pair00 = (long long)(kStored ? 2 * hh : hh) * p.pairs_cap + c.pair0 + (long long)I * (I + 1) / 2;
     char *out = kStored ? reinterpret_cast<char *>(p.az + (pair00 * kBM + r) * kBM) : reinterpret_cast<char *>(p.bnd_r1 + pair00 * (4 * kBM) + r);
-    const bool ragged = row0 + kBM > c.len;      // the sequence ends inside this tile
     const int u_diag = 2 * I, u_tail = c.len / kBN;   // a sub-tile with rows past the sequence is number u_tail
     // this warp's rows start at sub-tile u_warp (never, if they are past the sequence): before it, A and dz are zeros
     const int u_warp = row0 + (r & ~31) < c.len ? first_key(p, c, h, row0 + (r & ~31)) / kBN : 0x7fffffff;
     // Where the forward has said where each warp's rows start, hardly a chunk of zeros is left, and the test for them costs
     // every chunk a tenth of its instructions.
     const bool skip = p.tile_start == nullptr && !p.dense;
+    const long long s2_off = kStored ? 0 : p.bnd_s2 - p.bnd_r1;
     bool ok = true;
+    // One step: `pass` does the rows of sub-tile u, `dst` is its part of this row's workspace.  Zeros up to the warp's first
+    // key, then full sub-tiles, then the diagonal: three loops, because what the kinds of step need would otherwise be kept in
+    // registers for one another (see the forward's row loop).
     // u: 64-key sub-tile inside the sequence; the first one is even, so that phases follow from u alone
-    for (int u = w == 0 ? first_a : first_b; u < my_steps && ok; ++u) {
+    int u = w == 0 ? first_a : first_b;
+    auto step = [&](auto pass, auto tail) {
       ok = wait_or_abort(bars + 8u * bSFull, u & 1, abort_flag, p, 530);
-      if (!ok) break;
+      if (!ok) return;
       if (r == 0) trace_event(p, 2 + w, tr_cur, 4 + 16 * w, u);
       tc_fence_after();
-      const float r1f = r1 + r1_lo;
-      float gs = 0.f, logsum = 0.f;
-      bool pass_ok;
-      // a tile with rows past the sequence end takes the masking variant throughout: those rows must be zero in the
-      // stored tiles (the dK/dV GEMMs sum over all 128 query rows)
-      const bool on_diag = u >= u_diag;
-      void *dst;
-      long long s2_off = 0;
-      if constexpr (kStored) {
-        dst = out + ((long long)(u >> 1) * (kBM * kBM) + (u & 1) * kBN) * 2;
-      } else {
-        dst = out + (long long)u * (2 * kBM * sizeof(float));
-        s2_off = p.bnd_s2 - p.bnd_r1;
-        reinterpret_cast<float *>(dst)[0] = u < u_warp ? kNothingLeft : r1f;
-        reinterpret_cast<float *>(dst)[s2_off] = gpre;
-      }
-      if (u < u_warp)
-        pass_ok = zero_strip_row<kStored>(gZ, r, u, bars, dst, s2_off);
-      else if (on_diag || (kStored && ragged))
-        pass_ok = strip_row_pass<kFp16, true, kStored, false>(tS, tP, r, u, on_diag ? (u - u_diag) * kBN : 0,
-                                                       chunk_limit(valid || !kStored, on_diag, r, p.attend_current), scale2, r1f, gpre, dr,
-                                                       gs, logsum, gZ, bars, dst, s2_off);
-      else if (skip)
-        pass_ok = strip_row_pass<kFp16, false, kStored, true>(tS, tP, r, u, 0, 0, scale2, r1f, gpre, dr, gs, logsum, gZ, bars, dst, s2_off);
-      else
-        pass_ok = strip_row_pass<kFp16, false, kStored, false>(tS, tP, r, u, 0, 0, scale2, r1f, gpre, dr, gs, logsum, gZ, bars, dst, s2_off);
-      if (!pass_ok) {   // a bounded wait inside the pass gave up
+      void *dst = kStored ? out + ((long long)(u >> 1) * (kBM * kBM) + (u & 1) * kBN) * 2 : out + (long long)u * (2 * kBM * sizeof(float));
+      if (!pass(dst)) {   // a bounded wait inside the pass gave up
         *abort_flag = 1;
         if (p.status != nullptr) { p.status[0] = SB_DEV_WAIT_TIMEOUT; p.status[1] = 531; }
         ok = false;
       }
-      {   // r1 += logsum
-        const float sum = r1 + logsum, b = sum - r1;
-        r1_lo += (r1 - (sum - b)) + (logsum - b);
-        r1 = sum;
-      }
-      gpre += gs;
       // the sequence ends inside this sub-tile: its dz columns behind the end are exact zeros, the K rows there are
       // not this sequence's (see zero_tile_rows) and are cleared before this step's dz K MMA is released
-      if (u == u_tail)
+      if (decltype(tail)::value && u == u_tail)
         zero_tile_rows(gbase + (sKV - base) + ((u - item.first) % kStages) * kStageBytes, item.len - u * kBN, kBN, kBoxes, kKvBox, r, kBM);
       tc_fence_before();          // this step's TMEM reads are done before the slots are handed back
       fence_proxy_async_smem();
       __syncwarp();
       if (r == 0) trace_event(p, 2 + w, tr_cur, 5 + 16 * w, u);
       if (lane == 0) mbar_arrive(bars + 8u * bZFull);
+    };
+    auto record = [&](void *dst, float r1f) {
+      if constexpr (!kStored) {
+        reinterpret_cast<float *>(dst)[0] = r1f;
+        reinterpret_cast<float *>(dst)[s2_off] = gpre;
+      }
+    };
+    auto carry = [&](float logsum, float gs) {   // r1 += logsum, gpre += gs
+      const float sum = r1 + logsum, b = sum - r1;
+      r1_lo += (r1 - (sum - b)) + (logsum - b);
+      r1 = sum;
+      gpre += gs;
+    };
+    using std::false_type; using std::true_type;
+    for (; u < min(u_warp, my_steps) && ok; ++u)
+      step([&](void *dst) {
+        record(dst, kNothingLeft);
+        return zero_strip_row<kStored>(gZ, r, u, bars, dst, s2_off);
+      }, true_type());
+    // rows past the sequence end must be zero in the stored tiles (the dK/dV GEMMs sum over all 128 query rows): the warp that
+    // holds the end masks throughout
+    const int u_full = kStored && row0 + (r | 31) >= c.len ? 0 : min(u_diag, my_steps);
+    if (!skip) {
+      for (; u < u_full && ok; ++u)
+        step([&](void *dst) {
+          const float r1f = r1 + r1_lo;
+          float gs = 0.f, logsum = 0.f;
+          record(dst, r1f);
+          const bool good = strip_row_pass<kFp16, false, kStored, false>(tS, tP, r, u, 0, 0, scale2, r1f, gpre, dr, gs, logsum, gZ, bars, dst, s2_off);
+          carry(logsum, gs);
+          return good;
+        }, false_type());
+    } else {
+      for (; u < u_full && ok; ++u)
+        step([&](void *dst) {
+          const float r1f = r1 + r1_lo;
+          float gs = 0.f, logsum = 0.f;
+          record(dst, r1f);
+          const bool good = strip_row_pass<kFp16, false, kStored, true>(tS, tP, r, u, 0, 0, scale2, r1f, gpre, dr, gs, logsum, gZ, bars, dst, s2_off);
+          carry(logsum, gs);
+          return good;
+        }, false_type());
     }
+    for (; u < my_steps && ok; ++u)
+      step([&](void *dst) {
+        const bool on_diag = u >= u_diag;
+        const float r1f = r1 + r1_lo;
+        float gs = 0.f, logsum = 0.f;
+        record(dst, r1f);
+        const bool good = strip_row_pass<kFp16, true, kStored, false>(tS, tP, r, u, on_diag ? (u - u_diag) * kBN : 0,
+                                                                      chunk_limit(valid || !kStored, on_diag, r, p.attend_current), scale2, r1f,
+                                                                      gpre, dr, gs, logsum, gZ, bars, dst, s2_off);
+        carry(logsum, gs);
+        return good;
+      }, true_type());
     // the dz buffer is reused by the epilogue: its last tile has been read (in stored-tiles mode by the store as well)
     if (ok && my_steps > 0) ok = wait_or_abort(bars + 8u * bZEmpty, (my_steps - 1) & 1, abort_flag, p, 533);
     if (ok && my_steps > 0) ok = wait_or_abort(bar(bDqFull + w), 0, abort_flag, p, 532);
