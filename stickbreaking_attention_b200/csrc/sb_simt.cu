@@ -696,6 +696,9 @@ __global__ void __launch_bounds__(kSimtThreads, kSimtBlocks<DP>) simt_bwd_dq_ker
     __syncthreads();
     tile_dot<DP, kT, kStep>(Ps, Gs, Vs, 1.f);
     __syncthreads();
+    // V is done with: the next K goes into its buffer while this step goes on, and the next V into this K's
+    const bool more = key0 + kStep <= row0;
+    if (more) lk.issue(Vs, p.k, c, h, key0 + kStep, d, wide);
     {
       float z[16], dp[16];
       float *zrow = Zs + r * kLdS + seg * 16;
@@ -720,14 +723,12 @@ __global__ void __launch_bounds__(kSimtThreads, kSimtBlocks<DP>) simt_bwd_dq_ker
       gpre += gs;
     }
     __syncthreads();
-    const bool more = key0 + kStep <= row0;
     tile_pv<DP>(acc, Zs, Ks);
+    if (more) lk.land(Vs);
     __syncthreads();
-    if (more) {
-      lk.issue(Ks, p.k, c, h, key0 + kStep, d, wide);
-      lk.land(Ks);
-      __syncthreads();
-    }
+    float *tmp = Ks;
+    Ks = Vs;
+    Vs = tmp;
   }
 
   const int tx = t % 16, ty = t / 16;
@@ -784,30 +785,59 @@ __global__ void __launch_bounds__(kSimtThreads, kSimtBlocks<DP>) simt_bwd_dkv_ke
   }
   __syncthreads();
   float dk[4][DP / 16] = {}, dv[4][DP / 16] = {};
-  for (int off = 0; off < list.n;) {   // two of the query tiles that reach this key tile per step
-    const int I0 = J + off, off1 = list.next(off + 1), I1 = J + off1;   // I1 == n_tiles: rows past the sequence, zeros
-    off = list.next(off1 + 1);
+  // Two of the query tiles that reach this key tile per step: I0 and I1 (== n_tiles: rows past the sequence, zeros).
+  int off = 0, I0 = J, I1 = J + list.next(1);
+  auto advance = [&] {
+    off = list.next(I1 - J + 1);
+    I0 = J + off;
+    I1 = J + list.next(off + 1);
+  };
+  auto load_q = [&] {
     lq.issue(Qs, p.q, c, h, I0 * kT, d, wide);
-    lg.issue(Gs, p.d_o, c, h, I0 * kT, d, wide);
     lq1.issue(Qs + kT * kLd<DP>, p.q, c, h, I1 * kT, d, wide);
+  };
+  auto load_g = [&] {
+    lg.issue(Gs, p.d_o, c, h, I0 * kT, d, wide);
     lg1.issue(Gs + kT * kLd<DP>, p.d_o, c, h, I1 * kT, d, wide);
-    if constexpr (kStored) {   // 64 query rows x (32 A, 32 dz): 16 float4 per row
+  };
+  if constexpr (kStored) {
+    auto load_stored = [&](float *dst, int part) {   // 64 query rows of A (part 0) or dz (part 1): 8 float4 per row
 #pragma unroll
-      for (int i = 0; i < kStep * 16 / kSimtThreads; ++i) {
-        const int e = t + i * kSimtThreads, row = e >> 4, x = (e & 15) * 4;
+      for (int i = 0; i < kStep * 8 / kSimtThreads; ++i) {
+        const int e = t + i * kSimtThreads, row = e >> 3, x = (e & 7) * 4;
         const int Ir = row < kT ? I0 : I1;
         const bool take = Ir < c.n_tiles;
         const long long pair = (long long)hh * p.pairs_cap + c.pair0 + (long long)Ir * (Ir + 1) / 2 + J;
-        const float *src = reinterpret_cast<const float *>(p.az) + (take ? (pair * kT + (row & 31)) * (2 * kT) + x : 0);
-        cp_async16((x < kT ? Ps + row * kLdH + x : Zs + row * kLdH + x - kT), src, take);
+        const float *src = reinterpret_cast<const float *>(p.az) + (take ? (pair * kT + (row & 31)) * (2 * kT) + part * kT + x : 0);
+        cp_async16(dst + row * kLdH + x, src, take);
       }
+    };
+    // the operands of either product arrive while the other one runs
+    load_q();
+    load_stored(Zs, 1);
+    while (off < list.n) {
       lq.land(Qs);
-      lg.land(Gs);
       lq1.land(Qs + kT * kLd<DP>);
+      cp_async_wait();
+      __syncthreads();
+      load_g();
+      load_stored(Ps, 0);
+      tile_ptb<DP>(dk, Zs, Qs);
+      lg.land(Gs);
       lg1.land(Gs + kT * kLd<DP>);
       cp_async_wait();
       __syncthreads();
-    } else {
+      advance();
+      if (off < list.n) {
+        load_q();
+        load_stored(Zs, 1);
+      }
+      tile_ptb<DP>(dv, Ps, Gs);
+    }
+  } else {
+    for (; off < list.n; advance()) {
+      load_q();
+      load_g();
       lq.land(Qs);
       lg.land(Gs);
       lq1.land(Qs + kT * kLd<DP>);
@@ -833,10 +863,10 @@ __global__ void __launch_bounds__(kSimtThreads, kSimtBlocks<DP>) simt_bwd_dkv_ke
       store16(Zs + row * kLdH + seg * 16, z);
       store16(Ps + row * kLdH + seg * 16, dp);
       __syncthreads();
+      tile_ptb<DP>(dk, Zs, Qs);
+      tile_ptb<DP>(dv, Ps, Gs);
+      __syncthreads();
     }
-    tile_ptb<DP>(dk, Zs, Qs);
-    tile_ptb<DP>(dv, Ps, Gs);
-    __syncthreads();
   }
 
   const int tx = t % 16, ty = t / 16;
