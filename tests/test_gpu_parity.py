@@ -353,6 +353,29 @@ def test_cuda_core_kernels_at_tile_edges(sb, cuda_device, d, dtype, mode):
         H.assert_parity(got, want, dtype, f"CUDA-core d={d} {mode} ac={ac}")
 
 
+@pytest.mark.parametrize("mode", ["stored", "recompute"])
+@pytest.mark.parametrize("d,dtype", [(128, torch.bfloat16), (64, torch.float16), (64, torch.float32), (50, torch.bfloat16)])
+def test_starting_where_the_forward_stopped(sb, cuda_device, d, dtype, mode):
+    """N(0, 1) scores use the stick up after some 110 keys, so tiles of longer sequences stop early, at different keys per
+    warp; a second half of the heads with low scores does not stop.  Against a run that visits every key: the same bits on
+    the tensor cores, the same to rounding of the carried sums on the CUDA cores."""
+    lengths = [1500, 129, 700, 65, 192]
+    q, k, v, do, drem = H.make_inputs((4, sum(lengths), d), dtype, seed=5 + d)
+    q[2:] *= 0.05
+    k[3] -= 1.0
+    q[3] += 0.5
+    cu = cu_of(lengths)
+    with sb.small_backward_workspace(mode == "recompute"):
+        got = H.run_varlen(sb, q, k, v, do, drem, cu, cuda_device, max_seqlens=1500)
+        with sb.dense_row_pass():
+            want = H.run_varlen(sb, q, k, v, do, drem, cu, cuda_device, max_seqlens=1500)
+    for name, a, b in zip(("o", "rem", "dq", "dk", "dv"), got, want):
+        if dtype == torch.float32 or d % 8:
+            assert H.rel_l2(a, b) <= (1e-6 if dtype == torch.float32 else 1e-3), name
+        else:
+            assert torch.equal(a, b), name
+
+
 @pytest.mark.parametrize("dtype,d", [(torch.bfloat16, 64), (torch.bfloat16, 128), (torch.float32, 32)])
 @pytest.mark.parametrize("lengths", [[1], [300, 0, 5] * 20, [7] * 128, [7] * 129, [40] * 120 + [900], [1100, 1] * 3, [1500, 1, 130, 300]])
 def test_item_tables_at_their_limits(sb, cuda_device, dtype, d, lengths):
