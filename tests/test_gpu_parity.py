@@ -371,7 +371,7 @@ def test_starting_where_the_forward_stopped(sb, cuda_device, d, dtype, mode):
             want = H.run_varlen(sb, q, k, v, do, drem, cu, cuda_device, max_seqlens=1500)
     for name, a, b in zip(("o", "rem", "dq", "dk", "dv"), got, want):
         if dtype == torch.float32 or d % 8:
-            assert H.rel_l2(a, b) <= (1e-6 if dtype == torch.float32 else 1e-3), name
+            assert H.rel_l2(a, b) <= (2e-5 if dtype == torch.float32 else 1e-3), name
         else:
             assert torch.equal(a, b), name
 
