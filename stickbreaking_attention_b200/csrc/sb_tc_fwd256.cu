@@ -270,6 +270,10 @@ tc_fwd256_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
           if (!ok) break;
         } else if (!active) {
           release(0, w.n_steps);
+          // No accumulator to wait for, but the rows have to have seen the previous item's bOFull: with two idle items in a
+          // row this thread could complete two of its phases while they are in an epilogue or look an item up, and their
+          // parity wait would then be for a phase that only they could bring about.
+          if (ok && it >= 1) ok = wait_or_abort(bar(bOFree + wg), (it - 1) & 1, abort_flag, p, 327);
           if (!ok) break;
         }
         if (!active) mma_commit(bar_qfree);   // after this thread's earlier MMAs, like every arrival on these two

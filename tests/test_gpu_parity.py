@@ -353,6 +353,23 @@ def test_cuda_core_kernels_at_tile_edges(sb, cuda_device, d, dtype, mode):
         H.assert_parity(got, want, dtype, f"CUDA-core d={d} {mode} ac={ac}")
 
 
+@pytest.mark.parametrize("dtype,d", [(torch.bfloat16, 128), (torch.float16, 64)])
+@pytest.mark.parametrize("num,low,high", [(130, 8, 300), (60, 8, 300), (64, 64, 256), (300, 1, 140)])
+def test_items_with_and_without_a_second_tile_in_turn(sb, cuda_device, dtype, d, num, low, high):
+    """Sequences around 128 tokens: 256-row items whose second tile is missing follow each other and items that have both,
+    several times per block.  Enough heads for that; the first is compared with the oracle, its copies with it."""
+    gen = torch.Generator().manual_seed(num)
+    lengths = torch.randint(low, high + 1, (num,), generator=gen).tolist()
+    q, k, v, do, drem = (t.repeat(16, *[1] * (t.dim() - 1)) for t in H.make_inputs((1, sum(lengths), d), dtype, seed=num, recipe="reference"))
+    cu = cu_of(lengths)
+    for _ in range(3):
+        got = H.run_varlen(sb, q, k, v, do, drem, cu, cuda_device, max_seqlens=2048)   # (the 256-row kernel at either width)
+        sb.check_status(cuda_device)
+    for t in got:
+        assert torch.equal(t, t[:1].expand_as(t))
+    H.assert_parity([t[:1] for t in got], H.oracle_varlen(*(t[:1] for t in (q, k, v, do, drem)), cu), dtype, f"{num} sequences")
+
+
 @pytest.mark.parametrize("mode", ["stored", "recompute"])
 @pytest.mark.parametrize("d,dtype", [(128, torch.bfloat16), (64, torch.float16), (64, torch.float32), (50, torch.bfloat16)])
 def test_starting_where_the_forward_stopped(sb, cuda_device, d, dtype, mode):
