@@ -179,20 +179,24 @@ __device__ __forceinline__ bool build_small_table(const KParams &p, int group, S
   // of the same class in the sequences before, then the heavier ones of its own.
   for (int i = t; i < kSmallItems; i += blockDim.x) tb.order[i] = 0xffffffffu;
   __syncthreads();
-  for (int s = 0, first = 0; s < p.num_seq; ++s) {
-    const int m = ((int)tb.pair0[s] + group - 1) / group;
-    for (int e = t - first % (int)blockDim.x; e < m; e += blockDim.x) {   // spread over the threads across sequences
-      if (e < 0) continue;
-      const int lo = e / span * span, hi = lo + span;
-      int pos = min(hi, m) - 1 - e;
-      for (int q = 0; q < p.num_seq; ++q) {
-        const int mq = ((int)tb.pair0[q] + group - 1) / group;
-        pos += max(mq - hi, 0);
-        if (q < s) pos += min(max(mq - lo, 0), span);
-      }
-      tb.order[pos] = (uint32_t)s << 16 | (uint32_t)(e * group);
+  // One pass to find the thread's entry and one to place it: placing the entries while walking the sequences would let a
+  // warp run the inner loop once per sequence that its threads hold (8 heads, 16000 tokens in sequences of 32 to 1000: 77 us, now 55).
+  for (int i = t; i < kSmallItems; i += blockDim.x) {
+    int s = 0, e = i, m = 0;
+    for (; s < p.num_seq; ++s) {
+      m = ((int)tb.pair0[s] + group - 1) / group;
+      if (e < m) break;
+      e -= m;
     }
-    first += m;
+    if (s == p.num_seq) break;
+    const int lo = e / span * span, hi = lo + span;
+    int pos = min(hi, m) - 1 - e;
+    for (int q = 0; q < p.num_seq; ++q) {
+      const int mq = ((int)tb.pair0[q] + group - 1) / group;
+      pos += max(mq - hi, 0);
+      if (q < s) pos += min(max(mq - lo, 0), span);
+    }
+    tb.order[pos] = (uint32_t)s << 16 | (uint32_t)(e * group);
   }
   uint32_t before = 0;
   if (t < p.num_seq)
