@@ -450,11 +450,13 @@ __device__ __forceinline__ void tile_ptb(float (&acc)[4][DP / 16], const float *
 
 // One lane's 16 keys of a row: beta and 1 - beta per key, and the sum of softplus(z) over the allowed ones.
 //   u = e^-|z|, t = 1 + u in (1, 2]:  beta = (z > 0 ? 1 : u) / t,  1 - beta = (z > 0 ? u : 1) / t,
-//   softplus(z) = max(z, 0) + log t;  16 factors t share one logarithm, and what rounding 1 + u to fp32 dropped comes back
-//   to first order ((u - (t - 1)) / t), so that the sum is as good as 16 log1p.
+//   softplus(z) = max(z, 0) + log t;  16 factors t share one logarithm.  What the roundings of 1 + u and of the product
+//   dropped is carried along (`rest`, exact to first order) and comes back as rest / prod, so that the sum is as good as
+//   16 log1p.  (Without the product's part a head whose scores lie around -12 loses the factors near 1 altogether: log_rem
+//   off by 7e-5 instead of 2e-8.)
 // Keys [key0, key0 + 16) below `limit` are allowed, negative ones never.
 __device__ __forceinline__ float stick_segment(float (&z)[16], int key0, int limit, float (&beta)[16], float (&keep)[16]) {
-  float lin = 0.f, prod = 1.f, comp = 0.f;
+  float lin = 0.f, prod = 1.f, rest = 0.f;   // the product of the exact factors is prod + rest
 #pragma unroll
   for (int j = 0; j < 16; ++j) {
     const bool on = key0 + j >= 0 && key0 + j < limit;
@@ -463,10 +465,11 @@ __device__ __forceinline__ float stick_segment(float (&z)[16], int key0, int lim
     beta[j] = on ? (pos ? rt : u * rt) : 0.f;
     keep[j] = on ? (pos ? u * rt : rt) : 1.f;
     lin += on && pos ? z[j] : 0.f;
-    prod *= on ? t : 1.f;
-    comp += on ? (u - (t - 1.f)) * rt : 0.f;
+    const float factor = on ? t : 1.f, dropped = on ? u - (t - 1.f) : 0.f, next = prod * factor;
+    rest = fmaf(rest, factor, fmaf(prod, dropped, fmaf(prod, factor, -next)));
+    prod = next;
   }
-  return lin + (logf(prod) + comp);
+  return lin + (logf(prod) + rest * __frcp_rn(prod));
 }
 __device__ __forceinline__ void load16(float (&x)[16], const float *src) {
 #pragma unroll

@@ -532,6 +532,28 @@ def test_skipping_exact_zeros_changes_no_bit(sb, cuda_device, d, dtype, mode):
     H.assert_parity(fast, H.oracle_varlen(*ins, cu), dtype, "zeros skipped")
 
 
+@pytest.mark.parametrize("d,n,mean", [(64, 1024, -7.4), (33, 700, -12.0), (64, 300, -3.0), (128, 515, 0.0), (64, 130, 4.0)])
+def test_fp32_log_sums_against_64_bits(sb, cuda_device, d, n, mean):
+    """rem and log_rem of the CUDA-core kernels over score ranges from a stick that hardly gets shorter per key (all factors
+    1 + exp(z) next to 1) to one that is used up.  Bound on log_rem, a sum of softplus(z) terms of one sign: the relative error
+    of a term (two units of expf, one each for the logarithm and the sums of 64 in fp32, 2^-23 apiece), plus what z brings from
+    its own fp32 sums of d terms (random signs: 2^-24 sqrt(d) |z| per key, a root of n less over n keys)."""
+    gen = torch.Generator().manual_seed(d + n)
+    q, k, v = (torch.randn(2, n, d, generator=gen) for _ in range(3))
+    shift = math.sqrt(abs(mean) / math.sqrt(d))
+    q += shift
+    k += math.copysign(shift, mean)
+    cu = cu_of([n])
+    o, rem, log_rem = (t.cpu().double() for t in sb.ops.varlen_fwd(q.to(cuda_device), k.to(cuda_device), v.to(cuda_device), cu.to(cuda_device),
+                                                                   n, 1 / math.sqrt(d)))
+    z = q.double() @ k.double().transpose(1, 2) / math.sqrt(d)
+    lost = torch.nn.functional.softplus(z).tril(-1).sum(-1)
+    dz = 2.0 ** -24 * math.sqrt(d / n) * float(z.square().mean().sqrt())
+    bound = 4 * 2.0 ** -23 + dz
+    assert H.rel_l2(-log_rem * math.log(2.0), lost) <= bound
+    assert H.rel_l2(rem, (-lost).exp()) <= (1 + float(lost.max())) * bound
+
+
 # ---- error behaviour: failures are made on the host, never by faulting the device -----------------------
 
 def test_bad_cu_seqlens_is_reported_not_executed(sb, cuda_device):
