@@ -9,7 +9,8 @@
  *
  * Tensor convention (same as the reference operators): q, k, v, o and their gradients are
  * (batch, heads, tokens, head_dim) with arbitrary element strides for the first three axes and a
- * unit stride on head_dim.  A packed variable-length batch is batch == 1 with `cu_seqlens` holding
+ * unit stride on head_dim; the stride of an axis of one element does not matter, and a stride of 0 (an axis whose elements are
+ * all the same) is taken by the CUDA-core kernels.  A packed variable-length batch is batch == 1 with `cu_seqlens` holding
  * the END offset of every sequence (no leading zero), exactly what
  * stickbreaking_attention/sb_varlen/__init__.py:71-78 hands to its kernels after stripping the zero.
  * A fixed-length batch passes cu_seqlens == NULL.

@@ -59,10 +59,12 @@ static int check_tensor(const SbTensor &t, const char *name, bool required) {
   return SB_OK;
 }
 
-static bool tma_friendly(const SbTensor &t, int esize) {
-  if (reinterpret_cast<uintptr_t>(t.ptr) % 16) return false;
+// Whether tensor maps and 16-byte vectors can address the tensor.  An axis of one element has no stride to speak of; an axis
+// that repeats its elements (stride 0) has no place in a tensor map and is left to the CUDA-core kernels.
+static bool tma_friendly(const SbTensor &t, const SbParams &p, int esize) {
   const long long m = 16 / esize;
-  return t.stride_t % m == 0 && t.stride_h % m == 0 && t.stride_b % m == 0 && t.stride_t > 0;
+  auto axis = [m](long long extent, long long stride) { return extent <= 1 || (stride > 0 && stride % m == 0); };
+  return reinterpret_cast<uintptr_t>(t.ptr) % 16 == 0 && axis(p.tokens, t.stride_t) && axis(p.heads, t.stride_h) && axis(p.batch, t.stride_b);
 }
 
 static int make_plan(const SbParams *p, Plan &pl, bool backward) {
@@ -85,11 +87,11 @@ static int make_plan(const SbParams *p, Plan &pl, bool backward) {
   const int esize = p->dtype == SB_DTYPE_F32 ? 4 : 2;
   bool tc = !(p->flags & SB_FLAG_FORCE_SIMT) && !(p->attn_weights != nullptr && !backward) &&
             tc_supported(p->dtype, p->head_dim, backward) &&
-            tma_friendly(p->q, esize) && tma_friendly(p->k, esize) && tma_friendly(p->v, esize);
+            tma_friendly(p->q, *p, esize) && tma_friendly(p->k, *p, esize) && tma_friendly(p->v, *p, esize);
   // outputs and gradients are stored with 16-byte vectors on the tensor-core path
   const SbTensor *others[] = {&p->o, &p->d_o, &p->dq, &p->dk, &p->dv};
   for (const SbTensor *t : others)
-    if (t->ptr != nullptr && !tma_friendly(*t, esize)) tc = false;
+    if (t->ptr != nullptr && !tma_friendly(*t, *p, esize)) tc = false;
   pl.path = tc ? SB_PATH_TCGEN05 : SB_PATH_SIMT;
   const long long T = p->tokens;
   pl.max_seqlen = (p->max_seqlen == 0 || p->max_seqlen > T) ? (int)T : p->max_seqlen;

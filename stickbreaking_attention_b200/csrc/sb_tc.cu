@@ -77,10 +77,12 @@ static cudaError_t encode_cached(CUtensorMap *map, const void *ptr, const cuuint
 
 cudaError_t make_tile_map(CUtensorMap *map, const TensorRef &t, const KParams &p, int dtype, int box_rows) {
   const cuuint64_t esz = 2;
-  long long sb_el = t.sb > 0 ? t.sb : (t.sh > 0 ? t.sh * p.heads : (long long)p.tokens * p.head_dim);
-  long long sh_el = t.sh > 0 ? t.sh : (long long)p.tokens * p.head_dim;
+  // the stride of an axis of one element is the caller's to leave as it likes; every other one is a real one (make_plan)
+  const long long st_el = p.tokens > 1 ? t.st : p.head_dim;
+  const long long sh_el = p.heads > 1 ? t.sh : p.tokens * st_el;
+  const long long sb_el = p.batch > 1 ? t.sb : p.heads * sh_el;
   cuuint64_t dims[4] = {(cuuint64_t)p.head_dim, (cuuint64_t)p.tokens, (cuuint64_t)p.heads, (cuuint64_t)p.batch};
-  cuuint64_t strides[3] = {(cuuint64_t)t.st * esz, (cuuint64_t)sh_el * esz, (cuuint64_t)sb_el * esz};
+  cuuint64_t strides[3] = {(cuuint64_t)st_el * esz, (cuuint64_t)sh_el * esz, (cuuint64_t)sb_el * esz};
   return encode_cached(map, t.ptr, dims, strides, box_rows, dtype);
 }
 

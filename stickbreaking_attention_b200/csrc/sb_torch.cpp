@@ -63,14 +63,16 @@ int32_t *status_ptr(int device) {
   return p;
 }
 
-// Unit innermost stride, 16-byte aligned base and outer strides (what TMA and the vector accesses need); copies only
-// where that does not hold.  Rows that are no multiple of 16 bytes take the CUDA-core kernels: any stride will do.
+// Unit innermost stride, 16-byte aligned base and outer strides (what TMA and the vector accesses need) and, for the types
+// the tensor maps are for, no axis that repeats its elements (an expanded tensor: a key head shared by several heads, the
+// gradient of a sum); copies only where that does not hold, so that forward and backward take the same kernels whatever
+// the strides.  Rows that are no multiple of 16 bytes take the CUDA-core kernels: any stride will do.
 Tensor tma_ready(const Tensor &t) {
   const int64_t mult = 16 / t.element_size(), nd = t.dim();
   bool ok = t.stride(-1) == 1;
   if (ok && t.size(-1) % mult == 0) {
     ok = reinterpret_cast<uintptr_t>(t.data_ptr()) % 16 == 0;
-    for (int64_t i = 0; ok && i + 1 < nd; ++i) ok = t.stride(i) % mult == 0 || t.size(i) == 1;
+    for (int64_t i = 0; ok && i + 1 < nd; ++i) ok = t.size(i) == 1 || (t.stride(i) % mult == 0 && (t.stride(i) > 0 || mult < 8));
   }
   return ok ? t : t.contiguous();
 }
@@ -343,6 +345,7 @@ PYBIND11_MODULE(_sb_torch, m) {
   m.def("attention", &attention, py::call_guard<py::gil_scoped_release>());
   m.def("forward", &forward, py::call_guard<py::gil_scoped_release>());
   m.def("backward", &backward, py::call_guard<py::gil_scoped_release>());
+  m.def("tma_ready", &tma_ready);
   m.def("status_word", &status_word, py::call_guard<py::gil_scoped_release>());
   m.def("launches", [] { return g_launches.load(); });
 }

@@ -118,14 +118,7 @@ def _require(cond: bool, msg: str):
         raise ValueError(msg)
 
 
-def _tma_ready(t: torch.Tensor) -> torch.Tensor:
-    """Unit innermost stride, 16-byte aligned base and outer strides; copies only if needed."""
-    mult = 16 // t.element_size()
-    ok = t.stride(-1) == 1 and t.data_ptr() % 16 == 0 and all(
-        s % mult == 0 or n == 1 for s, n in zip(t.stride()[:-1], t.shape[:-1]))
-    if t.shape[-1] % mult != 0:          # rows cannot be 16-byte multiples anyway
-        ok = t.stride(-1) == 1
-    return t if ok else t.contiguous()
+_tma_ready = _sb_torch.tma_ready   # what the kernels can address as it is; copies only if needed
 
 
 def _fill(prm, *, fixed, q, k, v, cu_seqlens, max_seqlens, logit_scale, attend_current, leading_zero,

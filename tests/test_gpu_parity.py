@@ -452,6 +452,46 @@ def test_strided_views_and_scale(sb, cuda_device, dtype):
     H.assert_parity(got, want, dtype, "strided")
 
 
+@pytest.mark.parametrize("dtype,d", [(torch.bfloat16, 128), (torch.float16, 64), (torch.float32, 64), (torch.bfloat16, 50)])
+@pytest.mark.parametrize("packed", [True, False])
+def test_expanded_tensors_match_their_copies(sb, cuda_device, dtype, d, packed):
+    """Keys and values shared by several heads (or by the batch) and gradients that arrive expanded, as those of a sum over an
+    axis do, give the bits of the same tensors written out; so do axes of one element with a stride of their own."""
+    full = (3, 300, d) if packed else (2, 3, 300, d)
+    kv_shapes = [(1, 300, d)] if packed else [(2, 1, 300, d), (1, 3, 300, d)]
+    g_shapes = [(1, 300, d), (3, 1, d), (1, 1, d)] if packed else [(2, 1, 300, d), (1, 3, 300, d), (2, 3, 1, d), (1, 1, 1, 1)]
+    gen = torch.Generator().manual_seed(d)
+    rand = lambda shape: torch.randn(shape, generator=gen).to(dtype).to(cuda_device)
+    cu = cu_of([170, 130]).to(cuda_device)
+
+    def run(q, k, v, do):
+        q, k, v = (t.detach().requires_grad_(True) for t in (q, k, v))
+        o, rem = sb.sb_attn_varlen(q, k, v, cu, 170, zero_start=False) if packed else sb.sb_attn(q, k, v)
+        return (o, rem) + torch.autograd.grad(o, (q, k, v), do)
+
+    q, do = rand(full), rand(full)
+    cases = [(q, rand(s).expand(full), rand(s).expand(full), do) for s in kv_shapes]
+    cases += [(q, rand(full), rand(full), rand(s).expand(full)) for s in g_shapes]
+    one = full[:-3] + (1,) + full[-2:] if packed else (1,) + full[1:]
+    strides = (3, d, 1) if packed else (3, 300 * d, d, 1)
+    cases.append(tuple(rand(one).as_strided(one, strides) for _ in range(4)))
+    for ins in cases:
+        got, want = run(*ins), run(*(t.clone(memory_format=torch.contiguous_format) for t in ins))
+        for name, a, b in zip(("o", "rem", "dq", "dk", "dv"), got, want):
+            assert torch.equal(a, b), name
+
+
+def test_a_repeated_head_through_the_c_abi(sb, cuda_device):
+    """A caller of the C ABI may pass a stride of 0: the call takes the CUDA-core kernels."""
+    q, k, v, _, _ = (t.to(cuda_device) for t in H.make_inputs((3, 200, 64), torch.bfloat16, seed=4))
+    k = k[:1].expand_as(k)
+    o, rem, log_rem = torch.empty_like(q), torch.empty_like(q[..., 0]), torch.empty(3, 200, dtype=torch.float64, device=cuda_device)
+    sb.ops._fwd_impl(False, q, k, v, cu_of([200]).to(cuda_device), None, 0.125, False, False, o, rem, log_rem)
+    with sb.force_simt():
+        want = sb.ops.varlen_fwd(q, k.contiguous(), v, cu_of([200]).to(cuda_device), None, 0.125)
+    assert torch.equal(o, want[0]) and torch.equal(rem, want[1])
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 def test_backward_is_bitwise_deterministic(sb, cuda_device, dtype):
     lengths = [700, 324]

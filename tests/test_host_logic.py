@@ -4,7 +4,7 @@ import ctypes
 import pytest
 import torch
 
-from stickbreaking_attention_b200 import _cabi, shard
+from stickbreaking_attention_b200 import _cabi, ops, shard
 import stickbreaking_attention_b200 as sb
 
 
@@ -37,6 +37,38 @@ def test_kernel_selection():
         for dtype in (1, 2):
             assert lib.sb_kernel_path(params(dtype=dtype, d=d)) == _cabi.SB_PATH_TCGEN05
     assert lib.sb_kernel_path(params(dtype=1, d=128, stride_t=129)) == _cabi.SB_PATH_SIMT  # rows not 16-B aligned
+
+
+def test_repeated_axes_have_no_tensor_map():
+    """An axis with stride 0 (a key head shared by several heads) cannot be a tensor-map axis; an axis of one element can have any
+    stride, so that forward and backward choose the same kernels whatever torch leaves there."""
+    lib = _cabi.load()
+
+    def path(**strides):   # of k, in a fixed-length batch
+        p = params(num_seq=0, heads=strides.pop("heads", 4), tokens=strides.pop("tokens", 256), batch=strides.pop("batch", 2))
+        p.cu_seqlens = None
+        for name in ("q", "k", "v"):
+            setattr(p, name, _cabi.SbTensor(4096, 4 * 256 * 128, 256 * 128, 128))
+        p.k = _cabi.SbTensor(4096, strides.get("b", 4 * 256 * 128), strides.get("h", 256 * 128), strides.get("t", 128))
+        return lib.sb_kernel_path(p)
+
+    assert path() == _cabi.SB_PATH_TCGEN05
+    for axis in ("b", "h", "t"):
+        assert path(**{axis: 0}) == _cabi.SB_PATH_SIMT, axis
+    for extent, axis in (("batch", "b"), ("heads", "h"), ("tokens", "t")):
+        for stride in (0, 3):
+            assert path(**{extent: 1, axis: stride}) == _cabi.SB_PATH_TCGEN05, axis
+
+
+@pytest.mark.parametrize("dtype,d,copied", [(torch.bfloat16, 64, True), (torch.float16, 40, True), (torch.float32, 64, False),
+                                            (torch.bfloat16, 50, False)])
+def test_expanded_tensors_are_copied_where_a_tensor_map_would_be_built(dtype, d, copied):
+    for shape, full in (((2, 1, 8, d), (2, 3, 8, d)), ((1, 3, 8, d), (2, 3, 8, d)), ((2, 3, 1, d), (2, 3, 8, d))):
+        t = torch.randn(shape).to(dtype).expand(full)
+        got = ops._tma_ready(t)
+        assert torch.equal(got, t) and got.is_contiguous() == copied
+    one = torch.randn(64 * 8 * 64)[:8 * d].to(dtype).as_strided((1, 1, 8, d), (3, 5, d, 1))   # axes of one element: any stride
+    assert ops._tma_ready(one).data_ptr() == one.data_ptr()
 
 
 def test_invalid_parameters():
