@@ -95,12 +95,28 @@ void check_inputs(const Tensor &q, const Tensor &k, const Tensor &v, const std::
   dtype_code(q.scalar_type());
   TORCH_CHECK_VALUE(q.scalar_type() == k.scalar_type() && q.scalar_type() == v.scalar_type(), "q, k, v must share a dtype");
   TORCH_CHECK_VALUE(q.sizes() == k.sizes() && q.sizes() == v.sizes(), "q, k, v must share a shape");
+  TORCH_CHECK_VALUE(q.device() == k.device() && q.device() == v.device(), "q, k, v must share a device");
   TORCH_CHECK_VALUE(q.dim() == (c.fixed ? 4 : 3), "expected (B,H,T,d) for sb_attn and (H,T,d) for sb_attn_varlen");
   if (!c.fixed) {
     TORCH_CHECK_VALUE(cu->is_cuda() && cu->dim() == 1, "cu_seqlens must be a 1-D CUDA tensor");
+    TORCH_CHECK_VALUE(cu->device() == q.device(), "cu_seqlens must be on the device of q, k, v");
     TORCH_CHECK_VALUE(cu->scalar_type() == at::kInt || cu->scalar_type() == at::kLong, "cu_seqlens must be int32 or int64");
     TORCH_CHECK_VALUE(cu->numel() <= 1 || cu->stride(0) == 1, "cu_seqlens must be contiguous");
   }
+}
+
+// The backward's own inputs: the kernels go by the shapes of q.
+void check_gradients(const Tensor &dout, const Tensor &drem, const Tensor &q) {
+  if (dout.defined())
+    TORCH_CHECK_VALUE(dout.device() == q.device() && dout.sizes() == q.sizes(), "the gradient of o must have the shape and device of q");
+  if (drem.defined())
+    TORCH_CHECK_VALUE(drem.device() == q.device() && drem.numel() * q.size(-1) == q.numel(),
+                      "the gradient of rem must have one value per row of q, on its device");
+}
+void check_log_rem(const Tensor &log_rem, const Tensor &q) {
+  TORCH_CHECK_VALUE(log_rem.scalar_type() == at::kDouble && log_rem.is_contiguous() && log_rem.device() == q.device() &&
+                        log_rem.numel() * q.size(-1) == q.numel(),
+                    "log_rem must be what the forward returned: fp64, contiguous, one value per row of q");
 }
 
 void fill(SbParams &p, const Tensor &q, const Tensor &k, const Tensor &v, const std::optional<Tensor> &cu, const Call &c) {
@@ -207,6 +223,7 @@ Forward run_forward(const Tensor &q_in, const Tensor &k_in, const Tensor &v_in, 
 std::array<Tensor, 3> run_backward(const Tensor &dout_in, const Tensor &drem_in, const Tensor &q_in, const Tensor &k_in, const Tensor &v_in,
                                    const std::optional<Tensor> &cu, const Tensor &state, bool tile_starts, const Call &c) {
   check_inputs(q_in, k_in, v_in, cu, c);
+  check_gradients(dout_in, drem_in, q_in);
   c10::cuda::CUDAGuard guard(q_in.device());
   const Tensor q = tma_ready(q_in), k = tma_ready(k_in), v = tma_ready(v_in);
   const Tensor dout = dout_in.defined() ? tma_ready(dout_in.scalar_type() == q.scalar_type() ? dout_in : dout_in.to(q.scalar_type()))
@@ -327,6 +344,7 @@ std::tuple<Tensor, Tensor, Tensor> backward(const Tensor &dout, const std::optio
                                             const Tensor &log_rem, double scale, bool attend_current, bool leading_zero, bool fused,
                                             int64_t flags) {
   at::AutoDispatchBelowADInplaceOrView below;
+  check_log_rem(log_rem, q);
   std::array<Tensor, 3> g = run_backward(dout, drem.value_or(Tensor()), q, k, v, cu, log_rem, false,
                                          make_call(!cu.has_value(), max_seqlens, scale, attend_current, leading_zero, fused, flags));
   return {g[0], g[1], g[2]};

@@ -127,6 +127,7 @@ def _fill(prm, *, fixed, q, k, v, cu_seqlens, max_seqlens, logit_scale, attend_c
     _require(q.dtype in _cabi.SB_DTYPE, f"unsupported dtype {q.dtype}")
     _require(q.dtype == k.dtype == v.dtype, "q, k, v must share a dtype")
     _require(q.shape == k.shape == v.shape, "q, k, v must share a shape")
+    _require(q.device == k.device == v.device, "q, k, v must share a device")
     _require(q.dim() == (4 if fixed else 3), "expected (B,H,T,d) for sb_attn and (H,T,d) for sb_attn_varlen")
     prm.struct_bytes = _cabi.ctypes.sizeof(_cabi.SbParams)
     prm.dtype = _cabi.SB_DTYPE[q.dtype]
@@ -138,6 +139,7 @@ def _fill(prm, *, fixed, q, k, v, cu_seqlens, max_seqlens, logit_scale, attend_c
         prm.batch = 1
         prm.heads, prm.tokens, prm.head_dim = q.shape
         _require(cu_seqlens.is_cuda and cu_seqlens.dim() == 1, "cu_seqlens must be a 1-D CUDA tensor")
+        _require(cu_seqlens.device == q.device, "cu_seqlens must be on the device of q, k, v")
         _require(cu_seqlens.dtype in (torch.int32, torch.int64), "cu_seqlens must be int32 or int64")
         _require(cu_seqlens.stride(0) == 1, "cu_seqlens must be contiguous")
         prm.num_seq = cu_seqlens.numel()
@@ -207,6 +209,12 @@ def _bwd_impl(fixed, do, dr, q, k, v, cu_seqlens, max_seqlens, log_rem, logit_sc
     _fill(prm, fixed=fixed, q=q, k=k, v=v, cu_seqlens=cu_seqlens, max_seqlens=max_seqlens,
           logit_scale=logit_scale, attend_current=attend_current, leading_zero=leading_zero, fuse_rem_v=fuse_rem_v,
           switches=switches)
+    _require(do.device == q.device and do.shape == q.shape, "the gradient of o must have the shape and device of q")
+    _require(dr is None or (dr.device == q.device and dr.numel() * q.shape[-1] == q.numel()),
+             "the gradient of rem must have one value per row of q, on its device")
+    _require(log_rem.dtype == torch.float64 and log_rem.is_contiguous() and log_rem.device == q.device
+             and log_rem.numel() * q.shape[-1] == q.numel(),
+             "log_rem must be what the forward returned: fp64, contiguous, one value per row of q")
     prm.log_rem = log_rem.data_ptr()
     prm.d_o = _cabi.tensor_arg(do, fixed)
     prm.d_rem = dr.data_ptr() if dr is not None else None

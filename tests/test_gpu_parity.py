@@ -626,6 +626,17 @@ def test_argument_errors(sb, cuda_device):
         sb.sb_attn(q, q, q)
 
 
+def test_tensors_of_another_device_are_refused(sb, cuda_device):
+    q, cu = torch.randn(2, 64, 64, device=cuda_device), torch.tensor([64], device=cuda_device)
+    for args in ((q.cpu(), q), (q, q.cpu())):
+        with pytest.raises(ValueError):
+            sb.sb_attn_varlen(q, *args, cu, zero_start=False)
+    o, rem, log_rem = sb.ops.varlen_fwd(q, q, q, cu, 64, 0.125)
+    for args in ((o.cpu(), rem, log_rem), (o, rem.cpu(), log_rem), (o, rem, log_rem.cpu())):
+        with pytest.raises(ValueError):
+            sb.ops.varlen_bwd(args[0], args[1], q, q, q, cu, 64, args[2], 0.125)
+
+
 def test_cuda_graph_replay_matches_eager(sb, cuda_device):
     """Forward and backward enqueue only (no allocation of their own, no synchronisation, no host reads), so a step can
     be captured in a CUDA graph and replayed: the replay on new inputs must equal an eager call bit for bit."""

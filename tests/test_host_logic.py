@@ -28,6 +28,32 @@ def test_cpu_tensors_are_rejected_not_computed():
         sb.sb_attn(q[None], q[None], q[None])
 
 
+def test_tensors_of_another_device_or_size_are_refused_before_their_pointers_are_used():
+    """(Fake tensors: CUDA tensors as far as the checks can tell, with no device behind them.)"""
+    from torch._subclasses.fake_tensor import FakeTensorMode
+    from stickbreaking_attention_b200 import _sb_torch
+    with FakeTensorMode(allow_non_fake_inputs=True):
+        q = torch.empty(2, 8, 16, device="cuda")
+        cu = torch.empty(1, dtype=torch.int32, device="cuda")
+        log_rem = torch.empty(2, 8, dtype=torch.float64, device="cuda")
+        dr = torch.empty(2, 8, device="cuda")
+    host = torch.zeros(2, 8, 16)
+
+    def forward(q, k, v, cu):
+        _sb_torch.forward(q, k, v, cu, None, 1.0, False, False, False, 0)
+
+    def backward(do, dr, log_rem):
+        _sb_torch.backward(do, dr, q, q, q, cu, None, log_rem, 1.0, False, False, False, 0)
+
+    for args in ((q, host, q, cu), (q, q, host, cu), (q, q, q, torch.zeros(1, dtype=torch.int32))):
+        with pytest.raises(ValueError):
+            forward(*args)
+    for args in ((host, dr, log_rem), (q[:, :4], dr, log_rem), (q, dr.cpu(), log_rem), (q, dr[:1], log_rem), (q, dr, log_rem.float()),
+                 (q, dr, log_rem[:1]), (q, dr, log_rem.t()), (q, dr, torch.zeros(2, 8, dtype=torch.float64))):
+        with pytest.raises(ValueError):
+            backward(*args)
+
+
 def test_kernel_selection():
     lib = _cabi.load()
     assert lib.sb_kernel_path(params(dtype=0)) == _cabi.SB_PATH_SIMT            # fp32 -> CUDA cores
