@@ -308,6 +308,8 @@ variable_list attention(const Tensor &q, const Tensor &k, const Tensor &v, const
                         std::optional<int64_t> max_seqlens, double scale, bool attend_current, bool leading_zero, bool fused,
                         int64_t flags) {
   const Call c = make_call(!cu.has_value(), max_seqlens, scale, attend_current, leading_zero, fused, flags);
+  for (const Tensor *t : {&q, &k, &v})
+    TORCH_CHECK_NOT_IMPLEMENTED(!t->_fw_grad(0).defined(), "stick-breaking attention has no forward-mode derivative");
   const bool grad = torch::autograd::compute_requires_grad(q, k, v);
   Forward f;
   {

@@ -637,6 +637,16 @@ def test_tensors_of_another_device_are_refused(sb, cuda_device):
             sb.ops.varlen_bwd(args[0], args[1], q, q, q, cu, 64, args[2], 0.125)
 
 
+@pytest.mark.parametrize("which", range(3))
+def test_forward_mode_is_refused_not_ignored(sb, cuda_device, which):
+    import torch.autograd.forward_ad as fwAD
+    qkv = [torch.randn(1, 2, 40, 64, device=cuda_device, dtype=torch.bfloat16) for _ in range(3)]
+    with fwAD.dual_level():
+        qkv[which] = fwAD.make_dual(qkv[which], torch.ones_like(qkv[which]))
+        with pytest.raises(NotImplementedError):
+            sb.sb_attn(*qkv)
+
+
 def test_cuda_graph_replay_matches_eager(sb, cuda_device):
     """Forward and backward enqueue only (no allocation of their own, no synchronisation, no host reads), so a step can
     be captured in a CUDA graph and replayed: the replay on new inputs must equal an eager call bit for bit."""
