@@ -269,13 +269,14 @@ struct StickBreakingAttentionBackward : public torch::autograd::Node {
   }
   variable_list apply(variable_list &&grads) override {
     TORCH_CHECK(!released, torch::autograd::ERR_BACKWARD_TWICE);
+    // Saved-tensor hooks run here and may record operations of their own (activation checkpointing runs the forward again).
+    const Tensor sq = q.unpack(), sk = k.unpack(), sv = v.unpack(), saved = state.unpack();
     std::optional<Tensor> ends;
     if (!call.fixed) ends = cu.unpack();
     at::AutoDispatchBelowADInplaceOrView below;   // plain tensors from here on: conversions and copies record nothing
     std::array<Tensor, 3> g;
     try {
-      g = run_backward(grads[0], grads.size() > 1 ? grads[1] : Tensor(), q.unpack(), k.unpack(), v.unpack(), ends, state.unpack(), true,
-                       call);
+      g = run_backward(grads[0], grads.size() > 1 ? grads[1] : Tensor(), sq, sk, sv, ends, saved, true, call);
     } catch (const LibraryError &e) {   // on an autograd thread: the exception keeps its Python type on its way to the caller
       py::gil_scoped_acquire gil;
       set_python_error(e);

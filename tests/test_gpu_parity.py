@@ -647,6 +647,31 @@ def test_forward_mode_is_refused_not_ignored(sb, cuda_device, which):
             sb.sb_attn(*qkv)
 
 
+@pytest.mark.parametrize("packed", [False, True])
+@pytest.mark.parametrize("fused", [False, True])
+def test_activation_checkpointing(sb, cuda_device, packed, fused):
+    """The operator is the last one of the region that saves tensors, so its backward is what runs the region again."""
+    from torch.utils.checkpoint import checkpoint
+    gen = torch.Generator().manual_seed(1)
+    x, w = (torch.randn(s, generator=gen).to(cuda_device) for s in ((1, 2, 70, 64), (64, 64)))
+    cu = torch.tensor([30, 70], device=cuda_device)
+
+    def region(x):
+        q, k, v = x @ w, x @ w.T, x
+        if packed:
+            out = (sb.sb_attn_varlen_fused if fused else sb.sb_attn_varlen)(q[0], k[0], v[0], cu, 70, zero_start=False)
+        else:
+            out = (sb.sb_attn_fused if fused else sb.sb_attn)(q, k, v)
+        return out.sum() if fused else out[0].sum() + out[1].sum()
+
+    grads = []
+    for run in (region, lambda x: checkpoint(region, x, use_reentrant=False)):
+        leaf = x.clone().requires_grad_(True)
+        run(leaf).backward()
+        grads.append(leaf.grad)
+    assert torch.equal(*grads)
+
+
 def test_cuda_graph_replay_matches_eager(sb, cuda_device):
     """Forward and backward enqueue only (no allocation of their own, no synchronisation, no host reads), so a step can
     be captured in a CUDA graph and replayed: the replay on new inputs must equal an eager call bit for bit."""
