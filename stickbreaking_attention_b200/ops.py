@@ -367,6 +367,7 @@ def varlen_fwd(q, k, v, cu_seqlens, max_seqlens: Optional[int], logit_scale: flo
     ``W``, fp32 ``(heads, tokens, max_seqlens)``: row t holds the weights of token t over the keys of its own sequence,
     indexed from the sequence start, zeros elsewhere.  A debugging aid: O(tokens * max_seqlens) memory, and the call
     runs the CUDA-core kernels whatever the dtype."""
+    _require(cu_seqlens is not None, "a packed batch needs cu_seqlens")
     if not (return_attention or _compiling()):
         return _native_fwd(q, k, v, cu_seqlens, max_seqlens, logit_scale, attend_current, leading_zero, False)
     q, k, v = _tma_ready(q), _tma_ready(k), _tma_ready(v)
@@ -389,6 +390,7 @@ def varlen_bwd(do, dr, q, k, v, cu_seqlens, max_seqlens: Optional[int], log_rem,
                attend_current: bool = False, leading_zero: bool = False, switches: Optional[int] = None):
     """Packed backward; returns ``(dq, dk, dv)`` in the dtype of the inputs.  ``switches``: the ``switch_flags()`` of
     the forward call (default: the calling thread's)."""
+    _require(cu_seqlens is not None, "a packed batch needs cu_seqlens")
     if not _compiling():
         return _native_bwd(do, dr, q, k, v, cu_seqlens, max_seqlens, log_rem, logit_scale, attend_current, leading_zero, False,
                            switches)

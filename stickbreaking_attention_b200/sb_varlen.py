@@ -13,6 +13,11 @@ import torch
 from . import ops
 
 
+def _require_ends(cu_seqlens):
+    """(Without them the native call takes a batch for a fixed-length one.)"""
+    ops._require(cu_seqlens is not None, "a packed batch needs cu_seqlens")
+
+
 class StickBreakingAttention:
     """The reference's name for the differentiable operator (``sb_varlen/__init__.py:24-68``); the autograd node itself is
     native (``csrc/sb_torch.cpp``)."""
@@ -32,6 +37,7 @@ def sb_attn_varlen(q, k, v, cu_seqlens, max_seqlens=None, inv_temp=None, zero_st
     The leading zero is verified on the device (see ``ops.check_status``) rather than with the
     reference's host-side ``assert cu_seqlens[0] == 0`` (``sb_varlen/__init__.py:72-74``).
     """
+    _require_ends(cu_seqlens)
     if inv_temp is None:
         inv_temp = 1 / math.sqrt(q.size(-1))
     if torch.compiler.is_compiling():   # one traceable operator with its own autograd formula
@@ -41,6 +47,7 @@ def sb_attn_varlen(q, k, v, cu_seqlens, max_seqlens=None, inv_temp=None, zero_st
 
 
 def sb_attn_varlen_(q, k, v, inv_temp, cu_seqlens, max_seqlens, attend_current, leading_zero=False):
+    _require_ends(cu_seqlens)
     o, rem = ops.attention(q, k, v, cu_seqlens, max_seqlens, inv_temp, attend_current, leading_zero)
     return o, rem
 
@@ -49,6 +56,7 @@ def sb_attn_varlen_fused(q, k, v, cu_seqlens, max_seqlens=None, inv_temp=None, z
                          attend_current=False):
     """Same arguments as ``sb_attn_varlen``; returns the single tensor ``o + rem[..., None] * v`` that the reference's
     callers compute from its two outputs (``tests/test_varlen.py:101``), without the extra passes over o and v."""
+    _require_ends(cu_seqlens)
     if inv_temp is None:
         inv_temp = 1 / math.sqrt(q.size(-1))
     if torch.compiler.is_compiling():

@@ -28,6 +28,14 @@ def test_cpu_tensors_are_rejected_not_computed():
         sb.sb_attn(q[None], q[None], q[None])
 
 
+def test_packed_calls_without_sequence_ends_are_refused():
+    q = torch.zeros(1, 2, 8, 16)
+    for call in (lambda: sb.sb_attn_varlen(q, q, q, None), lambda: sb.sb_attn_varlen_fused(q, q, q, None, zero_start=False),
+                 lambda: ops.varlen_fwd(q, q, q, None, None, 1.0), lambda: ops.varlen_bwd(q, q, q, q, q, None, None, q, 1.0)):
+        with pytest.raises(ValueError, match="cu_seqlens"):
+            call()
+
+
 def test_tensors_of_another_device_or_size_are_refused_before_their_pointers_are_used():
     """(Fake tensors: CUDA tensors as far as the checks can tell, with no device behind them.)"""
     from torch._subclasses.fake_tensor import FakeTensorMode
