@@ -35,6 +35,14 @@ def sb_attn_(q, k, v, inv_temp, attend_current):
     return o, rem
 
 
+class StickBreakingAttentionFused:
+    """The fused form's operator by the same interface."""
+
+    @staticmethod
+    def apply(q, k, v, inv_temp, attend_current=False):
+        return ops.attention(q, k, v, None, None, inv_temp, attend_current, False, fused=True)[0]
+
+
 def sb_attn_fused(q, k, v, inv_temp=None, zero_start=True, attend_current=False):
     """Same arguments as ``sb_attn``; returns ``o + rem[..., None] * v`` (``tests/test_attn.py:64`` of the reference)."""
     if inv_temp is None:

@@ -52,6 +52,15 @@ def sb_attn_varlen_(q, k, v, inv_temp, cu_seqlens, max_seqlens, attend_current, 
     return o, rem
 
 
+class StickBreakingAttentionFused:
+    """The fused form's operator by the same interface."""
+
+    @staticmethod
+    def apply(q, k, v, cu_seqlens, max_seqlens, inv_temp, attend_current, leading_zero):
+        _require_ends(cu_seqlens)
+        return ops.attention(q, k, v, cu_seqlens, max_seqlens, inv_temp, attend_current, leading_zero, fused=True)[0]
+
+
 def sb_attn_varlen_fused(q, k, v, cu_seqlens, max_seqlens=None, inv_temp=None, zero_start=True,
                          attend_current=False):
     """Same arguments as ``sb_attn_varlen``; returns the single tensor ``o + rem[..., None] * v`` that the reference's

@@ -166,6 +166,17 @@ def test_slice_packed_round_trip():
     assert sl.shape[1] == 0 and lens == []
 
 
+def test_operator_classes_keep_their_names():
+    import importlib
+    fixed, packed = (importlib.import_module(f"stickbreaking_attention_b200.{m}") for m in ("sb_attn", "sb_varlen"))   # (not the functions)
+    q, cu = torch.zeros(2, 8, 16), torch.tensor([8])
+    for name in ("StickBreakingAttention", "StickBreakingAttentionFused"):
+        with pytest.raises(ValueError, match="CUDA"):
+            getattr(packed, name).apply(q, q, q, cu, 8, 1.0, False, False)
+        with pytest.raises(ValueError, match="CUDA"):
+            getattr(fixed, name).apply(q[None], q[None], q[None], 1.0)
+
+
 def test_dropin_alias():
     import sys
     sb.install_as_dropin("stickbreaking_attention_alias_for_test")
