@@ -192,6 +192,7 @@ tc_fwd128x2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
         // that step (issued earlier by this thread) has read.
         int steps = w.n_steps, used = w.n_steps;   // steps computed and stages taken
         bool early = false, halt = false;   // halt: the tile stops before step u
+        bool through = false;               // all rows were through by the step at hand: its P is zero
         for (int u = 0; ok && u <= steps; ++u) {
           if (halt) {
             early = true;
@@ -210,7 +211,7 @@ tc_fwd128x2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
             mma_commit(bar(bSFull + (gu & 1)));
             stop.word[gu & 1] = st;
             mbar_arrive(bar(bSFull + (gu & 1)));
-            halt = kStop && u >= 2 && u + 1 < w.n_steps && may_stop_before(w.s_top - u - 1) && all_through(stop, it);
+            halt = kStop && u >= 2 && u + 1 < w.n_steps && may_stop_before(w.s_top - u - 1) && all_through(stop, U, u);
             if (u == w.n_steps - 1) mma_commit(bar(bQFree + qb));   // the tile's last read of Q
           }
           if (u >= 1) {
@@ -220,8 +221,10 @@ tc_fwd128x2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
             if (ok && up == 0 && it >= 1) ok = wait_or_abort(bar(bOFree), (it - 1) & 1, abort_flag, p, 725);
             if (!ok) break;
             tc_fence_after();
-            mma_tmem_mnmajor<kBN, kKvTileBytes>(tmem + 128, tmem + (gu & 1) * 64 + kPCol,
-                                                sKV + st * kStageBytes + kKvTileBytes, idesc_pv, up > 0);
+            through = through || (kStop && all_through(stop, U, up));
+            if (!through)
+              mma_tmem_mnmajor<kBN, kKvTileBytes>(tmem + 128, tmem + (gu & 1) * 64 + kPCol,
+                                                  sKV + st * kStageBytes + kKvTileBytes, idesc_pv, up > 0);
             mma_commit(bar(bKvEmpty + st));
           }
         }
@@ -294,7 +297,7 @@ tc_fwd128x2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
       // well.  The sequence's tail is behind these steps.
       if (kStop && u < w.n_steps && ok) {
         s_reached = w.s_top - u + 1;
-        if (lane == 0) publish_through(stop, warp & 3, it);
+        if (lane == 0) publish_through(stop, warp & 3, U + u);
         for (bool first = true; u < w.n_steps && ok; ++u, first = false) {
           const int gu = U + u, buf = gu & 1;
           bool halt = false;

@@ -223,6 +223,7 @@ tc_fwd256_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
         // before p_full(u-2) was signalled, and that was waited for in iteration u-1.
         int steps = my_steps;          // steps computed
         bool early = false, halt = false;   // halt: the tile stops before step u
+        bool through = false;               // all rows were through by the step at hand: its P is zero
         for (int u = 0; ok && active && u <= steps; ++u) {
           if (halt) {
             early = true;
@@ -244,7 +245,7 @@ tc_fwd256_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
             mma_commit(bar(bSFull + wg * 2 + (gu & 1)));
             stop.word[gu & 1] = st;
             mbar_arrive(bar(bSFull + wg * 2 + (gu & 1)));
-            halt = may_stop && u >= 2 && u + 1 < my_steps && may_stop_before(w.s_top - t0 - u - 1) && all_through(stop, it);
+            halt = may_stop && u >= 2 && u + 1 < my_steps && may_stop_before(w.s_top - t0 - u - 1) && all_through(stop, U, u);
             if (u == my_steps - 1) mma_commit(bar_qfree);   // the item's last read of Q
             trace_event(p, 1 + 3 * wg, tr_cur, 3 + 16 * wg, t0 + u);
           }
@@ -256,9 +257,11 @@ tc_fwd256_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
             if (!ok) break;
             trace_event(p, 1 + 3 * wg, tr_cur, 6 + 16 * wg, t0 + up);
             tc_fence_after();
+            through = through || (may_stop && all_through(stop, U, up));
             // 16 keys per MMA; V: 64 rows x (2 x 64) columns, MN-major
-            mma_tmem_mnmajor<kBN, kKvBoxBytes>(tmem + 256 + wg * 128, tmem + wg * 128 + (gu & 1) * 64 + kPCol,
-                                               sKV + st * kStageBytes + kKvTileBytes, idesc_pv, up > 0);
+            if (!through)
+              mma_tmem_mnmajor<kBN, kKvBoxBytes>(tmem + 256 + wg * 128, tmem + wg * 128 + (gu & 1) * 64 + kPCol,
+                                                 sKV + st * kStageBytes + kKvTileBytes, idesc_pv, up > 0);
             mma_commit(bar(bKvEmpty + st));
             trace_event(p, 1 + 3 * wg, tr_cur, 7 + 16 * wg, t0 + up);
           }
@@ -347,7 +350,7 @@ tc_fwd256_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
       // well.  The sequence's tail is behind these steps.
       if (may_stop && u < my_steps && ok) {
         s_reached = w.s_top - (t0 + u) + 1;
-        if (lane == 0) publish_through(stop, warp & 3, it);
+        if (lane == 0) publish_through(stop, warp & 3, U + u);
         for (bool first = true; u < my_steps && ok; ++u, first = false) {
           const int gu = U + u, buf = gu & 1;
           bool halt = false;

@@ -186,28 +186,30 @@ __device__ __forceinline__ bool fwd256_row_pass(uint32_t ts, int key0, int row, 
 // ---- stopping early ------------------------------------------------------------------------------------------------
 // A row warp is through once the product R has underflowed to exactly 0 for all its rows: no earlier key can add anything
 // to O or rem.  From then on it only writes zeros for P, its log sum stays what it is, and the key it got to is recorded
-// for the backward.  Each of a query tile's four warps publishes that it is through; once all four are, the tile's MMA
-// issuer, who looks after each step's scores have been issued, stops before the next step and tells the rows with the word
-// that accompanies every step's scores.  Where exactly it stops depends on timing, what is stored does not: the steps in
-// between are zeros.  Rows that never finish pay nothing: the vote is the one the row pass takes anyway to skip its
-// arithmetic, and the issuer's look is one 16-byte read.
+// for the backward.  Each of a query tile's four warps publishes the step it was through at; from the step on in which all
+// four are, the tile's MMA issuer leaves P V out (P is zero), and it stops before the next step that it has not issued the
+// scores of yet and tells the rows with the word that accompanies every step's scores.  Where exactly it stops depends on
+// timing, what is stored does not: not even where a value of V behind the last warp's stop is not finite (0 times it would
+// be NaN).  Rows that never finish pay nothing: the vote is the one the row pass takes anyway to skip its arithmetic, and the
+// issuer's look is a 16-byte read.
 constexpr int kStepStop = -1;
 // No stop with fewer than three sub-tiles to go: what is left costs about as much as stopping and restarting the stream.
 __device__ __forceinline__ bool may_stop_before(int sub_tile) { return sub_tile >= 2; }
 struct alignas(16) EarlyStop {                // shared memory, one per query tile
-  int through[4];                             // per row warp: the last item it was through with, plus one
+  int through[4];                             // per row warp: the last step it was through at (counted over all items), plus one
   int word[2];                                // per S slot: K/V stage of the step, or kStepStop (read where it can matter)
   int stopped;                                // item + 1: the tile wants no more keys of this item
 };
-__device__ __forceinline__ void publish_through(volatile EarlyStop &e, int warp, int item) { e.through[warp] = item + 1; }
-__device__ __forceinline__ bool all_through(const volatile EarlyStop &e, int item) {
+__device__ __forceinline__ void publish_through(volatile EarlyStop &e, int warp, int step) { e.through[warp] = step + 1; }
+// Whether all four warps were through by step `u` of the item whose steps count from `first` on.
+__device__ __forceinline__ bool all_through(const volatile EarlyStop &e, int first, int u) {
   uint32_t a, b, c, d;
   asm volatile("ld.volatile.shared.v4.u32 {%0, %1, %2, %3}, [%4];"
                : "=r"(a), "=r"(b), "=r"(c), "=r"(d)
                : "r"(smem_u32(const_cast<const int *>(&e.through[0])))
                : "memory");
-  const uint32_t t = (uint32_t)item + 1u;
-  return ((a ^ t) | (b ^ t) | (c ^ t) | (d ^ t)) == 0u;
+  const uint32_t t = (uint32_t)first + 1u;   // entries of earlier items are smaller and wrap around
+  return max(max(a - t, b - t), max(c - t, d - t)) <= (uint32_t)u;
 }
 
 }  // namespace sb

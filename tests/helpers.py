@@ -143,3 +143,20 @@ def assert_fused_parity(got, want, dtype, what=""):
             assert max_abs(a, b) <= tol["out"], f"{what}: out max-abs {max_abs(a, b):.3e} > {tol['out']}"
         else:
             assert rel_l2(a, b) <= tol["grad_rel"], f"{what}: {name} rel-L2 {rel_l2(a, b):.3e} > {tol['grad_rel']}"
+
+
+def forward_state(sb, q, k, v, cu, max_seqlens, flags=0):
+    """Packed forward through the C ABI with its saved state: (o, rem, log_rem, tile_start), `tile_start` as (heads, groups of 32
+    tokens); entries the call does not write hold -1.  Device tensors, `cu` without a leading zero."""
+    ops, cabi = sb.ops, sb._cabi
+    heads, tokens, _ = q.shape
+    o, rem = torch.empty_like(q), torch.empty_like(q[..., 0])
+    log_rem = torch.empty(heads, tokens, dtype=torch.float64, device=q.device)
+    start = torch.full((heads, (tokens + 31) // 32), -1, dtype=torch.int32, device=q.device)
+    prm = cabi.SbParams()
+    ops._fill(prm, fixed=False, q=q, k=k, v=v, cu_seqlens=cu, max_seqlens=max_seqlens, logit_scale=1 / math.sqrt(q.shape[-1]),
+              attend_current=False, leading_zero=False, switches=flags)
+    prm.o, prm.rem, prm.log_rem = cabi.tensor_arg(o, False), rem.data_ptr(), log_rem.data_ptr()
+    prm.tile_start, prm.tile_start_stride = start.data_ptr(), start.shape[1]
+    ops._run(False, prm, q.device)
+    return o, rem, log_rem, start

@@ -572,6 +572,35 @@ def test_skipping_exact_zeros_changes_no_bit(sb, cuda_device, d, dtype, mode):
     H.assert_parity(fast, H.oracle_varlen(*ins, cu), dtype, "zeros skipped")
 
 
+@pytest.mark.parametrize("d,dtype,lengths", [(128, torch.bfloat16, [4000, 1111]), (64, torch.float16, [4000, 1111]),
+                                             (64, torch.bfloat16, [1000, 900] * 4), (64, torch.float32, [1500]), (50, torch.float16, [1500])])
+def test_values_that_are_not_finite_reach_the_tiles_that_visit_them(sb, cuda_device, d, dtype, lengths):
+    """One NaN per head in v.  A query tile (128 rows, on the CUDA cores 32) gets NaN if it visits that key, i.e. if one of its
+    groups of 32 rows does, and is finite otherwise -- at every call, however long the tile took to stop."""
+    heads, tokens, cu = 16, sum(lengths), cu_of(lengths).to(cuda_device)
+    q, k, v, _, _ = (t.to(cuda_device) for t in H.make_inputs((heads, tokens, d), dtype, seed=d))
+    rows = 32 if dtype == torch.float32 or d % 8 else 128
+    keys = [(97 + 61 * h) % tokens for h in range(heads)]
+    for h, key in enumerate(keys):
+        v[h, key] = float("nan")
+    finite = 0
+    for _ in range(4):
+        o, _, _, start = H.forward_state(sb, q, k, v, cu, max(lengths))
+        got, start = torch.isnan(o).cpu(), start.cpu()
+        for h, key in enumerate(keys):
+            tok0 = 0
+            for n in lengths:
+                for row0 in range(0, n, rows):
+                    groups = range(row0, min(row0 + rows, n), 32)
+                    first = 0 if row0 < 64 else min(int(start[h, (tok0 + g) // 32]) for g in groups)
+                    visits = first <= key - tok0 < min(row0 + rows, n)
+                    block = got[h, tok0 + row0:tok0 + min(row0 + rows, n)]
+                    assert bool(block.all()) if visits else not bool(block.any()), (h, key, tok0 + row0, first)
+                    finite += first > key - tok0 >= 0
+                tok0 += n
+    assert finite > 0   # (some tiles did stop before the key)
+
+
 @pytest.mark.parametrize("d,n,mean", [(64, 1024, -7.4), (33, 700, -12.0), (64, 300, -3.0), (128, 515, 0.0), (64, 130, 4.0)])
 def test_fp32_log_sums_against_64_bits(sb, cuda_device, d, n, mean):
     """rem and log_rem of the CUDA-core kernels over score ranges from a stick that hardly gets shorter per key (all factors
