@@ -572,6 +572,38 @@ def test_skipping_exact_zeros_changes_no_bit(sb, cuda_device, d, dtype, mode):
     H.assert_parity(fast, H.oracle_varlen(*ins, cu), dtype, "zeros skipped")
 
 
+@pytest.mark.parametrize("copies", [1, 40])   # an item table per block; a table in memory, from which the short-sequence kernel draws
+@pytest.mark.parametrize("d,dtype,longest", [(64, torch.bfloat16, 1000), (64, torch.float16, 1500), (128, torch.bfloat16, 1000),
+                                             (64, torch.float32, 1000), (50, torch.bfloat16, 1000)])
+def test_tiles_do_stop_and_say_so(sb, cuda_device, d, dtype, longest, copies):
+    """Heads with N(0, 1) scores stop early, heads with low scores and calls that are to visit every key do not, as the saved
+    state shows; where they stopped, outputs and gradients on the tensor cores are the bits of the call that visits every key."""
+    lengths = [longest, 129, 700, 65] * copies
+    ins = H.make_inputs((4, sum(lengths), d), dtype, seed=7 + d)
+    ins[0][2:] *= 0.05
+    cu = cu_of(lengths)
+    q, k, v = (t.to(cuda_device) for t in ins[:3])
+    o, rem, _, start = H.forward_state(sb, q, k, v, cu.to(cuda_device), longest)
+    o_all, rem_all, _, start_all = H.forward_state(sb, q, k, v, cu.to(cuda_device), longest, flags=sb._cabi.SB_FLAG_DENSE_ROW_PASS)
+    written = start >= 0
+    assert torch.equal(written, start_all >= 0) and int(start_all.max()) == 0 and int(start[2:].max()) == 0
+    tok0 = 0
+    for n in lengths:
+        groups = [(tok0 + row0) // 32 for row0 in range(64, n, 32)]
+        assert bool(written[:, groups].all())
+        late = [(tok0 + row0) // 32 for row0 in range(320, n, 32)]   # 320 keys back: N(0, 1) scores lose a bit or more of stick per key
+        assert not late or int(start[:2, late].min()) > 0
+        tok0 += n
+    assert int(written[0].sum()) == sum(max(0, (n + 31) // 32 - 2) for n in lengths)
+    if dtype != torch.float32 and d % 8 == 0:
+        assert torch.equal(o, o_all) and torch.equal(rem, rem_all)
+        got = H.run_varlen(sb, *ins, cu, cuda_device, max_seqlens=longest)
+        with sb.dense_row_pass():
+            want = H.run_varlen(sb, *ins, cu, cuda_device, max_seqlens=longest)
+        for name, a, b in zip(("o", "rem", "dq", "dk", "dv"), got, want):
+            assert torch.equal(a, b), name
+
+
 @pytest.mark.parametrize("d,dtype,lengths", [(128, torch.bfloat16, [4000, 1111]), (64, torch.float16, [4000, 1111]),
                                              (64, torch.bfloat16, [1000, 900] * 4), (64, torch.float32, [1500]), (50, torch.float16, [1500])])
 def test_values_that_are_not_finite_reach_the_tiles_that_visit_them(sb, cuda_device, d, dtype, lengths):
