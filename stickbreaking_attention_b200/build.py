@@ -11,6 +11,7 @@ leave it out because even the untaken branches cost a few percent.
 """
 from __future__ import annotations
 
+import importlib.util
 import os
 import shutil
 import subprocess
@@ -43,24 +44,29 @@ def _stale(target: str, deps) -> bool:
     return any(os.path.exists(d) and os.path.getmtime(d) > t for d in deps)
 
 
-def _start_ext(force: bool):
-    """Starts the compilation of the torch binding; returns the process, or None if it is up to date."""
+def _build_ext(force: bool) -> None:
+    """Compiles the torch binding if it is older than its source or than the torch it is built against; it links against the
+    kernels' library, which therefore comes first."""
     src = os.path.join(CSRC, EXT_SOURCE)
-    if not (force or _stale(EXT_PATH, [src, os.path.join(CSRC, "../../include/sb_b200.h")])):
-        return None
+    root = os.path.dirname(importlib.util.find_spec("torch").origin)
+    if not (force or _stale(EXT_PATH, [src, os.path.join(CSRC, "../../include/sb_b200.h"), os.path.join(root, "version.py")])):
+        return
     import sysconfig
 
     import torch
-    root = os.path.dirname(torch.__file__)
     cuda = os.path.dirname(os.path.dirname(os.path.realpath(find_nvcc())))
     inc = [os.path.join(root, "include"), os.path.join(root, "include", "torch", "csrc", "api", "include"),
            os.path.join(cuda, "include"), sysconfig.get_paths()["include"]]
-    cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden", "-w",
+    cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden", "-Wall",
            f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", "-DTORCH_API_INCLUDE_EXTENSION_H",
-           "-DTORCH_EXTENSION_NAME=_sb_torch", *[f"-I{i}" for i in inc], src, "-o", EXT_PATH + ".tmp",
+           "-DTORCH_EXTENSION_NAME=_sb_torch", *[f"-isystem{i}" for i in inc], src, "-o", EXT_PATH + ".tmp",
            f"-L{os.path.join(root, 'lib')}", "-lc10", "-lc10_cuda", "-ltorch", "-ltorch_cpu", "-ltorch_cuda", "-ltorch_python",
            f"-L{PKG_DIR}", "-l:libsb_b200.so", "-Wl,-rpath,$ORIGIN"]
-    return subprocess.Popen(cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
+    proc = subprocess.run(cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
+    sys.stderr.write(proc.stdout)
+    if proc.returncode != 0:
+        raise RuntimeError(f"the host compiler failed on {EXT_SOURCE}")
+    os.replace(EXT_PATH + ".tmp", EXT_PATH)
 
 
 def build(force: bool = False, verbose: bool = False) -> str:
@@ -88,13 +94,7 @@ def build(force: bool = False, verbose: bool = False) -> str:
     if force or procs or _stale(LIB_PATH, objs):
         cmd = [nvcc, "-shared", "-o", LIB_PATH, *objs, "-gencode", "arch=compute_100a,code=sm_100a"]
         subprocess.run(cmd, check=True)
-    ext = _start_ext(force)
-    if ext is not None:
-        out, _ = ext.communicate()
-        if ext.returncode != 0:
-            sys.stderr.write(out)
-            raise RuntimeError(f"the host compiler failed on {EXT_SOURCE}")
-        os.replace(EXT_PATH + ".tmp", EXT_PATH)
+    _build_ext(force)
     return LIB_PATH
 
 

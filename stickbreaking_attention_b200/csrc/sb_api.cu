@@ -230,7 +230,10 @@ static int fill_kparams(const SbParams *p, const Plan &pl, bool backward, KParam
   // tensor-core path has no shared memory left for the table.
   if (p->cu_seqlens != nullptr && p->num_seq <= kSmallSeqs && pl.tiles_cap <= kSmallItems) {
     const bool tc = pl.path == SB_PATH_TCGEN05;
-    k.small_table = (!backward && tc) || ((long long)pl.tiles_cap * p->heads <= 2 * 148 * (tc ? 2 : 4) && (pl.store_az || !tc));
+    int sms = 0;
+    const cudaError_t e = sm_count(&sms);
+    if (e != cudaSuccess) return fail(SB_ERR_CUDA, "SM count: %s", cudaGetErrorString(e));
+    k.small_table = (!backward && tc) || ((long long)pl.tiles_cap * p->heads <= 2 * sms * (tc ? 2 : 4) && (pl.store_az || !tc));
   }
   // Short sequences, forward, larger batches: the workers draw their items, and then the tiles of a sequence (eight at most:
   // see tc_tile) can be neighbours and share K/V through L2 (DRAM reads -38 %, time -1 %).

@@ -4,8 +4,8 @@
 // Two kernels per call, no atomics, no locks, fixed summation order:
 //   dq kernel (tc_bwd_dq2_kernel)   query-stationary, 256 query rows per block.  Walks the keys 0 -> diagonal in
 //               64-key sub-tiles; per step S = Q K^T and dP = dO V^T go to TMEM, one thread per query row recomputes
-//               A and dz = G - beta * C with the log-space suffix sum (fp64 across tiles, started from the saved
-//               log_rem) and the prefix sum C of G carried in registers, writes dz as a 16-bit tile, and
+//               A and dz = G - beta * C with the log-space suffix sum (a pair of floats across tiles, started from
+//               the saved fp64 log_rem) and the prefix sum C of G carried in registers, writes dz as a 16-bit tile, and
 //               dQ += dz K accumulates in TMEM.  It leaves for the second kernel either its A and dz tiles
 //               (stored-tiles mode) or, every 32 keys, the two carried values R1 and S2 (small-workspace mode).
 //   dK/dV kernel  key-stationary, one 128-key tile per block, query tiles diagonal -> end.

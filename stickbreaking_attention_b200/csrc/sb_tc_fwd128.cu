@@ -4,8 +4,8 @@
 // adjacent tiles share one stream of K/V sub-tiles; with sequences of a few hundred tokens that coupling costs more
 // than it saves: the earlier tile of a pair has no work in the first two steps of every item (half of a four-step
 // item), a sequence's last item often has no second tile at all, and both tiles stand still together at every item
-// boundary.  Here a block holds two WORKERS that share nothing but the SM: each has its own list of 128-row tiles
-// (weight-ordered, boustrophedon over all workers of the grid), its own TMA producer and MMA issuer, its own
+// boundary.  Here a block holds two WORKERS that share nothing but the SM: each gets its 128-row tiles one by one
+// (see fwd128_item: from a counter where a kernel has written the item table, else by a fixed walk), and has its own TMA producer and MMA issuer, its own
 // three-stage K/V ring, two Q buffers, S slots and O accumulator.  At 64 columns all of that fits twice.
 //   warps 0-3 / 4-7   rows of worker 0 / 1: one thread per query row (the row arithmetic of sb_tc_fwd_rows.cuh)
 //   warps 8 / 11      TMA producers of worker 0 / 1
@@ -302,7 +302,7 @@ tc_fwd128x2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
           const int gu = U + u, buf = gu & 1;
           bool halt = false;
           if (!first) {
-            ok = wait_or_abort(bar(bSFull + buf), (gu >> 1) & 1, abort_flag, p, 331);
+            ok = wait_or_abort(bar(bSFull + buf), (gu >> 1) & 1, abort_flag, p, 731);
             if (!ok) break;
             halt = stop.word[buf] == kStepStop;
           }

@@ -16,7 +16,7 @@ namespace sb {
 
 namespace fwd256 {
 constexpr int kThreads = 352;
-constexpr int kMaxStages = 6;
+constexpr int kMaxStages = 4;
 constexpr int kKvBoxBytes = kBN * 64 * 2;     // one 64-row x 64-column box
 constexpr int kBarBytes = 512;
 template <int D>                              // D: head size rounded up to 64 or 128
@@ -30,21 +30,21 @@ struct Cfg {
   // waiting ~1000 of 2800 clk for its keys.  Four fit next to one staging box per tile; at 64 columns six would, and are 1 %
   // slower (more keys in flight than L2 likes).
   static constexpr int kStages = 4;
+  static_assert(kStages <= kMaxStages, "barrier slots per stage");
   // Q tiles of two items at 64 columns (there is room): the next item's Q is loaded while the current item still
   // reads its own, so a short item does not wait a load latency for its first scores
   static constexpr int kQBufs = D == 64 ? 2 : 1;
   static constexpr int kSmem = 1024 + kQBufs * 2 * kQBytes + kStages * kStageBytes + 2 * kPBytes + kBarBytes + (int)sizeof(SmallTable);
   static_assert(kSmem <= 232448, "shared memory per block");
 };
-enum { bQ = 0, bKvFull = 1, bKvEmpty = 7, bSFull = 13, bQFree = 17, bOFree = 18, bPFull = 20, bOFull = 24, bQ2 = 26,
-       bQFree2 = 27, bNum = 28 };   // bQ2 / bQFree2: the second Q buffer
+enum { bQ = 0, bKvFull = 1, bKvEmpty = bKvFull + kMaxStages, bSFull = bKvEmpty + kMaxStages, bQFree = bSFull + 4, bOFree = bQFree + 1,
+       bPFull = bOFree + 2, bOFull = bPFull + 4, bQ2 = bOFull + 2, bQFree2 = bQ2 + 1, bNum = bQFree2 + 1 };   // bQ2 / bQFree2: the second Q buffer
 struct Shared {                     // behind the barriers
   Ctl ctl;
   EarlyStop stop[2];                // per tile
   int kv_end[kMaxStages];           // per stage: stage number + 1 if it holds no keys but marks the end of its item
 };
 static_assert(bNum * 8 + sizeof(Shared) <= kBarBytes, "barriers and control words");
-static_assert(bKvEmpty - bKvFull == kMaxStages && bSFull - bKvEmpty == kMaxStages, "barrier slots per stage");
 // per-warpgroup barrier index: base + wg * 2 + buf
 }  // namespace fwd256
 
