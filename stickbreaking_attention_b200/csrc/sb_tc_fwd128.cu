@@ -211,7 +211,6 @@ tc_fwd128x2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
             mma_commit(bar(bSFull + (gu & 1)));
             stop.word[gu & 1] = st;
             mbar_arrive(bar(bSFull + (gu & 1)));
-            halt = kStop && u >= 2 && u + 1 < w.n_steps && may_stop_before(w.s_top - u - 1) && all_through(stop, U, u);
             if (u == w.n_steps - 1) mma_commit(bar(bQFree + qb));   // the tile's last read of Q
           }
           if (u >= 1) {
@@ -221,11 +220,12 @@ tc_fwd128x2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
             if (ok && up == 0 && it >= 1) ok = wait_or_abort(bar(bOFree), (it - 1) & 1, abort_flag, p, 725);
             if (!ok) break;
             tc_fence_after();
-            through = through || (kStop && all_through(stop, U, up));
+            through = through || (kStop && up >= 2 && all_through(stop, U, up));
             if (!through)
               mma_tmem_mnmajor<kBN, kKvTileBytes>(tmem + 128, tmem + (gu & 1) * 64 + kPCol,
                                                   sKV + st * kStageBytes + kKvTileBytes, idesc_pv, up > 0);
             mma_commit(bar(bKvEmpty + st));
+            halt = kStop && u >= 2 && u + 1 < steps && may_stop_before(w.s_top - u - 1) && (through || all_through(stop, U, u));
           }
         }
         if (ok && early) {   // the stop word's slot has a P phase like every other; the rest of the tile's stages go unread

@@ -245,7 +245,6 @@ tc_fwd256_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
             mma_commit(bar(bSFull + wg * 2 + (gu & 1)));
             stop.word[gu & 1] = st;
             mbar_arrive(bar(bSFull + wg * 2 + (gu & 1)));
-            halt = may_stop && u >= 2 && u + 1 < my_steps && may_stop_before(w.s_top - t0 - u - 1) && all_through(stop, U, u);
             if (u == my_steps - 1) mma_commit(bar_qfree);   // the item's last read of Q
             trace_event(p, 1 + 3 * wg, tr_cur, 3 + 16 * wg, t0 + u);
           }
@@ -257,12 +256,13 @@ tc_fwd256_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
             if (!ok) break;
             trace_event(p, 1 + 3 * wg, tr_cur, 6 + 16 * wg, t0 + up);
             tc_fence_after();
-            through = through || (may_stop && all_through(stop, U, up));
+            through = through || (may_stop && up >= 2 && all_through(stop, U, up));
             // 16 keys per MMA; V: 64 rows x (2 x 64) columns, MN-major
             if (!through)
               mma_tmem_mnmajor<kBN, kKvBoxBytes>(tmem + 256 + wg * 128, tmem + wg * 128 + (gu & 1) * 64 + kPCol,
                                                  sKV + st * kStageBytes + kKvTileBytes, idesc_pv, up > 0);
             mma_commit(bar(bKvEmpty + st));
+            halt = may_stop && u >= 2 && u + 1 < steps && may_stop_before(w.s_top - t0 - u - 1) && (through || all_through(stop, U, u));
             trace_event(p, 1 + 3 * wg, tr_cur, 7 + 16 * wg, t0 + up);
           }
         }

@@ -191,7 +191,9 @@ __device__ __forceinline__ bool fwd256_row_pass(uint32_t ts, int key0, int row, 
 // scores of yet and tells the rows with the word that accompanies every step's scores.  Where exactly it stops depends on
 // timing, what is stored does not: not even where a value of V behind the last warp's stop is not finite (0 times it would
 // be NaN).  Rows that never finish pay nothing: the vote is the one the row pass takes anyway to skip its arithmetic, and the
-// issuer's look is a 16-byte read.
+// issuer's look is a 16-byte read.  It looks between the rows' word that P is there and P V (from the third step on: a tile's
+// first row has no keys in its own tile and loses at most 30 bits per key), and for the stop once P V is out: with that look
+// ahead of the wait for P the forward of 8 x 2048 x 16 heads N(0, 1) takes 82.5 us instead of 79.2.
 constexpr int kStepStop = -1;
 // No stop with fewer than three sub-tiles to go: what is left costs about as much as stopping and restarting the stream.
 __device__ __forceinline__ bool may_stop_before(int sub_tile) { return sub_tile >= 2; }
