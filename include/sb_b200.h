@@ -88,8 +88,9 @@ enum SbFlags {
                             there on everything a row computes per score (p in the forward; A, G and dz in the
                             backward) is exactly 0, and the tensor-core kernels skip that arithmetic wherever it
                             is 0 for all 32 rows of a warp: they keep only the running log-space sum.  With
-                            `tile_start` (below) whole tiles beyond that point are not visited either.  The
-                            results are bit-identical.  With this flag every tile is visited and the
+                            `tile_start` (below) whole tiles beyond that point are not visited either.  For
+                            finite inputs the tensor-core kernels' results are the same bit for bit (CUDA
+                            cores: see `tile_start`).  With this flag every tile is visited and the
                             arithmetic is done for every score regardless.                        */
 };
 
@@ -146,10 +147,18 @@ typedef struct SbParams {
                          * query rows where all of them have used their stick up (the product of (1 - beta) over *
                          * the keys visited is exactly 0 in fp32: no earlier key can add anything to o, rem or a *
                          * gradient), records here which key that was, and log_rem covers the visited keys only; *
-                         * the backward then starts at that key.  Results are the same bit for bit.              *
+                         * the backward then starts at that key.  Results for finite inputs: the same bit for   *
+                         * bit on the tensor cores, to rounding of the carried log sums on the CUDA cores.  A    *
+                         * key or value that is not finite is seen by the query tiles (128 rows; CUDA cores: 32) *
+                         * of which some row visits it (backward: visits its 128 keys) and by no others: 0 times *
+                         * it is left out there.                                                                 *
                          * Without it, or with SB_FLAG_DENSE_ROW_PASS in the forward, every key is visited and   *
                          * log_rem covers all of them.  Hand the same buffer (or NULL) to both calls, which have *
-                         * to take the same kernel path (sb_kernel_path).                                        */
+                         * to take the same kernel path (sb_kernel_path).                                        *
+                         * Entry (batch, head, (first token of the sequence + row) / 32) holds the first visited *
+                         * key, counted inside the sequence, of the rows row .. row + 31, row = 64, 96, ...; the *
+                         * first 64 rows of a sequence visit everything and have none.  All other entries are    *
+                         * left as they are.                                                                     */
   int64_t tile_start_stride; /* elements per (batch, head): at least ceil(tokens / 32)                           */
 } SbParams;
 

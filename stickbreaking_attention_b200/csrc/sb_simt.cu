@@ -279,7 +279,9 @@ cudaError_t launch_fused_dv(const KParams &p, int dtype, cudaStream_t s) {
 // ------------------------------------------------------------------------------------------------
 // CUDA-core kernels: fp32 arithmetic throughout, for fp32 tensors and head sizes the tensor-core kernels do not take.
 // ------------------------------------------------------------------------------------------------
-// What bounds them: shared-memory operand traffic of the fp32 products.  A block is 128 threads; every product of a step
+// What bounds them: latency at three blocks per SM, next to no single unit (2 x 8 heads x 1024 x 64 fp32: shared-memory and L1
+// pipe 59 to 66 % busy, FMA pipe 43 to 47 %, issue slots 41 to 46 %), and the tail of 512 blocks of unequal length (a quarter
+// of the SMs' time).  The products' operands come from shared memory: a block is 128 threads; every product of a step
 // gives each thread a 4 x 4 patch of the result (4 x DP/16 for the accumulators), so that eight 16-byte shared loads feed
 // 64 FMAs.  A step is 32 query rows x 64 keys (forward, dQ) or 64 query rows x 32 keys (dK/dV): small enough for three or
 // four blocks per SM at head size 64, and for a few heads of a few hundred tokens to spread over the GPU.  The scans over

@@ -66,7 +66,9 @@ def small_backward_workspace(enabled: bool = True):
 def dense_row_pass(enabled: bool = True):
     """Within the block (calling thread only) the tensor-core kernels do the per-score arithmetic for every score, also
     where the product of (1 - beta) over the keys in between has underflowed to exactly 0 for a whole warp and the
-    results are known to be exact zeros (``SB_FLAG_DENSE_ROW_PASS``).  Same results bit for bit; a measuring aid."""
+    results are known to be exact zeros, and all kernels visit every key (``SB_FLAG_DENSE_ROW_PASS``).  For finite inputs the
+    same results bit for bit on the tensor cores and to rounding on the CUDA cores; a measuring aid, and the way to have a
+    NaN or an infinity in a key far back show in every row that attends to it with weight 0."""
     old = _state.dense_row_pass
     _state.dense_row_pass = enabled
     try:
