@@ -28,7 +28,7 @@ static inline size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; 
 
 // Workspace layout, a pure function of the shapes:
 //   [hdr 256 B][pair_prefix int64 x (num_seq+1)]
-//   packed batches: [order int2 x tiles][order2 (backward) int2 x tiles]
+//   packed batches: [order int2 x tiles]
 //   backward, either: [A | dz tiles, 16-bit x chunk_heads x pairs_cap x 2 x 128 x 128]   (stored-tiles mode)
 //             or:     [R1 fp32 x chunk_heads x pairs_cap x halves x tile][S2 same]       (recompute mode)
 //   backward with SB_FLAG_FUSE_REM_V: [d_rem + <d_out, v>, one value of the tensors' dtype in a 4-byte slot budget x batch x heads x tokens]
@@ -39,7 +39,7 @@ struct Plan {
   int n_max;
   int max_seqlen;
   long long pairs_cap;
-  size_t off_pair_prefix, off_order, off_order2, off_bnd, off_drem;
+  size_t off_pair_prefix, off_order, off_bnd, off_drem;
   int bnd_halves;             // boundary records per (query tile, key tile) pair
   size_t bnd_bytes_per_head;  // one of the two arrays
   int chunk_heads;
@@ -110,8 +110,7 @@ static int make_plan(const SbParams *p, Plan &pl, bool backward) {
   pl.off_pair_prefix = 256;
   pl.off_order = align_up(pl.off_pair_prefix + sizeof(long long) * (size_t)(p->num_seq + 1), 256);
   const size_t order_bytes = p->cu_seqlens != nullptr ? align_up(sizeof(int2) * (size_t)pl.tiles_cap, 256) : 0;
-  pl.off_order2 = pl.off_order + order_bytes;                       // every second tile: the backward's dq kernel
-  pl.off_bnd = pl.off_order2 + ((backward && tc) ? order_bytes : 0);
+  pl.off_bnd = pl.off_order + order_bytes;
   // the tensor-core path records the carried values four times per 128-key tile
   pl.bnd_halves = tc ? 4 : 1;   // keys 0, 32, 64, 96 of every 128-key tile
   pl.bnd_bytes_per_head = align_up((size_t)pl.pairs_cap * pl.tile * pl.bnd_halves * sizeof(float), 256);
@@ -214,10 +213,7 @@ static int fill_kparams(const SbParams *p, const Plan &pl, bool backward, KParam
   char *ws = reinterpret_cast<char *>(p->workspace);
   k.hdr = reinterpret_cast<int *>(ws);
   k.pair_prefix = reinterpret_cast<long long *>(ws + pl.off_pair_prefix);
-  if (p->cu_seqlens != nullptr) {
-    k.order = reinterpret_cast<const int2 *>(ws + pl.off_order);
-    if (pl.off_bnd != pl.off_order2) k.order2 = reinterpret_cast<const int2 *>(ws + pl.off_order2);
-  }
+  if (p->cu_seqlens != nullptr) k.order = reinterpret_cast<const int2 *>(ws + pl.off_order);
   if (backward && pl.store_az) {
     k.az = reinterpret_cast<unsigned short *>(ws + pl.off_bnd);
   } else {

@@ -41,13 +41,12 @@ struct KParams {
   int dense;               // measuring aid: do the per-score arithmetic even where it is known to give exact zeros
   int small_table;         // packed batches: every block builds the item table itself (see SmallTable)
   const int2 *order;       // packed batches: work items by descending weight, see decode_item
-  const int2 *order2;      // the same for every second tile (backward only)
-  int order_span;          // entries of one sequence that stay neighbours in order / order2 (>= 1)
+  int order_span;          // entries of one sequence that stay neighbours in order (>= 1)
   int trace_mode;          // diagnostics builds: bit 1 = log every block's SM, start, first row work and end time
   int dbg;                 // experiments only (SbParams.reserved): 0 = normal arithmetic
   unsigned long long *trace;  // experiments only: event log of block (0,0) in the workspace tail, or nullptr
   // workspace views
-  int *hdr;            // [0] cu_seqlens refused, [1] end of the last sequence, [2] / [3] entries of order / order2
+  int *hdr;            // [0] cu_seqlens refused, [1] end of the last sequence, [2] entries of order
   unsigned *item_counter;  // hdr[4]: items the workers of a persistent kernel have drawn, or null: fixed assignment
   long long *pair_prefix;  // [num_seq] exclusive prefix of n(n+1)/2 (varlen)
   float *bnd_r1;       // [head_cnt][pairs_cap][tile]  suffix sums of log(1-beta) at tile starts
@@ -144,9 +143,8 @@ struct QueryList {
 // ---- which work items there are ---------------------------------------------------------------------------------------
 // Work items (query or key tiles) are ordered by weight across ALL sequences: the tile with the most key (or query) tiles
 // to visit comes first, so that the blocks that run longest start earliest and the last blocks of a launch are the short
-// ones.  An entry is (sequence, k), k = tile index counted so that larger means heavier; `group` > 1 lists every group-th
-// tile only.  For a fixed-length batch the order is arithmetic.  For a packed batch it is a table, either written by a
-// kernel that runs first (p.order, p.order2, p.pair_prefix, p.hdr), or, for small calls (p.small_table), built by every
+// ones.  An entry is (sequence, k), k = tile index counted so that larger means heavier.  For a fixed-length batch the order is arithmetic.  For a packed batch it is a table, either written by a
+// kernel that runs first (p.order, p.pair_prefix, p.hdr), or, for small calls (p.small_table), built by every
 // block for itself in shared memory: a launch and its hand-over cost more than the microsecond this takes.
 constexpr int kSmallSeqs = 128, kSmallItems = 256;
 struct SmallTable {                       // 1.5 KB: what the kernels' shared memory has left
@@ -159,7 +157,7 @@ __device__ __forceinline__ bool seq_valid(const KParams &p, long long start, lon
 }
 
 // By all threads of the block (at least kSmallSeqs of them); contains barriers.  Returns whether cu_seqlens was refused.
-__device__ __forceinline__ bool build_small_table(const KParams &p, int group, SmallTable &tb) {
+__device__ __forceinline__ bool build_small_table(const KParams &p, SmallTable &tb) {
   const int t = threadIdx.x, span = p.order_span;
   bool bad = false;
   uint32_t n = 0;
@@ -184,7 +182,7 @@ __device__ __forceinline__ bool build_small_table(const KParams &p, int group, S
   for (int i = t; i < kSmallItems; i += blockDim.x) {
     int s = 0, e = i, m = 0;
     for (; s < p.num_seq; ++s) {
-      m = ((int)tb.pair0[s] + group - 1) / group;
+      m = (int)tb.pair0[s];
       if (e < m) break;
       e -= m;
     }
@@ -192,11 +190,11 @@ __device__ __forceinline__ bool build_small_table(const KParams &p, int group, S
     const int lo = e / span * span, hi = lo + span;
     int pos = min(hi, m) - 1 - e;
     for (int q = 0; q < p.num_seq; ++q) {
-      const int mq = ((int)tb.pair0[q] + group - 1) / group;
+      const int mq = (int)tb.pair0[q];
       pos += max(mq - hi, 0);
       if (q < s) pos += min(max(mq - lo, 0), span);
     }
-    tb.order[pos] = (uint32_t)s << 16 | (uint32_t)(e * group);
+    tb.order[pos] = (uint32_t)s << 16 | (uint32_t)e;
   }
   uint32_t before = 0;
   if (t < p.num_seq)
@@ -209,15 +207,14 @@ __device__ __forceinline__ bool build_small_table(const KParams &p, int group, S
 
 // `reverse`: the heavy tiles are the late ones (a query tile sees all earlier keys); otherwise the early ones (a key tile
 // is seen by all later queries).
-__device__ __forceinline__ bool decode_item(const KParams &p, const SmallTable &tb, int item, int group, bool reverse, TileCoord &c) {
+__device__ __forceinline__ bool decode_item(const KParams &p, const SmallTable &tb, int item, bool reverse, TileCoord &c) {
   int s, k;
   if (p.cu == nullptr) {
     const int n = (int)((p.tokens + p.tile - 1) / p.tile);
-    const int m = (n + group - 1) / group;
-    if (item >= m * p.batch) return false;
+    if (item >= n * p.batch) return false;
     const int j = item / p.batch;
     s = item - j * p.batch;
-    k = (m - 1 - j) * group;
+    k = n - 1 - j;
     c.n_tiles = n;
     c.len = (int)p.tokens;
     c.tok0 = 0;
@@ -232,8 +229,8 @@ __device__ __forceinline__ bool decode_item(const KParams &p, const SmallTable &
       k = (int)(e & 0xffffu);
       c.pair0 = tb.pair0[s];
     } else {
-      if (item >= p.hdr[group == 1 ? 2 : 3]) return false;
-      const int2 e = (group == 1 ? p.order : p.order2)[item];
+      if (item >= p.hdr[2]) return false;
+      const int2 e = p.order[item];
       s = e.x;
       k = e.y;
       c.pair0 = p.pair_prefix[s];
@@ -248,10 +245,10 @@ __device__ __forceinline__ bool decode_item(const KParams &p, const SmallTable &
   return true;
 }
 // One-dimensional grids: block = item * head_cnt + head, so that equal-weight items of all heads are neighbours.
-__device__ __forceinline__ bool decode_block(const KParams &p, const SmallTable &tb, int group, bool reverse, TileCoord &c, int &hh) {
+__device__ __forceinline__ bool decode_block(const KParams &p, const SmallTable &tb, bool reverse, TileCoord &c, int &hh) {
   const int item = blockIdx.x / p.head_cnt;
   hh = blockIdx.x - item * p.head_cnt;
-  return decode_item(p, tb, item, group, reverse, c);
+  return decode_item(p, tb, item, reverse, c);
 }
 
 // ---- rows no sequence covers --------------------------------------------------------------------------------------------
@@ -293,7 +290,7 @@ __device__ __forceinline__ void fill_forward_rows(const KParams &p, long long fi
 }
 // A kernel's first step: its item table (by all threads; contains barriers for a small packed batch).  Returns the end of
 // the last sequence; `refused`: cu_seqlens was, nothing is to be computed and no row counts as covered.
-__device__ __forceinline__ long long open_table(const KParams &p, int group, SmallTable &tb, bool &refused) {
+__device__ __forceinline__ long long open_table(const KParams &p, SmallTable &tb, bool &refused) {
   refused = false;
   if (p.cu == nullptr) return p.tokens;
   if (!p.small_table) {
@@ -301,19 +298,13 @@ __device__ __forceinline__ long long open_table(const KParams &p, int group, Sma
     refused = h.x != 0;
     return h.y;
   }
-  refused = build_small_table(p, group, tb);
+  refused = build_small_table(p, tb);
   return refused ? 0 : load_cu(p, p.num_seq - 1);
 }
 
 // Blocks to launch for such a grid (an upper bound for packed batches: surplus blocks leave at once).
-inline long long item_blocks(const KParams &p, int group) {
-  long long items;
-  if (p.cu == nullptr) {
-    const long long n = (p.tokens + p.tile - 1) / p.tile;
-    items = ((n + group - 1) / group) * p.batch;
-  } else {
-    items = group == 1 ? p.tiles_cap : (p.tiles_cap + p.num_seq + 1) / 2;
-  }
+inline long long item_blocks(const KParams &p) {
+  const long long items = p.cu == nullptr ? (p.tokens + p.tile - 1) / p.tile * p.batch : p.tiles_cap;
   return items * p.head_cnt;
 }
 

@@ -9,8 +9,7 @@ namespace sb {
 // Sequence table of the larger packed batches: the first (query tile, key tile) pair of every sequence, and the work items
 // by descending weight (see decode_item).
 // ------------------------------------------------------------------------------------------------
-// The order is a counting sort over classes of `order_span` consecutive tiles (counted in units of `group`), the heaviest
-// class first.  The tiles of one sequence inside a class stay neighbours (they read the same keys or queries at about the
+// The order is a counting sort over classes of `order_span` consecutive tiles, the heaviest class first.  The tiles of one sequence inside a class stay neighbours (they read the same keys or queries at about the
 // same time and share them through L2); the order of the sequences inside a class is whatever the shared-memory atomics
 // give, which does not matter.
 // One block: what bounds it is latency, so every phase is a few steps of 1024 threads.  Sequences of few classes are taken
@@ -52,17 +51,16 @@ __device__ __forceinline__ int seq_tiles(const KParams &p, int s) {
   return (int)((end - start + p.tile - 1) / p.tile);
 }
 
-__device__ void build_order(const KParams &p, int group, int2 *out, int hdr_slot, int *s_cls, int *s_warp) {
+__device__ void build_order(const KParams &p, int2 *out, int *s_cls, int *s_warp) {
   const int t = threadIdx.x, lane = t & 31;
   const int span = p.order_span;                         // entries of one sequence that stay neighbours
-  const int m_max = (p.n_max + group - 1) / group;       // entries of the longest sequence
-  const int c_max = (m_max + span - 1) / span;           // classes
+  const int c_max = (p.n_max + span - 1) / span;         // classes
   if (c_max > kMaxClasses) {   // sequences beyond millions of tokens: sequence by sequence, serially
     if (t == 0) {
       int pos = 0;
       for (int s = 0; s < p.num_seq; ++s)
-        for (int j = (seq_tiles(p, s) + group - 1) / group - 1; j >= 0; --j) out[pos++] = make_int2(s, j * group);
-      p.hdr[hdr_slot] = pos;
+        for (int j = seq_tiles(p, s) - 1; j >= 0; --j) out[pos++] = make_int2(s, j);
+      p.hdr[2] = pos;
     }
     __syncthreads();
     return;
@@ -75,12 +73,12 @@ __device__ void build_order(const KParams &p, int group, int2 *out, int hdr_slot
     const int step = wide ? kPrepThreads / 32 : kPrepThreads;
     for (int s0 = 0; s0 < p.num_seq; s0 += step) {
       const int s = s0 + (wide ? t >> 5 : t);
-      const int m = s < p.num_seq ? (seq_tiles(p, s) + group - 1) / group : 0;
+      const int m = s < p.num_seq ? seq_tiles(p, s) : 0;
       if (wide) {
         for (int cl = lane; cl * span < m; cl += 32) {
           const int n = min(span, m - cl * span), pos = atomicAdd(&s_cls[cl], n);
           if (write)
-            for (int i = 0; i < n; ++i) out[pos + i] = make_int2(s, (cl * span + n - 1 - i) * group);   // heaviest first
+            for (int i = 0; i < n; ++i) out[pos + i] = make_int2(s, cl * span + n - 1 - i);   // heaviest first
         }
       } else {
         for (int cl = 0; cl < c_max; ++cl) {   // the same class in all lanes: one atomic per warp
@@ -97,7 +95,7 @@ __device__ void build_order(const KParams &p, int group, int2 *out, int hdr_slot
           if (lane == 0) base = atomicAdd(&s_cls[cl], sum);
           const int pos = __shfl_sync(0xffffffffu, base, 0) + incl - n;
           if (write)
-            for (int i = 0; i < n; ++i) out[pos + i] = make_int2(s, (cl * span + n - 1 - i) * group);
+            for (int i = 0; i < n; ++i) out[pos + i] = make_int2(s, cl * span + n - 1 - i);
         }
       }
     }
@@ -114,7 +112,7 @@ __device__ void build_order(const KParams &p, int group, int2 *out, int hdr_slot
     if (cl >= 0) s_cls[cl] = base + before;
     base += total;
   }
-  if (t == 0) p.hdr[hdr_slot] = base;
+  if (t == 0) p.hdr[2] = base;
   __syncthreads();
   sweep(true);
   __syncthreads();
@@ -153,9 +151,7 @@ __global__ void __launch_bounds__(kPrepThreads) prep_kernel(KParams p) {
     const long long n = seq_tiles(p, s);
     before += n * (n + 1) / 2;
   }
-  int *s_warp_i = reinterpret_cast<int *>(s_warp);
-  build_order(p, 1, const_cast<int2 *>(p.order), 2, s_cls, s_warp_i);
-  if (p.order2 != nullptr) build_order(p, 2, const_cast<int2 *>(p.order2), 3, s_cls, s_warp_i);
+  build_order(p, const_cast<int2 *>(p.order), s_cls, reinterpret_cast<int *>(s_warp));
 }
 
 #ifdef SB_TRACE
@@ -493,11 +489,11 @@ __global__ void __launch_bounds__(kSimtThreads, kSimtBlocks<DP>) simt_fwd_kernel
   extern __shared__ float4 smem4[];
   __shared__ SmallTable tb;
   bool refused;
-  const long long covered = open_table(p, 1, tb, refused);
+  const long long covered = open_table(p, tb, refused);
   const int block = blockIdx.y * gridDim.x + blockIdx.x, blocks = gridDim.x * gridDim.y;
   if (covered < p.tokens) fill_forward_rows<T>(p, covered, refused, block, blocks);
   TileCoord c;
-  if (refused || !decode_item(p, tb, blockIdx.x, 1, true, c)) return;
+  if (refused || !decode_item(p, tb, blockIdx.x, true, c)) return;
   const int d = p.head_dim, h = p.head0 + blockIdx.y, t = threadIdx.x;
   float *Qs = reinterpret_cast<float *>(smem4), *Ks = Qs + kT * kLd<DP>, *Vs = Ks + kStep * kLd<DP>, *Ss = Vs + kStep * kLd<DP>;
   const int row0 = c.idx * kT, ac = p.attend_current;
@@ -658,11 +654,11 @@ __global__ void __launch_bounds__(kSimtThreads, kSimtBlocks<DP>) simt_bwd_dq_ker
   extern __shared__ float4 smem4[];
   __shared__ SmallTable tb;
   bool refused;
-  const long long covered = open_table(p, 1, tb, refused);
+  const long long covered = open_table(p, tb, refused);
   const int block = blockIdx.y * gridDim.x + blockIdx.x, blocks = gridDim.x * gridDim.y;
   if (covered < p.tokens) fill_rows<T>(p.dq, fill_job(p, covered, refused, block, blocks));
   TileCoord c;
-  if (refused || !decode_item(p, tb, blockIdx.x, 1, true, c)) return;
+  if (refused || !decode_item(p, tb, blockIdx.x, true, c)) return;
   const int d = p.head_dim, hh = blockIdx.y, h = p.head0 + hh, t = threadIdx.x;
   float *Qs = reinterpret_cast<float *>(smem4), *Gs = Qs + kT * kLd<DP>, *Ks = Gs + kT * kLd<DP>, *Vs = Ks + kStep * kLd<DP>;
   float *Zs = Vs + kStep * kLd<DP>, *Ps = Zs + kT * kLdS;
@@ -759,14 +755,14 @@ __global__ void __launch_bounds__(kSimtThreads, kSimtBlocks<DP>) simt_bwd_dkv_ke
   extern __shared__ float4 smem4[];
   __shared__ SmallTable tb;
   bool refused;
-  const long long covered = open_table(p, 1, tb, refused);
+  const long long covered = open_table(p, tb, refused);
   const int block = blockIdx.y * gridDim.x + blockIdx.x, blocks = gridDim.x * gridDim.y;
   if (covered < p.tokens) {
     fill_rows<T>(p.dk, fill_job(p, covered, refused, block, blocks));
     fill_rows<T>(p.dv, fill_job(p, covered, refused, block, blocks));
   }
   TileCoord c;
-  if (refused || !decode_item(p, tb, blockIdx.x, 1, false, c)) return;
+  if (refused || !decode_item(p, tb, blockIdx.x, false, c)) return;
   const int d = p.head_dim, hh = blockIdx.y, h = p.head0 + hh, t = threadIdx.x;
   float *Qs = reinterpret_cast<float *>(smem4), *Gs = Qs + kStep * kLd<DP>, *Zs = Gs + kStep * kLd<DP>, *Ps = Zs + kStep * kLdH;
   float *Ks = Ps + kStep * kLdH, *Vs = Ks + kT * kLd<DP>;   // recomputation only

@@ -2,10 +2,10 @@
 // sb_varlen_bwd.py:297-481, which accumulates dK/dV across blocks under a global spin lock).
 //
 // Two kernels per call, no atomics, no locks, fixed summation order:
-//   dq kernel (tc_bwd_dq2_kernel)   query-stationary, 256 query rows per block.  Walks the keys 0 -> diagonal in
+//   dq kernel (tc_bwd_dq3_kernel)   query-stationary, 128 query rows per block.  Walks the keys 0 -> diagonal in
 //               64-key sub-tiles; per step S = Q K^T and dP = dO V^T go to TMEM, one thread per query row recomputes
 //               A and dz = G - beta * C with the log-space suffix sum (a pair of floats across tiles, started from
-//               the saved fp64 log_rem) and the prefix sum C of G carried in registers, writes dz as a 16-bit tile, and
+//               the saved fp64 log_rem) and the prefix sum C of G carried in registers, writes dz to TMEM in 16 bits, and
 //               dQ += dz K accumulates in TMEM.  It leaves for the second kernel either its A and dz tiles
 //               (stored-tiles mode) or, every 32 keys, the two carried values R1 and S2 (small-workspace mode).
 //   dK/dV kernel  key-stationary, one 128-key tile per block, query tiles diagonal -> end.
@@ -37,98 +37,83 @@ namespace sb {
 // Packed pairs (two fp32 per instruction) are used where a pair sits in adjacent registers anyway -- accumulator columns and
 // what is computed column by column from them.  Products across columns stay scalar: pairing their operands up costs as many
 // register moves as the packed instruction saves.
-struct BwdChunk {
-  float2 be01[4], be23[4];   // beta
-  float pa[16];              // A
-  bool zero;                 // the chunk is known to be zero for all rows of the warp
+struct BwdExp {                    // what follows from a chunk's scores alone
+  float2 e01[4], e23[4];           // e
+  float2 be01[4], be23[4];         // beta
+  float rpg[4], i23[4], ri1[4], ri3[4];   // per group: 1 / t0 t1 t2 t3, 1 / t2 t3, 1 / t1, 1 / t3
+  float log;                       // log2 of the product of t, added up like the forward's (see fwd256_row_chunk): the two agree bit for bit
 };
 
-// Sweeps 1 and 2, which do not need dP; `between` runs where the fewest registers are in use and half of sweep 2 is left.
-template <bool kMasked, bool kSkip, class Between>
-__device__ __forceinline__ void bwd_chunk_weights(const uint32_t (&s)[16], int mc0, int limit, float scale2, float r1, float g_before,
-                                                  float &logsum, BwdChunk &c, Between between, bool may_skip = true) {
-  float chunk_log = 0.f;   // summed per chunk, like the forward's (see fwd256_row_chunk): the two agree bit for bit
+// Sweep 1.
+template <bool kMasked>
+__device__ __forceinline__ void bwd_chunk_exp(const uint32_t (&s)[16], int mc0, int limit, float scale2, BwdExp &c) {
   const float2 sc = make_float2(scale2, scale2), one = make_float2(1.f, 1.f);
-  float2 e01[4], e23[4], t01[4], t23[4];
+  c.log = 0.f;
 #pragma unroll
   for (int g = 3; g >= 0; --g) {
     const float2 x01 = mul2(make_float2(__uint_as_float(s[4 * g]), __uint_as_float(s[4 * g + 1])), sc);
     const float2 x23 = mul2(make_float2(__uint_as_float(s[4 * g + 2]), __uint_as_float(s[4 * g + 3])), sc);
-    e01[g] = make_float2(ex2(fminf(x01.x, 30.f)), ex2(fminf(x01.y, 30.f)));
-    e23[g] = make_float2(ex2(fminf(x23.x, 30.f)), ex2(fminf(x23.y, 30.f)));
-    t01[g] = add2(e01[g], one);
-    t23[g] = add2(e23[g], one);
+    float2 e01 = make_float2(ex2(fminf(x01.x, 30.f)), ex2(fminf(x01.y, 30.f)));
+    float2 e23 = make_float2(ex2(fminf(x23.x, 30.f)), ex2(fminf(x23.y, 30.f)));
+    float2 t01 = add2(e01, one), t23 = add2(e23, one);
     if (kMasked) {
       const int col = mc0 + 4 * g;
-      if (!(col < limit)) { e01[g].x = 0.f; t01[g].x = 1.f; }
-      if (!(col + 1 < limit)) { e01[g].y = 0.f; t01[g].y = 1.f; }
-      if (!(col + 2 < limit)) { e23[g].x = 0.f; t23[g].x = 1.f; }
-      if (!(col + 3 < limit)) { e23[g].y = 0.f; t23[g].y = 1.f; }
+      if (!(col < limit)) { e01.x = 0.f; t01.x = 1.f; }
+      if (!(col + 1 < limit)) { e01.y = 0.f; t01.y = 1.f; }
+      if (!(col + 2 < limit)) { e23.x = 0.f; t23.x = 1.f; }
+      if (!(col + 3 < limit)) { e23.y = 0.f; t23.y = 1.f; }
     }
-    chunk_log += lg2((t01[g].x * t01[g].y) * (t23[g].x * t23[g].y));
-  }
-  logsum += chunk_log;
-  c.zero = kSkip && may_skip && __all_sync(0xffffffffu, ex2(r1 + logsum) == 0.f && g_before == 0.f);
-  if (c.zero) {
-#pragma unroll
-    for (int i = 0; i < 16; ++i) c.pa[i] = 0.f;
-    between();
-    return;
-  }
-  float rpg[4], i23[4], ri1[4], ri3[4];
-#pragma unroll
-  for (int g = 0; g < 4; ++g) {
-    const float p01 = t01[g].x * t01[g].y, p23 = t23[g].x * t23[g].y;
-    const float rp = rcp(p01 * p23);
+    const float p01 = t01.x * t01.y, p23 = t23.x * t23.y, prod = p01 * p23;
+    c.log += lg2(prod);
+    const float rp = rcp(prod);
     const float i01 = rp * p23;                 // 1 / t0 t1
-    i23[g] = rp * p01;                          // 1 / t2 t3
-    const float2 ri01 = make_float2(i01 * t01[g].y, i01 * t01[g].x);
-    const float2 ri23 = make_float2(i23[g] * t23[g].y, i23[g] * t23[g].x);
-    c.be01[g] = mul2(e01[g], ri01);
-    c.be23[g] = mul2(e23[g], ri23);
-    rpg[g] = rp;
-    ri1[g] = ri01.y;
-    ri3[g] = ri23.y;
-  }
-  between();
-  float wend = ex2(r1 + logsum);   // product of (1 - beta) over everything after the chunk
-#pragma unroll
-  for (int g = 3; g >= 0; --g) {
-    const float2 w23 = make_float2(wend * i23[g], wend * ri3[g]);   // inclusive products at columns 2, 3
-    wend *= rpg[g];                                                  // at column 0 = after the previous group
-    const float2 w01 = make_float2(wend, w23.x * ri1[g]);
-    const float2 a01 = mul2(e01[g], w01);
-    const float2 a23 = mul2(e23[g], w23);
-    c.pa[4 * g] = a01.x;
-    c.pa[4 * g + 1] = a01.y;
-    c.pa[4 * g + 2] = a23.x;
-    c.pa[4 * g + 3] = a23.y;
+    c.i23[g] = rp * p01;                        // 1 / t2 t3
+    const float2 ri01 = make_float2(i01 * t01.y, i01 * t01.x);
+    const float2 ri23 = make_float2(c.i23[g] * t23.y, c.i23[g] * t23.x);
+    c.e01[g] = e01;
+    c.e23[g] = e23;
+    c.be01[g] = mul2(e01, ri01);
+    c.be23[g] = mul2(e23, ri23);
+    c.rpg[g] = rp;
+    c.ri1[g] = ri01.y;
+    c.ri3[g] = ri23.y;
   }
 }
 
-// Sweep 3.  On entry `gs` is the pass's sum of G before the chunk; pz: dz.
-template <bool kMasked, bool kSkip>
-__device__ __forceinline__ void bwd_chunk_dz(const uint32_t (&dp)[16], int mc0, int limit, float gpre, float dr, float &gs, BwdChunk &c,
-                                             float (&pz)[16]) {
-  if (kSkip && c.zero) {
+// Sweep 2.  wend: the product of (1 - beta) over everything after the chunk.  pa: A.
+__device__ __forceinline__ void bwd_chunk_products(const BwdExp &c, float wend, float (&pa)[16]) {
 #pragma unroll
-    for (int i = 0; i < 16; ++i) pz[i] = 0.f;
-    return;
+  for (int g = 3; g >= 0; --g) {
+    const float2 w23 = make_float2(wend * c.i23[g], wend * c.ri3[g]);   // inclusive products at columns 2, 3
+    wend *= c.rpg[g];                                                    // at column 0 = after the previous group
+    const float2 w01 = make_float2(wend, w23.x * c.ri1[g]);
+    const float2 a01 = mul2(c.e01[g], w01);
+    const float2 a23 = mul2(c.e23[g], w23);
+    pa[4 * g] = a01.x;
+    pa[4 * g + 1] = a01.y;
+    pa[4 * g + 2] = a23.x;
+    pa[4 * g + 3] = a23.y;
   }
+}
+
+// Sweep 3.  On entry `gs` is the sum of G between gpre and the chunk; pz: dz.
+template <bool kMasked>
+__device__ __forceinline__ void bwd_chunk_dz(const BwdExp &c, const uint32_t (&dp)[16], int mc0, int limit, float gpre, float dr, float &gs,
+                                             float (&pa)[16], float (&pz)[16]) {
   const float2 ndr = make_float2(-dr, -dr);
   float cb = gpre + gs, csum = 0.f;   // C before the group; the chunk's own sum of G
 #pragma unroll
   for (int g = 0; g < 4; ++g) {
-    float2 g01 = mul2(make_float2(c.pa[4 * g], c.pa[4 * g + 1]),
+    float2 g01 = mul2(make_float2(pa[4 * g], pa[4 * g + 1]),
                       add2(make_float2(__uint_as_float(dp[4 * g]), __uint_as_float(dp[4 * g + 1])), ndr));
-    float2 g23 = mul2(make_float2(c.pa[4 * g + 2], c.pa[4 * g + 3]),
+    float2 g23 = mul2(make_float2(pa[4 * g + 2], pa[4 * g + 3]),
                       add2(make_float2(__uint_as_float(dp[4 * g + 2]), __uint_as_float(dp[4 * g + 3])), ndr));
     if (kMasked) {   // rows past the sequence end carry arbitrary values: select, do not rely on 0 * x
       const int col = mc0 + 4 * g;
-      if (!(col < limit)) { g01.x = 0.f; c.pa[4 * g] = 0.f; }
-      if (!(col + 1 < limit)) { g01.y = 0.f; c.pa[4 * g + 1] = 0.f; }
-      if (!(col + 2 < limit)) { g23.x = 0.f; c.pa[4 * g + 2] = 0.f; }
-      if (!(col + 3 < limit)) { g23.y = 0.f; c.pa[4 * g + 3] = 0.f; }
+      if (!(col < limit)) { g01.x = 0.f; pa[4 * g] = 0.f; }
+      if (!(col + 1 < limit)) { g01.y = 0.f; pa[4 * g + 1] = 0.f; }
+      if (!(col + 2 < limit)) { g23.x = 0.f; pa[4 * g + 2] = 0.f; }
+      if (!(col + 3 < limit)) { g23.y = 0.f; pa[4 * g + 3] = 0.f; }
     }
     const float t1 = g01.x + g01.y, t23 = g23.x + g23.y;
     const float tg = t1 + t23;
@@ -153,358 +138,326 @@ __device__ __forceinline__ int chunk_limit(bool row_valid, bool diag, int r, int
   return !row_valid ? -1 : (diag ? r + ac : 0x7fffffff);
 }
 
-// All three sweeps, A and dz written to the 16-bit tiles; c0 addresses the output tiles.
-template <bool kFp16, bool kMasked, bool kSkip>
-__device__ __forceinline__ void bwd_row_chunk(const uint32_t (&s)[16], const uint32_t (&dp)[16], int c0, int mc0, int r, int limit,
-                                              float scale2, float r1, float gpre, float dr, float &gs, float &logsum, uint8_t *tile_a,
-                                              uint8_t *tile_z, bool may_skip = true) {
-  BwdChunk c;
-  float pz[16];
-  bwd_chunk_weights<kMasked, kSkip>(s, mc0, limit, scale2, r1, gpre + gs, logsum, c, [] {}, may_skip);
-  bwd_chunk_dz<kMasked, kSkip>(dp, mc0, limit, gpre, dr, gs, c, pz);
-  store_row_chunk16<kFp16>(tile_a, r, c0, c.pa);
-  store_row_chunk16<kFp16>(tile_z, r, c0, pz);
-}
-
-// One row of a 64-key sub-tile of the dq kernel: four 16-column chunks.  What a pair of chunks still needs is requested
-// together in the first one's sweep 2, the second chunk's dP into the registers of the first one's scores, so that 48
-// registers do for everything in flight, and the last S and dP columns are in registers after two thirds of the pass:
-// bSpEmpty is signalled then (one arrival per warp), and the next sub-tile's scores are computed under the rest.  dP is not
-// waited for before half of the first chunk is done.
-// mc0: key index of the sub-tile's first column inside its 128-key tile (for the diagonal mask).  The dz tile of the
-// sub-tile before is waited for before the first store to it (in a tile's first sub-tile, an even one, that is the phase
-// before the barrier's first: no wait).  Returns false if a wait gave up.
-namespace dq2 {
-constexpr int kMaxStages = 4;
-enum { bQG = 0, bKvFull = 1, bKvEmpty = bKvFull + kMaxStages, bSFull = bKvEmpty + kMaxStages, bDpFull = bSFull + 2, bZFull = bDpFull + 2,
-       bZEmpty = bZFull + 2, bFirst = bZEmpty + 2, bSpEmpty = bFirst + 1, bDqFull = bSpEmpty + 2, bNum = bDqFull + 2 };
-}  // namespace dq2
-// `bars`: the dq kernel's barriers, offset by the tile's number.  out: stored-tiles mode: this row's 64 values of A in the
-// workspace; otherwise this row's record of R1 at the sub-tile's first key (S2 is `s2_off` floats further, both again kBM
-// floats further for the key 32 columns on).
-template <bool kFp16, bool kMasked, bool kStored, bool kSkip>
-__device__ __forceinline__ bool strip_row_pass(uint32_t ts, uint32_t tp, int r, int u, int mc0, int limit, float scale2, float r1, float gpre,
-                                              float dr, float &gs, float &logsum, uint8_t *tile_z, uint32_t bars, void *out,
-                                              long long s2_off) {
-  uint32_t s0[16], s1[16], d[16];
-  bool ok = true;
-  auto store = [&](int c0, const BwdChunk &c, const float (&pz)[16]) {
-    uint32_t wz[8];
-    pack_row_chunk16<kFp16>(pz, wz);
-    store_packed_chunk16(tile_z, r, c0, wz);
-    if constexpr (kStored) {
-      uint32_t wa[8];
-      pack_row_chunk16<kFp16>(c.pa, wa);
-      store_packed_global16(reinterpret_cast<unsigned short *>(out) + c0, wa);
-    }
-  };
-  tmem_ld16(ts, s0);
-#pragma unroll 1
-  for (int pair = 0; pair < 2; ++pair) {
-    const int c0 = pair * 32;
-    tmem_wait_ld_regs(s0);
-    {
-      BwdChunk c;
-      bwd_chunk_weights<kMasked, kSkip>(s0, mc0 + c0, limit, scale2, r1, gpre + gs, logsum, c, [&] {
-        if (pair == 0) {
-          ok = mbar_wait(bars + 8u * dq2::bDpFull, u & 1);
-          tc_fence_after();
-        }
-        tmem_ld16(tp + c0, d);
-        tmem_ld16(ts + c0 + 16, s1);
-        tmem_ld16(tp + c0 + 16, s0);
-      });
-      tmem_wait_ld_regs(d, s0);
-      asm volatile("" : "+r"(s1[0]), "+r"(s1[1]), "+r"(s1[2]), "+r"(s1[3]), "+r"(s1[4]), "+r"(s1[5]), "+r"(s1[6]), "+r"(s1[7]), "+r"(s1[8]),
-                   "+r"(s1[9]), "+r"(s1[10]), "+r"(s1[11]), "+r"(s1[12]), "+r"(s1[13]), "+r"(s1[14]), "+r"(s1[15])::"memory");
-      if (pair == 0) {
-        ok = mbar_wait(bars + 8u * dq2::bZEmpty, (u + 1) & 1) && ok;   // the previous sub-tile's dz has been read
-        tc_fence_after();
-      } else {               // the last columns are in registers: the S / dP slots can be overwritten
-        tc_fence_before();
-        __syncwarp();
-        if ((threadIdx.x & 31) == 0) mbar_arrive(bars + 8u * dq2::bSpEmpty);
-      }
-      float pz[16];
-      bwd_chunk_dz<kMasked, kSkip>(d, mc0 + c0, limit, gpre, dr, gs, c, pz);
-      store(c0, c, pz);
-    }
-    {
-      BwdChunk c;
-      float pz[16];
-      bwd_chunk_weights<kMasked, kSkip>(s1, mc0 + c0 + 16, limit, scale2, r1, gpre + gs, logsum, c, [] {});
-      bwd_chunk_dz<kMasked, kSkip>(s0, mc0 + c0 + 16, limit, gpre, dr, gs, c, pz);
-      store(c0 + 16, c, pz);
-    }
-    if (pair == 0) {
-      tmem_ld16(ts + 32, s0);
-      if constexpr (!kStored) {   // the carried values after 32 of the 64 columns
-        float *rec = reinterpret_cast<float *>(out) + kBM;
-        rec[0] = r1 + logsum;
-        rec[s2_off] = gpre + gs;
-      }
-    }
+// All three sweeps.  kSkip: see above.
+template <bool kMasked, bool kSkip>
+__device__ __forceinline__ void bwd_chunk(const uint32_t (&s)[16], const uint32_t (&dp)[16], int mc0, int limit, float scale2, float r1,
+                                          float gpre, float dr, float &gs, float &logsum, float (&pa)[16], float (&pz)[16], bool may_skip) {
+  BwdExp c;
+  bwd_chunk_exp<kMasked>(s, mc0, limit, scale2, c);
+  logsum += c.log;
+  const float wend = ex2(r1 + logsum);
+  if (kSkip && may_skip && __all_sync(0xffffffffu, wend == 0.f && gpre + gs == 0.f)) {
+#pragma unroll
+    for (int i = 0; i < 16; ++i) pa[i] = pz[i] = 0.f;
+    return;
   }
-  return ok;
+  bwd_chunk_products(c, wend, pa);
+  bwd_chunk_dz<kMasked>(c, dp, mc0, limit, gpre, dr, gs, pa, pz);
 }
 
 // What is recorded as R1 (a log2) where a row has not started: the product is 0, and so is all that follows from it.
 constexpr float kNothingLeft = -1e6f;
 
+namespace dq3 {
+enum { bQ = 0, bG, bKFull, bKEmpty = bKFull + 3, bVFull = bKEmpty + 3, bVEmpty = bVFull + 2, bSFull = bVEmpty + 2, bDpFull, bDqFull, bSEmpty,
+       bDpEmpty, bZFull, bNum = bZFull + 2 };
+}  // namespace dq3
+// One row of a 64-key sub-tile of the dq kernel, 16 columns at a time.  The loop's body is one chunk, about 330 instructions:
+// straight code over more of them is fetched more slowly than it is issued.  The next chunk's scores are requested as soon as
+// this one's are in use, dP under the products that do not need it; the S slot is handed back with a chunk and a half to go.
+// dz goes to tensor memory (key k of the sub-tile in column tz + k / 2, two per column), at 128 columns over the dP columns
+// that have been read by then.
+// mc0: key index of the sub-tile's first column inside its 128-key tile (for the diagonal mask).  Returns false if a wait gave up.
+// out: stored-tiles mode: this row's 64 values of A in the workspace, those of dz `off` elements further; otherwise this row's
+// record of R1 at the sub-tile's first key, S2 `off` floats further, both again kBM floats further for the key 32 columns on.
+template <bool kFp16, bool kMasked, bool kStored, bool kSkip>
+__device__ __forceinline__ bool strip_row_pass(uint32_t ts, uint32_t tp, uint32_t tz, int u, int mc0, int limit, float scale2, float r1,
+                                              float gpre, float dr, float &gs, float &logsum, uint32_t bars, void *out, long long off) {
+  uint32_t s[16], d[16];
+  bool ok = true;
+  tmem_ld16(ts, s);
+#pragma unroll 1
+  for (int c0 = 0; c0 < 64; c0 += 16) {
+    if (!kStored && c0 == 32) {   // the carried values after 32 of the 64 columns
+      float *rec = reinterpret_cast<float *>(out) + kBM;
+      rec[0] = r1 + logsum;
+      rec[off] = gpre + gs;
+    }
+    BwdExp x;
+    float pa[16], pz[16];
+    tmem_wait_ld_regs(s);
+    bwd_chunk_exp<kMasked>(s, mc0 + c0, limit, scale2, x);
+    if (c0 == 0) {
+      ok = mbar_wait(bars + 8u * dq3::bDpFull, u & 1);
+      tc_fence_after();
+    }
+    tmem_ld16(ts + min(c0 + 16, 48), s);   // (the last time: not used)
+    tmem_ld16(tp + c0, d);
+    logsum += x.log;
+    const float wend = ex2(r1 + logsum);
+    const bool zero = kSkip && __all_sync(0xffffffffu, wend == 0.f && gpre + gs == 0.f);
+    bwd_chunk_products(x, wend, pa);   // (not left out where `zero`: no branch while a tcgen05.ld is under way)
+    tmem_wait_ld_regs(s, d);
+    if (c0 >= 32) {   // the last columns of S (32: the chunk to come has them), then of dP are in registers
+      tc_fence_before();
+      __syncwarp();
+      if ((threadIdx.x & 31) == 0) mbar_arrive(bars + 8u * (c0 == 32 ? dq3::bSEmpty : dq3::bDpEmpty));
+    }
+    if (zero) {   // (A is zero as it is: e is finite)
+#pragma unroll
+      for (int i = 0; i < 16; ++i) pz[i] = 0.f;
+    } else {
+      bwd_chunk_dz<kMasked>(x, d, mc0 + c0, limit, gpre, dr, gs, pa, pz);
+    }
+    uint32_t w[8];
+    pack_row_chunk16<kFp16>(pz, w);
+    tmem_st8(tz + (c0 >> 1), w);
+    if constexpr (kStored) {
+      unsigned short *row = reinterpret_cast<unsigned short *>(out) + c0;
+      store_packed_global16(row + off, w);
+      pack_row_chunk16<kFp16>(pa, w);
+      store_packed_global16(row, w);
+    }
+  }
+  return ok;
+}
+
 // The same for a sub-tile before the first key of the warp's rows: dz (and the stored A) are zeros, the scores are not read.
 template <bool kStored>
-__device__ __forceinline__ bool zero_strip_row(uint8_t *tile_z, int r, int u, uint32_t bars, void *out, long long s2_off) {
+__device__ __forceinline__ bool zero_strip_row(uint32_t tz, int u, uint32_t bars, void *out, long long off) {
   const uint32_t z[8] = {0u, 0u, 0u, 0u, 0u, 0u, 0u, 0u};
-  const bool ok = mbar_wait(bars + 8u * dq2::bDpFull, u & 1) && mbar_wait(bars + 8u * dq2::bZEmpty, (u + 1) & 1);   // (every phase is followed)
+  const bool ok = mbar_wait(bars + 8u * dq3::bDpFull, u & 1);   // (every phase is followed; and dz may lie over dP)
+  tc_fence_after();
 #pragma unroll
   for (int c = 0; c < 64; c += 16) {
-    store_packed_chunk16(tile_z, r, c, z);
-    if constexpr (kStored) store_packed_global16(reinterpret_cast<unsigned short *>(out) + c, z);
+    tmem_st8(tz + (c >> 1), z);
+    if constexpr (kStored) {
+      unsigned short *row = reinterpret_cast<unsigned short *>(out) + c;
+      store_packed_global16(row, z);
+      store_packed_global16(row + off, z);
+    }
   }
   if constexpr (!kStored) {
     float *rec = reinterpret_cast<float *>(out) + kBM;
     rec[0] = kNothingLeft;
-    rec[s2_off] = 0.f;
+    rec[off] = 0.f;
   }
   __syncwarp();
-  if ((threadIdx.x & 31) == 0) mbar_arrive(bars + 8u * dq2::bSpEmpty);
+  if ((threadIdx.x & 31) == 0) {
+    mbar_arrive(bars + 8u * dq3::bSEmpty);
+    mbar_arrive(bars + 8u * dq3::bDpEmpty);
+  }
   return ok;
 }
 
 // =======================================================================================================
-// dq kernel: 256 query rows per CTA
+// dq kernel: 128 query rows per CTA, two CTAs per SM
 // =======================================================================================================
-// Two adjacent 128-row query tiles (a, b) share one stream of 64-key K/V sub-tiles, walked from the first key their rows
-// reach to tile b's diagonal.  Each tile has its own row-owning warpgroup (warps 0-3 / 4-7), MMA issuer (warps 9 / 10),
-// S/dP slots and dQ accumulator in TMEM and dz tile in shared memory.  Per sub-tile and tile: S = Q K^T and
-// dP = dO V^T (128 x 64), the row pass (which also records R1/S2 at the sub-tile's first key, i.e. at keys 0 and 64
-// of every 128-key tile), then dQ += dz K.
-// TMEM columns: S_a 0, dP_a 64, S_b 128, dP_b 192, dQ_a 256, dQ_b 384.
-// What bounds it: the row arithmetic (~2700 clk per sub-tile of both tiles in isolation, ~4200 here) and the MMAs'
-// shared-memory operand traffic (~80 clk per 128 x 64 x 16 instruction, ~3300 clk at 128 columns), so the two have to
-// overlap although S and dP fill all the tensor memory there is and cannot be double-buffered: rows start on S alone, dP
-// has until the middle of the first chunk, and both slots are handed back after two thirds of the pass (see strip_row_pass).
-namespace dq2 {
-constexpr int kThreads = 384;   // three warpgroups (one warp idles)
+// A block owns one 128-row query tile and walks the 64-key K/V sub-tiles from the first key its rows reach to its diagonal.
+// Per sub-tile: S = Q K^T and dP = dO V^T (128 x 64), the row pass (which also records R1/S2 at the sub-tile's first key,
+// i.e. at keys 0 and 64 of every 128-key tile), then dQ += dz K with dz read from tensor memory.
+//   warps 0-3  rows, one thread per query row;  warp 4  TMA;  warp 5  MMA issue;  warps 6, 7 fill their warpgroup up
+// Two blocks share an SM -- half of its tensor memory, of its registers and, to the byte, of its shared memory each --, so
+// that nothing ties the two tiles of an SM together: one's loads, first scores and epilogue run under the other's row passes.
+// What bounds it: the MMAs (an instruction of 64 keys takes as long as one of 128, ~64 clk: 2500 clk per step of both tiles)
+// and the row arithmetic (~2900), which overlap only in part, because S and dP fill what tensor memory dQ leaves and have a
+// single slot each.  A block of 256 rows, its two tiles sharing the K/V stream and dz in shared memory, took (us, then now)
+// 178 / 141 on 8 sequences of 2048 tokens x 16 heads N(0, 1), whose tiles visit two key tiles; 630 / 573 on 48 heads x 4096;
+// 377 / 338 at 64 columns; 165 / 128 on 131072 tokens without the stored tiles.  One tile per SM with 128 keys per step needs
+// half of the MMA time, but its lone row warp per scheduler makes less of the issue slots than two do: 145 / 622.
+// TMEM columns: S 0, dP 64, dQ 128.  At 128 columns dz lies over the first half of dP, which the next dP MMA therefore
+// overwrites behind this step's dQ; at 64 columns it has two tiles of its own (192, 224), so that the next S and dP both go
+// ahead of dQ (dP of step t + 2 is issued behind dQ of step t: who has seen the one may overwrite what the other read).
+namespace dq3 {
+constexpr int kThreads = 256;
 constexpr int kBN = 64;
 constexpr int kKvBox = kBN * 64 * 2;           // 64 keys x 64 columns
-constexpr int kZBytes = kBM * kBN * 2;         // dz tile: 128 rows x 64 keys
+constexpr uint32_t kCols = 256;
+constexpr uint32_t tcS = 0, tcP = 64, tcDQ = 128;
 template <int D>                               // head size rounded up to 64 or 128
 struct Cfg {
   static constexpr int kBoxes = D / 64;
   static constexpr int kTileBytes = kBoxes * kBoxBytes;   // Q or dO tile
   static constexpr int kKvTile = kBoxes * kKvBox;         // K or V sub-tile
-  static constexpr int kStageBytes = 2 * kKvTile;
-  static constexpr int kStages = D == 64 ? 4 : 2;         // what shared memory holds
-  static constexpr int kSmem = 1024 + 4 * kTileBytes + kStages * kStageBytes + 2 * kZBytes + 512 + (int)sizeof(SmallTable);
-  static_assert(kSmem <= 232448, "shared memory per block");
+  static constexpr int kKStages = D == 64 ? 3 : 2;        // K is read twice, by S and a pass later by dQ, V once
+  static constexpr int kVStages = D == 64 ? 2 : 1;
+  static constexpr bool kOwnDz = D == 64;                 // dz has columns of its own: the next dP need not wait for dQ
+  static constexpr uint32_t tcZ = kOwnDz ? 192 : tcP, kZToggle = kOwnDz ? 32 : 0;
+  static constexpr int kSmem = 2 * kTileBytes + (kKStages + kVStages) * kKvTile + 1024;
+  static_assert(2 * (kSmem + 1024) <= 233472, "two blocks per SM");
 };
 // What the rows need again after their loop, kept out of their registers meanwhile.
 struct Shared {
   Ctl ctl;
   int first;     // the sub-tile in stage 0
   int h, hh, len, idx;
-  long long tok0, boff, pair0;
+  long long tok0, boff;
 };
-static_assert(bNum * 8 + sizeof(Shared) <= 512, "barriers and control words");
-}  // namespace dq2
+static_assert(bNum * 8 + sizeof(Shared) <= 1024, "barriers and control words");
+}  // namespace dq3
 
 template <int D, bool kFp16, bool kStored>
-__global__ void __launch_bounds__(dq2::kThreads, 1)
-tc_bwd_dq2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
+__global__ void __launch_bounds__(dq3::kThreads, 2)
+tc_bwd_dq3_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                   const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_g,
-                  const __grid_constant__ CUtensorMap tm_dq, const __grid_constant__ CUtensorMap tm_az, const KParams p) {
-  using namespace dq2;
+                  const __grid_constant__ CUtensorMap tm_dq, const KParams p) {
+  using namespace dq3;
   using C = Cfg<D>;
-  constexpr int kTileBytes = C::kTileBytes, kKvTile = C::kKvTile, kStageBytes = C::kStageBytes, kStages = C::kStages, kBoxes = C::kBoxes;
-  extern __shared__ uint8_t smem_raw[];
+  constexpr int kTileBytes = C::kTileBytes, kKvTile = C::kKvTile, kKStages = C::kKStages, kVStages = C::kVStages, kBoxes = C::kBoxes;
+  extern __shared__ __align__(1024) uint8_t smem_tiles[];   // (no byte is left to align it here)
   if (threadIdx.x == 0) trace_block(p, 0);
-  const uint32_t raw = smem_u32(smem_raw);
-  const uint32_t base = (raw + 1023u) & ~1023u;
-  uint8_t *gbase = smem_raw + (base - raw);
-  const uint32_t sQ = base;                     // tile w: Q at sQ + w * 2 * kTileBytes, dO right behind it
-  const uint32_t sKV = sQ + 4 * kTileBytes;     // stage: K sub-tile then V sub-tile
-  const uint32_t sZ = sKV + kStages * kStageBytes;
-  const uint32_t sBar = sZ + 2 * kZBytes;
-  SmallTable &tb = *reinterpret_cast<SmallTable *>(gbase + (sBar - base) + 512);
+  const uint32_t sQ = smem_u32(smem_tiles);
+  const uint32_t sG = sQ + kTileBytes;
+  const uint32_t sK = sG + kTileBytes;
+  const uint32_t sV = sK + kKStages * kKvTile;
+  const uint32_t sBar = sV + kVStages * kKvTile;
+  // the item table lies where the second K sub-tile goes, which is not asked for before the block's barrier
+  static_assert(sizeof(SmallTable) <= kKvTile, "item table in a K stage");
+  SmallTable &tb = *reinterpret_cast<SmallTable *>(smem_tiles + 2 * kTileBytes + kKvTile);
   bool refused;
-  const long long covered = open_table(p, 2, tb, refused);
+  const long long covered = open_table(p, tb, refused);
   if (covered < p.tokens) fill_rows<typename std::conditional<kFp16, __half, __nv_bfloat16>::type>(p.dq, fill_job(p, covered, refused, blockIdx.x, gridDim.x));
   TileCoord c;
-  int hh_blk;
-  if (refused || !decode_block(p, tb, 2, true, c, hh_blk)) return;   // c.idx: the even tile of the pair (idx, idx + 1)
-  const int Ia = c.idx;
-  const bool b_active = Ia + 1 < c.n_tiles;
-  Shared *sh = reinterpret_cast<Shared *>(gbase + (sBar - base) + bNum * 8);
+  int hh;
+  if (refused || !decode_block(p, tb, true, c, hh)) return;
+  const int I = c.idx;
+  Shared *sh = reinterpret_cast<Shared *>(smem_tiles + (sBar - sQ) + bNum * 8);
   Ctl *ctl = &sh->ctl;
   volatile int *abort_flag = &ctl->abort;
   auto bar = [&](int i) { return sBar + 8u * i; };
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int hh = hh_blk, h = p.head0 + hh;
+  const int h = p.head0 + hh;
   const int n_sub = (c.len + kBN - 1) / kBN;
-  const int steps_a = min(2 * Ia + 2, n_sub);            // sub-tiles 0 .. 2 Ia + 1 reach tile a's diagonal
-  const int steps_b = b_active ? min(2 * Ia + 4, n_sub) : 0;
-  const int n_steps = b_active ? steps_b : steps_a;
-  const int issuers = b_active ? 2 : 1;
-  // the sub-tiles each tile starts at (even numbers: whole key tiles), and the block's: earlier keys have weight exactly 0
-  const int first_a = tile_first_key(p, c, p.head0 + hh_blk, Ia, kBM) / kBM * 2;
-  const int first_b = b_active ? tile_first_key(p, c, p.head0 + hh_blk, Ia + 1, kBM) / kBM * 2 : first_a;
-  const int first = min(first_a, first_b);
+  const int end = min(2 * I + 2, n_sub);       // sub-tiles 0 .. 2 I + 1 reach the tile's diagonal
+  // the sub-tile the tile starts at (an even number: whole key tiles): earlier keys have weight exactly 0
+  const int first = tile_first_key(p, c, h, I, kBM) / kBM * 2;
+  const int n_steps = end - first;
   int tr_cur = 0;   // cursor of this thread's event-log lane (diagnostics)
 
-  if (threadIdx.x == 0) {
-    mbar_init(bar(bQG), 1);
-    mbar_init(bar(bFirst), 1);
-    for (int s = 0; s < kStages; ++s) { mbar_init(bar(bKvFull + s), 1); mbar_init(bar(bKvEmpty + s), issuers); }
-    for (int w = 0; w < 2; ++w) {
-      mbar_init(bar(bSFull + w), 1);
-      mbar_init(bar(bDpFull + w), 1);
-      mbar_init(bar(bZFull + w), 4);
-      mbar_init(bar(bZEmpty + w), kStored ? 2 : 1);   // the dQ MMAs have read the dz tile, and it has left for the workspace
-      mbar_init(bar(bSpEmpty + w), 4);
-    }
-    mbar_init(bar(bDqFull), 1);
-    mbar_init(bar(bDqFull + 1), 1);
+  auto load_k = [&](int t) {
+    const int st = t % kKStages;
+    mbar_arrive_expect_tx(bar(bKFull + st), kKvTile);
+    for (int kb = 0; kb < kBoxes; ++kb)
+      tma_load_4d(sK + st * kKvTile + kb * kKvBox, &tm_k, bar(bKFull + st), kb * 64, (int)c.tok0 + (first + t) * kBN, h, (int)c.boff);
+  };
+  auto load_v = [&](int t) {
+    const int st = t % kVStages;
+    mbar_arrive_expect_tx(bar(bVFull + st), kKvTile);
+    for (int kb = 0; kb < kBoxes; ++kb)
+      tma_load_4d(sV + st * kKvTile + kb * kKvBox, &tm_v, bar(bVFull + st), kb * 64, (int)c.tok0 + (first + t) * kBN, h, (int)c.boff);
+  };
+  if (warp == 4 && lane == 0) {   // the first loads are on their way while the rest of the block gets ready
+    for (int i = 0; i < bNum; ++i) mbar_init(bar(i), i >= bSEmpty ? 4 : 1);
     ctl->abort = 0;
-    sh->first = first; sh->h = h; sh->hh = hh; sh->len = c.len; sh->idx = Ia;
-    sh->tok0 = c.tok0; sh->boff = c.boff; sh->pair0 = c.pair0;
+    sh->first = first; sh->h = h; sh->hh = hh; sh->len = c.len; sh->idx = I;
+    sh->tok0 = c.tok0; sh->boff = c.boff;
     fence_barrier_init();
+    const int qrow = (int)c.tok0 + I * kBM;
+    mbar_arrive_expect_tx(bar(bQ), kTileBytes);
+    for (int kb = 0; kb < kBoxes; ++kb) tma_load_4d(sQ + kb * kBoxBytes, &tm_q, bar(bQ), kb * 64, qrow, h, (int)c.boff);
+    load_k(0);
+    mbar_arrive_expect_tx(bar(bG), kTileBytes);
+    for (int kb = 0; kb < kBoxes; ++kb) tma_load_4d(sG + kb * kBoxBytes, &tm_g, bar(bG), kb * 64, qrow, h, (int)c.boff);
+    load_v(0);
   }
-  if (warp == 9) {
-    tmem_alloc(smem_u32(&ctl->tmem_base), kTmemCols);
+  if (warp == 5) {
+    tmem_alloc(smem_u32(&ctl->tmem_base), kCols);
     tmem_relinquish();
   }
+  fence_proxy_async_smem();   // the item table's bytes are TMA's from here on
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = ctl->tmem_base;
 
-  // The row warps take over registers the other warpgroup does not need (8 x 32 x 216 + 4 x 32 x 64 of the launch's
-  // 12 x 32 x 168): at 168 they spill.
-  if (warp >= 8) {
+  // The row warps take over registers the other warpgroup does not need (128 x 192 + 128 x 64 of the launch's 256 x 128).
+  if (warp >= 4) {
   reg_dec<64>();
-  if (warp == 8) {
+  if (warp == 4) {
     if (lane == 0) {
-      prefetch_tensormap(&tm_q); prefetch_tensormap(&tm_k); prefetch_tensormap(&tm_v); prefetch_tensormap(&tm_g);
-      const int qrow = (int)c.tok0 + Ia * kBM;
-      mbar_arrive_expect_tx(bar(bQG), 4 * kTileBytes);
-      for (int w = 0; w < 2; ++w)
-        for (int kb = 0; kb < kBoxes; ++kb) {
-          tma_load_4d(sQ + w * 2 * kTileBytes + kb * kBoxBytes, &tm_q, bar(bQG), kb * 64, qrow + w * kBM, h, (int)c.boff);
-          tma_load_4d(sQ + w * 2 * kTileBytes + kTileBytes + kb * kBoxBytes, &tm_g, bar(bQG), kb * 64, qrow + w * kBM, h, (int)c.boff);
-        }
-      for (int t = 0; t < n_steps - first; ++t) {
-        const int st = t % kStages;
-        if (t >= kStages && !wait_or_abort(bar(bKvEmpty + st), ((t / kStages) - 1) & 1, abort_flag, p, 510)) break;
+      for (int t = 1; t < n_steps; ++t) {
+        if (t >= kKStages && !wait_or_abort(bar(bKEmpty + t % kKStages), ((t / kKStages) - 1) & 1, abort_flag, p, 510)) break;
         if (*abort_flag) break;
-        const int krow = (int)c.tok0 + (first + t) * kBN;
-        const uint32_t dst = sKV + st * kStageBytes;
-        mbar_arrive_expect_tx(bar(bKvFull + st), kStageBytes);
-        for (int kb = 0; kb < kBoxes; ++kb) {
-          tma_load_4d(dst + kb * kKvBox, &tm_k, bar(bKvFull + st), kb * 64, krow, h, (int)c.boff);
-          tma_load_4d(dst + kKvTile + kb * kKvBox, &tm_v, bar(bKvFull + st), kb * 64, krow, h, (int)c.boff);
-        }
+        load_k(t);
+        if (t >= kVStages && !wait_or_abort(bar(bVEmpty + t % kVStages), ((t / kVStages) - 1) & 1, abort_flag, p, 511)) break;
+        if (*abort_flag) break;
+        load_v(t);
       }
     }
-  } else if (warp == 9 || warp == 10) {
-    // ------------------------------------------------ MMA issuers, one per tile
-    const int w = warp - 9;
-    if (lane == 0 && w < issuers) {
+  } else if (warp == 5) {
+    // ------------------------------------------------ MMA issuer
+    if (lane == 0) {
       constexpr uint32_t idesc_s = idesc_f16(kBM, kBN, kFp16, false, false);
       constexpr uint32_t idesc_dq = idesc_f16(kBM, D, kFp16, false, true);
-      const uint32_t qaddr = sQ + w * 2 * kTileBytes, gaddr = qaddr + kTileBytes, zaddr = sZ + w * kZBytes;
-      const uint32_t tS = tmem + w * 128, tP = tS + 64, tDQ = tmem + 256 + w * 128;
-      // this tile takes part in stages t_first .. t_end - 1 of the block's n_stages; u counts from its first one
-      const int n_stages = n_steps - first;
-      const int t_first = (w == 0 ? first_a : first_b) - first, t_end = (w == 0 ? steps_a : steps_b) - first;
-      const int my_steps = t_end - t_first;
-      const int z_row = (int)((c.pair0 + (long long)(Ia + w) * (Ia + w + 1) / 2) * kBM);   // of the stored dz tiles
-      auto issue_sp = [&](int u) {
-        const uint32_t kaddr = sKV + ((t_first + u) % kStages) * kStageBytes;
-        mma_kmajor_kmajor<D, kBoxBytes, kKvBox>(tS, qaddr, kaddr, idesc_s, false);            // S = Q K^T
-        mma_commit(bar(bSFull + w));
-        mma_kmajor_kmajor<D, kBoxBytes, kKvBox>(tP, gaddr, kaddr + kKvTile, idesc_s, false);  // dP = dO V^T
-        mma_commit(bar(bDpFull + w));
-      };
       bool ok = true;
-      // stages the tile does not read are released on its behalf once they have arrived
-      auto release = [&](int t, int t_stop) {
-        for (; ok && t < t_stop; ++t) {
-          ok = wait_or_abort(bar(bKvFull + t % kStages), (t / kStages) & 1, abort_flag, p, 524);
-          if (ok) mbar_arrive(bar(bKvEmpty + t % kStages));
-        }
+      auto issue_s = [&](int t) {   // S = Q K^T
+        const int st = t % kKStages;
+        ok = ok && wait_or_abort(bar(bKFull + st), (t / kKStages) & 1, abort_flag, p, 521);
+        if (!ok) return;
+        tc_fence_after();
+        mma_kmajor_kmajor<D, kBoxBytes, kKvBox>(tmem + tcS, sQ, sK + st * kKvTile, idesc_s, false);
+        mma_commit(bar(bSFull));
       };
-      release(0, t_first);
-      ok = ok && wait_or_abort(bar(bQG), 0, abort_flag, p, 520) &&
-           wait_or_abort(bar(bKvFull + t_first % kStages), (t_first / kStages) & 1, abort_flag, p, 521);
-      // if both tiles start at the same stage, tile b starts once tile a's first scores are done, so that one tile's MMAs fall into the other's row pass
-      // (bFirst completes exactly once: this waiter does not follow the phases of tile a's own barriers)
-      if (ok && w == 1 && first_a == first_b) ok = wait_or_abort(bar(bFirst), 0, abort_flag, p, 525);
-      if (ok) {
+      auto issue_dp = [&](int t) {   // dP = dO V^T
+        const int st = t % kVStages;
+        ok = ok && wait_or_abort(bar(bVFull + st), (t / kVStages) & 1, abort_flag, p, 523);
+        if (!ok) return;
         tc_fence_after();
-        issue_sp(0);
-        if (w == 0) mma_commit(bar(bFirst));
-      }
-      for (int u = 0; ok && u < my_steps; ++u) {
-        // the rows of step u have read their S/dP (they are still computing): the next scores go first ...
-        if (u + 1 < my_steps) {
-          ok = wait_or_abort(bar(bSpEmpty + w), u & 1, abort_flag, p, 526) &&
-               wait_or_abort(bar(bKvFull + (t_first + u + 1) % kStages), ((t_first + u + 1) / kStages) & 1, abort_flag, p, 523);
-          if (!ok) break;
-          trace_event(p, 1 + 3 * w, tr_cur, 2 + 16 * w, u + 1);
-          tc_fence_after();
-          issue_sp(u + 1);
-          trace_event(p, 1 + 3 * w, tr_cur, 3 + 16 * w, u + 1);
+        mma_kmajor_kmajor<D, kBoxBytes, kKvBox>(tmem + tcP, sG, sV + st * kKvTile, idesc_s, false);
+        mma_commit(bar(bDpFull));
+        mma_commit(bar(bVEmpty + st));
+      };
+      ok = wait_or_abort(bar(bQ), 0, abort_flag, p, 520);
+      issue_s(0);
+      ok = ok && wait_or_abort(bar(bG), 0, abort_flag, p, 524);
+      issue_dp(0);
+      for (int t = 0; ok && t < n_steps; ++t) {
+        // the rows of step t have read their S (they are still computing): the next scores go first ...
+        if (t + 1 < n_steps) {
+          ok = wait_or_abort(bar(bSEmpty), t & 1, abort_flag, p, 526);
+          trace_event(p, 1, tr_cur, 2, t + 1);
+          issue_s(t + 1);
+          if (C::kOwnDz) {
+            ok = ok && wait_or_abort(bar(bDpEmpty), t & 1, abort_flag, p, 527);
+            issue_dp(t + 1);
+          }
+          trace_event(p, 1, tr_cur, 3, t + 1);
         }
-        // ... then, once its dz tile is written, this step's dQ
-        ok = wait_or_abort(bar(bZFull + w), u & 1, abort_flag, p, 522);
+        // ... then, once its dz is written, this step's dQ += dz K (K sub-tile: 64 keys x (2 x 64) columns, MN-major)
+        ok = ok && wait_or_abort(bar(bZFull + (t & 1)), (t >> 1) & 1, abort_flag, p, 522);
         if (!ok) break;
-        trace_event(p, 1 + 3 * w, tr_cur, 6 + 16 * w, u);
+        trace_event(p, 1, tr_cur, 6, t);
         tc_fence_after();
-        // dQ += dz K: dz [128 x 64] K-major, K sub-tile [64 keys x (2 x 64) columns] MN-major
-        mma_kmajor_mnmajor<kBN, kKvBox>(tDQ, zaddr, sKV + ((t_first + u) % kStages) * kStageBytes, idesc_dq, u > 0);
-        mma_commit(bar(bZEmpty + w));
-        mma_commit(bar(bKvEmpty + (t_first + u) % kStages));
-        if constexpr (kStored) {
-          // The dz tile also leaves for the workspace.  (Issued by the row warps, 32 rows each, these stores held every one of
-          // them up for ~900 clk a step; this thread has nothing to do before two thirds of the next pass.)
-          const int ub = u + (w == 0 ? first_a : first_b);   // sub-tile inside the sequence
-          tma_store_4d(&tm_az, zaddr, (ub & 1) * kBN, z_row + (ub >> 1) * kBM, 1, hh);
-          tma_store_commit();
-          tma_store_wait_read();
-          mbar_arrive(bar(bZEmpty + w));
-        }
+        mma_tmem_mnmajor<kBN, kKvBox>(tmem + tcDQ, tmem + C::tcZ + (t & 1) * C::kZToggle, sK + (t % kKStages) * kKvTile, idesc_dq, t > 0);
+        mma_commit(bar(bKEmpty + t % kKStages));
+        // ... and, where dz lay over it, the next dP
+        if (!C::kOwnDz && t + 1 < n_steps) issue_dp(t + 1);
+        trace_event(p, 1, tr_cur, 7, t);
       }
-      if (ok) mma_commit(bar(bDqFull + w));   // this tile's dQ is complete: its rows store it while the other tile goes on
-      release(t_end, n_stages);   // tile a does not read the last sub-tiles
-      if constexpr (kStored) tma_store_wait_all();
+      if (ok) mma_commit(bar(bDqFull));
     }
   }
   } else {
-    reg_inc<216>();
-    // ------------------------------------------------ rows: warpgroup w owns query tile Ia + w
+    reg_inc<192>();
+    // ------------------------------------------------ rows: one thread per query row
     using T = typename std::conditional<kFp16, __half, __nv_bfloat16>::type;
-    const int w = warp >> 2;
-    const int r = threadIdx.x & 127;
-    const uint32_t lane_off = (uint32_t)((warp & 3) * 32) << 16;
+    const int r = threadIdx.x;
+    const uint32_t lane_off = (uint32_t)(warp * 32) << 16;
     const float scale2 = p.scale * kLog2e;
     const volatile Shared &item = *sh;
-    const int I = Ia + w, row0 = I * kBM;
-    const int my_steps = w == 0 ? steps_a : steps_b;
+    const int row0 = I * kBM;
     const bool valid = row0 + r < c.len;
     const long long idx = (c.boff * p.heads + h) * p.tokens + c.tok0 + row0 + r;
     // sum of log2(1 - beta) over the keys from the current sub-tile on, as an unevaluated pair (see LogSum in the forward)
     float r1 = 0.f, r1_lo = 0.f, dr = 0.f, gpre = 0.f;
-    if (valid && my_steps > 0) {
+    if (valid) {
       const double total = p.log_rem[idx];
       r1 = (float)total;
       r1_lo = (float)(total - (double)r1);
       dr = load_drem<T>(p, idx);
     }
-    uint8_t *gZ = gbase + (sZ - base) + w * kZBytes;
-    const uint32_t tS = tmem + w * 128 + lane_off, tP = tS + 64;
-    const uint32_t bars = sBar + 8u * w;
+    const uint32_t tS = tmem + tcS + lane_off, tP = tmem + tcP + lane_off, tZ = tmem + C::tcZ + lane_off;
     // this row's part of the workspace for sub-tile 0: A, or the boundary records [pair (I, J)][quarter of the key tile][row]
     const long long pair00 = (long long)(kStored ? 2 * hh : hh) * p.pairs_cap + c.pair0 + (long long)I * (I + 1) / 2;
     char *out = kStored ? reinterpret_cast<char *>(p.az + (pair00 * kBM + r) * kBM) : reinterpret_cast<char *>(p.bnd_r1 + pair00 * (4 * kBM) + r);
@@ -514,17 +467,18 @@ tc_bwd_dq2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
     // Where the forward has said where each warp's rows start, hardly a chunk of zeros is left, and the test for them costs
     // every chunk a tenth of its instructions.
     const bool skip = p.tile_start == nullptr && !p.dense;
-    const long long s2_off = kStored ? 0 : p.bnd_s2 - p.bnd_r1;
+    // stored tiles: elements from A to dz; records: floats from R1 to S2
+    const long long off = kStored ? p.pairs_cap * (kBM * kBM) : p.bnd_s2 - p.bnd_r1;
     bool ok = true;
     // One step: `pass` does the rows of sub-tile u, `dst` is its part of this row's workspace.  Zeros up to the warp's first
     // key, then full sub-tiles, then the diagonal: three loops, because what the kinds of step need would otherwise be kept in
     // registers for one another (see the forward's row loop).
     // u: 64-key sub-tile inside the sequence; the first one is even, so that phases follow from u alone
-    int u = w == 0 ? first_a : first_b;
+    int u = first;
     auto step = [&](auto pass, auto tail) {
-      ok = wait_or_abort(bars + 8u * bSFull, u & 1, abort_flag, p, 530);
+      ok = wait_or_abort(bar(bSFull), u & 1, abort_flag, p, 530);
       if (!ok) return;
-      if (r == 0) trace_event(p, 2 + w, tr_cur, 4 + 16 * w, u);
+      if (r == 0) trace_event(p, 2, tr_cur, 4, u);
       tc_fence_after();
       void *dst = kStored ? out + ((long long)(u >> 1) * (kBM * kBM) + (u & 1) * kBN) * 2 : out + (long long)u * (2 * kBM * sizeof(float));
       if (!pass(dst)) {   // a bounded wait inside the pass gave up
@@ -534,18 +488,21 @@ tc_bwd_dq2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
       }
       // the sequence ends inside this sub-tile: its dz columns behind the end are exact zeros, the K rows there are
       // not this sequence's (see zero_tile_rows) and are cleared before this step's dz K MMA is released
-      if (decltype(tail)::value && u == u_tail)
-        zero_tile_rows(gbase + (sKV - base) + ((u - item.first) % kStages) * kStageBytes, item.len - u * kBN, kBN, kBoxes, kKvBox, r, kBM);
-      tc_fence_before();          // this step's TMEM reads are done before the slots are handed back
-      fence_proxy_async_smem();
+      if (decltype(tail)::value && u == u_tail) {
+        zero_tile_rows(smem_tiles + (sK - sQ) + ((u - item.first) % kKStages) * kKvTile, item.len - u * kBN, kBN, kBoxes, kKvBox, r, kBM);
+        fence_proxy_async_smem();
+      }
+      tmem_wait_st();
+      tc_fence_before();          // this step's TMEM reads and its writes of dz are done before the slots are handed back
       __syncwarp();
-      if (r == 0) trace_event(p, 2 + w, tr_cur, 5 + 16 * w, u);
-      if (lane == 0) mbar_arrive(bars + 8u * bZFull);
+      if (r == 0) trace_event(p, 2, tr_cur, 5, u);
+      // (two barriers in turn: a warp whose dz is zeros may get to the next step's before another has got to this one's)
+      if (lane == 0) mbar_arrive(bar(bZFull + (u & 1)));
     };
     auto record = [&](void *dst, float r1f) {
       if constexpr (!kStored) {
         reinterpret_cast<float *>(dst)[0] = r1f;
-        reinterpret_cast<float *>(dst)[s2_off] = gpre;
+        reinterpret_cast<float *>(dst)[off] = gpre;
       }
     };
     auto carry = [&](float logsum, float gs) {   // r1 += logsum, gpre += gs
@@ -555,21 +512,21 @@ tc_bwd_dq2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
       gpre += gs;
     };
     using std::false_type; using std::true_type;
-    for (; u < min(u_warp, my_steps) && ok; ++u)
+    for (; u < min(u_warp, end) && ok; ++u)
       step([&](void *dst) {
         record(dst, kNothingLeft);
-        return zero_strip_row<kStored>(gZ, r, u, bars, dst, s2_off);
+        return zero_strip_row<kStored>(tZ + (u & 1) * C::kZToggle, u, sBar, dst, off);
       }, true_type());
     // rows past the sequence end must be zero in the stored tiles (the dK/dV GEMMs sum over all 128 query rows): the warp that
     // holds the end masks throughout
-    const int u_full = kStored && row0 + (r | 31) >= c.len ? 0 : min(u_diag, my_steps);
+    const int u_full = kStored && row0 + (r | 31) >= c.len ? 0 : min(u_diag, end);
     if (!skip) {
       for (; u < u_full && ok; ++u)
         step([&](void *dst) {
           const float r1f = r1 + r1_lo;
           float gs = 0.f, logsum = 0.f;
           record(dst, r1f);
-          const bool good = strip_row_pass<kFp16, false, kStored, false>(tS, tP, r, u, 0, 0, scale2, r1f, gpre, dr, gs, logsum, gZ, bars, dst, s2_off);
+          const bool good = strip_row_pass<kFp16, false, kStored, false>(tS, tP, tZ + (u & 1) * C::kZToggle, u, 0, 0, scale2, r1f, gpre, dr, gs, logsum, sBar, dst, off);
           carry(logsum, gs);
           return good;
         }, false_type());
@@ -579,58 +536,42 @@ tc_bwd_dq2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
           const float r1f = r1 + r1_lo;
           float gs = 0.f, logsum = 0.f;
           record(dst, r1f);
-          const bool good = strip_row_pass<kFp16, false, kStored, true>(tS, tP, r, u, 0, 0, scale2, r1f, gpre, dr, gs, logsum, gZ, bars, dst, s2_off);
+          const bool good = strip_row_pass<kFp16, false, kStored, true>(tS, tP, tZ + (u & 1) * C::kZToggle, u, 0, 0, scale2, r1f, gpre, dr, gs, logsum, sBar, dst, off);
           carry(logsum, gs);
           return good;
         }, false_type());
     }
-    for (; u < my_steps && ok; ++u)
+    for (; u < end && ok; ++u)
       step([&](void *dst) {
         const bool on_diag = u >= u_diag;
         const float r1f = r1 + r1_lo;
         float gs = 0.f, logsum = 0.f;
         record(dst, r1f);
-        const bool good = strip_row_pass<kFp16, true, kStored, false>(tS, tP, r, u, on_diag ? (u - u_diag) * kBN : 0,
+        const bool good = strip_row_pass<kFp16, true, kStored, false>(tS, tP, tZ + (u & 1) * C::kZToggle, u, on_diag ? (u - u_diag) * kBN : 0,
                                                                       chunk_limit(valid || !kStored, on_diag, r, p.attend_current), scale2, r1f,
-                                                                      gpre, dr, gs, logsum, gZ, bars, dst, s2_off);
+                                                                      gpre, dr, gs, logsum, sBar, dst, off);
         carry(logsum, gs);
         return good;
       }, true_type());
-    // the dz buffer is reused by the epilogue: its last tile has been read (in stored-tiles mode by the store as well)
-    if (ok && my_steps > 0) ok = wait_or_abort(bars + 8u * bZEmpty, (my_steps - 1) & 1, abort_flag, p, 533);
-    if (ok && my_steps > 0) ok = wait_or_abort(bar(bDqFull + w), 0, abort_flag, p, 532);
-    if (ok && my_steps > 0) {
+    if (ok) ok = wait_or_abort(bar(bDqFull), 0, abort_flag, p, 532);
+    if (ok) {
       tc_fence_after();
-      const uint32_t t_acc = tmem + 256 + w * 128 + lane_off;
+      const uint32_t t_acc = tmem + tcDQ + lane_off;
       const long long tok0 = item.tok0, boff = item.boff;
-      const int hd = item.h, tile_row0 = (item.idx + w) * kBM;
+      const int hd = item.h, tile_row0 = item.idx * kBM;
       if (tile_row0 + kBM <= item.len) {
-        // full tile: two 64-column halves through this tile's dz buffer (its last dQ MMA is done), one TMA store per
-        // warp and half -- full lines instead of 16 bytes per thread and row
-        const uint32_t src = sZ + w * kZBytes + (warp & 3) * 32 * 128;
-        const int trow = (int)tok0 + tile_row0 + (warp & 3) * 32;
-#pragma unroll 1
-        for (int half = 0; half < (D > 64 && p.head_dim > 64 ? 2 : 1); ++half) {   // columns past head_dim do not exist
-#pragma unroll 1
-          for (int ch = 0; ch < 2; ++ch) {
-            uint32_t v[32];
-            tmem_ld32(t_acc + half * 64 + ch * 32, v);
-            tmem_wait_ld();
-            float x[32];
-#pragma unroll
-            for (int i = 0; i < 32; ++i) x[i] = __uint_as_float(v[i]) * p.scale;
-            store_row_chunk<kFp16>(gZ, r, ch * 32, x);
-          }
-          fence_proxy_async_smem();
-          __syncwarp();
-          if (lane == 0) {
-            tma_store_4d(&tm_dq, src, half * 64, trow, hd, (int)boff);
-            tma_store_commit();
-            tma_store_wait_read();   // the buffer is rewritten by the next half
-          }
-          __syncwarp();
+        // full tile: through Q's memory (every MMA is done), one TMA store per warp and 64 columns -- full lines instead of
+        // 16 bytes per thread and row
+        stage_acc_rows<D, kFp16>(t_acc, smem_tiles, r, p.scale);
+        fence_proxy_async_smem();
+        __syncwarp();
+        if (lane == 0) {
+          const int trow = (int)tok0 + tile_row0 + warp * 32;
+          tma_store_4d(&tm_dq, sQ + warp * 32 * 128, 0, trow, hd, (int)boff);
+          if (D > 64 && p.head_dim > 64) tma_store_4d(&tm_dq, sQ + kBoxBytes + warp * 32 * 128, 64, trow, hd, (int)boff);
+          tma_store_commit();
+          tma_store_wait_all();
         }
-        if (lane == 0) tma_store_wait_all();
       } else {
         // the sequence ends inside the tile: row by row, rows past the end are left alone
         T *grow = reinterpret_cast<T *>(p.dq.ptr) + boff * p.dq.sb + (long long)hd * p.dq.sh + (tok0 + tile_row0 + r) * p.dq.st;
@@ -642,7 +583,7 @@ tc_bwd_dq2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
   tc_fence_before();
   __syncthreads();
   if (threadIdx.x == 0) trace_block(p, 2);
-  if (warp == 9) tmem_dealloc(tmem, kTmemCols);
+  if (warp == 5) tmem_dealloc(tmem, kCols);
 }
 
 // =======================================================================================================
@@ -680,7 +621,7 @@ tc_bwd_dkv4_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
   if (threadIdx.x == 0) trace_block(p, 0);
   SmallTable &tb = *reinterpret_cast<SmallTable *>(smem_raw);   // never used: the launch sees to that, there is no room for it
   bool refused;
-  const long long covered = open_table(p, 1, tb, refused);
+  const long long covered = open_table(p, tb, refused);
   if (covered < p.tokens) {
     using T = typename std::conditional<kFp16, __half, __nv_bfloat16>::type;
     fill_rows<T>(p.dk, fill_job(p, covered, refused, blockIdx.x, gridDim.x));
@@ -688,7 +629,7 @@ tc_bwd_dkv4_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
   }
   TileCoord c;
   int hh_blk;
-  if (refused || !decode_block(p, tb, 1, false, c, hh_blk)) return;
+  if (refused || !decode_block(p, tb, false, c, hh_blk)) return;
   const int J = c.idx;                         // the 128-key tile
   const int n_halves = J * kBM + kBN < c.len ? 2 : 1;   // the sequence may end inside the first strip
 
@@ -862,31 +803,28 @@ tc_bwd_dkv4_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
         tmem_ld16(tP + 16, d1);
         const int limit = chunk_limit(valid, diag, r, p.attend_current);
         {
-          BwdChunk k;
-          float pz[16];
-          if (masked) {
-            bwd_chunk_weights<true, false>(s0, quarter * 32, limit, scale2, r1f, gpre, logsum, k, [] {});
-            bwd_chunk_dz<true, false>(d0, quarter * 32, limit, gpre, dr, gs, k, pz);
-          } else {
-            bwd_chunk_weights<false, true>(s0, 0, limit, scale2, r1f, gpre, logsum, k, [] {}, !p.dense);
-            bwd_chunk_dz<false, true>(d0, 0, limit, gpre, dr, gs, k, pz);
-          }
+          float pa[16], pz[16];
+          if (masked) bwd_chunk<true, false>(s0, d0, quarter * 32, limit, scale2, r1f, gpre, dr, gs, logsum, pa, pz, false);
+          else bwd_chunk<false, true>(s0, d0, 0, limit, scale2, r1f, gpre, dr, gs, logsum, pa, pz, !p.dense);
           // the A/dz tiles are still being read by the previous step's MMAs
           if (g >= 1) {
             ok = wait_or_abort(bar(bAzEmpty), (g - 1) & 1, abort_flag, p, 631);
             tc_fence_after();
           }
-          store_row_chunk16<kFp16>(gA, r, w * 32, k.pa);
+          store_row_chunk16<kFp16>(gA, r, w * 32, pa);
           store_row_chunk16<kFp16>(gZ, r, w * 32, pz);
         }
         tmem_wait_ld_regs(s1, d1);
         tc_fence_before();          // this step's TMEM reads are done: the S/dP slot is handed back
         __syncwarp();
         if (lane == 0) mbar_arrive(bar(bSpEmpty + slot));
-        if (masked)
-          bwd_row_chunk<kFp16, true, false>(s1, d1, w * 32 + 16, quarter * 32 + 16, r, limit, scale2, r1f, gpre, dr, gs, logsum, gA, gZ);
-        else
-          bwd_row_chunk<kFp16, false, true>(s1, d1, w * 32 + 16, 0, r, limit, scale2, r1f, gpre, dr, gs, logsum, gA, gZ, !p.dense);
+        {
+          float pa[16], pz[16];
+          if (masked) bwd_chunk<true, false>(s1, d1, quarter * 32 + 16, limit, scale2, r1f, gpre, dr, gs, logsum, pa, pz, false);
+          else bwd_chunk<false, true>(s1, d1, 0, limit, scale2, r1f, gpre, dr, gs, logsum, pa, pz, !p.dense);
+          store_row_chunk16<kFp16>(gA, r, w * 32 + 16, pa);
+          store_row_chunk16<kFp16>(gZ, r, w * 32 + 16, pz);
+        }
       } else {
         if (g >= 1) {
           ok = wait_or_abort(bar(bAzEmpty), (g - 1) & 1, abort_flag, p, 631);
@@ -1018,7 +956,7 @@ tc_bwd_dkv5_kernel(const __grid_constant__ CUtensorMap tm_az, const __grid_const
   const uint32_t sBar = base + kStages * kStageBytes;
   SmallTable &tb = *reinterpret_cast<SmallTable *>(gbase + (sBar - base) + 512 + kListBits / 8);
   bool refused;
-  const long long covered = open_table(p, 1, tb, refused);
+  const long long covered = open_table(p, tb, refused);
   if (covered < p.tokens) {
     using T = typename std::conditional<kFp16, __half, __nv_bfloat16>::type;
     fill_rows<T>(p.dk, fill_job(p, covered, refused, blockIdx.x, gridDim.x));
@@ -1026,7 +964,7 @@ tc_bwd_dkv5_kernel(const __grid_constant__ CUtensorMap tm_az, const __grid_const
   }
   TileCoord c;
   int hh;
-  if (refused || !decode_block(p, tb, 1, false, c, hh)) return;
+  if (refused || !decode_block(p, tb, false, c, hh)) return;
   const int h = p.head0 + hh;
   const int J = c.idx;                        // the 128-key tile
   // The sequence may end inside the last query tile.  The A and dz rows behind the end are zeros in the workspace; the
@@ -1185,21 +1123,18 @@ static cudaError_t launch_bwd_t(const KParams &p, int dtype, cudaStream_t s) {
   if ((e = make_tile_map(&mk, p.k, p, dtype)) != cudaSuccess) return e;
   if ((e = make_tile_map(&mv, p.v, p, dtype)) != cudaSuccess) return e;
   if ((e = make_tile_map(&mg, p.d_o, p, dtype)) != cudaSuccess) return e;
-  const dim3 grid((unsigned)item_blocks(p, 1)), grid_pairs((unsigned)item_blocks(p, 2));
+  const dim3 grid((unsigned)item_blocks(p));
   if (!p.skip_dq) {
     const bool narrow = p.head_dim <= 64;
-    auto kernel = p.az != nullptr ? (narrow ? tc_bwd_dq2_kernel<64, kFp16, true> : tc_bwd_dq2_kernel<128, kFp16, true>)
-                                  : (narrow ? tc_bwd_dq2_kernel<64, kFp16, false> : tc_bwd_dq2_kernel<128, kFp16, false>);
-    const int smem = narrow ? dq2::Cfg<64>::kSmem : dq2::Cfg<128>::kSmem;
+    auto kernel = p.az != nullptr ? (narrow ? tc_bwd_dq3_kernel<64, kFp16, true> : tc_bwd_dq3_kernel<128, kFp16, true>)
+                                  : (narrow ? tc_bwd_dq3_kernel<64, kFp16, false> : tc_bwd_dq3_kernel<128, kFp16, false>);
+    const int smem = narrow ? dq3::Cfg<64>::kSmem : dq3::Cfg<128>::kSmem;
     if ((e = allow_dynamic_smem(reinterpret_cast<const void *>(kernel), smem)) != cudaSuccess) return e;
-    CUtensorMap mk64, mv64;   // 64-row boxes: the kernel streams 64-key sub-tiles
+    CUtensorMap mk64, mv64, mdq;   // 64-row boxes: the kernel streams 64-key sub-tiles; dQ leaves 32 rows per warp
     if ((e = make_tile_map(&mk64, p.k, p, dtype, 64)) != cudaSuccess) return e;
     if ((e = make_tile_map(&mv64, p.v, p, dtype, 64)) != cudaSuccess) return e;
-    CUtensorMap mdq, maz128;   // stores: dQ 32 rows per warp, dz one tile at a time
     if ((e = make_tile_map(&mdq, p.dq, p, dtype, 32)) != cudaSuccess) return e;
-    if (p.az != nullptr) { if ((e = make_az_map(&maz128, p, dtype, kBM)) != cudaSuccess) return e; }
-    else maz128 = mdq;         // not used
-    kernel<<<grid_pairs, dq2::kThreads, smem, s>>>(mq, mk64, mv64, mg, mdq, maz128, p);
+    kernel<<<grid, dq3::kThreads, smem, s>>>(mq, mk64, mv64, mg, mdq, p);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
   }
   if (!p.skip_dkv && p.az != nullptr) {

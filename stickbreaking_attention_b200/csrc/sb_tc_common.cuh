@@ -207,17 +207,8 @@ __device__ __forceinline__ void mma_kmajor_kmajor(uint32_t d_tmem, uint32_t a_ad
   for (int k = 0; k < KDIM / 16; ++k)
     mma_f16_ss(d_tmem, a0 + kstep_kmajor(k, A_BOX), b0 + kstep_kmajor(k, B_BOX), idesc, accumulate || k > 0);
 }
-// A: K-major [128 x KDIM];  B: rows = K (KDIM), columns = N in blocks of 64 that are B_BOX bytes apart, MN-major.
-template <int KDIM = kBM, int B_BOX = kBoxBytes>
-__device__ __forceinline__ void mma_kmajor_mnmajor(uint32_t d_tmem, uint32_t a_addr, uint32_t b_addr, uint32_t idesc,
-                                                   bool accumulate) {
-  const uint64_t a0 = smem_desc_sw128(a_addr, 16, 1024), b0 = smem_desc_sw128(b_addr, B_BOX, 1024);
-#pragma unroll
-  for (int ks = 0; ks < KDIM / 16; ++ks)
-    mma_f16_ss(d_tmem, a0 + kstep_kmajor(ks, kBoxBytes), b0 + (uint64_t)(ks * 128), idesc, accumulate || ks > 0);
-}
 // A: [128 x KDIM] 16-bit rows in tensor memory (KDIM / 2 columns starting at a_tmem, two K elements per column);
-// B as in mma_kmajor_mnmajor.
+// B: rows = K (KDIM), columns = N in blocks of 64 that are B_BOX bytes apart, MN-major.
 template <int KDIM, int B_BOX = kBoxBytes>
 __device__ __forceinline__ void mma_tmem_mnmajor(uint32_t d_tmem, uint32_t a_tmem, uint32_t b_addr, uint32_t idesc,
                                                  bool accumulate) {

@@ -65,7 +65,7 @@ __device__ __forceinline__ void fwd128_item(const KParams &p, const SmallTable &
   const long long lin = p.item_counter != nullptr ? (long long)atomicAdd(p.item_counter, 1u) : (long long)it * V + ((it & 1) ? V - 1 - v : v);
   const long long item = lin / p.head_cnt;
   w.n_steps = 0;
-  if (item > 0x7fffffffLL || !decode_item(p, tb, (int)item, 1, true, w.c)) return;
+  if (item > 0x7fffffffLL || !decode_item(p, tb, (int)item, true, w.c)) return;
   w.h = p.head0 + (int)(lin - item * p.head_cnt);
   const int n_sub = (w.c.len + fwd128::kBN - 1) / fwd128::kBN;
   w.row0 = w.c.idx * kBM;
@@ -87,7 +87,7 @@ tc_fwd128x2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
   const uint32_t sBar = base + 2 * kWorkerBytes;
   SmallTable &tb = *reinterpret_cast<SmallTable *>(gbase + (sBar - base) + kBarBytes);
   bool refused;
-  const long long covered = open_table(p, 1, tb, refused);
+  const long long covered = open_table(p, tb, refused);
   if (covered < p.tokens) fill_forward_rows<typename std::conditional<kFp16, __half, __nv_bfloat16>::type>(p, covered, refused, blockIdx.x, gridDim.x);
   if (refused) return;
   Shared *sh = reinterpret_cast<Shared *>(gbase + (sBar - base) + 2 * bPerWorker * 8);
@@ -376,7 +376,7 @@ static cudaError_t launch128_t(const KParams &p, int dtype, cudaStream_t s) {
   if ((e = make_tile_map(&mv, p.v, p, dtype, fwd128::kBN)) != cudaSuccess) return e;
   int sms = 0;
   if ((e = sm_count(&sms)) != cudaSuccess) return e;
-  const long long blocks = (item_blocks(p, 1) + 1) / 2;       // two workers per block
+  const long long blocks = (item_blocks(p) + 1) / 2;       // two workers per block
   const dim3 grid((unsigned)(blocks < sms ? blocks : sms));   // one resident block per SM
   auto kernel = tc_fwd128x2_kernel<kFp16, kStop>;
   if ((e = allow_dynamic_smem(reinterpret_cast<const void *>(kernel), fwd128::kSmem)) != cudaSuccess) return e;

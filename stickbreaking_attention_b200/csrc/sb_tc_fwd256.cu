@@ -65,7 +65,7 @@ __device__ __forceinline__ bool fwd256_item(const KParams &p, const SmallTable &
   const long long G = gridDim.x;
   const long long lin = (long long)it * G + ((it & 1) ? G - 1 - blockIdx.x : blockIdx.x);
   const long long item = lin / p.head_cnt;
-  if (item > 0x7fffffffLL || !decode_item(p, tb, (int)item, 1, true, w.c)) return false;
+  if (item > 0x7fffffffLL || !decode_item(p, tb, (int)item, true, w.c)) return false;
   w.h = p.head0 + (int)(lin - item * p.head_cnt);
   const int m = w.c.idx;
   const int n_sub = (w.c.len + fwd256::kBN - 1) / fwd256::kBN;   // 64-key sub-tiles of the sequence
@@ -103,7 +103,7 @@ tc_fwd256_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
   uint8_t *gP = gbase + (sP - base);
   SmallTable &tb = *reinterpret_cast<SmallTable *>(gbase + (sBar - base) + kBarBytes);
   bool refused;
-  const long long covered = open_table(p, 1, tb, refused);
+  const long long covered = open_table(p, tb, refused);
   if (covered < p.tokens) fill_forward_rows<typename std::conditional<kFp16, __half, __nv_bfloat16>::type>(p, covered, refused, blockIdx.x, gridDim.x);
   if (refused) return;
   Shared *sh = reinterpret_cast<Shared *>(gbase + (sBar - base) + bNum * 8);
@@ -448,7 +448,7 @@ static cudaError_t launch_t(const KParams &p, int dtype, cudaStream_t s) {
   if ((e = make_tile_map(&mv, p.v, p, dtype, fwd256::kBN)) != cudaSuccess) return e;
   int sms = 0;
   if ((e = sm_count(&sms)) != cudaSuccess) return e;
-  const long long blocks = item_blocks(p, 1);
+  const long long blocks = item_blocks(p);
   const dim3 grid((unsigned)(blocks < sms ? blocks : sms));   // one resident block per SM
   auto kernel = tc_fwd256_kernel<D, kFp16>;
   constexpr int smem = fwd256::Cfg<D>::kSmem;

@@ -768,3 +768,21 @@ def test_cuda_graph_replay_matches_eager(sb, cuda_device):
         for name, a, b in zip(("o", "rem", "dq", "dk", "dv"), outs, want):
             assert torch.equal(a, b), name
     sb.check_status(cuda_device)
+
+
+@pytest.mark.parametrize("mode", ["stored", "recompute"])
+@pytest.mark.parametrize("d,dtype", [(128, torch.bfloat16), (64, torch.float16), (72, torch.bfloat16)])
+def test_dq_tiles_that_share_an_sm(sb, cuda_device, d, dtype, mode):
+    """Query tiles that end in either half of a 64-key sub-tile or a 128-key tile, with one to eight steps, from the first key
+    or from a later one; enough heads that two of them share every SM several times over.  The first head is compared with the
+    oracle, the others, which hold copies of it, with the first."""
+    lengths = [1, 63, 64, 65, 127, 128, 129, 191, 193, 257, 450]
+    cu = cu_of(lengths)
+    one = H.make_inputs((1, sum(lengths), d), dtype, seed=d)   # N(0, 1): the later tiles of the longest start late
+    q, k, v, do, drem = (t.repeat(40, *[1] * (t.dim() - 1)) for t in one)
+    with sb.small_backward_workspace(mode == "recompute"):
+        got = H.run_varlen(sb, q, k, v, do, drem, cu, cuda_device, max_seqlens=max(lengths))
+    sb.check_status(cuda_device)
+    for t in got:
+        assert torch.equal(t, t[:1].expand_as(t))
+    H.assert_parity([t[:1] for t in got], H.oracle_varlen(*one, cu), dtype, f"d={d} {mode}")
