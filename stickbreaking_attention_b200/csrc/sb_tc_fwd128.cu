@@ -73,9 +73,11 @@ __device__ __forceinline__ void fwd128_item(const KParams &p, const SmallTable &
   w.n_steps = w.s_top + 1;
 }
 
-// kStop: tiles may stop early.  A tile of a sequence of up to 512 tokens has no four sub-tiles left by the time it could
-// (see may_stop_before), and the code for it costs short tiles 6 %: the launch leaves it out for such calls.
-template <bool kFp16, bool kStop>
+// kDrop: from the sub-tile on where a warp's weights are exactly 0 it only writes zeros for P, and log_rem ends there (the
+// caller keeps the tile starts); where all four warps are that far, P V is left out.  kStop: tiles may stop altogether.  A tile of a sequence of up to 512 tokens has no four
+// sub-tiles left by the time it could (see may_stop_before), and the code for it costs short tiles 6 %: the launch leaves it
+// out for such calls.
+template <bool kFp16, bool kStop, bool kDrop>
 __global__ void __launch_bounds__(fwd128::kThreads, 1)
 tc_fwd128x2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                    const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_o, const __grid_constant__ KParams p) {
@@ -220,7 +222,7 @@ tc_fwd128x2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
             if (ok && up == 0 && it >= 1) ok = wait_or_abort(bar(bOFree), (it - 1) & 1, abort_flag, p, 725);
             if (!ok) break;
             tc_fence_after();
-            through = through || (kStop && up >= 2 && all_through(stop, U, up));
+            through = through || (kDrop && up >= 2 && all_through(stop, U, up));
             if (!through)
               mma_tmem_mnmajor<kBN, kKvTileBytes>(tmem + 128, tmem + (gu & 1) * 64 + kPCol,
                                                   sKV + st * kStageBytes + kKvTileBytes, idesc_pv, up > 0);
@@ -284,7 +286,7 @@ tc_fwd128x2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
           if (kStop) break;
         } else if (s >= s_diag0) {
           fwd256_row_pass<kFp16, true>(ts, s * kBN, row, ac, scale2, run, logsum, ts + kPCol, true);
-        } else if (fwd256_row_pass<kFp16, false>(ts, 0, 0, ac, scale2, run, logsum, ts + kPCol, row < w.c.len, !p.dense, kStop)) {
+        } else if (fwd256_row_pass<kFp16, false>(ts, 0, 0, ac, scale2, run, logsum, ts + kPCol, row < w.c.len, !p.dense, kDrop)) {
           break;
         }
         run.add(logsum);
@@ -295,7 +297,7 @@ tc_fwd128x2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
       }
       // Through (the scores of step u are there, and count for nothing): zeros for P until the other warps of the tile are as
       // well.  The sequence's tail is behind these steps.
-      if (kStop && u < w.n_steps && ok) {
+      if (kDrop && u < w.n_steps && ok) {
         s_reached = w.s_top - u + 1;
         if (lane == 0) publish_through(stop, warp & 3, U + u);
         for (bool first = true; u < w.n_steps && ok; ++u, first = false) {
@@ -304,7 +306,7 @@ tc_fwd128x2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
           if (!first) {
             ok = wait_or_abort(bar(bSFull + buf), (gu >> 1) & 1, abort_flag, p, 731);
             if (!ok) break;
-            halt = stop.word[buf] == kStepStop;
+            halt = kStop && stop.word[buf] == kStepStop;
           }
           if (!halt) {
             tc_fence_after();
@@ -366,7 +368,7 @@ tc_fwd128x2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
   if (warp == 9) tmem_dealloc(ctl->tmem_base, kTmemCols);
 }
 
-template <bool kFp16, bool kStop>
+template <bool kFp16, bool kStop, bool kDrop>
 static cudaError_t launch128_t(const KParams &p, int dtype, cudaStream_t s) {
   CUtensorMap mq, mk, mv, mo;
   cudaError_t e;
@@ -378,16 +380,20 @@ static cudaError_t launch128_t(const KParams &p, int dtype, cudaStream_t s) {
   if ((e = sm_count(&sms)) != cudaSuccess) return e;
   const long long blocks = (item_blocks(p) + 1) / 2;       // two workers per block
   const dim3 grid((unsigned)(blocks < sms ? blocks : sms));   // one resident block per SM
-  auto kernel = tc_fwd128x2_kernel<kFp16, kStop>;
+  auto kernel = tc_fwd128x2_kernel<kFp16, kStop, kDrop>;
   if ((e = allow_dynamic_smem(reinterpret_cast<const void *>(kernel), fwd128::kSmem)) != cudaSuccess) return e;
   kernel<<<grid, fwd128::kThreads, fwd128::kSmem, s>>>(mq, mk, mv, mo, p);
   return cudaGetLastError();
 }
 
+template <bool kFp16>
+static cudaError_t launch128(const KParams &p, int dtype, cudaStream_t s) {
+  if (p.tile_start == nullptr || p.dense) return launch128_t<kFp16, false, false>(p, dtype, s);
+  return p.max_seqlen > 512 ? launch128_t<kFp16, true, true>(p, dtype, s) : launch128_t<kFp16, false, true>(p, dtype, s);
+}
+
 cudaError_t launch_tc_fwd128(const KParams &p, int dtype, cudaStream_t s) {
-  if (p.tile_start != nullptr && !p.dense && p.max_seqlen > 512)
-    return dtype == SB_DTYPE_F16 ? launch128_t<true, true>(p, dtype, s) : launch128_t<false, true>(p, dtype, s);
-  return dtype == SB_DTYPE_F16 ? launch128_t<true, false>(p, dtype, s) : launch128_t<false, false>(p, dtype, s);
+  return dtype == SB_DTYPE_F16 ? launch128<true>(p, dtype, s) : launch128<false>(p, dtype, s);
 }
 
 }  // namespace sb

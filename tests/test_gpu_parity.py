@@ -786,3 +786,16 @@ def test_dq_tiles_that_share_an_sm(sb, cuda_device, d, dtype, mode):
     for t in got:
         assert torch.equal(t, t[:1].expand_as(t))
     H.assert_parity([t[:1] for t in got], H.oracle_varlen(*one, cu), dtype, f"d={d} {mode}")
+
+
+@pytest.mark.parametrize("lengths", [[512, 300], [512] * 20 + [385, 129, 64]])   # an item table per block; one in memory
+def test_keys_without_weight_are_left_out_of_short_sequences_too(sb, cuda_device, lengths):
+    """Up to 512 tokens no tile stops altogether, but its rows form no log sums of keys whose weight is exactly 0."""
+    cu = cu_of(lengths)
+    inputs = H.make_inputs((16, sum(lengths), 64), torch.bfloat16, seed=5)
+    got = H.run_varlen(sb, *inputs, cu, cuda_device, max_seqlens=512)
+    with sb.dense_row_pass():
+        want = H.run_varlen(sb, *inputs, cu, cuda_device, max_seqlens=512)
+    for name, a, b in zip(("o", "rem", "dq", "dk", "dv"), got, want):
+        assert torch.equal(a, b), name
+    test_values_that_are_not_finite_reach_the_tiles_that_visit_them(sb, cuda_device, 64, torch.float16, lengths)
