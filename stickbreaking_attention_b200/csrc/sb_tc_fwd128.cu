@@ -284,6 +284,7 @@ tc_fwd128x2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
         // (the P rows of a warp that is not live keep whatever was there: they only reach accumulator rows that are never stored)
         if (!warp_live) {
           if (kStop) break;
+          if (kDrop && u == 0 && lane == 0) publish_through(stop, warp & 3, U);
         } else if (s >= s_diag0) {
           fwd256_row_pass<kFp16, true>(ts, s * kBN, row, ac, scale2, run, logsum, ts + kPCol, true);
         } else if (fwd256_row_pass<kFp16, false>(ts, 0, 0, ac, scale2, run, logsum, ts + kPCol, row < w.c.len, !p.dense, kDrop)) {
@@ -389,7 +390,9 @@ static cudaError_t launch128_t(const KParams &p, int dtype, cudaStream_t s) {
 template <bool kFp16>
 static cudaError_t launch128(const KParams &p, int dtype, cudaStream_t s) {
   if (p.tile_start == nullptr || p.dense) return launch128_t<kFp16, false, false>(p, dtype, s);
-  return p.max_seqlen > 512 ? launch128_t<kFp16, true, true>(p, dtype, s) : launch128_t<kFp16, false, true>(p, dtype, s);
+  if (p.max_seqlen > 512) return launch128_t<kFp16, true, true>(p, dtype, s);
+  // (up to 256 tokens: a tile has no sub-tile left by the time its rows could be through)
+  return p.max_seqlen > 256 ? launch128_t<kFp16, false, true>(p, dtype, s) : launch128_t<kFp16, false, false>(p, dtype, s);
 }
 
 cudaError_t launch_tc_fwd128(const KParams &p, int dtype, cudaStream_t s) {
