@@ -277,21 +277,23 @@ cudaError_t launch_fused_dv(const KParams &p, int dtype, cudaStream_t s) {
 // ------------------------------------------------------------------------------------------------
 // What bounds them: latency at three blocks per SM, next to no single unit (2 x 8 heads x 1024 x 64 fp32: shared-memory and L1
 // pipe 59 to 66 % busy, FMA pipe 43 to 47 %, issue slots 41 to 46 %), and the tail of 512 blocks of unequal length (a quarter
-// of the SMs' time).  The products' operands come from shared memory: a block is 128 threads; every product of a step
-// gives each thread a 4 x 4 patch of the result (4 x DP/16 for the accumulators), so that eight 16-byte shared loads feed
-// 64 FMAs.  A step is 32 query rows x 64 keys (forward, dQ) or 64 query rows x 32 keys (dK/dV): small enough for three or
-// four blocks per SM at head size 64, and for a few heads of a few hundred tokens to spread over the GPU.  The scans over
-// the keys of a row are shared by four (two) lanes with 16 keys each.  Next operands are requested while the other product
+// of the SMs' time).  The products' operands come from shared memory: a block is one or two groups of 128 threads; every
+// product of a step gives each thread a 4 x 4 patch of the result (4 x DP/16 for the accumulators), so that eight 16-byte
+// shared loads feed 64 FMAs.  Per group a step is 32 query rows x 64 keys (forward, dQ) or 64 query rows x 32 keys (dK/dV):
+// small enough for three or four blocks of one group per SM at head size 64, and for a few heads of a few hundred tokens to
+// spread over the GPU.  The groups' accumulators are added up at the end.  The scans over the keys of a row are shared by
+// four (eight; dK/dV: two) lanes with 16 keys each.  Next operands are requested while the other product
 // of the step runs: cp.async for fp32, registers for 16-bit tensors (which are widened on their way to shared memory).
 // Measured, forward + backward: 2 x 8 heads x 1024 tokens, head size 64, fp32: 419 us; one thread per row scanning
 // serially and one shared load per FMA before: 2290 us.
 constexpr int kT = kSimtTile;      // 32 rows or keys per tile
-constexpr int kStep = 2 * kT;      // keys (or query rows) per step
-constexpr int kSimtThreads = 128;
-constexpr int kLdS = kStep + 4;    // row stride of a score tile with 64 columns
-constexpr int kLdH = kT + 4;       // ... with 32 columns
-template <int DP> constexpr int kSimtBlocks = DP == 64 ? 3 : 1;   // blocks per SM the register allocation leaves room for
 template <int DP> constexpr int kLd = DP + 4;   // row stride of an operand tile: 16-byte rows, four banks apart
+constexpr int kLdH = kT + 4;       // row stride of a score tile with 32 columns
+// A block is G groups of 128 threads, and a step is 64 keys (or query rows) per group (see simt_run for which is taken).
+template <int G> constexpr int kThreads = 128 * G;
+template <int G> constexpr int kStep = 2 * kT * G;
+template <int G> constexpr int kLdS = kStep<G> + 4;            // row stride of a score tile with kStep columns
+template <int DP, int G> constexpr int kBlocks = DP == 64 ? (G == 1 ? 3 : 2) : 1;   // blocks per SM the register allocation leaves room for
 
 __device__ __forceinline__ void cp_async16(float *dst, const void *src, bool take) {
   const uint32_t d = static_cast<uint32_t>(__cvta_generic_to_shared(dst));
@@ -305,9 +307,9 @@ __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_al
 
 // A tile of ROWS rows of one tensor on its way into shared memory: issue() requests it, land() makes it visible to the
 // issuing thread's next barrier.  Rows outside [0, len) become zeros; columns past head_dim are zeroed once by clear().
-template <typename T, int DP, int ROWS>
+template <typename T, int DP, int ROWS, int G>
 struct TileLoad {
-  static constexpr int kWords = ROWS * DP / 2 / kSimtThreads;   // 16-bit tensors: two elements per register
+  static constexpr int kWords = ROWS * DP / 2 / kThreads<G>;   // 16-bit tensors: two elements per register
   uint32_t w[sizeof(T) == 4 ? 1 : kWords];
 
   __device__ __forceinline__ static const T *row_ptr(const TensorRef &t, const TileCoord &c, int h) {
@@ -318,14 +320,14 @@ struct TileLoad {
     if constexpr (sizeof(T) == 4) {
       if (wide) {   // rows of whole 16-byte chunks
 #pragma unroll 4
-        for (int e = threadIdx.x; e < ROWS * (DP / 4); e += kSimtThreads) {
+        for (int e = threadIdx.x; e < ROWS * (DP / 4); e += kThreads<G>) {
           const int r = e / (DP / 4), x = (e % (DP / 4)) * 4, row = row0 + r;
           const bool take = row >= 0 && row < c.len;
           if (x < d) cp_async16(dst + r * kLd<DP> + x, base + (take ? row * t.st + x : 0), take);
         }
       } else {
 #pragma unroll 4
-        for (int e = threadIdx.x; e < ROWS * DP; e += kSimtThreads) {
+        for (int e = threadIdx.x; e < ROWS * DP; e += kThreads<G>) {
           const int r = e / DP, x = e % DP, row = row0 + r;
           const bool take = row >= 0 && row < c.len;
           if (x < d) cp_async4(dst + r * kLd<DP> + x, base + (take ? row * t.st + x : 0), take);
@@ -335,7 +337,7 @@ struct TileLoad {
       const unsigned short *b16 = reinterpret_cast<const unsigned short *>(base);
 #pragma unroll
       for (int i = 0; i < kWords; ++i) {
-        const int e = threadIdx.x + i * kSimtThreads;
+        const int e = threadIdx.x + i * kThreads<G>;
         const int r = e / (DP / 2), x = (e % (DP / 2)) * 2, row = row0 + r;
         w[i] = 0u;
         if (row >= 0 && row < c.len && x < d) {
@@ -352,7 +354,7 @@ struct TileLoad {
     } else {
 #pragma unroll
       for (int i = 0; i < kWords; ++i) {
-        const int e = threadIdx.x + i * kSimtThreads;
+        const int e = threadIdx.x + i * kThreads<G>;
         const int r = e / (DP / 2), x = (e % (DP / 2)) * 2;
         const unsigned short lo = (unsigned short)(w[i] & 0xffffu), hi = (unsigned short)(w[i] >> 16);
         *reinterpret_cast<float2 *>(dst + r * kLd<DP> + x) =
@@ -361,13 +363,13 @@ struct TileLoad {
     }
   }
 };
-template <int DP, int ROWS>
+template <int DP, int ROWS, int G>
 __device__ __forceinline__ void clear_tile(float *dst, int d) {   // columns past head_dim stay zero from here on
   if (d == DP) return;
-  for (int e = threadIdx.x; e < ROWS * DP; e += kSimtThreads) dst[(e / DP) * kLd<DP> + e % DP] = 0.f;
+  for (int e = threadIdx.x; e < ROWS * DP; e += kThreads<G>) dst[(e / DP) * kLd<DP> + e % DP] = 0.f;
 }
 
-// S[m][n] = mul * <A_m, B_n>, M x N with M N = 2048: thread (ty, tx) owns rows ty + i * (M / 4), columns tx + j * (N / 4).
+// S[m][n] = mul * <A_m, B_n>, M x N with 16 results per thread: thread (ty, tx) owns rows ty + i * (M / 4), columns tx + j * (N / 4).
 template <int DP, int M, int N>
 __device__ __forceinline__ void tile_dot(float *S, const float *A, const float *B, float mul) {
   constexpr int kTx = N / 4, kTy = M / 4, kLdO = N + 4;
@@ -402,16 +404,16 @@ __device__ __forceinline__ void add_scaled(float *acc, float s, const float4 &b)
   acc[0] = lo.x; acc[1] = lo.y; acc[2] = hi.x; acc[3] = hi.y;
 }
 
-// acc (32 rows x DP, thread: rows 4 ty .. + 3, columns 4 tx + 64 u ..) += P (32 x 64) B (64 x DP)
-template <int DP>
+// acc (32 rows x DP, thread: rows 4 ty .. + 3, columns 4 tx + 64 u ..) += P (32 x 64 G) B (64 G x DP), 64 keys per group
+template <int DP, int G>
 __device__ __forceinline__ void tile_pv(float (&acc)[4][DP / 16], const float *P, const float *B) {
-  const int tx = threadIdx.x % 16, ty = threadIdx.x / 16;
-  const float *pp = P + 4 * ty * kLdS, *b = B + 4 * tx;
+  const int tx = threadIdx.x % 16, ty = threadIdx.x / 16 % 8, first = threadIdx.x / 128 * 64;
+  const float *pp = P + 4 * ty * kLdS<G> + first, *b = B + first * kLd<DP> + 4 * tx;
 #pragma unroll 2
-  for (int k = 0; k < kStep; k += 4) {
+  for (int k = 0; k < 64; k += 4) {
     float4 pv[4];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) pv[i] = *reinterpret_cast<const float4 *>(pp + i * kLdS + k);
+    for (int i = 0; i < 4; ++i) pv[i] = *reinterpret_cast<const float4 *>(pp + i * kLdS<G> + k);
 #pragma unroll
     for (int kk = 0; kk < 4; ++kk) {
 #pragma unroll
@@ -426,13 +428,13 @@ __device__ __forceinline__ void tile_pv(float (&acc)[4][DP / 16], const float *P
     }
   }
 }
-// acc (32 keys x DP) += P^T B with P (64 query rows x 32 keys), B (64 x DP)
+// acc (32 keys x DP) += P^T B with P (64 G query rows x 32 keys), B (64 G x DP), 64 rows per group
 template <int DP>
 __device__ __forceinline__ void tile_ptb(float (&acc)[4][DP / 16], const float *P, const float *B) {
-  const int tx = threadIdx.x % 16, ty = threadIdx.x / 16;
-  const float *pp = P + 4 * ty, *b = B + 4 * tx;
+  const int tx = threadIdx.x % 16, ty = threadIdx.x / 16 % 8, first = threadIdx.x / 128 * 64;
+  const float *pp = P + first * kLdH + 4 * ty, *b = B + first * kLd<DP> + 4 * tx;
 #pragma unroll 4
-  for (int k = 0; k < kStep; ++k) {
+  for (int k = 0; k < 64; ++k) {
     const float4 pv = *reinterpret_cast<const float4 *>(pp + k * kLdH);
 #pragma unroll
     for (int u = 0; u < DP / 64; ++u) {
@@ -442,6 +444,26 @@ __device__ __forceinline__ void tile_ptb(float (&acc)[4][DP / 16], const float *
         const float s = i == 0 ? pv.x : i == 1 ? pv.y : i == 2 ? pv.z : pv.w;
         add_scaled(&acc[i][4 * u], s, bv);
       }
+    }
+  }
+}
+// The groups' parts of an accumulator, summed into the first group's; `scratch`: 32 x DP floats that are free.
+template <int DP, int G>
+__device__ __forceinline__ void sum_groups(float (&acc)[4][DP / 16], float *scratch) {
+  if constexpr (G == 2) {
+    const int t = threadIdx.x & 127;
+    if (threadIdx.x >= 128) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int x = 0; x < DP / 16; ++x) scratch[(i * (DP / 16) + x) * 128 + t] = acc[i][x];
+    }
+    __syncthreads();
+    if (threadIdx.x < 128) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int x = 0; x < DP / 16; ++x) acc[i][x] += scratch[(i * (DP / 16) + x) * 128 + t];
     }
   }
 }
@@ -484,8 +506,8 @@ __device__ __forceinline__ void store16(float *dst, const float (&x)[16]) {
 // Forward: one block per (sequence, 32-row query tile, head), keys walked from the diagonal back to the sequence start in
 // steps of 64; every row carries sum softplus(z) over the keys already visited, in fp64 (reference: _forward_one_row,
 // sb_varlen_fwd.py:81-215).
-template <typename T, int DP>
-__global__ void __launch_bounds__(kSimtThreads, kSimtBlocks<DP>) simt_fwd_kernel(const __grid_constant__ KParams p, bool wide) {
+template <typename T, int DP, int G>
+__global__ void __launch_bounds__(kThreads<G>, kBlocks<DP, G>) simt_fwd_kernel(const __grid_constant__ KParams p, bool wide) {
   extern __shared__ float4 smem4[];
   __shared__ SmallTable tb;
   bool refused;
@@ -495,18 +517,19 @@ __global__ void __launch_bounds__(kSimtThreads, kSimtBlocks<DP>) simt_fwd_kernel
   TileCoord c;
   if (refused || !decode_item(p, tb, blockIdx.x, true, c)) return;
   const int d = p.head_dim, h = p.head0 + blockIdx.y, t = threadIdx.x;
-  float *Qs = reinterpret_cast<float *>(smem4), *Ks = Qs + kT * kLd<DP>, *Vs = Ks + kStep * kLd<DP>, *Ss = Vs + kStep * kLd<DP>;
+  float *Qs = reinterpret_cast<float *>(smem4), *Ks = Qs + kT * kLd<DP>, *Vs = Ks + kStep<G> * kLd<DP>, *Ss = Vs + kStep<G> * kLd<DP>;
   const int row0 = c.idx * kT, ac = p.attend_current;
-  const int r = t >> 2, seg = t & 3, gi = row0 + r;   // the row this thread scans, and which 16 of the step's keys
+  constexpr int kLanes = 4 * G;
+  const int r = t / kLanes, seg = t % kLanes, gi = row0 + r;   // the row this thread scans, and which 16 of the step's keys
   const int limit = gi < c.len ? gi + ac : 0;
 
-  clear_tile<DP, kT>(Qs, d);
-  clear_tile<DP, kStep>(Ks, d);
-  clear_tile<DP, kStep>(Vs, d);
+  clear_tile<DP, kT, G>(Qs, d);
+  clear_tile<DP, kStep<G>, G>(Ks, d);
+  clear_tile<DP, kStep<G>, G>(Vs, d);
   if (d != DP) __syncthreads();
-  TileLoad<T, DP, kT> lq;
-  TileLoad<T, DP, kStep> lk, lv;
-  int key0 = row0 - kT;                     // first key of the step (negative: keys before the sequence, masked)
+  TileLoad<T, DP, kT, G> lq;
+  TileLoad<T, DP, kStep<G>, G> lk, lv;
+  int key0 = row0 + kT - kStep<G>;          // first key of the step (negative: keys before the sequence, masked)
   lq.issue(Qs, p.q, c, h, row0, d, wide);
   lk.issue(Ks, p.k, c, h, key0, d, wide);
   lq.land(Qs);
@@ -516,36 +539,39 @@ __global__ void __launch_bounds__(kSimtThreads, kSimtBlocks<DP>) simt_fwd_kernel
   double run = 0.0;                         // sum of softplus(z) over the keys of the earlier steps
   const bool may_stop = p.tile_start != nullptr && !p.dense;
   int reached = 0;                          // first key visited
-  for (; key0 > -kStep; key0 -= kStep) {
+  for (; key0 > -kStep<G>; key0 -= kStep<G>) {
     lv.issue(Vs, p.v, c, h, key0, d, wide);
-    tile_dot<DP, kT, kStep>(Ss, Qs, Ks, p.scale);
+    tile_dot<DP, kT, kStep<G>>(Ss, Qs, Ks, p.scale);
     lv.land(Vs);
     __syncthreads();
     bool more = key0 > 0;
-    if (more) lk.issue(Ks, p.k, c, h, key0 - kStep, d, wide);
+    if (more) lk.issue(Ks, p.k, c, h, key0 - kStep<G>, d, wide);
     {
       float z[16], beta[16], keep[16];
-      float *srow = Ss + r * kLdS + seg * 16;
+      float *srow = Ss + r * kLdS<G> + seg * 16;
       load16(z, srow);
       const float sp = stick_segment(z, key0 + seg * 16, limit, beta, keep);
       float prod = 1.f;
 #pragma unroll
       for (int j = 0; j < 16; ++j) prod *= keep[j];
       // product over the lanes with later keys, then down the lane's own keys
-      const float p1 = __shfl_down_sync(0xffffffffu, prod, 1, 4), p2 = __shfl_down_sync(0xffffffffu, prod, 2, 4),
-                  p3 = __shfl_down_sync(0xffffffffu, prod, 3, 4);
+#pragma unroll
+      for (int o = 1; o < kLanes; o <<= 1) {
+        const float later = __shfl_down_sync(0xffffffffu, prod, o, kLanes);
+        if (seg + o < kLanes) prod *= later;
+      }
+      const float after = __shfl_down_sync(0xffffffffu, prod, 1, kLanes);
       float R = expf(-(float)run);
-      if (seg < 3) R *= p1;
-      if (seg < 2) R *= p2;
-      if (seg < 1) R *= p3;
+      if (seg + 1 < kLanes) R *= after;
 #pragma unroll
       for (int j = 15; j >= 0; --j) {
         z[j] = beta[j] * R;
         R *= keep[j];
       }
       store16(srow, z);
-      float sum = sp + __shfl_xor_sync(0xffffffffu, sp, 1);
-      sum += __shfl_xor_sync(0xffffffffu, sum, 2);
+      float sum = sp;
+#pragma unroll
+      for (int o = 1; o < kLanes; o <<= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
       run += (double)sum;
     }
     if (may_stop) {   // once every row's product has underflowed to 0, no earlier key has any weight
@@ -557,19 +583,20 @@ __global__ void __launch_bounds__(kSimtThreads, kSimtBlocks<DP>) simt_fwd_kernel
       __syncthreads();
     }
     if (p.attn != nullptr) {   // debugging aid: the attention weights of this step, keys indexed inside the sequence
-      for (int e = t; e < kT * kStep; e += kSimtThreads) {
-        const int ri = row0 + e / kStep, gj = key0 + e % kStep;
+      for (int e = t; e < kT * kStep<G>; e += kThreads<G>) {
+        const int ri = row0 + e / kStep<G>, gj = key0 + e % kStep<G>;
         if (ri < c.len && gj >= 0 && gj < c.len && gj < p.attn_cols)
-          p.attn[((c.boff * p.heads + h) * p.tokens + c.tok0 + ri) * p.attn_cols + gj] = Ss[(e / kStep) * kLdS + e % kStep];
+          p.attn[((c.boff * p.heads + h) * p.tokens + c.tok0 + ri) * p.attn_cols + gj] = Ss[(e / kStep<G>) * kLdS<G> + e % kStep<G>];
       }
     }
-    tile_pv<DP>(acc, Ss, Vs);
+    tile_pv<DP, G>(acc, Ss, Vs);
     if (!more) break;
     lk.land(Ks);
     __syncthreads();
   }
   if constexpr (sizeof(T) == 4) cp_async_wait();   // keys requested before the stop was known
   __syncthreads();
+  sum_groups<DP, G>(acc, Ss);
   if (p.tile_start != nullptr && t == 0 && row0 >= 64) *tile_start_entry(p, c, h, row0) = reached;
 
   const float rem = expf(-(float)run);
@@ -579,9 +606,11 @@ __global__ void __launch_bounds__(kSimtThreads, kSimtBlocks<DP>) simt_fwd_kernel
     p.log_rem[idx] = -run * kLog2eD;
   }
   if (p.fuse_rem_v) {   // out = o + rem * v: the row owners publish rem through the free score tile
+    if (G > 1) __syncthreads();
     if (seg == 0) Ss[r] = rem;
     __syncthreads();
   }
+  if (t >= 128) return;
   const int tx = t % 16, ty = t / 16;
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
@@ -649,8 +678,8 @@ __device__ __forceinline__ void bwd_segment(float (&z)[16], float (&dp)[16], int
 // dQ: query-stationary, keys from the sequence start to the diagonal (reference: _backward_one_row,
 // sb_varlen_bwd.py:297-481, which adds dK/dV under a spin lock instead).  Leaves A and dz of every (query tile, key tile)
 // pair in the workspace (p.az), or, where those would not fit the scratch budget, the carried R1 and S2 per pair and row.
-template <typename T, int DP>
-__global__ void __launch_bounds__(kSimtThreads, kSimtBlocks<DP>) simt_bwd_dq_kernel(const __grid_constant__ KParams p, bool wide) {
+template <typename T, int DP, int G>
+__global__ void __launch_bounds__(kThreads<G>, kBlocks<DP, G>) simt_bwd_dq_kernel(const __grid_constant__ KParams p, bool wide) {
   extern __shared__ float4 smem4[];
   __shared__ SmallTable tb;
   bool refused;
@@ -660,19 +689,21 @@ __global__ void __launch_bounds__(kSimtThreads, kSimtBlocks<DP>) simt_bwd_dq_ker
   TileCoord c;
   if (refused || !decode_item(p, tb, blockIdx.x, true, c)) return;
   const int d = p.head_dim, hh = blockIdx.y, h = p.head0 + hh, t = threadIdx.x;
-  float *Qs = reinterpret_cast<float *>(smem4), *Gs = Qs + kT * kLd<DP>, *Ks = Gs + kT * kLd<DP>, *Vs = Ks + kStep * kLd<DP>;
-  float *Zs = Vs + kStep * kLd<DP>, *Ps = Zs + kT * kLdS;
+  float *Qs = reinterpret_cast<float *>(smem4), *Gs = Qs + kT * kLd<DP>, *Ks = Gs + kT * kLd<DP>, *Vs = Ks + kStep<G> * kLd<DP>;
+  // the scores, later dz, and dP; with two groups dP follows the scores into the one tile, so that two blocks fit an SM
+  float *Zs = Vs + kStep<G> * kLd<DP>, *Ps = G == 1 ? Zs + kT * kLdS<G> : Zs;
   const int I = c.idx, row0 = I * kT;
-  const int r = t >> 2, seg = t & 3, gi = row0 + r;
+  constexpr int kLanes = 4 * G;
+  const int r = t / kLanes, seg = t % kLanes, gi = row0 + r;
   const int limit = gi < c.len ? gi + p.attend_current : 0;
 
-  clear_tile<DP, kT>(Qs, d);
-  clear_tile<DP, kT>(Gs, d);
-  clear_tile<DP, kStep>(Ks, d);
-  clear_tile<DP, kStep>(Vs, d);
+  clear_tile<DP, kT, G>(Qs, d);
+  clear_tile<DP, kT, G>(Gs, d);
+  clear_tile<DP, kStep<G>, G>(Ks, d);
+  clear_tile<DP, kStep<G>, G>(Vs, d);
   if (d != DP) __syncthreads();
-  TileLoad<T, DP, kT> lq, lg;
-  TileLoad<T, DP, kStep> lk, lv;
+  TileLoad<T, DP, kT, G> lq, lg;
+  TileLoad<T, DP, kStep<G>, G> lk, lv;
   lq.issue(Qs, p.q, c, h, row0, d, wide);
   lg.issue(Gs, p.d_o, c, h, row0, d, wide);
   const int key_first = first_key(p, c, h, row0);
@@ -690,24 +721,28 @@ __global__ void __launch_bounds__(kSimtThreads, kSimtBlocks<DP>) simt_bwd_dq_ker
   __syncthreads();
   float acc[4][DP / 16] = {};
   const long long pair0 = (long long)hh * p.pairs_cap + c.pair0 + (long long)I * (I + 1) / 2;
-  for (int key0 = key_first; key0 <= row0; key0 += kStep) {
+  for (int key0 = key_first; key0 <= row0; key0 += kStep<G>) {
     lv.issue(Vs, p.v, c, h, key0, d, wide);
-    tile_dot<DP, kT, kStep>(Zs, Qs, Ks, p.scale);
+    tile_dot<DP, kT, kStep<G>>(Zs, Qs, Ks, p.scale);
     lv.land(Vs);
     __syncthreads();
-    tile_dot<DP, kT, kStep>(Ps, Gs, Vs, 1.f);
+    float z[16], dp[16];
+    float *zrow = Zs + r * kLdS<G> + seg * 16;
+    if (G > 1) {
+      load16(z, zrow);
+      __syncthreads();
+    }
+    tile_dot<DP, kT, kStep<G>>(Ps, Gs, Vs, 1.f);
     __syncthreads();
     // V is done with: the next K goes into its buffer while this step goes on, and the next V into this K's
-    const bool more = key0 + kStep <= row0;
-    if (more) lk.issue(Vs, p.k, c, h, key0 + kStep, d, wide);
+    const bool more = key0 + kStep<G> <= row0;
+    if (more) lk.issue(Vs, p.k, c, h, key0 + kStep<G>, d, wide);
     {
-      float z[16], dp[16];
-      float *zrow = Zs + r * kLdS + seg * 16;
-      load16(z, zrow);
-      load16(dp, Ps + r * kLdS + seg * 16);
+      if (G == 1) load16(z, zrow);
+      load16(dp, Ps + r * kLdS<G> + seg * 16);
       double r1_seg, sp;
       float g_seg, gs;
-      bwd_segment<4>(z, dp, key0 + seg * 16, limit, r1, gpre, dr, r1_seg, g_seg, sp, gs);
+      bwd_segment<kLanes>(z, dp, key0 + seg * 16, limit, r1, gpre, dr, r1_seg, g_seg, sp, gs);
       store16(zrow, z);
       const int J = key0 / kT + (seg >> 1);
       if (J <= I) {
@@ -724,13 +759,15 @@ __global__ void __launch_bounds__(kSimtThreads, kSimtBlocks<DP>) simt_bwd_dq_ker
       gpre += gs;
     }
     __syncthreads();
-    tile_pv<DP>(acc, Zs, Ks);
+    tile_pv<DP, G>(acc, Zs, Ks);
     if (more) lk.land(Vs);
     __syncthreads();
     float *tmp = Ks;
     Ks = Vs;
     Vs = tmp;
   }
+  sum_groups<DP, G>(acc, Zs);
+  if (t >= 128) return;
 
   const int tx = t % 16, ty = t / 16;
 #pragma unroll
@@ -750,8 +787,8 @@ __global__ void __launch_bounds__(kSimtThreads, kSimtBlocks<DP>) simt_bwd_dq_ker
 
 // dK, dV: key-stationary, one block per 32-key tile, query tiles diagonal -> end two at a time; accumulators in registers,
 // fixed summation order, no atomics.  kStored: A and dz come from the workspace; otherwise they are computed again.
-template <typename T, int DP, bool kStored>
-__global__ void __launch_bounds__(kSimtThreads, kSimtBlocks<DP>) simt_bwd_dkv_kernel(const __grid_constant__ KParams p, bool wide) {
+template <typename T, int DP, int G, bool kStored>
+__global__ void __launch_bounds__(kThreads<G>, kBlocks<DP, G>) simt_bwd_dkv_kernel(const __grid_constant__ KParams p, bool wide) {
   extern __shared__ float4 smem4[];
   __shared__ SmallTable tb;
   bool refused;
@@ -764,21 +801,22 @@ __global__ void __launch_bounds__(kSimtThreads, kSimtBlocks<DP>) simt_bwd_dkv_ke
   TileCoord c;
   if (refused || !decode_item(p, tb, blockIdx.x, false, c)) return;
   const int d = p.head_dim, hh = blockIdx.y, h = p.head0 + hh, t = threadIdx.x;
-  float *Qs = reinterpret_cast<float *>(smem4), *Gs = Qs + kStep * kLd<DP>, *Zs = Gs + kStep * kLd<DP>, *Ps = Zs + kStep * kLdH;
-  float *Ks = Ps + kStep * kLdH, *Vs = Ks + kT * kLd<DP>;   // recomputation only
+  float *Qs = reinterpret_cast<float *>(smem4), *Gs = Qs + kStep<G> * kLd<DP>, *Zs = Gs + kStep<G> * kLd<DP>, *Ps = Zs + kStep<G> * kLdH;
+  float *Ks = Ps + kStep<G> * kLdH, *Vs = Ks + kT * kLd<DP>;   // recomputation only
   const int J = c.idx;
   __shared__ uint32_t list_bits[kListBits / 32];
   QueryList list{p, c, h, J, kT, c.n_tiles - J, list_bits};
   list.build();
 
-  clear_tile<DP, kStep>(Qs, d);
-  clear_tile<DP, kStep>(Gs, d);
-  TileLoad<T, DP, kT> lq, lg, lq1, lg1;
+  constexpr int kTiles = 2 * G;   // query tiles per step
+  clear_tile<DP, kStep<G>, G>(Qs, d);
+  clear_tile<DP, kStep<G>, G>(Gs, d);
+  TileLoad<T, DP, kT, G> lq[kTiles], lg[kTiles];
   if constexpr (!kStored) {
-    clear_tile<DP, kT>(Ks, d);
-    clear_tile<DP, kT>(Vs, d);
+    clear_tile<DP, kT, G>(Ks, d);
+    clear_tile<DP, kT, G>(Vs, d);
     if (d != DP) __syncthreads();
-    TileLoad<T, DP, kT> lk, lv;
+    TileLoad<T, DP, kT, G> lk, lv;
     lk.issue(Ks, p.k, c, h, J * kT, d, wide);
     lv.issue(Vs, p.v, c, h, J * kT, d, wide);
     lk.land(Ks);
@@ -786,27 +824,32 @@ __global__ void __launch_bounds__(kSimtThreads, kSimtBlocks<DP>) simt_bwd_dkv_ke
   }
   __syncthreads();
   float dk[4][DP / 16] = {}, dv[4][DP / 16] = {};
-  // Two of the query tiles that reach this key tile per step: I0 and I1 (== n_tiles: rows past the sequence, zeros).
-  int off = 0, I0 = J, I1 = J + list.next(1);
-  auto advance = [&] {
-    off = list.next(I1 - J + 1);
-    I0 = J + off;
-    I1 = J + list.next(off + 1);
+  // The next query tiles that reach this key tile (n_tiles where there are no more: rows past the sequence, zeros).
+  int off = 0, I[kTiles];
+  auto advance = [&](int from) {
+    off = list.next(from);
+    int o = off;
+#pragma unroll
+    for (int i = 0; i < kTiles; ++i) {
+      I[i] = J + o;
+      o = list.next(o + 1);
+    }
   };
-  auto load_q = [&] {
-    lq.issue(Qs, p.q, c, h, I0 * kT, d, wide);
-    lq1.issue(Qs + kT * kLd<DP>, p.q, c, h, I1 * kT, d, wide);
+  advance(0);
+  auto load_rows = [&](TileLoad<T, DP, kT, G> (&l)[kTiles], float *dst, const TensorRef &x) {
+#pragma unroll
+    for (int i = 0; i < kTiles; ++i) l[i].issue(dst + i * kT * kLd<DP>, x, c, h, I[i] * kT, d, wide);
   };
-  auto load_g = [&] {
-    lg.issue(Gs, p.d_o, c, h, I0 * kT, d, wide);
-    lg1.issue(Gs + kT * kLd<DP>, p.d_o, c, h, I1 * kT, d, wide);
+  auto land_rows = [&](TileLoad<T, DP, kT, G> (&l)[kTiles], float *dst) {
+#pragma unroll
+    for (int i = 0; i < kTiles; ++i) l[i].land(dst + i * kT * kLd<DP>);
   };
   if constexpr (kStored) {
-    auto load_stored = [&](float *dst, int part) {   // 64 query rows of A (part 0) or dz (part 1): 8 float4 per row
+    auto load_stored = [&](float *dst, int part) {   // the query rows of A (part 0) or dz (part 1): 8 float4 per row
 #pragma unroll
-      for (int i = 0; i < kStep * 8 / kSimtThreads; ++i) {
-        const int e = t + i * kSimtThreads, row = e >> 3, x = (e & 7) * 4;
-        const int Ir = row < kT ? I0 : I1;
+      for (int i = 0; i < kStep<G> * 8 / kThreads<G>; ++i) {
+        const int e = t + i * kThreads<G>, row = e >> 3, x = (e & 7) * 4;
+        const int Ir = I[i * kThreads<G> / (8 * kT)];
         const bool take = Ir < c.n_tiles;
         const long long pair = (long long)hh * p.pairs_cap + c.pair0 + (long long)Ir * (Ir + 1) / 2 + J;
         const float *src = reinterpret_cast<const float *>(p.az) + (take ? (pair * kT + (row & 31)) * (2 * kT) + part * kT + x : 0);
@@ -814,40 +857,37 @@ __global__ void __launch_bounds__(kSimtThreads, kSimtBlocks<DP>) simt_bwd_dkv_ke
       }
     };
     // the operands of either product arrive while the other one runs
-    load_q();
+    load_rows(lq, Qs, p.q);
     load_stored(Zs, 1);
     while (off < list.n) {
-      lq.land(Qs);
-      lq1.land(Qs + kT * kLd<DP>);
+      land_rows(lq, Qs);
       cp_async_wait();
       __syncthreads();
-      load_g();
+      load_rows(lg, Gs, p.d_o);
       load_stored(Ps, 0);
       tile_ptb<DP>(dk, Zs, Qs);
-      lg.land(Gs);
-      lg1.land(Gs + kT * kLd<DP>);
+      land_rows(lg, Gs);
       cp_async_wait();
       __syncthreads();
-      advance();
+      advance(I[kTiles - 1] - J + 1);
       if (off < list.n) {
-        load_q();
+        load_rows(lq, Qs, p.q);
         load_stored(Zs, 1);
       }
       tile_ptb<DP>(dv, Ps, Gs);
     }
   } else {
-    for (; off < list.n; advance()) {
-      load_q();
-      load_g();
-      lq.land(Qs);
-      lg.land(Gs);
-      lq1.land(Qs + kT * kLd<DP>);
-      lg1.land(Gs + kT * kLd<DP>);
+    static_assert(kStored || G == 1, "a row's keys are shared by two lanes");
+    for (; off < list.n; advance(I[kTiles - 1] - J + 1)) {
+      load_rows(lq, Qs, p.q);
+      load_rows(lg, Gs, p.d_o);
+      land_rows(lq, Qs);
+      land_rows(lg, Gs);
       __syncthreads();
-      tile_dot<DP, kStep, kT>(Zs, Qs, Ks, p.scale);
-      tile_dot<DP, kStep, kT>(Ps, Gs, Vs, 1.f);
+      tile_dot<DP, kStep<G>, kT>(Zs, Qs, Ks, p.scale);
+      tile_dot<DP, kStep<G>, kT>(Ps, Gs, Vs, 1.f);
       __syncthreads();
-      const int row = t >> 1, seg = t & 1, Ir = row < kT ? I0 : I1, gi = Ir * kT + (row & 31);
+      const int row = t >> 1, seg = t & 1, Ir = row < kT ? I[0] : I[1], gi = Ir * kT + (row & 31);
       float r1 = 0.f, gpre = 0.f, dr = 0.f;
       if (gi < c.len) {
         const long long slot = ((long long)hh * p.pairs_cap + c.pair0 + (long long)Ir * (Ir + 1) / 2 + J) * kT + (row & 31);
@@ -868,6 +908,12 @@ __global__ void __launch_bounds__(kSimtThreads, kSimtBlocks<DP>) simt_bwd_dkv_ke
       tile_ptb<DP>(dv, Ps, Gs);
       __syncthreads();
     }
+  }
+  if (G > 1) {
+    __syncthreads();
+    sum_groups<DP, G>(dk, Zs);
+    sum_groups<DP, G>(dv, Ps);
+    if (t >= 128) return;
   }
 
   const int tx = t % 16, ty = t / 16;
@@ -893,13 +939,13 @@ __global__ void __launch_bounds__(kSimtThreads, kSimtBlocks<DP>) simt_bwd_dkv_ke
   }
 }
 
-template <typename K>
+template <int G, typename K>
 static cudaError_t launch_one(K kernel, const KParams &p, size_t floats, bool wide, cudaStream_t s) {
   const size_t smem = floats * sizeof(float);
   cudaError_t e = allow_dynamic_smem(reinterpret_cast<const void *>(kernel), (int)smem);
   if (e != cudaSuccess) return e;
   dim3 grid(p.tiles_cap, p.head_cnt);
-  kernel<<<grid, kSimtThreads, smem, s>>>(p, wide);
+  kernel<<<grid, kThreads<G>, smem, s>>>(p, wide);
   return cudaGetLastError();
 }
 
@@ -911,23 +957,37 @@ static bool wide_rows(const TensorRef &t, int head_dim) {
                               t.sh % m == 0 && t.st % m == 0);
 }
 
-template <typename T, int DP>
+template <typename T, int DP, int G>
 static cudaError_t simt_run(const KParams &p, bool backward, cudaStream_t s) {
   const bool wide = wide_rows<T>(p.q, p.head_dim) && wide_rows<T>(p.k, p.head_dim) && wide_rows<T>(p.v, p.head_dim) &&
                     (!backward || wide_rows<T>(p.d_o, p.head_dim));
   constexpr size_t kRow = kT * kLd<DP>;
-  if (!backward) return launch_one(simt_fwd_kernel<T, DP>, p, 5 * kRow + kT * kLdS, wide, s);
+  if (!backward) return launch_one<G>(simt_fwd_kernel<T, DP, G>, p, (1 + 4 * G) * kRow + kT * kLdS<G>, wide, s);
   cudaError_t e = cudaSuccess;
-  if (!p.skip_dq) e = launch_one(simt_bwd_dq_kernel<T, DP>, p, 6 * kRow + 2 * kT * kLdS, wide, s);
+  if (!p.skip_dq) e = launch_one<G>(simt_bwd_dq_kernel<T, DP, G>, p, (2 + 4 * G) * kRow + (G == 1 ? 2 : 1) * kT * kLdS<G>, wide, s);
   if (e != cudaSuccess || p.skip_dkv) return e;
-  if (p.az != nullptr) return launch_one(simt_bwd_dkv_kernel<T, DP, true>, p, 4 * kRow + 2 * kStep * kLdH, wide, s);
-  return launch_one(simt_bwd_dkv_kernel<T, DP, false>, p, 6 * kRow + 2 * kStep * kLdH, wide, s);
+  if (p.az != nullptr) return launch_one<G>(simt_bwd_dkv_kernel<T, DP, G, true>, p, 4 * G * kRow + 2 * kStep<G> * kLdH, wide, s);
+  return launch_one<1>(simt_bwd_dkv_kernel<T, DP, 1, false>, p, 6 * kRow + 2 * kStep<1> * kLdH, wide, s);
+}
+// Two groups per block where there is no more than one block for every SM: the SM would idle with one block's four warps
+// (bf16, 7 heads x 500 tokens x 50, 112 blocks: forward + backward 98 us instead of 111).  With more blocks, one group each
+// makes better use of it: the steps at the diagonal waste less, and three blocks' barriers bind fewer threads (fp32, 512
+// blocks of 2 x 8 heads x 1024 x 64: 419 us instead of 462).  256 columns: two groups' operands do not fit.
+template <typename T, int DP>
+static cudaError_t simt_run_g(const KParams &p, bool backward, cudaStream_t s) {
+  if constexpr (DP <= 128) {
+    int sms = 0;
+    const cudaError_t e = sm_count(&sms);
+    if (e != cudaSuccess) return e;
+    if ((long long)p.tiles_cap * p.head_cnt <= sms) return simt_run<T, DP, 2>(p, backward, s);
+  }
+  return simt_run<T, DP, 1>(p, backward, s);
 }
 template <typename T>
 static cudaError_t simt_run_t(const KParams &p, bool backward, cudaStream_t s) {
-  if (p.head_dim <= 64) return simt_run<T, 64>(p, backward, s);
-  if (p.head_dim <= 128) return simt_run<T, 128>(p, backward, s);
-  return simt_run<T, 256>(p, backward, s);
+  if (p.head_dim <= 64) return simt_run_g<T, 64>(p, backward, s);
+  if (p.head_dim <= 128) return simt_run_g<T, 128>(p, backward, s);
+  return simt_run_g<T, 256>(p, backward, s);
 }
 static cudaError_t simt_dispatch(const KParams &p, int dtype, bool backward, cudaStream_t s) {
   if (dtype == SB_DTYPE_F32) return simt_run_t<float>(p, backward, s);

@@ -799,3 +799,19 @@ def test_keys_without_weight_are_left_out_of_short_sequences_too(sb, cuda_device
     for name, a, b in zip(("o", "rem", "dq", "dk", "dv"), got, want):
         assert torch.equal(a, b), name
     test_values_that_are_not_finite_reach_the_tiles_that_visit_them(sb, cuda_device, 64, torch.float16, lengths)
+
+
+@pytest.mark.parametrize("mode", ["stored", "recompute"])
+@pytest.mark.parametrize("d,dtype", [(64, torch.float32), (50, torch.bfloat16), (100, torch.float32)])
+@pytest.mark.parametrize("heads", [3, 60])   # two groups of threads per block; one (more blocks than SMs)
+def test_cuda_core_blocks_of_one_and_two_groups(sb, cuda_device, heads, d, dtype, mode):
+    """Steps of 128 and of 64 keys (query rows): sequences that end a row before, at and after either, and short ones."""
+    lengths = [1, 33, 64, 95, 127, 128, 129, 161, 300]
+    cu = cu_of(lengths)
+    one = H.make_inputs((1, sum(lengths), d), dtype, seed=d)
+    q, k, v, do, drem = (t.repeat(heads, *[1] * (t.dim() - 1)) for t in one)
+    with sb.small_backward_workspace(mode == "recompute"):
+        got = H.run_varlen(sb, q, k, v, do, drem, cu, cuda_device, attend_current=True)
+    for t in got:
+        assert torch.equal(t, t[:1].expand_as(t))
+    H.assert_parity([t[:1] for t in got], H.oracle_varlen(*one, cu, attend_current=True), dtype, f"{heads} heads d={d} {mode}")
