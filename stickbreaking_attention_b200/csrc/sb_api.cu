@@ -267,7 +267,8 @@ static int run(const SbParams *p, void *stream, bool backward) {
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
   cudaError_t e = launch_prep(k, s, &g_launches);
   if (e != cudaSuccess) return fail(SB_ERR_CUDA, "prep launch: %s", cudaGetErrorString(e));
-  if (backward && k.fuse_rem_v) {
+  k.drem_in_dq = backward && k.fuse_rem_v && pl.path == SB_PATH_TCGEN05 && pl.store_az;
+  if (backward && k.fuse_rem_v && !k.drem_in_dq) {
     e = launch_fused_drem(k, p->dtype, s);
     g_launches += 1;
     if (e != cudaSuccess) return fail(SB_ERR_CUDA, "d_rem launch: %s", cudaGetErrorString(e));

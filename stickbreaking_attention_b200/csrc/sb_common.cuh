@@ -61,6 +61,7 @@ struct KParams {
   int fuse_rem_v;      // forward writes o + rem * v; backward folds the two extra gradient terms in
   char *d_rem_fused;   // backward with fuse_rem_v: [batch][heads][tokens] d_rem + <d_out, v> in the tensors' dtype,
                        // written by the first kernel of the call; `d_rem` then points here for the other kernels
+  int drem_in_dq;      // ... or formed by the tensor-core dQ kernel, where no other kernel reads it (d_rem may be null then)
   int *status;
 };
 

@@ -296,6 +296,23 @@ struct Shared {
 static_assert(bNum * 8 + sizeof(Shared) <= 1024, "barriers and control words");
 }  // namespace dq3
 
+// d_rem + <d_out, v> of one row (g, v: its d_out and v), rounded like a caller's d_rem.  (Not inlined, and by value: see
+// fill_rows.)
+template <bool kFp16, typename T>
+__device__ __noinline__ float fused_drem_row(const T *g, const T *v, int head_dim, float d_rem) {
+  float s = 0.f;
+#pragma unroll 2
+  for (int x = 0; x < head_dim; x += 8) {
+    float gx[8], vx[8], part = 0.f;
+    load_row8<kFp16>(g + x, gx);
+    load_row8<kFp16>(v + x, vx);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) part = fmaf(gx[i], vx[i], part);
+    s += part;
+  }
+  return to_f32<T>(from_f32<T>(s + d_rem));
+}
+
 template <int D, bool kFp16, bool kStored>
 __global__ void __launch_bounds__(dq3::kThreads, 2)
 tc_bwd_dq3_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
@@ -455,7 +472,14 @@ tc_bwd_dq3_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
       const double total = p.log_rem[idx];
       r1 = (float)total;
       r1_lo = (float)(total - (double)r1);
-      dr = load_drem<T>(p, idx);
+      // out = o + rem * v: its gradient reaches rem through <d_out, v>.  (Formed here, the row of either comes from L2 while the
+      // SM's other block works; a kernel of its own took 21 us for 16 heads x 16384 x 64.)
+      if (p.d_rem != nullptr) dr = load_drem<T>(p, idx);
+      if (p.drem_in_dq) {
+        const long long tok = c.tok0 + row0 + r;
+        dr = fused_drem_row<kFp16, T>(reinterpret_cast<const T *>(p.d_o.ptr) + c.boff * p.d_o.sb + (long long)h * p.d_o.sh + tok * p.d_o.st,
+                                      reinterpret_cast<const T *>(p.v.ptr) + c.boff * p.v.sb + (long long)h * p.v.sh + tok * p.v.st, p.head_dim, dr);
+      }
     }
     const uint32_t tS = tmem + tcS + lane_off, tP = tmem + tcP + lane_off, tZ = tmem + C::tcZ + lane_off;
     // this row's part of the workspace for sub-tile 0: A, or the boundary records [pair (I, J)][quarter of the key tile][row]
