@@ -75,7 +75,9 @@ enum SbFlags {
                             unless sb_set_backward_scratch_budget changed it) -- and the dK/dV kernel is
                             two plain GEMMs over them.  With this flag, or when one head alone exceeds the
                             budget, the dK/dV kernel recomputes the tiles from boundary values (a few KiB
-                            per pair).  Same tiles either way.                                    */
+                            per pair).  Without the flag, and with `tile_start`, such a call on the tensor
+                            cores still stores the tiles of the pairs the forward visited if these fit the
+                            workspace; the device decides.  Same tiles either way.                */
   SB_FLAG_FUSE_REM_V = 32,  /* the caller wants out = o + rem[..., None] * v, what every caller of the
                             reference computes right after the operator (tests/test_varlen.py:101,
                             tests/test_attn.py:64).  sb_fwd writes `out` to `o` (rem and log_rem as usual).
@@ -209,7 +211,7 @@ SB_EXPORT int sb_fwd_static_scratch(const SbParams *p, void *stream);
  * value, and with bytes == 0 only reports it.  Process-wide; affects sb_workspace_bytes(p, 1) and sb_bwd alike, so
  * set it before sizing a workspace.  The backward works through the heads in chunks whose stored attention tiles
  * (64 KiB per 128 x 128 tile pair and head) fit the bound, and takes the recomputing dK/dV kernel when one head alone
- * does not fit.  The reference has no counterpart: its backward keeps nothing but lock arrays
+ * does not fit (or stores the tiles of the visited pairs only: SB_FLAG_BWD_RECOMPUTE).  The reference has no counterpart: its backward keeps nothing but lock arrays
  * (sb_varlen_bwd.py:568-573). */
 SB_EXPORT size_t sb_set_backward_scratch_budget(size_t bytes);
 

@@ -29,6 +29,7 @@ static inline size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; 
 // Workspace layout, a pure function of the shapes:
 //   [hdr 256 B][pair_prefix int64 x (num_seq+1)]
 //   packed batches: [order int2 x tiles]
+//   backward whose stored tiles would exceed the budget: [first slot int32 x heads x tiles][span int32 x heads] (see KParams)
 //   backward, either: [A | dz tiles, 16-bit x chunk_heads x pairs_cap x 2 x 128 x 128]   (stored-tiles mode)
 //             or:     [R1 fp32 x chunk_heads x pairs_cap x halves x tile][S2 same]       (recompute mode)
 //   backward with SB_FLAG_FUSE_REM_V: [d_rem + <d_out, v>, one value of the tensors' dtype in a 4-byte slot budget x batch x heads x tokens]
@@ -39,12 +40,14 @@ struct Plan {
   int n_max;
   int max_seqlen;
   long long pairs_cap;
-  size_t off_pair_prefix, off_order, off_bnd, off_drem;
+  size_t off_pair_prefix, off_order, off_slots, off_bnd, off_drem;
   int bnd_halves;             // boundary records per (query tile, key tile) pair
   size_t bnd_bytes_per_head;  // one of the two arrays
   int chunk_heads;
   bool store_az;              // backward: the dq kernel stores its A and dz tiles for the dK/dV kernel
   size_t az_bytes_per_head;
+  bool try_slots;             // backward: the visited pairs' tiles may fit although all pairs' do not
+  long long slots_cap;        // ... if there are no more than this
   size_t total_fwd, total_bwd;
 };
 
@@ -110,7 +113,6 @@ static int make_plan(const SbParams *p, Plan &pl, bool backward) {
   pl.off_pair_prefix = 256;
   pl.off_order = align_up(pl.off_pair_prefix + sizeof(long long) * (size_t)(p->num_seq + 1), 256);
   const size_t order_bytes = p->cu_seqlens != nullptr ? align_up(sizeof(int2) * (size_t)pl.tiles_cap, 256) : 0;
-  pl.off_bnd = pl.off_order + order_bytes;
   // the tensor-core path records the carried values four times per 128-key tile
   pl.bnd_halves = tc ? 4 : 1;   // keys 0, 32, 64, 96 of every 128-key tile
   pl.bnd_bytes_per_head = align_up((size_t)pl.pairs_cap * pl.tile * pl.bnd_halves * sizeof(float), 256);
@@ -120,11 +122,19 @@ static int make_plan(const SbParams *p, Plan &pl, bool backward) {
   const size_t budget = g_scratch_budget.load(std::memory_order_relaxed);
   pl.az_bytes_per_head = (size_t)pl.pairs_cap * 2 * pl.tile * pl.tile * (tc ? 2 : 4);
   pl.store_az = backward && !(p->flags & SB_FLAG_BWD_RECOMPUTE) && pl.az_bytes_per_head <= budget;
+  // A call that is too large for that keeps the visited pairs' tiles where the records would be, if they fit and the forward
+  // has said which pairs are visited (see run).
+  const bool slots = backward && tc && !pl.store_az && !(p->flags & SB_FLAG_BWD_RECOMPUTE);
+  pl.off_slots = pl.off_order + order_bytes;
+  pl.off_bnd = pl.off_slots + (slots ? align_up(sizeof(int) * (size_t)p->heads * ((size_t)pl.tiles_cap + 1), 256) : 0);
+  pl.try_slots = slots && p->struct_bytes > kShortParams && p->tile_start != nullptr && !(p->flags & SB_FLAG_DENSE_ROW_PASS);
   const size_t per_head = pl.store_az ? pl.az_bytes_per_head : 2 * pl.bnd_bytes_per_head;
   size_t chunk = per_head ? budget / per_head : (size_t)p->heads;
   if (chunk < 1) chunk = 1;
   if (chunk > (size_t)p->heads) chunk = p->heads;
   pl.chunk_heads = (int)chunk;
+  pl.slots_cap = (long long)(per_head * chunk / ((size_t)2 * kTcTile * kTcTile * 2));
+  if (pl.slots_cap < 1) pl.try_slots = false;
 #ifdef SB_TRACE   // diagnostic builds: reserved & 0x100 appends the event log to the workspace
   const size_t trace_bytes = (p->reserved & 0x100) ? kTraceBytes : 0;
 #else
@@ -273,6 +283,26 @@ static int run(const SbParams *p, void *stream, bool backward) {
     g_launches += 1;
     if (e != cudaSuccess) return fail(SB_ERR_CUDA, "d_rem launch: %s", cudaGetErrorString(e));
     k.d_rem = k.d_rem_fused;   // what the backward kernels read from here on
+  }
+  if (pl.try_slots) {
+    // Heads whose stick does not last visit a few key tiles per query tile whatever the sequence's length (one sequence of
+    // 131072 tokens, N(0, 0.5^2): 2 or 3 of up to 1024).  Which case it is is known on the device only: both are launched, the
+    // kernels of one of them leave at once (2 heads: 23 us for both).  dK/dV 266 -> 106 us for those 2 heads, dQ, which stores
+    // its tiles now, 127 -> 153.
+    KParams ks = k;
+    ks.head0 = 0;
+    ks.head_cnt = p->heads;
+    ks.az = reinterpret_cast<unsigned short *>(reinterpret_cast<char *>(p->workspace) + pl.off_bnd);
+    ks.pairs_cap = pl.slots_cap;
+    ks.pair_slot = reinterpret_cast<int *>(reinterpret_cast<char *>(p->workspace) + pl.off_slots);
+    ks.pair_span = ks.pair_slot + (size_t)p->heads * pl.tiles_cap;
+    ks.gate = k.gate = k.hdr + 5;
+    ks.gate_want = 1;
+    k.gate_want = 0;
+    e = launch_pair_slots(ks, s);
+    if (e == cudaSuccess) e = launch_tc_bwd(ks, p->dtype, s, &g_launches);
+    g_launches += 1;
+    if (e != cudaSuccess) return fail(SB_ERR_CUDA, "backward launch: %s", cudaGetErrorString(e));
   }
   const int chunk = backward ? pl.chunk_heads : p->heads;
   for (int h0 = 0; h0 < p->heads; h0 += chunk) {

@@ -54,6 +54,13 @@ struct KParams {
   unsigned short *az;  // stored-tiles mode: [head_cnt][pairs_cap][A, dz][128 query rows][128 keys], 16-bit; else null
                        // (CUDA-core kernels: fp32, [head_cnt][pairs_cap][32 query rows][32 A, 32 dz])
   long long pairs_cap;
+  // Stored-tiles mode where the tiles of all pairs would not fit, but those that the saved tile starts leave may (see
+  // launch_pair_slots): the slots of a query tile's visited pairs follow one another, slot = pair_slot[head][tile_id] + key
+  // tile, and `az` holds pairs_cap of them for all heads together.  Null otherwise.
+  int *pair_slot;      // [heads][tiles_cap]
+  int *pair_span;      // [heads] the most key tiles before its own that a query tile of the head visits
+  const int *gate;     // kernels of a launch whose gate_want is not *gate do nothing (null: no gate)
+  int gate_want;
   float *attn;         // forward, CUDA-core kernels only: [batch][heads][tokens][attn_cols] attention weights, or null
   long long attn_cols;
   int *tile_start;     // [batch * heads][tile_start_stride]: first key a group of 32 query rows reaches (see first_key), or null
@@ -108,13 +115,20 @@ __device__ __forceinline__ int tile_first_key(const KParams &p, const TileCoord 
   return first;
 }
 
+// A number for query tile I that no other tile of the call has, below tiles_cap: the tiles of a packed sequence begin at least
+// one after where the sequence before them ends.
+__device__ __forceinline__ int tile_id(const KParams &p, const TileCoord &c, int I) {
+  return (p.cu == nullptr ? c.seq * c.n_tiles : (int)(c.tok0 / p.tile) + c.seq) + I;
+}
+__device__ __forceinline__ bool gated(const KParams &p) { return p.gate != nullptr && *p.gate != p.gate_want; }
+
 // The query tiles I = J + off that reach key tile J (the others stopped before it), as a bit per tile in shared memory for
 // the first kListBits of them; later ones are looked up.  Tile J itself always does.
 constexpr int kListBits = 8192;
 struct QueryList {
   const KParams &p;
   const TileCoord &c;
-  int h, J, tile, n;      // n: query tiles J .. n_tiles - 1
+  int h, J, tile, n;      // n: query tiles J .. n_tiles - 1, or the first of them if none behind those reaches J
   uint32_t *bits;         // [kListBits / 32]
   __device__ __forceinline__ bool reaches(int off) const { return tile_first_key(p, c, h, J + off, tile) < (J + 1) * tile; }
   // by all threads of the block, before a barrier; one global read per query tile, all in flight together
@@ -319,6 +333,7 @@ __device__ __forceinline__ float load_drem(const KParams &p, long long idx) {
 cudaError_t launch_fused_drem(const KParams &p, int dtype, cudaStream_t s);   // fills d_rem_fused (all heads)
 cudaError_t launch_fused_dv(const KParams &p, int dtype, cudaStream_t s);     // dv += rem * d_out (all heads)
 cudaError_t launch_prep(const KParams &p, cudaStream_t s, int *launches);   // the sequence table, where the call needs one
+cudaError_t launch_pair_slots(const KParams &p, cudaStream_t s);   // fills pair_slot, pair_span and the gate
 cudaError_t launch_simt_fwd(const KParams &p, int dtype, cudaStream_t s, int *launches);
 cudaError_t launch_simt_bwd(const KParams &p, int dtype, cudaStream_t s, int *launches);
 cudaError_t launch_tc_fwd(const KParams &p, int dtype, cudaStream_t s, int *launches);

@@ -170,6 +170,47 @@ cudaError_t launch_prep(const KParams &p, cudaStream_t s, int *launches) {
   return cudaGetLastError();
 }
 
+// Where the stored tiles go if there is room for the visited pairs only: the slots are given out query tile by query tile, and
+// whether they suffice is known before the first kernel that would need them -- *gate says so, and the launches for either
+// case are made, one of which then does nothing.  One block: latency (two dependent reads per 1024 tiles and heads).
+__global__ void __launch_bounds__(kPrepThreads) pair_slots_kernel(KParams p, int *gate) {
+  __shared__ int s_warp[32];
+  __shared__ SmallTable tb;   // (not used: such calls have a table in memory)
+  const int t = threadIdx.x;
+  bool refused;
+  open_table(p, tb, refused);
+  if (refused) {              // the kernels of one of the two launches fill the outputs
+    if (t == 0) *gate = 1;
+    return;
+  }
+  for (int h = t; h < p.heads; h += kPrepThreads) p.pair_span[h] = 0;
+  __syncthreads();
+  const long long items = (p.cu == nullptr ? (p.tokens + p.tile - 1) / p.tile * p.batch : (long long)p.hdr[2]) * p.heads;
+  long long base = 0;
+  for (long long i0 = 0; i0 < items; i0 += kPrepThreads) {
+    const long long i = i0 + t;
+    TileCoord c;
+    int n = 0, h = 0, first = 0;
+    if (i < items && decode_item(p, tb, (int)(i / p.heads), true, c)) {
+      h = (int)(i % p.heads);
+      first = tile_first_key(p, c, h, c.idx, p.tile) / p.tile;
+      n = c.idx + 1 - first;
+      atomicMax(&p.pair_span[h], c.idx - first);
+    }
+    int total;
+    const int before = block_exclusive_scan(n, s_warp, total);
+    // (slots beyond the room there is are never used)
+    if (n > 0) p.pair_slot[(long long)h * p.tiles_cap + tile_id(p, c, c.idx)] = (int)min(base + before, (long long)0x3fffffff) - first;
+    base += total;
+  }
+  if (t == 0) *gate = base <= p.pairs_cap;
+}
+
+cudaError_t launch_pair_slots(const KParams &p, cudaStream_t s) {
+  pair_slots_kernel<<<1, kPrepThreads, 0, s>>>(p, const_cast<int *>(p.gate));
+  return cudaGetLastError();
+}
+
 // Backward with out = o + rem * v: the upstream gradient of rem gains <d_out, v> per row, and dv gains rem * d_out
 // (rem = 2^log_rem, from the saved fp64 value) on the rows that belong to a sequence.  Two elementwise kernels over
 // the (batch, heads, tokens) rows: grid (token blocks, heads, batch); `group` consecutive lanes share a row, each
@@ -213,6 +254,7 @@ __global__ void __launch_bounds__(256) fused_drem_kernel(KParams p, int group) {
 
 template <typename T, int kVec>
 __global__ void __launch_bounds__(256) fused_dv_kernel(KParams p, int group) {
+  if (gated(p)) return;
   if (p.cu != nullptr && p.hdr[0]) return;   // (a small call's table never comes with this kernel)
   const long long covered = p.cu != nullptr ? (long long)p.hdr[1] : p.tokens;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;

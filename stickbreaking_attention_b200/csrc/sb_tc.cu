@@ -103,7 +103,7 @@ cudaError_t allow_dynamic_smem(const void *kernel, int bytes) {
 
 cudaError_t make_az_map(CUtensorMap *map, const KParams &p, int dtype, int box_rows) {
   const cuuint64_t tile_bytes = (cuuint64_t)kBM * kBM * 2;
-  cuuint64_t dims[4] = {(cuuint64_t)kBM, (cuuint64_t)p.pairs_cap * kBM, 2, (cuuint64_t)p.head_cnt};
+  cuuint64_t dims[4] = {(cuuint64_t)kBM, (cuuint64_t)p.pairs_cap * kBM, 2, (cuuint64_t)(p.pair_slot != nullptr ? 1 : p.head_cnt)};
   cuuint64_t strides[3] = {(cuuint64_t)kBM * 2, (cuuint64_t)p.pairs_cap * tile_bytes, 2 * (cuuint64_t)p.pairs_cap * tile_bytes};
   return encode_cached(map, p.az, dims, strides, box_rows, dtype);
 }

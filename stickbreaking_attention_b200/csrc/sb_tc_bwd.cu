@@ -322,6 +322,7 @@ tc_bwd_dq3_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
   using C = Cfg<D>;
   constexpr int kTileBytes = C::kTileBytes, kKvTile = C::kKvTile, kKStages = C::kKStages, kVStages = C::kVStages, kBoxes = C::kBoxes;
   extern __shared__ __align__(1024) uint8_t smem_tiles[];   // (no byte is left to align it here)
+  if (gated(p)) return;
   if (threadIdx.x == 0) trace_block(p, 0);
   const uint32_t sQ = smem_u32(smem_tiles);
   const uint32_t sG = sQ + kTileBytes;
@@ -483,7 +484,9 @@ tc_bwd_dq3_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
     }
     const uint32_t tS = tmem + tcS + lane_off, tP = tmem + tcP + lane_off, tZ = tmem + C::tcZ + lane_off;
     // this row's part of the workspace for sub-tile 0: A, or the boundary records [pair (I, J)][quarter of the key tile][row]
-    const long long pair00 = (long long)(kStored ? 2 * hh : hh) * p.pairs_cap + c.pair0 + (long long)I * (I + 1) / 2;
+    const long long pair00 = kStored && p.pair_slot != nullptr
+                                 ? p.pair_slot[(long long)h * p.tiles_cap + tile_id(p, c, I)]
+                                 : (long long)(kStored ? 2 * hh : hh) * p.pairs_cap + c.pair0 + (long long)I * (I + 1) / 2;
     char *out = kStored ? reinterpret_cast<char *>(p.az + (pair00 * kBM + r) * kBM) : reinterpret_cast<char *>(p.bnd_r1 + pair00 * (4 * kBM) + r);
     const int u_diag = 2 * I, u_tail = c.len / kBN;   // a sub-tile with rows past the sequence is number u_tail
     // this warp's rows start at sub-tile u_warp (never, if they are past the sequence): before it, A and dz are zeros
@@ -642,6 +645,7 @@ tc_bwd_dkv4_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
   using namespace dkv4;
   constexpr int D = 128;
   extern __shared__ uint8_t smem_raw[];
+  if (gated(p)) return;
   if (threadIdx.x == 0) trace_block(p, 0);
   SmallTable &tb = *reinterpret_cast<SmallTable *>(smem_raw);   // never used: the launch sees to that, there is no room for it
   bool refused;
@@ -974,6 +978,7 @@ tc_bwd_dkv5_kernel(const __grid_constant__ CUtensorMap tm_az, const __grid_const
   using namespace dkv5;
   constexpr int D = 128;
   extern __shared__ uint8_t smem_raw[];
+  if (gated(p)) return;
   const uint32_t raw = smem_u32(smem_raw);
   const uint32_t base = (raw + 1023u) & ~1023u;
   uint8_t *gbase = smem_raw + (base - raw);
@@ -1005,7 +1010,9 @@ tc_bwd_dkv5_kernel(const __grid_constant__ CUtensorMap tm_az, const __grid_const
   auto bar = [&](int i) { return sBar + 8u * i; };
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   // the query tiles that reach this key tile, kSub stages each
-  QueryList list{p, c, h, J, kBM, c.n_tiles - J, reinterpret_cast<uint32_t *>(gbase + (sBar - base) + 512)};
+  const int last = c.n_tiles - J - 1;
+  QueryList list{p, c, h, J, kBM, p.pair_span == nullptr ? last + 1 : min(last, p.pair_span[h]) + 1,
+                 reinterpret_cast<uint32_t *>(gbase + (sBar - base) + 512)};
   list.build();
 
   if (threadIdx.x == 0) {
@@ -1033,14 +1040,16 @@ tc_bwd_dkv5_kernel(const __grid_constant__ CUtensorMap tm_az, const __grid_const
         if (t >= kStages && !wait_or_abort(bar(bEmpty + st), ((t / kStages) - 1) & 1, abort_flag, p, 640)) break;
         if (*abort_flag) break;
         const int I = J + off, hq = t % kSub;
-        const long long pair = c.pair0 + (long long)I * (I + 1) / 2 + J;
+        const bool packed = p.pair_slot != nullptr;
+        const long long pair = (packed ? (long long)p.pair_slot[(long long)h * p.tiles_cap + tile_id(p, c, I)] : c.pair0 + (long long)I * (I + 1) / 2) + J;
+        const int az_head = packed ? 0 : hh;
         const int az_row = (int)(pair * kBM) + hq * kRows;
         const int qrow = (int)c.tok0 + I * kBM + hq * kRows;
         const uint32_t dst = base + st * kStageBytes;
         mbar_arrive_expect_tx(bar(bFull + st), kStageBytes);
         for (int kb = 0; kb < 2; ++kb) {
-          tma_load_4d(dst + (0 + kb) * kBox, &tm_az, bar(bFull + st), kb * 64, az_row, 0, hh);   // A
-          tma_load_4d(dst + (2 + kb) * kBox, &tm_az, bar(bFull + st), kb * 64, az_row, 1, hh);   // dz
+          tma_load_4d(dst + (0 + kb) * kBox, &tm_az, bar(bFull + st), kb * 64, az_row, 0, az_head);   // A
+          tma_load_4d(dst + (2 + kb) * kBox, &tm_az, bar(bFull + st), kb * 64, az_row, 1, az_head);   // dz
           tma_load_4d(dst + (4 + kb) * kBox, &tm_q, bar(bFull + st), kb * 64, qrow, h, (int)c.boff);
           tma_load_4d(dst + (6 + kb) * kBox, &tm_g, bar(bFull + st), kb * 64, qrow, h, (int)c.boff);
         }
@@ -1055,7 +1064,7 @@ tc_bwd_dkv5_kernel(const __grid_constant__ CUtensorMap tm_az, const __grid_const
       for (int t = 0, off = 0; ok && off < list.n; ++t, off = t % kSub == 0 ? list.next(off + 1) : off) {
         const int st = t % kStages;
         ok = wait_or_abort(bar(bFull + st), (t / kStages) & 1, abort_flag, p, 641);
-        if (ok && off == list.n - 1 && t % kSub >= clean_from) {
+        if (ok && off == last && t % kSub >= clean_from) {
           *clean_stage = st;
           mbar_arrive(bar(bLanded));
           ok = wait_or_abort(bar(bClean), cleaned++ & 1, abort_flag, p, 643);
@@ -1081,7 +1090,7 @@ tc_bwd_dkv5_kernel(const __grid_constant__ CUtensorMap tm_az, const __grid_const
     const int r = threadIdx.x;
     const uint32_t lane_off = (uint32_t)(warp * 32) << 16;
     bool ok = true;
-    const bool last_listed = list.next(list.n - 1) < list.n;
+    const bool last_listed = last < list.n && list.next(last) == last;
     for (int hq = clean_from; ok && last_listed && hq < kSub; ++hq) {
       ok = wait_or_abort(bar(bLanded), (hq - clean_from) & 1, abort_flag, p, 644);
       if (!ok) break;

@@ -815,3 +815,29 @@ def test_cuda_core_blocks_of_one_and_two_groups(sb, cuda_device, heads, d, dtype
     for t in got:
         assert torch.equal(t, t[:1].expand_as(t))
     H.assert_parity([t[:1] for t in got], H.oracle_varlen(*one, cu, attend_current=True), dtype, f"{heads} heads d={d} {mode}")
+
+
+@pytest.mark.parametrize("d,dtype,form", [(128, torch.bfloat16, "packed"), (64, torch.float16, "fixed"), (96, torch.bfloat16, "packed")])
+@pytest.mark.parametrize("recipe", ["normal", "reference"])   # few pairs are visited and fit; nearly all are, and do not
+def test_tiles_of_the_visited_pairs_only(sb, cuda_device, recipe, d, dtype, form):
+    """A budget that one head's stored tiles exceed: those of the visited pairs take their place where they fit, otherwise the
+    dK/dV kernel recomputes.  Bit for bit what the stored tiles of all pairs give, or the recomputing kernels."""
+    from stickbreaking_attention_b200 import ops
+    lengths = [16000, 77, 300] if recipe == "normal" else [2500, 77, 300]
+    if form == "packed":
+        cu = cu_of(lengths)
+        ins = H.make_inputs((1, sum(lengths), d), dtype, seed=d, recipe=recipe)
+        run = lambda: H.run_varlen(sb, *ins, cu, cuda_device, max_seqlens=max(lengths))
+    else:
+        ins = H.make_inputs((1, 1, lengths[0], d), dtype, seed=d, recipe=recipe)
+        run = lambda: H.run_fixed(sb, *ins, cuda_device)
+    with sb.small_backward_workspace(recipe != "normal"):
+        want = run()
+    old = ops.set_backward_scratch_budget(1 << 20)
+    try:
+        got = run()
+        sb.check_status(cuda_device)
+    finally:
+        ops.set_backward_scratch_budget(old)
+    for a, b, name in zip(got, want, ("o", "rem", "dq", "dk", "dv")):
+        assert torch.equal(a, b), name
