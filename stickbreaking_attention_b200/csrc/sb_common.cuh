@@ -6,6 +6,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <utility>
+
 #include "../../include/sb_b200.h"
 
 namespace sb {
@@ -327,6 +329,32 @@ inline long long item_blocks(const KParams &p) {
 template <typename T>
 __device__ __forceinline__ float load_drem(const KParams &p, long long idx) {
   return to_f32<T>(reinterpret_cast<const T *>(p.d_rem)[idx]);
+}
+
+// Kernels follow one another without a gap: each may be launched before the one ahead of it has ended (programmatic dependent
+// launch) and, as its first step, waits for that; nothing is read or written, no tensor memory taken, before.  kLetGo: the
+// next kernel's blocks may take their places as soon as all of this one's have theirs.  That hides a launch's way to the GPU:
+// one 200-token forward after the other 11.7 -> 9.6 us, 2 heads x 131072 tokens, seven kernels, 390 -> 381.  The CUDA-core
+// kernels do not let go: where an SM's place is free for two blocks, the next kernel's few blocks would share the SMs that
+// are idle instead of having one each (7 heads x 500 x 50: 98 us without any of this, 134, 92).
+template <bool kLetGo = true>
+__device__ __forceinline__ void enter_kernel() {
+  if (kLetGo) asm volatile("griddepcontrol.launch_dependents;");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+template <typename... Params, typename... Args>
+inline cudaError_t launch_kernel(void (*kernel)(Params...), dim3 grid, int threads, size_t smem, cudaStream_t s, Args &&...args) {
+  cudaLaunchAttribute early = {};
+  early.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  early.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3((unsigned)threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cfg.attrs = &early;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);
 }
 
 // Host-side launch helpers implemented in the .cu files; all return cudaError_t of the launch.

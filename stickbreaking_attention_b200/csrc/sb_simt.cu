@@ -119,6 +119,7 @@ __device__ void build_order(const KParams &p, int2 *out, int *s_cls, int *s_warp
 }
 
 __global__ void __launch_bounds__(kPrepThreads) prep_kernel(KParams p) {
+  enter_kernel();
   __shared__ int s_cls[kMaxClasses];
   __shared__ long long s_warp[32];
   const int t = threadIdx.x;
@@ -166,14 +167,14 @@ cudaError_t launch_prep(const KParams &p, cudaStream_t s, int *launches) {
 #endif
   if (p.cu == nullptr || p.small_table) return cudaSuccess;
   *launches += 1;
-  prep_kernel<<<1, kPrepThreads, 0, s>>>(p);
-  return cudaGetLastError();
+  return launch_kernel(prep_kernel, dim3(1), kPrepThreads, 0, s, p);
 }
 
 // Where the stored tiles go if there is room for the visited pairs only: the slots are given out query tile by query tile, and
 // whether they suffice is known before the first kernel that would need them -- *gate says so, and the launches for either
 // case are made, one of which then does nothing.  One block: latency (two dependent reads per 1024 tiles and heads).
 __global__ void __launch_bounds__(kPrepThreads) pair_slots_kernel(KParams p, int *gate) {
+  enter_kernel();
   __shared__ int s_warp[32];
   __shared__ SmallTable tb;   // (not used: such calls have a table in memory)
   const int t = threadIdx.x;
@@ -207,8 +208,7 @@ __global__ void __launch_bounds__(kPrepThreads) pair_slots_kernel(KParams p, int
 }
 
 cudaError_t launch_pair_slots(const KParams &p, cudaStream_t s) {
-  pair_slots_kernel<<<1, kPrepThreads, 0, s>>>(p, const_cast<int *>(p.gate));
-  return cudaGetLastError();
+  return launch_kernel(pair_slots_kernel, dim3(1), kPrepThreads, 0, s, p, const_cast<int *>(p.gate));
 }
 
 // Backward with out = o + rem * v: the upstream gradient of rem gains <d_out, v> per row, and dv gains rem * d_out
@@ -229,6 +229,7 @@ __device__ __forceinline__ RowVec<T, kVec> load_vec(const T *src) {
 
 template <typename T, int kVec>
 __global__ void __launch_bounds__(256) fused_drem_kernel(KParams p, int group) {
+  enter_kernel();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int rows_per_warp = 32 / group;
   const long long tok = ((long long)blockIdx.x * 8 + warp) * rows_per_warp + lane / group;
@@ -254,6 +255,7 @@ __global__ void __launch_bounds__(256) fused_drem_kernel(KParams p, int group) {
 
 template <typename T, int kVec>
 __global__ void __launch_bounds__(256) fused_dv_kernel(KParams p, int group) {
+  enter_kernel();
   if (gated(p)) return;
   if (p.cu != nullptr && p.hdr[0]) return;   // (a small call's table never comes with this kernel)
   const long long covered = p.cu != nullptr ? (long long)p.hdr[1] : p.tokens;
@@ -292,14 +294,8 @@ static cudaError_t launch_fused_t(const KParams &p, cudaStream_t s) {
   while (group < 32 && group * per_lane < p.head_dim) group <<= 1;
   const long long rows_per_block = 8 * (32 / group);
   const dim3 grid((unsigned)((p.tokens + rows_per_block - 1) / rows_per_block), p.heads, p.batch);
-  if (kDv) {
-    if (vec) fused_dv_kernel<T, kVec><<<grid, 256, 0, s>>>(p, group);
-    else fused_dv_kernel<T, 1><<<grid, 256, 0, s>>>(p, group);
-  } else {
-    if (vec) fused_drem_kernel<T, kVec><<<grid, 256, 0, s>>>(p, group);
-    else fused_drem_kernel<T, 1><<<grid, 256, 0, s>>>(p, group);
-  }
-  return cudaGetLastError();
+  auto kernel = kDv ? (vec ? fused_dv_kernel<T, kVec> : fused_dv_kernel<T, 1>) : (vec ? fused_drem_kernel<T, kVec> : fused_drem_kernel<T, 1>);
+  return launch_kernel(kernel, grid, 256, 0, s, p, group);
 }
 
 cudaError_t launch_fused_drem(const KParams &p, int dtype, cudaStream_t s) {
@@ -550,6 +546,7 @@ __device__ __forceinline__ void store16(float *dst, const float (&x)[16]) {
 // sb_varlen_fwd.py:81-215).
 template <typename T, int DP, int G>
 __global__ void __launch_bounds__(kThreads<G>, kBlocks<DP, G>) simt_fwd_kernel(const __grid_constant__ KParams p, bool wide) {
+  enter_kernel<false>();
   extern __shared__ float4 smem4[];
   __shared__ SmallTable tb;
   bool refused;
@@ -722,6 +719,7 @@ __device__ __forceinline__ void bwd_segment(float (&z)[16], float (&dp)[16], int
 // pair in the workspace (p.az), or, where those would not fit the scratch budget, the carried R1 and S2 per pair and row.
 template <typename T, int DP, int G>
 __global__ void __launch_bounds__(kThreads<G>, kBlocks<DP, G>) simt_bwd_dq_kernel(const __grid_constant__ KParams p, bool wide) {
+  enter_kernel<false>();
   extern __shared__ float4 smem4[];
   __shared__ SmallTable tb;
   bool refused;
@@ -831,6 +829,7 @@ __global__ void __launch_bounds__(kThreads<G>, kBlocks<DP, G>) simt_bwd_dq_kerne
 // fixed summation order, no atomics.  kStored: A and dz come from the workspace; otherwise they are computed again.
 template <typename T, int DP, int G, bool kStored>
 __global__ void __launch_bounds__(kThreads<G>, kBlocks<DP, G>) simt_bwd_dkv_kernel(const __grid_constant__ KParams p, bool wide) {
+  enter_kernel<false>();
   extern __shared__ float4 smem4[];
   __shared__ SmallTable tb;
   bool refused;
@@ -987,8 +986,7 @@ static cudaError_t launch_one(K kernel, const KParams &p, size_t floats, bool wi
   cudaError_t e = allow_dynamic_smem(reinterpret_cast<const void *>(kernel), (int)smem);
   if (e != cudaSuccess) return e;
   dim3 grid(p.tiles_cap, p.head_cnt);
-  kernel<<<grid, kThreads<G>, smem, s>>>(p, wide);
-  return cudaGetLastError();
+  return launch_kernel(kernel, dim3(grid), kThreads<G>, smem, s, p, wide);
 }
 
 // Whether rows can be fetched in the loader's wide unit: 16 bytes of fp32, 4 bytes (two elements) of 16-bit tensors.

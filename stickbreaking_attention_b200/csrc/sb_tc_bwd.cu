@@ -318,6 +318,7 @@ __global__ void __launch_bounds__(dq3::kThreads, 2)
 tc_bwd_dq3_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                   const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_g,
                   const __grid_constant__ CUtensorMap tm_dq, const KParams p) {
+  enter_kernel();
   using namespace dq3;
   using C = Cfg<D>;
   constexpr int kTileBytes = C::kTileBytes, kKvTile = C::kKvTile, kKStages = C::kKStages, kVStages = C::kVStages, kBoxes = C::kBoxes;
@@ -642,6 +643,7 @@ __global__ void __launch_bounds__(dkv4::kThreads, 1)
 tc_bwd_dkv4_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                    const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_g,
                    const __grid_constant__ CUtensorMap tm_dk, const __grid_constant__ CUtensorMap tm_dv, const KParams p) {
+  enter_kernel();
   using namespace dkv4;
   constexpr int D = 128;
   extern __shared__ uint8_t smem_raw[];
@@ -975,6 +977,7 @@ __global__ void __launch_bounds__(dkv5::kThreads, 2)
 tc_bwd_dkv5_kernel(const __grid_constant__ CUtensorMap tm_az, const __grid_constant__ CUtensorMap tm_q,
                    const __grid_constant__ CUtensorMap tm_g, const __grid_constant__ CUtensorMap tm_dk,
                    const __grid_constant__ CUtensorMap tm_dv, const KParams p) {
+  enter_kernel();
   using namespace dkv5;
   constexpr int D = 128;
   extern __shared__ uint8_t smem_raw[];
@@ -1167,8 +1170,7 @@ static cudaError_t launch_bwd_t(const KParams &p, int dtype, cudaStream_t s) {
     if ((e = make_tile_map(&mk64, p.k, p, dtype, 64)) != cudaSuccess) return e;
     if ((e = make_tile_map(&mv64, p.v, p, dtype, 64)) != cudaSuccess) return e;
     if ((e = make_tile_map(&mdq, p.dq, p, dtype, 32)) != cudaSuccess) return e;
-    kernel<<<grid, dq3::kThreads, smem, s>>>(mq, mk64, mv64, mg, mdq, p);
-    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    if ((e = launch_kernel(kernel, grid, dq3::kThreads, smem, s, mq, mk64, mv64, mg, mdq, p)) != cudaSuccess) return e;
   }
   if (!p.skip_dkv && p.az != nullptr) {
     auto kernel = tc_bwd_dkv5_kernel<kFp16>;
@@ -1180,8 +1182,7 @@ static cudaError_t launch_bwd_t(const KParams &p, int dtype, cudaStream_t s) {
     if ((e = make_tile_map(&mg64, p.d_o, p, dtype, dkv5::kRows)) != cudaSuccess) return e;
     if ((e = make_tile_map(&mdk, p.dk, p, dtype, 32)) != cudaSuccess) return e;   // stores: 32 rows per warp
     if ((e = make_tile_map(&mdv, p.dv, p, dtype, 32)) != cudaSuccess) return e;
-    kernel<<<grid, dkv5::kThreads, dkv5::kSmem, s>>>(maz, mq64, mg64, mdk, mdv, p);
-    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    if ((e = launch_kernel(kernel, grid, dkv5::kThreads, dkv5::kSmem, s, maz, mq64, mg64, mdk, mdv, p)) != cudaSuccess) return e;
   } else if (!p.skip_dkv) {
     auto kernel = tc_bwd_dkv4_kernel<kFp16>;
     e = allow_dynamic_smem(reinterpret_cast<const void *>(kernel), dkv4::kSmem);
@@ -1189,8 +1190,7 @@ static cudaError_t launch_bwd_t(const KParams &p, int dtype, cudaStream_t s) {
     CUtensorMap mdk, mdv;   // stores: one 64-key strip at a time
     if ((e = make_tile_map(&mdk, p.dk, p, dtype, 64)) != cudaSuccess) return e;
     if ((e = make_tile_map(&mdv, p.dv, p, dtype, 64)) != cudaSuccess) return e;
-    kernel<<<grid, dkv4::kThreads, dkv4::kSmem, s>>>(mq, mk, mv, mg, mdk, mdv, p);
-    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    if ((e = launch_kernel(kernel, grid, dkv4::kThreads, dkv4::kSmem, s, mq, mk, mv, mg, mdk, mdv, p)) != cudaSuccess) return e;
   }
   return cudaSuccess;
 }

@@ -81,6 +81,7 @@ template <bool kFp16, bool kStop, bool kDrop>
 __global__ void __launch_bounds__(fwd128::kThreads, 1)
 tc_fwd128x2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                    const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_o, const __grid_constant__ KParams p) {
+  enter_kernel();
   using namespace fwd128;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
@@ -383,8 +384,7 @@ static cudaError_t launch128_t(const KParams &p, int dtype, cudaStream_t s) {
   const dim3 grid((unsigned)(blocks < sms ? blocks : sms));   // one resident block per SM
   auto kernel = tc_fwd128x2_kernel<kFp16, kStop, kDrop>;
   if ((e = allow_dynamic_smem(reinterpret_cast<const void *>(kernel), fwd128::kSmem)) != cudaSuccess) return e;
-  kernel<<<grid, fwd128::kThreads, fwd128::kSmem, s>>>(mq, mk, mv, mo, p);
-  return cudaGetLastError();
+  return launch_kernel(kernel, dim3(grid), fwd128::kThreads, fwd128::kSmem, s, mq, mk, mv, mo, p);
 }
 
 template <bool kFp16>

@@ -87,6 +87,7 @@ template <int D, bool kFp16>
 __global__ void __launch_bounds__(fwd256::kThreads, 1)
 tc_fwd256_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                  const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_o, const __grid_constant__ KParams p) {
+  enter_kernel();
   using namespace fwd256;
   using C = Cfg<D>;
   constexpr int kQBytes = C::kQBytes, kKvTileBytes = C::kKvTileBytes, kStageBytes = C::kStageBytes, kBoxes = C::kBoxes;
@@ -453,8 +454,7 @@ static cudaError_t launch_t(const KParams &p, int dtype, cudaStream_t s) {
   auto kernel = tc_fwd256_kernel<D, kFp16>;
   constexpr int smem = fwd256::Cfg<D>::kSmem;
   if ((e = allow_dynamic_smem(reinterpret_cast<const void *>(kernel), smem)) != cudaSuccess) return e;
-  kernel<<<grid, fwd256::kThreads, smem, s>>>(mq, mk, mv, mo, p);
-  return cudaGetLastError();
+  return launch_kernel(kernel, dim3(grid), fwd256::kThreads, smem, s, mq, mk, mv, mo, p);
 }
 
 cudaError_t launch_tc_fwd256(const KParams &p, int dtype, cudaStream_t s) {
