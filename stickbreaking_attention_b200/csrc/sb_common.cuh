@@ -331,12 +331,13 @@ __device__ __forceinline__ float load_drem(const KParams &p, long long idx) {
   return to_f32<T>(reinterpret_cast<const T *>(p.d_rem)[idx]);
 }
 
-// Kernels follow one another without a gap: each may be launched before the one ahead of it has ended (programmatic dependent
+// Kernels follow one another without a gap: each is launched before the one ahead of it has ended (programmatic dependent
 // launch) and, as its first step, waits for that; nothing is read or written, no tensor memory taken, before.  kLetGo: the
-// next kernel's blocks may take their places as soon as all of this one's have theirs.  That hides a launch's way to the GPU:
-// one 200-token forward after the other 11.7 -> 9.6 us, 2 heads x 131072 tokens, seven kernels, 390 -> 381.  The CUDA-core
-// kernels do not let go: where an SM's place is free for two blocks, the next kernel's few blocks would share the SMs that
-// are idle instead of having one each (7 heads x 500 x 50: 98 us without any of this, 134, 92).
+// next kernel's blocks may take their places as soon as all of this one's have theirs.  That hides a launch's way to the GPU
+// (one 200-token forward after the other: 11.7 us without any of this, 9.6) and is right for kernels of few blocks ahead of a
+// kernel of many.  Where this kernel's blocks are many or long, the next one's would sit in the places that its SMs have free
+// and be spread unevenly over them: kernels that let go / do not, 16 heads x 8 x 2048, d 64: 847 / 826 us forward + backward,
+// 2 heads x 131072: 384 / 376; CUDA cores, 7 heads x 500 x 50: 134 / 92 (98 without any of this).
 template <bool kLetGo = true>
 __device__ __forceinline__ void enter_kernel() {
   if (kLetGo) asm volatile("griddepcontrol.launch_dependents;");

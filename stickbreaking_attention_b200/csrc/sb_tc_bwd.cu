@@ -318,7 +318,7 @@ __global__ void __launch_bounds__(dq3::kThreads, 2)
 tc_bwd_dq3_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                   const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_g,
                   const __grid_constant__ CUtensorMap tm_dq, const KParams p) {
-  enter_kernel();
+  enter_kernel<false>();
   using namespace dq3;
   using C = Cfg<D>;
   constexpr int kTileBytes = C::kTileBytes, kKvTile = C::kKvTile, kKStages = C::kKStages, kVStages = C::kVStages, kBoxes = C::kBoxes;
@@ -643,7 +643,7 @@ __global__ void __launch_bounds__(dkv4::kThreads, 1)
 tc_bwd_dkv4_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                    const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_g,
                    const __grid_constant__ CUtensorMap tm_dk, const __grid_constant__ CUtensorMap tm_dv, const KParams p) {
-  enter_kernel();
+  enter_kernel<false>();
   using namespace dkv4;
   constexpr int D = 128;
   extern __shared__ uint8_t smem_raw[];
@@ -977,7 +977,7 @@ __global__ void __launch_bounds__(dkv5::kThreads, 2)
 tc_bwd_dkv5_kernel(const __grid_constant__ CUtensorMap tm_az, const __grid_constant__ CUtensorMap tm_q,
                    const __grid_constant__ CUtensorMap tm_g, const __grid_constant__ CUtensorMap tm_dk,
                    const __grid_constant__ CUtensorMap tm_dv, const KParams p) {
-  enter_kernel();
+  enter_kernel<false>();
   using namespace dkv5;
   constexpr int D = 128;
   extern __shared__ uint8_t smem_raw[];

@@ -87,7 +87,7 @@ template <int D, bool kFp16>
 __global__ void __launch_bounds__(fwd256::kThreads, 1)
 tc_fwd256_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                  const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_o, const __grid_constant__ KParams p) {
-  enter_kernel();
+  enter_kernel<false>();
   using namespace fwd256;
   using C = Cfg<D>;
   constexpr int kQBytes = C::kQBytes, kKvTileBytes = C::kKvTileBytes, kStageBytes = C::kStageBytes, kBoxes = C::kBoxes;
