@@ -32,8 +32,8 @@ namespace sb {
 // mc0: key index of the first column inside the 128-key tile (for the diagonal mask).
 // kSkip (unmasked chunks only): where the product of (1 - beta) at the END of the chunk -- its largest value in
 // the chunk -- has underflowed to exactly 0 and the prefix of G is still exactly 0, for all 32 rows of the warp, every
-// A, G and dz of the chunk is exactly 0 (e, the reciprocals and dP - dR are finite): only the log-space sum is formed,
-// with the same operations as otherwise, and the rest is not computed.
+// A, G and dz of the chunk is exactly 0 (e, the reciprocals and dP - dR are finite): the log-space sum is formed with the same
+// operations as otherwise, and sweep 3 (in the recomputing dK/dV kernel sweep 2 as well) is left out.
 // Packed pairs (two fp32 per instruction) are used where a pair sits in adjacent registers anyway -- accumulator columns and
 // what is computed column by column from them.  Products across columns stay scalar: pairing their operands up costs as many
 // register moves as the packed instruction saves.
