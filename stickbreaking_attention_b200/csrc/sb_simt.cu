@@ -608,10 +608,11 @@ __global__ void __launch_bounds__(kThreads<G>, kBlocks<DP, G>) simt_fwd_kernel(c
         R *= keep[j];
       }
       store16(srow, z);
-      float sum = sp;
+      // (in fp64: the backward subtracts its own sums from log_rem, and what an fp32 sum over the lanes rounds off is seen there)
+      double sum = (double)sp;
 #pragma unroll
       for (int o = 1; o < kLanes; o <<= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
-      run += (double)sum;
+      run += sum;
     }
     if (may_stop) {   // once every row's product has underflowed to 0, no earlier key has any weight
       if (!__syncthreads_or(gi < c.len && expf(-(float)run) != 0.f) && more) {

@@ -841,3 +841,18 @@ def test_tiles_of_the_visited_pairs_only(sb, cuda_device, recipe, d, dtype, form
         ops.set_backward_scratch_budget(old)
     for a, b, name in zip(got, want, ("o", "rem", "dq", "dk", "dv")):
         assert torch.equal(a, b), name
+
+
+@pytest.mark.parametrize("heads", [4, 40])   # two groups of threads per block; one
+def test_fp32_gradients_against_64_bits_where_rows_stop(sb, cuda_device, heads):
+    """The backward subtracts its own sums of softplus from the forward's, some 100 in all where a row's stick is used up, and
+    exponentiates: an error of the sums is one of the weights.  A lane's fp32 sum of 16 keys, about 13, is off by up to half a
+    unit of 2^-20, that is 5e-7; eight of them, at random, stay below 1e-6 as long as everything behind them is fp64."""
+    lengths = [64, 128, 256, 512]
+    cu = cu_of(lengths)
+    one = H.make_inputs((1, sum(lengths), 64), torch.float32, seed=3)
+    got = H.run_varlen(sb, *(t.repeat(heads, *[1] * (t.dim() - 1)) for t in one), cu, cuda_device, max_seqlens=512)
+    q, k, v, do, drem = (t.double() for t in one)
+    want = H.O.varlen_dense_grads(q, k, v, cu, do, drem, scale=None, attend_current=False, zero_start=False)
+    for name, a, b in zip(("dq", "dk", "dv"), got[2:], want[2:]):
+        assert H.rel_l2(a[:1], b) < 1e-6, name
