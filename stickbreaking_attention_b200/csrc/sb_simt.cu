@@ -1010,17 +1010,19 @@ static cudaError_t simt_run(const KParams &p, bool backward, cudaStream_t s) {
   if (p.az != nullptr) return launch_one<G>(simt_bwd_dkv_kernel<T, DP, G, true>, p, 4 * G * kRow + 2 * kStep<G> * kLdH, wide, s);
   return launch_one<1>(simt_bwd_dkv_kernel<T, DP, 1, false>, p, 6 * kRow + 2 * kStep<1> * kLdH, wide, s);
 }
-// Two groups per block where there is no more than one block for every SM: the SM would idle with one block's four warps
-// (bf16, 7 heads x 500 tokens x 50, 112 blocks: forward + backward 98 us instead of 111).  With more blocks, one group each
-// makes better use of it: the steps at the diagonal waste less, and three blocks' barriers bind fewer threads (fp32, 512
-// blocks of 2 x 8 heads x 1024 x 64: 419 us instead of 462).  256 columns: two groups' operands do not fit.
+// Two groups per block where there are no more than two blocks for every SM: one group each would leave the SMs with one or
+// two warps per scheduler.  With more blocks, one group makes better use of the SM: the steps at the diagonal waste less, and
+// three blocks' barriers bind fewer threads.  Forward + backward, one group / two (us): fp32, 64 columns, 1024 tokens, 160
+// blocks 203 / 184, 288 blocks 238 / 230, 384 blocks 284 / 295, 512 blocks 419 / 462; 100 columns, 154 blocks 314 / 253, 264
+// blocks 421 / 398, 308 blocks 445 / 447; bf16, 50 columns, 500 tokens, 224 blocks 180 / 159.  256 columns: two groups'
+// operands do not fit.
 template <typename T, int DP>
 static cudaError_t simt_run_g(const KParams &p, bool backward, cudaStream_t s) {
   if constexpr (DP <= 128) {
     int sms = 0;
     const cudaError_t e = sm_count(&sms);
     if (e != cudaSuccess) return e;
-    if ((long long)p.tiles_cap * p.head_cnt <= sms) return simt_run<T, DP, 2>(p, backward, s);
+    if ((long long)p.tiles_cap * p.head_cnt <= 2 * sms) return simt_run<T, DP, 2>(p, backward, s);
   }
   return simt_run<T, DP, 1>(p, backward, s);
 }

@@ -803,7 +803,7 @@ def test_keys_without_weight_are_left_out_of_short_sequences_too(sb, cuda_device
 
 @pytest.mark.parametrize("mode", ["stored", "recompute"])
 @pytest.mark.parametrize("d,dtype", [(64, torch.float32), (50, torch.bfloat16), (100, torch.float32)])
-@pytest.mark.parametrize("heads", [3, 60])   # two groups of threads per block; one (more blocks than SMs)
+@pytest.mark.parametrize("heads", [3, 60])   # two groups of threads per block; one (more than two blocks per SM)
 def test_cuda_core_blocks_of_one_and_two_groups(sb, cuda_device, heads, d, dtype, mode):
     """Steps of 128 and of 64 keys (query rows): sequences that end a row before, at and after either, and short ones."""
     lengths = [1, 33, 64, 95, 127, 128, 129, 161, 300]
