@@ -442,13 +442,15 @@ __device__ __forceinline__ void add_scaled(float *acc, float s, const float4 &b)
   acc[0] = lo.x; acc[1] = lo.y; acc[2] = hi.x; acc[3] = hi.y;
 }
 
-// acc (32 rows x DP, thread: rows 4 ty .. + 3, columns 4 tx + 64 u ..) += P (32 x 64 G) B (64 G x DP), 64 keys per group
+// acc (32 rows x DP, thread: rows 4 ty .. + 3, columns 4 tx + 64 u ..) += P (32 x 64 G) B (64 G x DP), 64 keys per group;
+// keys: the first of the step's that count, a multiple of 32 (the others' rows of B need not be finite)
 template <int DP, int G>
-__device__ __forceinline__ void tile_pv(float (&acc)[4][DP / 16], const float *P, const float *B) {
+__device__ __forceinline__ void tile_pv(float (&acc)[4][DP / 16], const float *P, const float *B, int keys = kStep<G>) {
   const int tx = threadIdx.x % 16, ty = threadIdx.x / 16 % 8, first = threadIdx.x / 128 * 64;
   const float *pp = P + 4 * ty * kLdS<G> + first, *b = B + first * kLd<DP> + 4 * tx;
+  const int mine = min(keys - first, 64);
 #pragma unroll 2
-  for (int k = 0; k < 64; k += 4) {
+  for (int k = 0; k < mine; k += 4) {
     float4 pv[4];
 #pragma unroll
     for (int i = 0; i < 4; ++i) pv[i] = *reinterpret_cast<const float4 *>(pp + i * kLdS<G> + k);
@@ -800,7 +802,7 @@ __global__ void __launch_bounds__(kThreads<G>, kBlocks<DP, G>) simt_bwd_dq_kerne
       gpre += gs;
     }
     __syncthreads();
-    tile_pv<DP, G>(acc, Zs, Ks);
+    tile_pv<DP, G>(acc, Zs, Ks, row0 + kT - key0);   // dz of the keys behind the tile is 0, and K may hold anything there
     if (more) lk.land(Vs);
     __syncthreads();
     float *tmp = Ks;

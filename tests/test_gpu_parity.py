@@ -856,3 +856,23 @@ def test_fp32_gradients_against_64_bits_where_rows_stop(sb, cuda_device, heads):
     want = H.O.varlen_dense_grads(q, k, v, cu, do, drem, scale=None, attend_current=False, zero_start=False)
     for name, a, b in zip(("dq", "dk", "dv"), got[2:], want[2:]):
         assert H.rel_l2(a[:1], b) < 1e-6, name
+
+
+@pytest.mark.parametrize("mode", ["stored", "recompute"])
+@pytest.mark.parametrize("d,dtype", [(64, torch.float32), (50, torch.bfloat16), (100, torch.float32), (200, torch.float16), (128, torch.bfloat16)])
+@pytest.mark.parametrize("heads", [8, 60])   # CUDA cores up to 128 columns: two groups of threads per block; one
+def test_later_tokens_that_are_not_finite_leave_earlier_query_tiles_alone(sb, cuda_device, heads, d, dtype, mode):
+    """A NaN or an infinity in k and v of one token per head, another one in each: o, rem and dq of the query tiles that end
+    before it are what they are without it."""
+    n, cu = 300, cu_of([300])
+    q, k, v, do, drem = H.make_inputs((heads, n, d), dtype, seed=d)
+    rows = 32 if dtype == torch.float32 or d % 8 or d > 128 else 128
+    with sb.small_backward_workspace(mode == "recompute"):
+        want = H.run_varlen(sb, q, k, v, do, drem, cu, cuda_device)
+        tokens = [(40 + 37 * h) % n for h in range(heads)]
+        for h, t in enumerate(tokens):
+            k[h, t] = v[h, t] = float("nan") if h % 2 else float("inf")
+        got = H.run_varlen(sb, q, k, v, do, drem, cu, cuda_device)
+    for h, t in enumerate(tokens):
+        for name, a, b in zip(("o", "rem", "dq"), got, want):
+            assert torch.equal(a[h, :t // rows * rows], b[h, :t // rows * rows]), (name, h, t)
