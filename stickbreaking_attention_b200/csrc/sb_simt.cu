@@ -313,17 +313,20 @@ cudaError_t launch_fused_dv(const KParams &p, int dtype, cudaStream_t s) {
 // ------------------------------------------------------------------------------------------------
 // CUDA-core kernels: fp32 arithmetic throughout, for fp32 tensors and head sizes the tensor-core kernels do not take.
 // ------------------------------------------------------------------------------------------------
-// What bounds them: latency at three blocks per SM, next to no single unit (2 x 8 heads x 1024 x 64 fp32: shared-memory and L1
-// pipe 59 to 66 % busy, FMA pipe 43 to 47 %, issue slots 41 to 46 %), and the tail of 512 blocks of unequal length (a quarter
-// of the SMs' time).  The products' operands come from shared memory: a block is one or two groups of 128 threads; every
-// product of a step gives each thread a 4 x 4 patch of the result (4 x DP/16 for the accumulators), so that eight 16-byte
-// shared loads feed 64 FMAs.  Per group a step is 32 query rows x 64 keys (forward, dQ) or 64 query rows x 32 keys (dK/dV):
-// small enough for three or four blocks of one group per SM at head size 64, and for a few heads of a few hundred tokens to
-// spread over the GPU.  The groups' accumulators are added up at the end.  The scans over the keys of a row are shared by
-// four (eight; dK/dV: two) lanes with 16 keys each.  Next operands are requested while the other product
-// of the step runs: cp.async for fp32, registers for 16-bit tensors (which are widened on their way to shared memory).
-// Measured, forward + backward: 2 x 8 heads x 1024 tokens, head size 64, fp32: 419 us; one thread per row scanning
+// What bounds them: latency at three blocks per SM, next to no single unit (one group per block, 2 x 8 heads x 1024 x 64 fp32:
+// shared-memory and L1 pipe 59 to 66 % busy, FMA pipe 43 to 47 %, issue slots 41 to 46 %), and the tail of 512 blocks of unequal
+// length (a quarter of the SMs' time).  The products' operands come from shared memory: a block is one or two groups of 128
+// threads; a product of scores gives each thread a 4 x 4 patch, so that eight 16-byte shared loads feed 64 FMAs, and of an
+// accumulator each thread has four rows and a sixteenth of its group's columns.  Per group a step is 32 query rows x 64 keys
+// (forward, dQ) or 64 query rows x 32 keys (dK/dV): small enough for three or four blocks of one group per SM at head size 64,
+// and for a few heads of a few hundred tokens to spread over the GPU.  The scans over the keys of a row are shared by four
+// (dK/dV: two) lanes per 64 (32) keys, 16 keys each.  Next operands are requested while the other product of the step runs:
+// cp.async for fp32, registers for 16-bit tensors (which are widened on their way to shared memory).
+// Measured, forward + backward: 2 x 8 heads x 1024 tokens, head size 64, fp32: 408 us; one thread per row scanning
 // serially and one shared load per FMA before: 2290 us.
+// Two groups give the bits of one: what a sequence's results are does not depend on what else is in the launch.  So the groups
+// share an accumulator's columns, and a step of 128 keys carries its sums and stops like two of 64.  With half of the keys each
+// and a sum over the groups at the end, a shared load fed twice the FMAs (7 heads x 500 x 64, fp32: 118 us instead of 124).
 constexpr int kT = kSimtTile;      // 32 rows or keys per tile
 template <int DP> constexpr int kLd = DP + 4;   // row stride of an operand tile: 16-byte rows, four banks apart
 constexpr int kLdH = kT + 4;       // row stride of a score tile with 32 columns
@@ -435,76 +438,68 @@ __device__ __forceinline__ void tile_dot(float *S, const float *A, const float *
     for (int j = 0; j < 4; ++j) S[(ty + i * kTy) * kLdO + tx + j * kTx] = (acc[i][j].x + acc[i][j].y) * mul;
 }
 
-__device__ __forceinline__ void add_scaled(float *acc, float s, const float4 &b) {   // four columns, two at a time
-  const float2 ss = make_float2(s, s);
-  const float2 lo = ptx::fma2(ss, make_float2(b.x, b.y), make_float2(acc[0], acc[1]));
-  const float2 hi = ptx::fma2(ss, make_float2(b.z, b.w), make_float2(acc[2], acc[3]));
-  acc[0] = lo.x; acc[1] = lo.y; acc[2] = hi.x; acc[3] = hi.y;
-}
-
-// acc (32 rows x DP, thread: rows 4 ty .. + 3, columns 4 tx + 64 u ..) += P (32 x 64 G) B (64 G x DP), 64 keys per group;
-// keys: the first of the step's that count, a multiple of 32 (the others' rows of B need not be finite)
+// A thread's part of a 32-row accumulator: rows 4 ty .. + 3 and, of the group's DP / G columns, kWide next to each other at
+// column(u) for every u < kChunks.  Each element is one thread's, who adds its terms up in the order of the keys (query
+// rows) as they are walked: one group or two, the sum has the same bits.
 template <int DP, int G>
-__device__ __forceinline__ void tile_pv(float (&acc)[4][DP / 16], const float *P, const float *B, int keys = kStep<G>) {
-  const int tx = threadIdx.x % 16, ty = threadIdx.x / 16 % 8, first = threadIdx.x / 128 * 64;
-  const float *pp = P + 4 * ty * kLdS<G> + first, *b = B + first * kLd<DP> + 4 * tx;
-  const int mine = min(keys - first, 64);
+struct Patch {
+  static constexpr int kCols = DP / 16 / G, kWide = kCols < 4 ? kCols : 4, kChunks = kCols / kWide;
+  float x[4][kCols] = {};
+  __device__ __forceinline__ static int row() { return threadIdx.x / 16 % 8 * 4; }
+  __device__ __forceinline__ static int column(int u) { return threadIdx.x / 128 * (DP / G) + threadIdx.x % 16 * kWide + 16 * kWide * u; }
+  // x[i][..] += s[i] * b[column(u) ..], b: a row of the operand from column(0) on
+  __device__ __forceinline__ void add_scaled(const float (&s)[4], const float *b) {
+#pragma unroll
+    for (int u = 0; u < kChunks; ++u) {
+      float2 bv[kWide / 2];
+      if constexpr (kWide == 4) {
+        const float4 f = *reinterpret_cast<const float4 *>(b + 16 * kWide * u);
+        bv[0] = make_float2(f.x, f.y);
+        bv[1] = make_float2(f.z, f.w);
+      } else {
+        bv[0] = *reinterpret_cast<const float2 *>(b + 16 * kWide * u);
+      }
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int w = 0; w < kWide; w += 2) {   // two columns at a time
+          float *a = &x[i][kWide * u + w];
+          const float2 r = ptx::fma2(make_float2(s[i], s[i]), bv[w / 2], make_float2(a[0], a[1]));
+          a[0] = r.x;
+          a[1] = r.y;
+        }
+    }
+  }
+};
+
+// acc (32 rows x DP) += P (32 x keys) B (keys x DP) for the keys [first, last) of the step, multiples of 32 (the rows of B
+// outside need not be finite)
+template <int DP, int G>
+__device__ __forceinline__ void tile_pv(Patch<DP, G> &acc, const float *P, const float *B, int first, int last) {
+  const float *pp = P + acc.row() * kLdS<G>, *b = B + acc.column(0);
 #pragma unroll 2
-  for (int k = 0; k < mine; k += 4) {
+  for (int k = first; k < last; k += 4) {
     float4 pv[4];
 #pragma unroll
     for (int i = 0; i < 4; ++i) pv[i] = *reinterpret_cast<const float4 *>(pp + i * kLdS<G> + k);
 #pragma unroll
     for (int kk = 0; kk < 4; ++kk) {
+      float sv[4];
 #pragma unroll
-      for (int u = 0; u < DP / 64; ++u) {
-        const float4 bv = *reinterpret_cast<const float4 *>(b + (k + kk) * kLd<DP> + 64 * u);
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const float s = kk == 0 ? pv[i].x : kk == 1 ? pv[i].y : kk == 2 ? pv[i].z : pv[i].w;
-          add_scaled(&acc[i][4 * u], s, bv);
-        }
-      }
+      for (int i = 0; i < 4; ++i) sv[i] = kk == 0 ? pv[i].x : kk == 1 ? pv[i].y : kk == 2 ? pv[i].z : pv[i].w;
+      acc.add_scaled(sv, b + (k + kk) * kLd<DP>);
     }
   }
 }
-// acc (32 keys x DP) += P^T B with P (64 G query rows x 32 keys), B (64 G x DP), 64 rows per group
-template <int DP>
-__device__ __forceinline__ void tile_ptb(float (&acc)[4][DP / 16], const float *P, const float *B) {
-  const int tx = threadIdx.x % 16, ty = threadIdx.x / 16 % 8, first = threadIdx.x / 128 * 64;
-  const float *pp = P + first * kLdH + 4 * ty, *b = B + first * kLd<DP> + 4 * tx;
-#pragma unroll 4
-  for (int k = 0; k < 64; ++k) {
-    const float4 pv = *reinterpret_cast<const float4 *>(pp + k * kLdH);
-#pragma unroll
-    for (int u = 0; u < DP / 64; ++u) {
-      const float4 bv = *reinterpret_cast<const float4 *>(b + k * kLd<DP> + 64 * u);
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const float s = i == 0 ? pv.x : i == 1 ? pv.y : i == 2 ? pv.z : pv.w;
-        add_scaled(&acc[i][4 * u], s, bv);
-      }
-    }
-  }
-}
-// The groups' parts of an accumulator, summed into the first group's; `scratch`: 32 x DP floats that are free.
+// acc (32 keys x DP) += P^T B with P (rows x 32 keys), B (rows x DP), rows: a multiple of 32
 template <int DP, int G>
-__device__ __forceinline__ void sum_groups(float (&acc)[4][DP / 16], float *scratch) {
-  if constexpr (G == 2) {
-    const int t = threadIdx.x & 127;
-    if (threadIdx.x >= 128) {
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int x = 0; x < DP / 16; ++x) scratch[(i * (DP / 16) + x) * 128 + t] = acc[i][x];
-    }
-    __syncthreads();
-    if (threadIdx.x < 128) {
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int x = 0; x < DP / 16; ++x) acc[i][x] += scratch[(i * (DP / 16) + x) * 128 + t];
-    }
+__device__ __forceinline__ void tile_ptb(Patch<DP, G> &acc, const float *P, const float *B, int rows) {
+  const float *pp = P + acc.row(), *b = B + acc.column(0);
+#pragma unroll 4
+  for (int k = 0; k < rows; ++k) {
+    const float4 pv = *reinterpret_cast<const float4 *>(pp + k * kLdH);
+    const float sv[4] = {pv.x, pv.y, pv.z, pv.w};
+    acc.add_scaled(sv, b + k * kLd<DP>);
   }
 }
 
@@ -544,7 +539,7 @@ __device__ __forceinline__ void store16(float *dst, const float (&x)[16]) {
 }
 
 // Forward: one block per (sequence, 32-row query tile, head), keys walked from the diagonal back to the sequence start in
-// steps of 64; every row carries sum softplus(z) over the keys already visited, in fp64 (reference: _forward_one_row,
+// steps of 64 per group; every row carries sum softplus(z) over the keys already visited, in fp64 (reference: _forward_one_row,
 // sb_varlen_fwd.py:81-215).
 template <typename T, int DP, int G>
 __global__ void __launch_bounds__(kThreads<G>, kBlocks<DP, G>) simt_fwd_kernel(const __grid_constant__ KParams p, bool wide) {
@@ -576,8 +571,8 @@ __global__ void __launch_bounds__(kThreads<G>, kBlocks<DP, G>) simt_fwd_kernel(c
   lq.land(Qs);
   lk.land(Ks);
   __syncthreads();
-  float acc[4][DP / 16] = {};
-  double run = 0.0;                         // sum of softplus(z) over the keys of the earlier steps
+  Patch<DP, G> acc;
+  double run = 0.0;                         // sum of softplus(z) over the keys visited
   const bool may_stop = p.tile_start != nullptr && !p.dense;
   int reached = 0;                          // first key visited
   for (; key0 > -kStep<G>; key0 -= kStep<G>) {
@@ -587,6 +582,7 @@ __global__ void __launch_bounds__(kThreads<G>, kBlocks<DP, G>) simt_fwd_kernel(c
     __syncthreads();
     bool more = key0 > 0;
     if (more) lk.issue(Ks, p.k, c, h, key0 - kStep<G>, d, wide);
+    double mid = 0.0;                       // two groups: `run` after the later 64 keys of the step
     {
       float z[16], beta[16], keep[16];
       float *srow = Ss + r * kLdS<G> + seg * 16;
@@ -595,28 +591,42 @@ __global__ void __launch_bounds__(kThreads<G>, kBlocks<DP, G>) simt_fwd_kernel(c
       float prod = 1.f;
 #pragma unroll
       for (int j = 0; j < 16; ++j) prod *= keep[j];
-      // product over the lanes with later keys, then down the lane's own keys
-#pragma unroll
-      for (int o = 1; o < kLanes; o <<= 1) {
-        const float later = __shfl_down_sync(0xffffffffu, prod, o, kLanes);
-        if (seg + o < kLanes) prod *= later;
+      // product over the lanes with later keys of the same 64, then down the lane's own keys
+      const float p1 = __shfl_down_sync(0xffffffffu, prod, 1, 4), p2 = __shfl_down_sync(0xffffffffu, prod, 2, 4),
+                  p3 = __shfl_down_sync(0xffffffffu, prod, 3, 4);
+      // (in fp64: the backward subtracts its own sums from log_rem, and what an fp32 sum over the lanes rounds off is seen there)
+      double sum = (double)sp;
+      sum += __shfl_xor_sync(0xffffffffu, sum, 1);
+      sum += __shfl_xor_sync(0xffffffffu, sum, 2);
+      double from = run;                    // ... over the keys after this lane's 64
+      if (G == 2) {
+        const double other = __shfl_xor_sync(0xffffffffu, sum, 4);
+        mid = run + (seg >= 4 ? sum : other);
+        if (seg < 4) from = mid;
+        run = mid + (seg >= 4 ? other : sum);
+      } else {
+        run += sum;
       }
-      const float after = __shfl_down_sync(0xffffffffu, prod, 1, kLanes);
-      float R = expf(-(float)run);
-      if (seg + 1 < kLanes) R *= after;
+      float R = expf(-(float)from);
+      if ((seg & 3) < 3) R *= p1;
+      if ((seg & 3) < 2) R *= p2;
+      if ((seg & 3) < 1) R *= p3;
 #pragma unroll
       for (int j = 15; j >= 0; --j) {
         z[j] = beta[j] * R;
         R *= keep[j];
       }
       store16(srow, z);
-      // (in fp64: the backward subtracts its own sums from log_rem, and what an fp32 sum over the lanes rounds off is seen there)
-      double sum = (double)sp;
-#pragma unroll
-      for (int o = 1; o < kLanes; o <<= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
-      run += sum;
     }
-    if (may_stop) {   // once every row's product has underflowed to 0, no earlier key has any weight
+    // Once every row's product has underflowed to 0, no earlier key has any weight.  With two groups a step is two of one
+    // group's: the tile stops where one group's would.
+    int from_key = 0;                       // the first key of the step that is visited, counted from key0
+    if (may_stop && G == 2 && !__syncthreads_or(gi < c.len && expf(-(float)mid) != 0.f) && key0 + 64 > 0) {
+      more = false;
+      reached = key0 + 64;
+      run = mid;
+      from_key = 64;
+    } else if (may_stop) {
       if (!__syncthreads_or(gi < c.len && expf(-(float)run) != 0.f) && more) {
         more = false;
         reached = key0;
@@ -627,18 +637,18 @@ __global__ void __launch_bounds__(kThreads<G>, kBlocks<DP, G>) simt_fwd_kernel(c
     if (p.attn != nullptr) {   // debugging aid: the attention weights of this step, keys indexed inside the sequence
       for (int e = t; e < kT * kStep<G>; e += kThreads<G>) {
         const int ri = row0 + e / kStep<G>, gj = key0 + e % kStep<G>;
-        if (ri < c.len && gj >= 0 && gj < c.len && gj < p.attn_cols)
+        if (ri < c.len && gj >= 0 && e % kStep<G> >= from_key && gj < c.len && gj < p.attn_cols)
           p.attn[((c.boff * p.heads + h) * p.tokens + c.tok0 + ri) * p.attn_cols + gj] = Ss[(e / kStep<G>) * kLdS<G> + e % kStep<G>];
       }
     }
-    tile_pv<DP, G>(acc, Ss, Vs);
+    if (G == 2) tile_pv(acc, Ss, Vs, 64, 128);   // the later keys first
+    if (from_key == 0 && key0 + 64 > 0) tile_pv(acc, Ss, Vs, 0, 64);
     if (!more) break;
     lk.land(Ks);
     __syncthreads();
   }
   if constexpr (sizeof(T) == 4) cp_async_wait();   // keys requested before the stop was known
   __syncthreads();
-  sum_groups<DP, G>(acc, Ss);
   if (p.tile_start != nullptr && t == 0 && row0 >= 64) *tile_start_entry(p, c, h, row0) = reached;
 
   const float rem = expf(-(float)run);
@@ -648,35 +658,35 @@ __global__ void __launch_bounds__(kThreads<G>, kBlocks<DP, G>) simt_fwd_kernel(c
     p.log_rem[idx] = -run * kLog2eD;
   }
   if (p.fuse_rem_v) {   // out = o + rem * v: the row owners publish rem through the free score tile
-    if (G > 1) __syncthreads();
     if (seg == 0) Ss[r] = rem;
     __syncthreads();
   }
-  if (t >= 128) return;
-  const int tx = t % 16, ty = t / 16;
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
-    const int row = row0 + 4 * ty + i;
+    const int row = row0 + acc.row() + i;
     if (row >= c.len) continue;
     T *o = reinterpret_cast<T *>(p.o.ptr) + c.boff * p.o.sb + (long long)h * p.o.sh + (c.tok0 + row) * p.o.st;
     const T *v = reinterpret_cast<const T *>(p.v.ptr) + c.boff * p.v.sb + (long long)h * p.v.sh + (c.tok0 + row) * p.v.st;
 #pragma unroll
-    for (int u = 0; u < DP / 64; ++u)
+    for (int u = 0; u < acc.kChunks; ++u)
 #pragma unroll
-      for (int x = 0; x < 4; ++x) {
-        const int col = 64 * u + 4 * tx + x;
-        if (col < d) o[col] = from_f32<T>(p.fuse_rem_v ? fmaf(Ss[4 * ty + i], to_f32<T>(v[col]), acc[i][4 * u + x]) : acc[i][4 * u + x]);
+      for (int x = 0; x < acc.kWide; ++x) {
+        const int col = acc.column(u) + x;
+        const float sum = acc.x[i][acc.kWide * u + x];
+        if (col < d) o[col] = from_f32<T>(p.fuse_rem_v ? fmaf(Ss[acc.row() + i], to_f32<T>(v[col]), sum) : sum);
       }
   }
 }
 
-// The backward of one lane's 16 keys: z, dP in; dz, A out.  LANES lanes share a row.
-// r1: minus the sum of softplus over the allowed keys from the step's first key on; gpre: sum of G over the keys before it.
-// On return r1_seg / g_seg hold the same two at this lane's first key and sp / gs the row's sums over the step.
-template <int LANES>
-__device__ __forceinline__ void bwd_segment(float (&z)[16], float (&dp)[16], int key0, int limit, double r1, float gpre, float dr,
-                                            double &r1_seg, float &g_seg, double &sp, float &gs) {
+// The backward of one lane's 16 keys: z, dP in; dz, A out.  LANES lanes share a row's keys of a step, or, with G == 2, of
+// either half of it; the second half goes on where the first one ends, as the next step of one group would.
+// r1: minus the sum of softplus over the allowed keys from the step's first key on; gpre: sum of G over the keys before it;
+// on return the same for the next step.  r1_seg / g_seg: both at this lane's first key.
+template <int LANES, int G>
+__device__ __forceinline__ void bwd_segment(float (&z)[16], float (&dp)[16], int key0, int limit, double &r1, float &gpre, float dr,
+                                            double &r1_seg, float &g_seg) {
   const int lane = threadIdx.x & (LANES - 1);
+  const bool second = G == 2 && (threadIdx.x & LANES);
   float beta[16], keep[16];
   const float own = stick_segment(z, key0, limit, beta, keep);
   double incl = own;                       // through this lane's last key
@@ -685,9 +695,13 @@ __device__ __forceinline__ void bwd_segment(float (&z)[16], float (&dp)[16], int
     const double up = __shfl_up_sync(0xffffffffu, incl, o, LANES);
     if (lane >= o) incl += up;
   }
-  sp = __shfl_sync(0xffffffffu, incl, LANES - 1, LANES);
+  const double sp = __shfl_sync(0xffffffffu, incl, LANES - 1, LANES);
+  const double sp_other = G == 2 ? __shfl_xor_sync(0xffffffffu, sp, LANES) : 0.0;
+  if (second) r1 += sp_other;
   r1_seg = r1 + (incl - (double)own);
   float W = expf((float)(r1 + incl));      // product of (1 - beta) over the keys after this lane's
+  r1 += sp;
+  if (G == 2 && !second) r1 += sp_other;
   float loc = 0.f;
 #pragma unroll
   for (int j = 15; j >= 0; --j) {
@@ -704,10 +718,14 @@ __device__ __forceinline__ void bwd_segment(float (&z)[16], float (&dp)[16], int
     const float up = __shfl_up_sync(0xffffffffu, gi, o, LANES);
     if (lane >= o) gi += up;
   }
-  gs = __shfl_sync(0xffffffffu, gi, LANES - 1, LANES);
+  const float gs = __shfl_sync(0xffffffffu, gi, LANES - 1, LANES);
+  const float gs_other = G == 2 ? __shfl_xor_sync(0xffffffffu, gs, LANES) : 0.f;
   const float before = __shfl_up_sync(0xffffffffu, gi, 1, LANES);
+  if (second) gpre += gs_other;
   g_seg = gpre + (lane > 0 ? before : 0.f);
   float C = g_seg;
+  gpre += gs;
+  if (G == 2 && !second) gpre += gs_other;
 #pragma unroll
   for (int j = 0; j < 16; ++j) {
     const float g = dp[j];
@@ -762,7 +780,7 @@ __global__ void __launch_bounds__(kThreads<G>, kBlocks<DP, G>) simt_bwd_dq_kerne
     dr = load_drem<T>(p, idx);
   }
   __syncthreads();
-  float acc[4][DP / 16] = {};
+  Patch<DP, G> acc;
   const long long pair0 = (long long)hh * p.pairs_cap + c.pair0 + (long long)I * (I + 1) / 2;
   for (int key0 = key_first; key0 <= row0; key0 += kStep<G>) {
     lv.issue(Vs, p.v, c, h, key0, d, wide);
@@ -783,9 +801,9 @@ __global__ void __launch_bounds__(kThreads<G>, kBlocks<DP, G>) simt_bwd_dq_kerne
     {
       if (G == 1) load16(z, zrow);
       load16(dp, Ps + r * kLdS<G> + seg * 16);
-      double r1_seg, sp;
-      float g_seg, gs;
-      bwd_segment<kLanes>(z, dp, key0 + seg * 16, limit, r1, gpre, dr, r1_seg, g_seg, sp, gs);
+      double r1_seg;
+      float g_seg;
+      bwd_segment<4, G>(z, dp, key0 + seg * 16, limit, r1, gpre, dr, r1_seg, g_seg);
       store16(zrow, z);
       const int J = key0 / kT + (seg >> 1);
       if (J <= I) {
@@ -798,37 +816,32 @@ __global__ void __launch_bounds__(kThreads<G>, kBlocks<DP, G>) simt_bwd_dq_kerne
           p.bnd_s2[(pair0 + J) * kT + r] = g_seg;
         }
       }
-      r1 += sp;
-      gpre += gs;
     }
     __syncthreads();
-    tile_pv<DP, G>(acc, Zs, Ks, row0 + kT - key0);   // dz of the keys behind the tile is 0, and K may hold anything there
+    tile_pv(acc, Zs, Ks, 0, min(kStep<G>, row0 + kT - key0));   // dz of the keys behind the tile is 0, and K may hold anything there
     if (more) lk.land(Vs);
     __syncthreads();
     float *tmp = Ks;
     Ks = Vs;
     Vs = tmp;
   }
-  sum_groups<DP, G>(acc, Zs);
-  if (t >= 128) return;
 
-  const int tx = t % 16, ty = t / 16;
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
-    const int row = row0 + 4 * ty + i;
+    const int row = row0 + acc.row() + i;
     if (row >= c.len) continue;
     T *o = reinterpret_cast<T *>(p.dq.ptr) + c.boff * p.dq.sb + (long long)h * p.dq.sh + (c.tok0 + row) * p.dq.st;
 #pragma unroll
-    for (int u = 0; u < DP / 64; ++u)
+    for (int u = 0; u < acc.kChunks; ++u)
 #pragma unroll
-      for (int x = 0; x < 4; ++x) {
-        const int col = 64 * u + 4 * tx + x;
-        if (col < d) o[col] = from_f32<T>(acc[i][4 * u + x] * p.scale);
+      for (int x = 0; x < acc.kWide; ++x) {
+        const int col = acc.column(u) + x;
+        if (col < d) o[col] = from_f32<T>(acc.x[i][acc.kWide * u + x] * p.scale);
       }
   }
 }
 
-// dK, dV: key-stationary, one block per 32-key tile, query tiles diagonal -> end two at a time; accumulators in registers,
+// dK, dV: key-stationary, one block per 32-key tile, query tiles diagonal -> end two per group at a time; accumulators in registers,
 // fixed summation order, no atomics.  kStored: A and dz come from the workspace; otherwise they are computed again.
 template <typename T, int DP, int G, bool kStored>
 __global__ void __launch_bounds__(kThreads<G>, kBlocks<DP, G>) simt_bwd_dkv_kernel(const __grid_constant__ KParams p, bool wide) {
@@ -867,15 +880,17 @@ __global__ void __launch_bounds__(kThreads<G>, kBlocks<DP, G>) simt_bwd_dkv_kern
     lv.land(Vs);
   }
   __syncthreads();
-  float dk[4][DP / 16] = {}, dv[4][DP / 16] = {};
+  Patch<DP, G> dk, dv;
   // The next query tiles that reach this key tile (n_tiles where there are no more: rows past the sequence, zeros).
-  int off = 0, I[kTiles];
+  int off = 0, rows = 0, I[kTiles];   // rows: those of the tiles there are
   auto advance = [&](int from) {
     off = list.next(from);
     int o = off;
+    rows = 0;
 #pragma unroll
     for (int i = 0; i < kTiles; ++i) {
       I[i] = J + o;
+      rows += o < list.n ? kT : 0;
       o = list.next(o + 1);
     }
   };
@@ -909,16 +924,17 @@ __global__ void __launch_bounds__(kThreads<G>, kBlocks<DP, G>) simt_bwd_dkv_kern
       __syncthreads();
       load_rows(lg, Gs, p.d_o);
       load_stored(Ps, 0);
-      tile_ptb<DP>(dk, Zs, Qs);
+      tile_ptb(dk, Zs, Qs, rows);
       land_rows(lg, Gs);
       cp_async_wait();
       __syncthreads();
+      const int rows_now = rows;
       advance(I[kTiles - 1] - J + 1);
       if (off < list.n) {
         load_rows(lq, Qs, p.q);
         load_stored(Zs, 1);
       }
-      tile_ptb<DP>(dv, Ps, Gs);
+      tile_ptb(dv, Ps, Gs, rows_now);
     }
   } else {
     static_assert(kStored || G == 1, "a row's keys are shared by two lanes");
@@ -932,7 +948,8 @@ __global__ void __launch_bounds__(kThreads<G>, kBlocks<DP, G>) simt_bwd_dkv_kern
       tile_dot<DP, kStep<G>, kT>(Ps, Gs, Vs, 1.f);
       __syncthreads();
       const int row = t >> 1, seg = t & 1, Ir = row < kT ? I[0] : I[1], gi = Ir * kT + (row & 31);
-      float r1 = 0.f, gpre = 0.f, dr = 0.f;
+      double r1 = 0.0;
+      float gpre = 0.f, dr = 0.f;
       if (gi < c.len) {
         const long long slot = ((long long)hh * p.pairs_cap + c.pair0 + (long long)Ir * (Ir + 1) / 2 + J) * kT + (row & 31);
         r1 = p.bnd_r1[slot];
@@ -942,28 +959,21 @@ __global__ void __launch_bounds__(kThreads<G>, kBlocks<DP, G>) simt_bwd_dkv_kern
       float z[16], dp[16];
       load16(z, Zs + row * kLdH + seg * 16);
       load16(dp, Ps + row * kLdH + seg * 16);
-      double r1_seg, sp;
-      float g_seg, gs;
-      bwd_segment<2>(z, dp, J * kT + seg * 16, gi < c.len ? gi + p.attend_current : 0, r1, gpre, dr, r1_seg, g_seg, sp, gs);
+      double r1_seg;
+      float g_seg;
+      bwd_segment<2, 1>(z, dp, J * kT + seg * 16, gi < c.len ? gi + p.attend_current : 0, r1, gpre, dr, r1_seg, g_seg);
       store16(Zs + row * kLdH + seg * 16, z);
       store16(Ps + row * kLdH + seg * 16, dp);
       __syncthreads();
-      tile_ptb<DP>(dk, Zs, Qs);
-      tile_ptb<DP>(dv, Ps, Gs);
+      tile_ptb(dk, Zs, Qs, rows);
+      tile_ptb(dv, Ps, Gs, rows);
       __syncthreads();
     }
   }
-  if (G > 1) {
-    __syncthreads();
-    sum_groups<DP, G>(dk, Zs);
-    sum_groups<DP, G>(dv, Ps);
-    if (t >= 128) return;
-  }
 
-  const int tx = t % 16, ty = t / 16;
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
-    const int key = J * kT + 4 * ty + i;
+    const int key = J * kT + dk.row() + i;
     if (key >= c.len) continue;
     T *ok = reinterpret_cast<T *>(p.dk.ptr) + c.boff * p.dk.sb + (long long)h * p.dk.sh + (c.tok0 + key) * p.dk.st;
     T *ov = reinterpret_cast<T *>(p.dv.ptr) + c.boff * p.dv.sb + (long long)h * p.dv.sh + (c.tok0 + key) * p.dv.st;
@@ -971,13 +981,14 @@ __global__ void __launch_bounds__(kThreads<G>, kBlocks<DP, G>) simt_bwd_dkv_kern
     const T *g = reinterpret_cast<const T *>(p.d_o.ptr) + c.boff * p.d_o.sb + (long long)h * p.d_o.sh + (c.tok0 + key) * p.d_o.st;
     const float rem = p.fuse_rem_v ? exp2f((float)p.log_rem[(c.boff * p.heads + h) * p.tokens + c.tok0 + key]) : 0.f;
 #pragma unroll
-    for (int u = 0; u < DP / 64; ++u)
+    for (int u = 0; u < dk.kChunks; ++u)
 #pragma unroll
-      for (int x = 0; x < 4; ++x) {
-        const int col = 64 * u + 4 * tx + x;
+      for (int x = 0; x < dk.kWide; ++x) {
+        const int col = dk.column(u) + x;
+        const float sum = dv.x[i][dv.kWide * u + x];
         if (col < d) {
-          ok[col] = from_f32<T>(dk[i][4 * u + x] * p.scale);
-          ov[col] = from_f32<T>(p.fuse_rem_v ? fmaf(rem, to_f32<T>(g[col]), dv[i][4 * u + x]) : dv[i][4 * u + x]);
+          ok[col] = from_f32<T>(dk.x[i][dk.kWide * u + x] * p.scale);
+          ov[col] = from_f32<T>(p.fuse_rem_v ? fmaf(rem, to_f32<T>(g[col]), sum) : sum);
         }
       }
   }

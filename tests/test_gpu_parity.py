@@ -876,3 +876,34 @@ def test_later_tokens_that_are_not_finite_leave_earlier_query_tiles_alone(sb, cu
     for h, t in enumerate(tokens):
         for name, a, b in zip(("o", "rem", "dq"), got, want):
             assert torch.equal(a[h, :t // rows * rows], b[h, :t // rows * rows]), (name, h, t)
+
+
+@pytest.mark.parametrize("mode", ["stored", "recompute"])
+@pytest.mark.parametrize("d,dtype", [(64, torch.float32), (50, torch.bfloat16), (100, torch.float32), (33, torch.float16)])
+def test_cuda_core_bits_do_not_depend_on_the_rest_of_the_launch(sb, cuda_device, d, dtype, mode):
+    """Three heads by themselves, among so many that a block has one group of threads, and one at a time: the same bits, with
+    rows that stop early and with an infinity that only some of the tiles reach."""
+    from stickbreaking_attention_b200 import ops
+    lengths = [500, 1, 129, 31, 700]
+    cu = cu_of(lengths)
+    q, k, v, do, drem = H.make_inputs((3, sum(lengths), d), dtype, seed=d)
+    q[1] += 0.3                                  # head 1 does not stop
+    k[1] -= 0.7
+    v[2, 100] = float("inf")
+    run = lambda copies: H.run_varlen(sb, *(t.repeat(copies, *[1] * (t.dim() - 1)) for t in (q, k, v, do, drem)), cu, cuda_device)
+    state = lambda copies: H.forward_state(sb, *(t.repeat(copies, 1, 1).to(cuda_device) for t in (q, k, v)), cu.to(cuda_device), 700)
+    with sb.small_backward_workspace(mode == "recompute"):
+        few, many = run(1), run(20)
+        # stored: (43 tiles and one more per sequence) x 23 / 2 pairs of 8 KiB per head, three heads per chunk; records: one
+        old = ops.set_backward_scratch_budget(1 if mode == "recompute" else 3 * 552 * 8192)
+        try:
+            chunked = run(20)
+        finally:
+            ops.set_backward_scratch_budget(old)
+    for what, got in (("many", many), ("chunked", chunked)):
+        for name, a, b in zip(("o", "rem", "dq", "dk", "dv"), got, few):
+            a = a.unflatten(0, (20, 3))
+            assert torch.equal(a.nan_to_num(nan=77.0), b.nan_to_num(nan=77.0).expand_as(a)), (what, name)
+    for name, a, b in zip(("o", "rem", "log_rem", "tile_start"), state(20), state(1)):
+        a = a.unflatten(0, (20, 3))
+        assert torch.equal(a.nan_to_num(nan=77.0), b.nan_to_num(nan=77.0).expand_as(a)), name
