@@ -347,7 +347,7 @@ __device__ __forceinline__ void cp_async4(float *dst, const void *src, bool take
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
 // A tile of ROWS rows of one tensor on its way into shared memory: issue() requests it, land() makes it visible to the
-// issuing thread's next barrier.  Rows outside [0, len) become zeros; columns past head_dim are zeroed once by clear().
+// issuing thread's next barrier.  Rows outside [0, end) become zeros; columns past head_dim are zeroed once by clear().
 template <typename T, int DP, int ROWS, int G>
 struct TileLoad {
   static constexpr int kWords = ROWS * DP / 2 / kThreads<G>;   // 16-bit tensors: two elements per register
@@ -357,20 +357,23 @@ struct TileLoad {
     return reinterpret_cast<const T *>(t.ptr) + c.boff * t.sb + (long long)h * t.sh + c.tok0 * t.st;
   }
   __device__ __forceinline__ void issue(float *dst, const TensorRef &t, const TileCoord &c, int h, int row0, int d, bool wide) {
+    issue(dst, t, c, h, row0, d, wide, c.len);
+  }
+  __device__ __forceinline__ void issue(float *dst, const TensorRef &t, const TileCoord &c, int h, int row0, int d, bool wide, int end) {
     const T *base = row_ptr(t, c, h);
     if constexpr (sizeof(T) == 4) {
       if (wide) {   // rows of whole 16-byte chunks
 #pragma unroll 4
         for (int e = threadIdx.x; e < ROWS * (DP / 4); e += kThreads<G>) {
           const int r = e / (DP / 4), x = (e % (DP / 4)) * 4, row = row0 + r;
-          const bool take = row >= 0 && row < c.len;
+          const bool take = row >= 0 && row < end;
           if (x < d) cp_async16(dst + r * kLd<DP> + x, base + (take ? row * t.st + x : 0), take);
         }
       } else {
 #pragma unroll 4
         for (int e = threadIdx.x; e < ROWS * DP; e += kThreads<G>) {
           const int r = e / DP, x = e % DP, row = row0 + r;
-          const bool take = row >= 0 && row < c.len;
+          const bool take = row >= 0 && row < end;
           if (x < d) cp_async4(dst + r * kLd<DP> + x, base + (take ? row * t.st + x : 0), take);
         }
       }
@@ -381,7 +384,7 @@ struct TileLoad {
         const int e = threadIdx.x + i * kThreads<G>;
         const int r = e / (DP / 2), x = (e % (DP / 2)) * 2, row = row0 + r;
         w[i] = 0u;
-        if (row >= 0 && row < c.len && x < d) {
+        if (row >= 0 && row < end && x < d) {
           const unsigned short *src = b16 + row * t.st + x;
           if (wide) w[i] = *reinterpret_cast<const uint32_t *>(src);   // even head size, 4-byte aligned rows
           else w[i] = (uint32_t)src[0] | (x + 1 < d ? (uint32_t)src[1] << 16 : 0u);
@@ -472,13 +475,14 @@ struct Patch {
   }
 };
 
-// acc (32 rows x DP) += P (32 x keys) B (keys x DP) for the keys [first, last) of the step, multiples of 32 (the rows of B
-// outside need not be finite)
+// acc (32 rows x DP) += P (32 x 64) B (64 x DP): 64 of the step's keys, from key `first` on.  (A trip count that is known only
+// as it runs costs the 16-bit kernels, short of registers at 128 columns, a tenth: dQ + dK/dV of 20 bf16 heads x 640 x 100,
+// one group, 455 us instead of 409.)
 template <int DP, int G>
-__device__ __forceinline__ void tile_pv(Patch<DP, G> &acc, const float *P, const float *B, int first, int last) {
-  const float *pp = P + acc.row() * kLdS<G>, *b = B + acc.column(0);
+__device__ __forceinline__ void tile_pv(Patch<DP, G> &acc, const float *P, const float *B, int first) {
+  const float *pp = P + acc.row() * kLdS<G> + first, *b = B + first * kLd<DP> + acc.column(0);
 #pragma unroll 2
-  for (int k = first; k < last; k += 4) {
+  for (int k = 0; k < 64; k += 4) {
     float4 pv[4];
 #pragma unroll
     for (int i = 0; i < 4; ++i) pv[i] = *reinterpret_cast<const float4 *>(pp + i * kLdS<G> + k);
@@ -491,12 +495,12 @@ __device__ __forceinline__ void tile_pv(Patch<DP, G> &acc, const float *P, const
     }
   }
 }
-// acc (32 keys x DP) += P^T B with P (rows x 32 keys), B (rows x DP), rows: a multiple of 32
+// acc (32 keys x DP) += P^T B with P (64 x 32 keys), B (64 x DP): 64 of the step's query rows, from row `first` on
 template <int DP, int G>
-__device__ __forceinline__ void tile_ptb(Patch<DP, G> &acc, const float *P, const float *B, int rows) {
-  const float *pp = P + acc.row(), *b = B + acc.column(0);
+__device__ __forceinline__ void tile_ptb(Patch<DP, G> &acc, const float *P, const float *B, int first) {
+  const float *pp = P + first * kLdH + acc.row(), *b = B + first * kLd<DP> + acc.column(0);
 #pragma unroll 4
-  for (int k = 0; k < rows; ++k) {
+  for (int k = 0; k < 64; ++k) {
     const float4 pv = *reinterpret_cast<const float4 *>(pp + k * kLdH);
     const float sv[4] = {pv.x, pv.y, pv.z, pv.w};
     acc.add_scaled(sv, b + k * kLd<DP>);
@@ -641,8 +645,8 @@ __global__ void __launch_bounds__(kThreads<G>, kBlocks<DP, G>) simt_fwd_kernel(c
           p.attn[((c.boff * p.heads + h) * p.tokens + c.tok0 + ri) * p.attn_cols + gj] = Ss[(e / kStep<G>) * kLdS<G> + e % kStep<G>];
       }
     }
-    if (G == 2) tile_pv(acc, Ss, Vs, 64, 128);   // the later keys first
-    if (from_key == 0 && key0 + 64 > 0) tile_pv(acc, Ss, Vs, 0, 64);
+    if (G == 2) tile_pv(acc, Ss, Vs, 64);   // the later keys first
+    if (G == 1 || (from_key == 0 && key0 + 64 > 0)) tile_pv(acc, Ss, Vs, 0);
     if (!more) break;
     lk.land(Ks);
     __syncthreads();
@@ -768,7 +772,9 @@ __global__ void __launch_bounds__(kThreads<G>, kBlocks<DP, G>) simt_bwd_dq_kerne
   lq.issue(Qs, p.q, c, h, row0, d, wide);
   lg.issue(Gs, p.d_o, c, h, row0, d, wide);
   const int key_first = first_key(p, c, h, row0);
-  lk.issue(Ks, p.k, c, h, key_first, d, wide);
+  // The last step runs past the tile.  dz is 0 there, and so is K to be: whatever later tokens hold, it is none of these rows'.
+  const int key_end = min(c.len, row0 + kT);
+  lk.issue(Ks, p.k, c, h, key_first, d, wide, key_end);
   lq.land(Qs);
   lg.land(Gs);
   lk.land(Ks);
@@ -797,7 +803,7 @@ __global__ void __launch_bounds__(kThreads<G>, kBlocks<DP, G>) simt_bwd_dq_kerne
     __syncthreads();
     // V is done with: the next K goes into its buffer while this step goes on, and the next V into this K's
     const bool more = key0 + kStep<G> <= row0;
-    if (more) lk.issue(Vs, p.k, c, h, key0 + kStep<G>, d, wide);
+    if (more) lk.issue(Vs, p.k, c, h, key0 + kStep<G>, d, wide, key_end);
     {
       if (G == 1) load16(z, zrow);
       load16(dp, Ps + r * kLdS<G> + seg * 16);
@@ -818,7 +824,8 @@ __global__ void __launch_bounds__(kThreads<G>, kBlocks<DP, G>) simt_bwd_dq_kerne
       }
     }
     __syncthreads();
-    tile_pv(acc, Zs, Ks, 0, min(kStep<G>, row0 + kT - key0));   // dz of the keys behind the tile is 0, and K may hold anything there
+    tile_pv(acc, Zs, Ks, 0);
+    if (G == 2 && key0 + 64 <= row0) tile_pv(acc, Zs, Ks, 64);
     if (more) lk.land(Vs);
     __syncthreads();
     float *tmp = Ks;
@@ -882,15 +889,13 @@ __global__ void __launch_bounds__(kThreads<G>, kBlocks<DP, G>) simt_bwd_dkv_kern
   __syncthreads();
   Patch<DP, G> dk, dv;
   // The next query tiles that reach this key tile (n_tiles where there are no more: rows past the sequence, zeros).
-  int off = 0, rows = 0, I[kTiles];   // rows: those of the tiles there are
+  int off = 0, I[kTiles];
   auto advance = [&](int from) {
     off = list.next(from);
     int o = off;
-    rows = 0;
 #pragma unroll
     for (int i = 0; i < kTiles; ++i) {
       I[i] = J + o;
-      rows += o < list.n ? kT : 0;
       o = list.next(o + 1);
     }
   };
@@ -924,17 +929,19 @@ __global__ void __launch_bounds__(kThreads<G>, kBlocks<DP, G>) simt_bwd_dkv_kern
       __syncthreads();
       load_rows(lg, Gs, p.d_o);
       load_stored(Ps, 0);
-      tile_ptb(dk, Zs, Qs, rows);
+      const bool wider = G == 2 && I[2 * (G - 1)] < c.n_tiles;   // there is a third tile
+      tile_ptb(dk, Zs, Qs, 0);
+      if (wider) tile_ptb(dk, Zs, Qs, 64);
       land_rows(lg, Gs);
       cp_async_wait();
       __syncthreads();
-      const int rows_now = rows;
       advance(I[kTiles - 1] - J + 1);
       if (off < list.n) {
         load_rows(lq, Qs, p.q);
         load_stored(Zs, 1);
       }
-      tile_ptb(dv, Ps, Gs, rows_now);
+      tile_ptb(dv, Ps, Gs, 0);
+      if (wider) tile_ptb(dv, Ps, Gs, 64);
     }
   } else {
     static_assert(kStored || G == 1, "a row's keys are shared by two lanes");
@@ -965,8 +972,8 @@ __global__ void __launch_bounds__(kThreads<G>, kBlocks<DP, G>) simt_bwd_dkv_kern
       store16(Zs + row * kLdH + seg * 16, z);
       store16(Ps + row * kLdH + seg * 16, dp);
       __syncthreads();
-      tile_ptb(dk, Zs, Qs, rows);
-      tile_ptb(dv, Ps, Gs, rows);
+      tile_ptb(dk, Zs, Qs, 0);
+      tile_ptb(dv, Ps, Gs, 0);
       __syncthreads();
     }
   }
