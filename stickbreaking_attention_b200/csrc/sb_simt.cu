@@ -1030,19 +1030,42 @@ static cudaError_t simt_run(const KParams &p, bool backward, cudaStream_t s) {
   if (p.az != nullptr) return launch_one<G>(simt_bwd_dkv_kernel<T, DP, G, true>, p, 4 * G * kRow + 2 * kStep<G> * kLdH, wide, s);
   return launch_one<1>(simt_bwd_dkv_kernel<T, DP, 1, false>, p, 6 * kRow + 2 * kStep<1> * kLdH, wide, s);
 }
-// Two groups per block where there are no more than two blocks for every SM: one group each would leave the SMs with one or
-// two warps per scheduler.  With more blocks, one group makes better use of the SM: the steps at the diagonal waste less, and
-// three blocks' barriers bind fewer threads.  Forward + backward, one group / two (us): fp32, 64 columns, 1024 tokens, 160
-// blocks 203 / 184, 288 blocks 238 / 230, 384 blocks 284 / 295, 512 blocks 419 / 462; 100 columns, 154 blocks 314 / 253, 264
-// blocks 421 / 398, 308 blocks 445 / 447; bf16, 50 columns, 500 tokens, 224 blocks 180 / 159.  256 columns: two groups'
-// operands do not fit.
+// Two groups per block are taken where one would leave the SMs with few warps and the longest sequence is worth their steps of
+// 128 keys.  Forward + backward, one group / two (us; fp32, 64 columns unless said otherwise):
+// * up to 64 tokens a tile is one step either way, at least half of the wider one masked: 8 heads x 4 x 64 tokens 33.6 / 38.9,
+//   200 x 12 tokens 44.5 / 54.8, at 100 columns 74.5 / 105;
+// * up to one block per SM: 80 tokens 47 / 41, 250 tokens 79.8 / 70.3, 500 tokens 143 / 124, 100 columns 184 / 135 (768 tokens:
+//   365 / 271);
+// * up to two, 64 columns: two steps of 64 in one are what is gained, half of the last step of an odd number of them is lost:
+//   192 tokens take 75 / 85, 320 118 / 126, 448 160 / 167, but 256 96 / 95, 384 138 / 135, 512 169 / 162, 1024 202 / 191;
+// * up to two, 128 columns: one group's operands leave room for a second block, two groups' do not.  fp32, 100 columns, up to 1.5
+//   blocks per SM: 256 tokens 152 / 147, 448 tokens 245 / 227, but 192 tokens 127 / 137; up to two: 256 tokens 183 / 195, 448
+//   tokens 290 / 307, 512 tokens 332 / 324.  16-bit tensors, which are widened on their way, gain from 256 tokens on (151 / 108
+//   to 211 / 201); 192 tokens 146 / 142, with two blocks per SM 170 / 184; 96 tokens 101 / 105, with two 120 / 113;
+// * beyond that one group makes better use of the SM: 512 blocks 413 / 482.
+// 256 columns: two groups' operands do not fit.
+template <typename T, int DP>
+static bool two_groups(const KParams &p, int sms) {
+  long long tiles = p.tiles_cap, longest = p.max_seqlen;
+  if (p.cu != nullptr) {
+    if ((long long)p.num_seq * p.n_max < tiles) tiles = (long long)p.num_seq * p.n_max;
+    // a bound that says nothing was most likely not given: four times the mean length instead
+    if (p.num_seq > 1 && longest >= p.tokens) longest = 4 * p.tokens / p.num_seq;
+  }
+  const long long blocks = tiles * p.head_cnt, steps = (longest + 63) / 64;
+  if (steps <= 1 || blocks > 2 * sms) return false;
+  if (blocks <= sms || steps >= 8) return true;
+  if (DP == 64) return steps % 2 == 0;
+  const bool few = 2 * blocks <= 3 * sms;
+  return sizeof(T) == 2 ? steps > 3 || (steps == 3) == few : steps > 3 && few;
+}
 template <typename T, int DP>
 static cudaError_t simt_run_g(const KParams &p, bool backward, cudaStream_t s) {
   if constexpr (DP <= 128) {
     int sms = 0;
     const cudaError_t e = sm_count(&sms);
     if (e != cudaSuccess) return e;
-    if ((long long)p.tiles_cap * p.head_cnt <= 2 * sms) return simt_run<T, DP, 2>(p, backward, s);
+    if (two_groups<T, DP>(p, sms)) return simt_run<T, DP, 2>(p, backward, s);
   }
   return simt_run<T, DP, 1>(p, backward, s);
 }
