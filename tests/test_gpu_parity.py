@@ -907,3 +907,69 @@ def test_cuda_core_bits_do_not_depend_on_the_rest_of_the_launch(sb, cuda_device,
     for name, a, b in zip(("o", "rem", "log_rem", "tile_start"), state(20), state(1)):
         a = a.unflatten(0, (20, 3))
         assert torch.equal(a.nan_to_num(nan=77.0), b.nan_to_num(nan=77.0).expand_as(a)), name
+
+
+@pytest.mark.parametrize("fits", [True, False])
+@pytest.mark.parametrize("form", ["packed", "fixed"])
+@pytest.mark.parametrize("fused", [False, True])
+def test_tiles_of_the_visited_pairs_of_several_heads(sb, cuda_device, fused, form, fits):
+    """Three heads that reach back differently, sequences and batch elements after the first, tokens behind the last sequence,
+    each token's own key, chunks of two heads: the visited pairs' stored tiles where they fit, the recomputing kernels where a
+    head reaches all keys.  Bit for bit what either gives when asked for, which are not the same bits."""
+    from stickbreaking_attention_b200 import ops
+    n, heads = 32000 if fits else 6000, 3
+    lead, tokens = ((2, heads), n) if form == "fixed" else ((heads,), 77 + n + 300 + 150)
+    q, k, v, do, drem = H.make_inputs((*lead, tokens, 64), torch.bfloat16, seed=9)
+    # <q, k> / 8 around -1 in the second head: some 0.6 bits of stick per key, 210 keys; around -12: 1e-4 bits, all 6000
+    shift = 1.0 if fits else 3.4
+    q[..., 1, :, :] += shift * 0.36
+    k[..., 1, :, :] -= shift * 0.36
+    cu = cu_of([77, n, 300])
+    kw = dict(attend_current=True)
+    if form == "packed":
+        kw.update(max_seqlens=n, zero_start=False)
+
+    def run():
+        if fused:
+            return H.run_fused(sb, q, k, v, do, cuda_device, cu if form == "packed" else None, **kw)
+        if form == "packed":
+            return H.run_varlen(sb, q, k, v, do, drem, cu, cuda_device, **kw)
+        return H.run_fixed(sb, q, k, v, do, drem, cuda_device, **kw)
+
+    with sb.small_backward_workspace(not fits):
+        want = run()
+    with sb.small_backward_workspace(fits):
+        other = run()
+    tiles = (n + 127) // 128
+    pairs = tiles * (tiles + 1) if form == "fixed" else ((tokens + 127) // 128 + 3) * (tiles + 1) // 2 + 1
+    old = ops.set_backward_scratch_budget(4096 * pairs * 5 // 2)   # records of two heads; 64 KiB per pair do not fit
+    try:
+        got = run()
+        sb.check_status(cuda_device)
+    finally:
+        ops.set_backward_scratch_budget(old)
+    for i, (a, b) in enumerate(zip(got, want)):
+        assert torch.equal(a, b), i
+    assert any(not torch.equal(a, b) for a, b in zip(got[-2:], other[-2:]))
+    if form == "packed":
+        for t in got:
+            assert torch.all(t[:, 77 + n + 300:] == 0)
+
+
+def test_refused_sequences_where_only_the_visited_pairs_would_fit(sb, cuda_device):
+    """Whichever kernels the device picks, they fill every row with NaN."""
+    from stickbreaking_attention_b200 import ops
+    ins = H.make_inputs((2, 3000, 64), torch.bfloat16, seed=2)
+    old = ops.set_backward_scratch_budget(1 << 20)
+    try:
+        for fused in (False, True):
+            if fused:
+                got = H.run_fused(sb, *ins[:4], cuda_device, cu_of([2000, 900]).flip(0), max_seqlens=3000, zero_start=False)
+            else:
+                got = H.run_varlen(sb, *ins, cu_of([2000, 900]).flip(0), cuda_device, max_seqlens=3000)
+            with pytest.raises(sb._cabi.SbError):
+                sb.check_status(cuda_device)
+            for t in got:
+                assert torch.isnan(t).all()
+    finally:
+        ops.set_backward_scratch_budget(old)
