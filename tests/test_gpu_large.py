@@ -38,8 +38,7 @@ def oracle_rows(q, k, v, do, drem, i0, i1, scale, tail_keys=0):
 
 @pytest.mark.parametrize("mode", ["stored", "recompute"])
 def test_16k_sequence_full_oracle(sb, cuda_device, mode):
-    """One 16384-token sequence against the row-blocked oracle, in both modes of the backward (the recomputing dK/dV
-    kernel is the one the 131072-token configuration takes)."""
+    """One 16384-token sequence against the row-blocked oracle, in both modes of the backward."""
     dtype = torch.bfloat16
     L = 16384
     q, k, v, do, drem = H.make_inputs((1, L, 128), dtype, seed=16, recipe="reference")
@@ -52,9 +51,16 @@ def test_16k_sequence_full_oracle(sb, cuda_device, mode):
           f"dk {rep['dk'][1]:.2e} dv {rep['dv'][1]:.2e}")
 
 
+@pytest.mark.parametrize("mode", ["visited", "recompute"])
 @pytest.mark.parametrize("std", [0.5, 1.0])
-def test_131072_sequence_sampled_rows_and_properties(sb, cuda_device, std):
-    """One head of the long-context configuration (131072 tokens, head_dim 128, q/k/v ~ N(0, std^2))."""
+def test_131072_sequence_sampled_rows_and_properties(sb, cuda_device, std, mode):
+    """One head of the long-context configuration (131072 tokens, head_dim 128, q/k/v ~ N(0, std^2)).  The stored tiles of all
+    its pairs do not fit; those of the pairs it visits do, and are what the dK/dV kernel reads unless it is told to recompute."""
+    with sb.small_backward_workspace(mode == "recompute"):
+        _check_131072_sequence(sb, cuda_device, std)
+
+
+def _check_131072_sequence(sb, cuda_device, std):
     dtype = torch.bfloat16
     L, d = 131072, 128
     q, k, v, do, drem = H.make_inputs((1, L, d), dtype, seed=131, std=std)
@@ -72,7 +78,7 @@ def test_131072_sequence_sampled_rows_and_properties(sb, cuda_device, std):
         assert H.max_abs(rem[:, i0:i1], wr) <= 2e-2
         assert H.rel_l2(dq[:, i0:i1], wdq) <= 5e-2
     # dk and dv of the last 256 keys receive contributions from the last 256 query rows only (a key is seen by later
-    # queries), so the oracle on those rows gives them in full; this workload runs the recomputing dK/dV kernel
+    # queries), so the oracle on those rows gives them in full
     _, _, _, wdk, wdv = oracle_rows(q, k, v, do, drem, L - 256, L, scale, tail_keys=256)
     assert H.rel_l2(dk[:, L - 256:], wdk) <= 5e-2
     assert H.rel_l2(dv[:, L - 256:], wdv) <= 5e-2
