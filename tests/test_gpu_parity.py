@@ -735,6 +735,30 @@ def test_activation_checkpointing(sb, cuda_device, packed, fused):
     assert torch.equal(*grads)
 
 
+@pytest.mark.parametrize("d,dtype", [(64, torch.bfloat16), (128, torch.float16), (64, torch.float32)])
+@pytest.mark.parametrize("backward", [False, True])
+def test_a_thread_whose_first_cuda_call_is_the_operator(sb, cuda_device, backward, d, dtype):
+    """A new thread has no CUDA context until a call binds it one, and where the allocator has the blocks at hand the operator
+    is that call: the autograd engine's thread, for one, if the operator's backward is the first node it runs."""
+    import threading
+    q, k, v, do, drem = (t.to(cuda_device) for t in H.make_inputs((3, 300, d), dtype, seed=d))
+    cu = cu_of([100, 200]).to(cuda_device)
+    o, rem, log_rem = sb.ops.varlen_fwd(q, k, v, cu, 200, 0.125)
+    if backward:
+        call = lambda: sb.ops.varlen_bwd(do, drem, q, k, v, cu, 200, log_rem, 0.125)
+    else:
+        call = lambda: sb.ops.varlen_fwd(q, k, v, cu, 200, 0.125)
+    want = call()                      # (and the blocks go back to the allocator)
+    got, spare = [], call()
+    del spare
+    thread = threading.Thread(target=lambda: got.extend(call()))
+    thread.start()
+    thread.join()
+    assert len(got) == len(want)
+    for a, b in zip(got, want):
+        assert torch.equal(a, b)
+
+
 def test_cuda_graph_replay_matches_eager(sb, cuda_device):
     """Forward and backward enqueue only (no allocation of their own, no synchronisation, no host reads), so a step can
     be captured in a CUDA graph and replayed: the replay on new inputs must equal an eager call bit for bit."""
