@@ -77,7 +77,7 @@ enum SbFlags {
                             budget, the dK/dV kernel recomputes the tiles from boundary values (a few KiB
                             per pair).  Without the flag, and with `tile_start`, such a call on the tensor
                             cores still stores the tiles of the pairs the forward visited if these fit the
-                            workspace; the device decides.  Same tiles either way.                */
+                            workspace; the device decides.  Same tiles either way, dK and dV to rounding. */
   SB_FLAG_FUSE_REM_V = 32,  /* the caller wants out = o + rem[..., None] * v, what every caller of the
                             reference computes right after the operator (tests/test_varlen.py:101,
                             tests/test_attn.py:64).  sb_fwd writes `out` to `o` (rem and log_rem as usual).
@@ -92,8 +92,9 @@ enum SbFlags {
                             is 0 for all 32 rows of a warp: they keep only the running log-space sum.  With
                             `tile_start` (below) whole tiles beyond that point are not visited either.  For
                             finite inputs the tensor-core kernels' results are the same bit for bit (CUDA
-                            cores: see `tile_start`).  With this flag every tile is visited and the
-                            arithmetic is done for every score regardless.                        */
+                            cores, and dK / dV of calls beyond the scratch budget: see `tile_start`).
+                            With this flag every tile is visited and the arithmetic is done for every
+                            score regardless.                                                     */
 };
 
 typedef struct SbTensor {
@@ -150,7 +151,11 @@ typedef struct SbParams {
                          * the keys visited is exactly 0 in fp32: no earlier key can add anything to o, rem or a *
                          * gradient), records here which key that was, and log_rem covers the visited keys only; *
                          * the backward then starts at that key.  Results for finite inputs: the same bit for   *
-                         * bit on the tensor cores, to rounding of the carried log sums on the CUDA cores.  A    *
+                         * bit on the tensor cores, to rounding of the carried log sums on the CUDA cores; dK    *
+                         * and dV to rounding (7e-5 relative, bf16) where one head's stored tiles exceed the     *
+                         * scratch budget, since with it, without SB_FLAG_DENSE_ROW_PASS and without             *
+                         * SB_FLAG_BWD_RECOMPUTE such a call stores the tiles of the visited pairs if these fit, *
+                         * and the recomputing dK/dV kernel runs otherwise.  A                                   *
                          * key or value that is not finite is seen by the query tiles (128 rows; CUDA cores: 32) *
                          * of which some row visits it (backward: visits its 128 keys) and by no others: 0 times *
                          * it is left out there.                                                                 *
@@ -210,9 +215,9 @@ SB_EXPORT int sb_fwd_static_scratch(const SbParams *p, void *stream);
 /* Upper bound, in bytes, on the scratch one chunk of heads of sb_bwd may take (default 8 GiB); returns the previous
  * value, and with bytes == 0 only reports it.  Process-wide; affects sb_workspace_bytes(p, 1) and sb_bwd alike, so
  * set it before sizing a workspace.  The backward works through the heads in chunks whose stored attention tiles
- * (64 KiB per 128 x 128 tile pair and head) fit the bound, and takes the recomputing dK/dV kernel when one head alone
- * does not fit (or stores the tiles of the visited pairs only: SB_FLAG_BWD_RECOMPUTE).  The reference has no counterpart: its backward keeps nothing but lock arrays
- * (sb_varlen_bwd.py:568-573). */
+ * (64 KiB per 128 x 128 tile pair and head) fit the bound.  When one head alone does not fit, it stores the tiles of the
+ * visited pairs only, if those do, or takes the recomputing dK/dV kernel (see SB_FLAG_BWD_RECOMPUTE).  The reference has no
+ * counterpart: its backward keeps nothing but lock arrays (sb_varlen_bwd.py:568-573). */
 SB_EXPORT size_t sb_set_backward_scratch_budget(size_t bytes);
 
 /* Which kernels sb_fwd / sb_bwd run for these parameters (an SbKernelPath), or -1 if invalid. */

@@ -52,8 +52,8 @@ struct Plan {
 };
 
 // Upper bound on the backward's per-chunk scratch (stored tiles, or R1 + S2): heads are processed in chunks that fit
-// it, and a call whose single head does not fit the stored tiles takes the recomputing dK/dV kernel.  Process-wide,
-// set through sb_set_backward_scratch_budget.
+// it; a call whose single head does not fit stores the tiles of the visited pairs where these fit (Plan::try_slots) and
+// takes the recomputing dK/dV kernel otherwise.  Process-wide, set through sb_set_backward_scratch_budget.
 static std::atomic<size_t> g_scratch_budget{(size_t)8 << 30};
 
 static int check_tensor(const SbTensor &t, const char *name, bool required) {

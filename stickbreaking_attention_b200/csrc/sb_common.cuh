@@ -160,9 +160,10 @@ struct QueryList {
 // ---- which work items there are ---------------------------------------------------------------------------------------
 // Work items (query or key tiles) are ordered by weight across ALL sequences: the tile with the most key (or query) tiles
 // to visit comes first, so that the blocks that run longest start earliest and the last blocks of a launch are the short
-// ones.  An entry is (sequence, k), k = tile index counted so that larger means heavier.  For a fixed-length batch the order is arithmetic.  For a packed batch it is a table, either written by a
-// kernel that runs first (p.order, p.pair_prefix, p.hdr), or, for small calls (p.small_table), built by every
-// block for itself in shared memory: a launch and its hand-over cost more than the microsecond this takes.
+// ones.  An entry is (sequence, k), k = tile index counted so that larger means heavier.  For a fixed-length batch the order is
+// arithmetic.  For a packed batch it is a table, either written by a kernel that runs first (p.order, p.pair_prefix, p.hdr),
+// or, for small calls (p.small_table), built by every block for itself in shared memory: a launch and its hand-over cost more
+// than the microsecond this takes.
 constexpr int kSmallSeqs = 128, kSmallItems = 256;
 struct SmallTable {                       // 1.5 KB: what the kernels' shared memory has left
   uint32_t pair0[kSmallSeqs];             // first (query tile, key tile) pair of each sequence; while building: its entries

@@ -9,9 +9,9 @@ namespace sb {
 // Sequence table of the larger packed batches: the first (query tile, key tile) pair of every sequence, and the work items
 // by descending weight (see decode_item).
 // ------------------------------------------------------------------------------------------------
-// The order is a counting sort over classes of `order_span` consecutive tiles, the heaviest class first.  The tiles of one sequence inside a class stay neighbours (they read the same keys or queries at about the
-// same time and share them through L2); the order of the sequences inside a class is whatever the shared-memory atomics
-// give, which does not matter.
+// The order is a counting sort over classes of `order_span` consecutive tiles, the heaviest class first.  The tiles of one
+// sequence inside a class stay neighbours (they read the same keys or queries at about the same time and share them through
+// L2); the order of the sequences inside a class is whatever the shared-memory atomics give, which does not matter.
 // One block: what bounds it is latency, so every phase is a few steps of 1024 threads.  Sequences of few classes are taken
 // one per thread, with one atomic per warp and class; long ones one per warp.  One 131072-token sequence: 8.3 us (one thread
 // per sequence and serial prefix sums before: 82 us); 1024 sequences of up to 512 tokens: 9.4 us (16.3).

@@ -254,8 +254,8 @@ __device__ __forceinline__ bool zero_strip_row(uint32_t tz, int u, uint32_t bars
 // dq kernel: 128 query rows per CTA, two CTAs per SM
 // =======================================================================================================
 // A block owns one 128-row query tile and walks the 64-key K/V sub-tiles from the first key its rows reach to its diagonal.
-// Per sub-tile: S = Q K^T and dP = dO V^T (128 x 64), the row pass (which also records R1/S2 at the sub-tile's first key,
-// i.e. at keys 0 and 64 of every 128-key tile), then dQ += dz K with dz read from tensor memory.
+// Per sub-tile: S = Q K^T and dP = dO V^T (128 x 64), the row pass (which, where the tiles are not stored, records R1/S2
+// every 32 keys), then dQ += dz K with dz read from tensor memory.
 //   warps 0-3  rows, one thread per query row;  warp 4  TMA;  warp 5  MMA issue;  warps 6, 7 fill their warpgroup up
 // Two blocks share an SM -- half of its tensor memory, of its registers and, to the byte, of its shared memory each --, so
 // that nothing ties the two tiles of an SM together: one's loads, first scores and epilogue run under the other's row passes.

@@ -13,7 +13,6 @@ namespace sb {
 using namespace ptx;
 
 constexpr int kBM = kTcTile;  // 128 query rows per CTA, 128 keys per tile
-constexpr int kTcThreads = 192;  // warps 0-3: one thread per tile row; warp 4: TMA; warp 5: MMA issue
 constexpr uint32_t kTmemCols = 512;
 constexpr int kBoxBytes = kBM * 64 * 2;  // one TMA box: 128 rows x 64 16-bit elements, 128-byte swizzled
 
@@ -216,14 +215,6 @@ __device__ __forceinline__ void mma_tmem_mnmajor(uint32_t d_tmem, uint32_t a_tme
 #pragma unroll
   for (int ks = 0; ks < KDIM / 16; ++ks)
     mma_f16_ts(d_tmem, a_tmem + ks * 8, b0 + (uint64_t)(ks * 128), idesc, accumulate || ks > 0);
-}
-// A and B both stored with rows = K (128): A^T B.
-__device__ __forceinline__ void mma_mnmajor_mnmajor(uint32_t d_tmem, uint32_t a_addr, uint32_t b_addr, uint32_t idesc,
-                                                    bool accumulate) {
-  const uint64_t a0 = smem_desc_sw128(a_addr, kBoxBytes, 1024), b0 = smem_desc_sw128(b_addr, kBoxBytes, 1024);
-#pragma unroll
-  for (int ks = 0; ks < kBM / 16; ++ks)
-    mma_f16_ss(d_tmem, a0 + (uint64_t)(ks * 128), b0 + (uint64_t)(ks * 128), idesc, accumulate || ks > 0);
 }
 
 // host: 4-D TMA map (head_dim, tokens, heads, batch), [64 x 128 x 1 x 1] box, 128-byte swizzle, zero fill

@@ -74,9 +74,9 @@ __device__ __forceinline__ void fwd128_item(const KParams &p, const SmallTable &
 }
 
 // kDrop: from the sub-tile on where a warp's weights are exactly 0 it only writes zeros for P, and log_rem ends there (the
-// caller keeps the tile starts); where all four warps are that far, P V is left out.  kStop: tiles may stop altogether.  A tile of a sequence of up to 512 tokens has no four
-// sub-tiles left by the time it could (see may_stop_before), and the code for it costs short tiles 6 %: the launch leaves it
-// out for such calls.
+// caller keeps the tile starts); where all four warps are that far, P V is left out.  kStop: tiles may stop altogether.  A tile
+// of a sequence of up to 512 tokens has no four sub-tiles left by the time it could (see may_stop_before), and the code for it
+// costs short tiles 6 %: the launch leaves it out for such calls.
 template <bool kFp16, bool kStop, bool kDrop>
 __global__ void __launch_bounds__(fwd128::kThreads, 1)
 tc_fwd128x2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
@@ -391,7 +391,8 @@ template <bool kFp16>
 static cudaError_t launch128(const KParams &p, int dtype, cudaStream_t s) {
   if (p.tile_start == nullptr || p.dense) return launch128_t<kFp16, false, false>(p, dtype, s);
   if (p.max_seqlen > 512) return launch128_t<kFp16, true, true>(p, dtype, s);
-  // (up to 256 tokens: a tile has no sub-tile left by the time its rows could be through)
+  // (Up to 256 tokens a sub-tile or two could be left out at most.  32 heads x 512 sequences, without / with it: N(0, 1), 256
+  // tokens 502 / 506 us, 192 tokens 425 / 440, 130 tokens 439 / 456; four times the scores 520 / 510, 419 / 420, 437 / 425.)
   return p.max_seqlen > 256 ? launch128_t<kFp16, false, true>(p, dtype, s) : launch128_t<kFp16, false, false>(p, dtype, s);
 }
 

@@ -67,7 +67,8 @@ def dense_row_pass(enabled: bool = True):
     """Within the block (calling thread only) the tensor-core kernels do the per-score arithmetic for every score, also
     where the product of (1 - beta) over the keys in between has underflowed to exactly 0 for a whole warp and the
     results are known to be exact zeros, and all kernels visit every key (``SB_FLAG_DENSE_ROW_PASS``).  For finite inputs the
-    same results bit for bit on the tensor cores and to rounding on the CUDA cores; a measuring aid, and the way to have a
+    same results bit for bit on the tensor cores and to rounding on the CUDA cores (and dk, dv of a call whose single head
+    exceeds the backward's scratch budget, see ``set_backward_scratch_budget``); a measuring aid, and the way to have a
     NaN or an infinity in a key far back show in every row that attends to it with weight 0."""
     old = _state.dense_row_pass
     _state.dense_row_pass = enabled
@@ -93,8 +94,9 @@ def kernel_launches() -> int:
 def set_backward_scratch_budget(nbytes: int) -> int:
     """Process-wide upper bound on the scratch one chunk of heads of the backward may take (default 8 GiB); returns
     the previous bound.  The backward stores 64 KiB per (query tile, key tile) pair and head for its dK/dV kernel and
-    works through the heads in chunks that fit the bound; a call whose single head does not fit recomputes the tiles
-    instead (slower, O(tokens) scratch).  Raising the bound on a GPU with memory to spare lets long sequences take the
+    works through the heads in chunks that fit the bound.  Where a single head does not fit, it stores the tiles of the
+    pairs that the forward visited, if those fit into the scratch of the recomputing kernels (4 KiB per pair of all pairs),
+    and otherwise recomputes the tiles (slower); the device decides, and dk and dv are the same to rounding.  Raising the bound on a GPU with memory to spare lets long sequences take the
     stored-tiles kernels; lowering it bounds the transient allocation of every backward call."""
     return int(_cabi.load().sb_set_backward_scratch_budget(int(nbytes)))
 
