@@ -944,7 +944,7 @@ __global__ void __launch_bounds__(kThreads<G>, kBlocks<DP, G>) simt_bwd_dkv_kern
       if (wider) tile_ptb(dv, Ps, Gs, 64);
     }
   } else {
-    static_assert(kStored || G == 1, "a row's keys are shared by two lanes");
+    static_assert(kStored || G == 1, "64 query rows per step, the 32 keys of a row shared by two lanes");
     for (; off < list.n; advance(I[kTiles - 1] - J + 1)) {
       load_rows(lq, Qs, p.q);
       load_rows(lg, Gs, p.d_o);
